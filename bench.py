@@ -154,10 +154,18 @@ def measured_peaks():
 
 
 def algorithmic_bytes(name, npx, nk, d2, s, tm):
-    """Bytes one launch of a CG-iteration kernel must move (per RHS)."""
+    """Bytes one launch of a CG-iteration kernel must move (per RHS).  The mixed method's
+    passes (disp.cuh) are counted for finite strain in 3-D: vectors of 3 complex values per
+    k-point, 6 components along axis 0, 9 along the others."""
     u = npx * d2 * s        # one real field
     spec = nk * d2 * 2 * s  # one half spectrum
+    comp = nk * 2 * s       # one component of it
     return {
+        'axis0_inv_update': 27 * comp,               # r, q, p, x in; r, p, x out; 6 components out
+        'axis1_inv_expand': 15 * comp,               # 6 in, 9 out
+        'last_axis_tangent': 18 * comp + tm * npx,   # 9 in and out, tangent data
+        'axis1_fwd_contract': 15 * comp,             # 9 in, 6 out
+        'axis0_fwd_dots': 15 * comp,                 # 6 in, q out; p, r in
         'last_axis_fwd_tangent': 3 * u + tm * npx + spec,  # r, p_old -> p; tangent data; spectrum out
         'axis1_fwd': 2 * spec,
         'green_axis0': 2 * spec,
@@ -278,7 +286,7 @@ def lognormal_config(mu, workloads, peak, n=256, repeats=3):
     solves; FP64: one batched solve of the same cells; per load case the
     homogenised-stress error of the mixed result against the FP64 one.  px.it/s counts
     pixels x CG iterations x right-hand sides; its roofline fraction uses the CG
-    iteration's algorithmic bytes (16 field passes + the Lame planes per px.it, FP32),
+    iteration's algorithmic bytes (78 component spectra + the Lame planes per px.it, FP32),
     so the Newton-level FP64 work makes it a lower bound."""
     import torch
     w = workloads.lognormal(n)
@@ -313,7 +321,7 @@ def lognormal_config(mu, workloads, peak, n=256, repeats=3):
     errs = [hom_err(a, b[0].hom_stress) for a, b in zip(hm, r64)]
     dt = statistics.median(times)
     pxit = npx * sum(per_solve) / dt
-    bpx = 16 * 9 * 4 + 8  # FP32 fields per px.it of the fused CG iteration + lambda, mu
+    bpx = 78 * 4 + 8  # FP32 component spectra per px.it of the small-strain iteration + lambda, mu
     return {'seconds_median': dt, 'seconds_all': times, 'rhs_solves_per_s': len(cells) / dt,
             'cg_iters_per_rhs': per_solve, 'newton_steps': [r[0].nb_it for r in res],
             'pxit_per_s': pxit, 'cg_bytes_per_pxit': bpx,

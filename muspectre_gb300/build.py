@@ -25,6 +25,10 @@ LIB = os.path.join(HERE, 'libmusg.so')
 
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
+# the out-of-line tile transforms are linked into kernels of 80 registers (device code is
+# relocatable; a kernel takes the registers of the functions it calls)
+EXTRA = {'tile_stages.cu': ['-maxrregcount=80']}
+
 
 def _nvcc():
     for cand in (os.environ.get('NVCC'), shutil.which('nvcc'), '/usr/local/cuda/bin/nvcc'):
@@ -73,7 +77,8 @@ def build(force=False, verbose=False, jobs=None):
     for src in cu:
         obj = os.path.join(BUILD, os.path.basename(src) + '.o')
         objs.append(obj)
-        cmds.append([nvcc] + ARCH + common + ['-lineinfo', '-Xcompiler', '-fPIC', '-c', src, '-o', obj])
+        cmds.append([nvcc] + ARCH + common + ['-lineinfo', '-Xcompiler', '-fPIC', '-dc', src, '-o', obj] +
+                    EXTRA.get(os.path.basename(src), []))
     for src in cpp:
         obj = os.path.join(BUILD, os.path.basename(src) + '.o')
         objs.append(obj)

@@ -161,20 +161,20 @@ struct musg_cell {
   bool tangent_valid = false;
   bool need32 = false;
   int plan_flags = 0;      // FFT_PlanFlags: estimate 0, measure 1, patient 2
-  bool tuned64 = false, tuned32 = false;
+  bool tuned64 = false;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::vector<Material> materials;
   Spectral sp;
   int tkind = TK_SMALL, tkind32 = TK_SMALL;  // CG operator kind of the FP64 / FP32 path
-  template <typename R> int tk() const { return sizeof(R) == 4 ? tkind32 : tkind; }
   int hep_cur = 0;
   bool has_le2 = false, has_hep = false;
   bool has_consistent = false;  // an HEP1 material with the consistent tangent: TK_FULL cell
   // device fields (FP64 component planes)
   DevBuf F, P, rhs, io, io2, F0;  // F0: the line search's Newton iterate
-  DevBuf Pk, dP32;                // the stress of the last projected residual; FP32 projection input
-  bool residual_kept = false;     // Pk and rhs belong together (incremental residual)
+  DevBuf Pk;                      // the stress of the last projected residual (incremental residual)
+  DevBuf rhat;                    // the mixed method's residual G(-P) in displacement space (disp.cuh)
+  bool residual_kept = false;     // Pk and rhat belong together (incremental residual)
   DevBuf mat, params, law_kind, Ctab64, Ctab32;
   bool has_generic = false;
   DevBuf lam64, mu64, lam32, mu32, eig;
@@ -403,15 +403,12 @@ struct musg_cell {
       autotune_with_wisdom<double>(sp, stream, plan_flags);
       tuned64 = true;
     }
-    if (need32 && !tuned32) {
-      autotune_with_wisdom<float>(sp, stream, plan_flags);
-      tuned32 = true;
-    }
   }
 
   void alloc32() {
     need32 = true;
     sp.ensure32();
+    if (!rhat.p) rhat.alloc(disp_vector_bytes(sp));
     if (!initialised && !lam64.p) return;  // done at initialise
     if (!lam32.p) {
       lam32.alloc((size_t)npx * sizeof(float));
@@ -484,31 +481,42 @@ struct musg_cell {
     for (int k = 0; k < 9; ++k) out[k] = k < D2 ? hscal[40 + k] : 0.0;
   }
 
-  // rhs = -G(P) for the current stress.  Incremental (the mixed path's default): the
-  // first residual after residual_kept is cleared is projected in FP64 and its P kept
-  // in Pk; each later one is G(rhs - (P - Pk)) projected in FP32 (rhs is in the range
-  // of G, so this is rhs - G(P - Pk) = -G(P)), and the new P is kept.  The FP32
-  // input is the previous residual minus the stress change since, whose size
-  // shrinks with the Newton increments: the result carries FP32 rounding of that
-  // change (not of P, whose mean and fluctuation are far larger), its part outside
-  // the range of G is rounding of the result itself (the fused CG iteration needs
-  // the right-hand side in that range), and the FP64 projections, bound by the FP64
-  // pipe, drop to one per load step.
-  void project_residual(bool incremental) {
-    if (!incremental || !residual_kept) {
-      spectral_project<double>(sp, P.as<double>(), rhs.as<double>(), -1.0, stream);
-      if (incremental) {
-        if (Pk.bytes < field_bytes()) Pk.alloc(field_bytes());
-        MUSG_CUDA(cudaMemcpyAsync(Pk.p, P.p, field_bytes(), cudaMemcpyDeviceToDevice, stream));
-        residual_kept = true;
-      }
+  // rhs = -G(P) for the current stress (FP64, the plain method), its norm's square in
+  // scal[32]
+  void project_residual() {
+    spectral_project<double>(sp, P.as<double>(), rhs.as<double>(), -1.0, stream);
+    dot_device<double, double>(rhs.as<double>(), rhs.as<double>(), nb_dof(), partial.as<double>(),
+                               scal.as<double>() + 32, stream);
+  }
+  // The mixed method's residual rhat = -G(P) in displacement space, its norm's square in
+  // scal[32].  Incremental (the default): the first residual after residual_kept is
+  // cleared is projected in FP64 and its P kept in Pk; each later one is rhat + G(Pk - P)
+  // with the stress change projected in FP32, and the new P is kept.  The FP32 rounding
+  // is relative to that change and not to P (whose mean and fluctuation are far larger),
+  // and in displacement space no part of it can leave the range of G.  The FP64
+  // projections, bound by the FP64 pipe, drop to one per load step.
+  void project_residual_mixed(bool incremental) {
+    double *part = partial.as<double>(), *norm2 = scal.as<double>() + 32;
+    if (incremental && residual_kept) {
+      disp_residual(sp, rhat.p, P.as<double>(), Pk.as<double>(), 1.0, true, part, norm2, stream);
       return;
     }
-    const long long n = nb_dof();
-    if (dP32.bytes < (size_t)n * sizeof(float)) dP32.alloc((size_t)n * sizeof(float));
-    residual_input(rhs.as<double>(), P.as<double>(), Pk.as<double>(), dP32.as<float>(), n, stream);
-    spectral_project<float>(sp, dP32.as<float>(), dP32.as<float>(), 1.0f, stream);
-    convert<double, float>(rhs.as<double>(), dP32.as<float>(), n, 1.0, stream);
+    spectral_project<double>(sp, P.as<double>(), rhs.as<double>(), -1.0, stream);
+    residual_from_rhs();
+    if (incremental) {
+      if (Pk.bytes < field_bytes()) Pk.alloc(field_bytes());
+      MUSG_CUDA(cudaMemcpyAsync(Pk.p, P.p, field_bytes(), cudaMemcpyDeviceToDevice, stream));
+      residual_kept = true;
+    }
+  }
+  // rhat of the projected field in rhs
+  void residual_from_rhs() {
+    disp_residual(sp, rhat.p, rhs.as<double>(), nullptr, 1.0, false, partial.as<double>(), scal.as<double>() + 32,
+                  stream);
+  }
+  void residual(bool mixed, bool incremental) {
+    if (mixed) project_residual_mixed(incremental);
+    else project_residual();
   }
 
   // host AoS vector -> device SoA planes (dst)
@@ -562,7 +570,9 @@ struct musg_solver {
   int precision = MUSG_PRECISION_FP64;
   bool converged = false;
   unsigned long long counter = 0;
-  DevBuf x, r, p, Ap, st;
+  // FP64: the CG vectors; mixed: r, q, p, xh in displacement space (DispVectors) and x,
+  // the solution in real space
+  DevBuf x, r, p, Ap, q, xh, st;
   CGState *hst = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned long long graph_nodes = 0;
@@ -601,10 +611,11 @@ struct musg_solver {
     if (precision == MUSG_PRECISION_MIXED) cell->alloc32();
     const size_t n = (size_t)cell->nb_dof();
     x.alloc(n * rbytes());
-    r.alloc(n * rbytes());
-    p.alloc(n * rbytes());
-    // the FP32 inner solve never stores Ap (its last pass updates r directly)
-    if (precision != MUSG_PRECISION_MIXED) Ap.alloc(n * rbytes());
+    if (precision == MUSG_PRECISION_MIXED) {
+      for (DevBuf *b : {&r, &q, &p, &xh}) b->alloc(disp_vector_bytes(cell->sp));
+    } else {
+      for (DevBuf *b : {&r, &p, &Ap}) b->alloc(n * rbytes());
+    }
     st.alloc(sizeof(CGState));
     MUSG_CUDA(cudaMemset(st.p, 0, sizeof(CGState)));
     MUSG_CUDA(cudaMallocHost(&hst, sizeof(CGState)));
@@ -614,40 +625,46 @@ struct musg_solver {
     if (verbose) chunk = 1;
   }
 
-  // one CG iteration (solver_cg.cc:76-97); ev, when given, receives an event
-  // before the first and after every kernel (profiling).  FP64: the operator passes
-  // (alpha by the last one) and cg_update (x, r, beta); FP32: the operator passes and
-  // cg_update_x, which carry the whole iteration (alpha from p.(K:p) in the first pass;
-  // r and beta in the last).
-  template <typename R> int iteration(cudaStream_t s, cudaEvent_t *ev = nullptr) {
-    musg_cell &c = *cell;
-    const long long n = c.nb_dof();
-    CGState *d = st.as<CGState>();
-    double *part = c.partial.as<double>();
-    const TangentData<R> td = c.tangent<R>();
-    R *ap = sizeof(R) == 8 ? Ap.as<R>() : nullptr;
-    const int nop = cg_operator<R>(c.sp, c.tk<R>(), td, d, r.as<R>(), x.as<R>(), p.as<R>(), ap, part, s, ev);
-    (void)nop;
-    const int k = nb_kernels();
-    if (sizeof(R) == 4) return k;
-    cg_update<R>(d, x.as<R>(), r.as<R>(), p.as<R>(), Ap.as<R>(), n, part, s);  // and beta
-    if (ev) MUSG_CUDA(cudaEventRecord(ev[k], s));
-    return k;  // number of kernels
+  DispVectors vectors() const {
+    DispVectors v;
+    v.r = r.p;
+    v.q = q.p;
+    v.p = p.p;
+    v.x = xh.p;
+    return v;
   }
 
-  // kernels per CG iteration: five (3-D) or three (2-D) passes and one vector kernel
-  int nb_kernels() const { return cell->dim == 3 ? 6 : 4; }
+  // one CG iteration (solver_cg.cc:76-97); ev, when given, receives an event
+  // before the first and after every kernel (profiling).  FP64: the operator passes
+  // (alpha by the last one) and cg_update (x, r, beta); mixed: the displacement-space
+  // passes, whose first one applies the updates of the iteration before.
+  template <typename R> void iteration(cudaStream_t s, cudaEvent_t *ev = nullptr) {
+    musg_cell &c = *cell;
+    CGState *d = st.as<CGState>();
+    double *part = c.partial.as<double>();
+    if constexpr (sizeof(R) == 4) {
+      disp_iteration(c.sp, c.tkind32, c.tangent<float>(), vectors(), d, part, s, ev);
+    } else {
+      cg_operator<double>(c.sp, c.tkind, c.tangent<double>(), d, r.as<double>(), p.as<double>(), Ap.as<double>(), part, s,
+                          ev);
+      cg_update<double>(d, x.as<double>(), r.as<double>(), p.as<double>(), Ap.as<double>(), c.nb_dof(), part, s);
+      if (ev) MUSG_CUDA(cudaEventRecord(ev[nb_kernels()], s));
+    }
+  }
+
+  // kernels per CG iteration: five (3-D) or three (2-D) passes, in FP64 and the update
+  int nb_kernels() const { return (cell->dim == 3 ? 5 : 3) + (precision == MUSG_PRECISION_MIXED ? 0 : 1); }
 
   static const char *kernel_name(int dim, int precision, int k) {
     static const char *n3[] = {"last_axis_fwd_tangent", "axis1_fwd", "green_axis0", "axis1_inv", "last_axis_inv_dot",
                                "cg_update"};
     static const char *n2[] = {"last_axis_fwd_tangent", "green_axis0", "last_axis_inv_dot", "cg_update"};
-    static const char *f3[] = {"last_axis_fwd_tangent_alpha", "cg_update_x", "axis1_fwd", "green_axis0",
-                               "axis1_inv", "last_axis_inv_update_r"};
-    static const char *f2[] = {"last_axis_fwd_tangent_alpha", "cg_update_x", "green_axis0",
-                               "last_axis_inv_update_r"};
-    const char *const *t = precision == MUSG_PRECISION_MIXED ? (dim == 3 ? f3 : f2) : (dim == 3 ? n3 : n2);
-    const int nk = dim == 3 ? 6 : 4;
+    static const char *f3[] = {"axis0_inv_update", "axis1_inv_expand", "last_axis_tangent", "axis1_fwd_contract",
+                               "axis0_fwd_dots"};
+    static const char *f2[] = {"axis0_inv_update", "last_axis_tangent", "axis0_fwd_dots"};
+    const bool mixed = precision == MUSG_PRECISION_MIXED;
+    const char *const *t = mixed ? (dim == 3 ? f3 : f2) : (dim == 3 ? n3 : n2);
+    const int nk = (dim == 3 ? 5 : 3) + (mixed ? 0 : 1);
     return (k >= 0 && k < nk) ? t[k] : "";
   }
 
@@ -659,7 +676,10 @@ struct musg_solver {
     require(c.tangent_valid, MUSG_ERR_RUNTIME, "profile needs an evaluated tangent");
     const long long n = c.nb_dof();
     double *part = c.partial.as<double>();
-    cg_init<R>(st.as<CGState>(), c.rhs.as<double>(), r.as<R>(), x.as<R>(), n, 0.0, iters, part, part + 4096, s);
+    if constexpr (sizeof(R) == 4)
+      disp_start(c.sp, vectors(), c.rhat.p, st.as<CGState>(), 0.0, iters, nullptr, c.scal.as<double>() + 32, s);
+    else
+      cg_init<R>(st.as<CGState>(), c.rhs.as<double>(), r.as<R>(), x.as<R>(), n, 0.0, iters, part, part + 4096, s);
     const int nk = nb_kernels();
     std::vector<cudaEvent_t> ev(nk + 1);
     for (auto &e : ev) MUSG_CUDA(cudaEventCreate(&e));
@@ -705,42 +725,51 @@ struct musg_solver {
     cudaGraphDestroy(g);
   }
 
-  // SolverCG::solve (solver_cg.cc:54-110) on a device rhs (FP64 SoA planes)
-  template <typename R> void solve_device(const double *rhs) {
+  // SolverCG::solve (solver_cg.cc:54-110) on a device rhs (FP64 SoA planes; mixed: null
+  // for the cell's own residual rhat, whose norm's square is in scal[32])
+  void solve_device(const double *rhs) {
     musg_cell &c = *cell;
     cudaStream_t s = c.stream;
     const long long n = c.nb_dof();
-    double *part = c.partial.as<double>();
+    double *part = c.partial.as<double>(), *dscal = c.scal.as<double>();
+    const bool mixed = precision == MUSG_PRECISION_MIXED;
     // r = A 0 - rhs = -rhs, p = -r (first iteration), x = 0
-    const double t = (precision == MUSG_PRECISION_MIXED) ? std::max(tol, inner_tol) : tol;
-    cg_init<R>(st.as<CGState>(), rhs, r.as<R>(), x.as<R>(), n, t, (int)maxiter, part, part + 4096, s);
+    if (mixed) {
+      const double t = std::max(tol, inner_tol);
+      if (rhs) {
+        dot_device<double, double>(rhs, rhs, n, part, dscal + 36, s);
+        disp_residual(c.sp, q.p, rhs, nullptr, 1.0, false, part, dscal + 37, s);
+        disp_start(c.sp, vectors(), q.p, st.as<CGState>(), t, (int)maxiter, dscal + 36, dscal + 37, s);
+      } else {
+        disp_start(c.sp, vectors(), c.rhat.p, st.as<CGState>(), t, (int)maxiter, nullptr, dscal + 32, s);
+      }
+    } else {
+      cg_init<double>(st.as<CGState>(), rhs, r.as<double>(), x.as<double>(), n, tol, (int)maxiter, part, part + 4096, s);
+    }
     converged = false;
-    if (graphs && !verbose) build_graph<R>();
+    if (graphs && !verbose) {
+      if (mixed) build_graph<float>();
+      else build_graph<double>();
+    }
     for (;;) {
       if (exec) {
         MUSG_CUDA(cudaGraphLaunch(exec, s));
         g_launches.fetch_add(graph_nodes);
       } else {
-        for (int k = 0; k < chunk; ++k) iteration<R>(s);
+        for (int k = 0; k < chunk; ++k) {
+          if (mixed) iteration<float>(s);
+          else iteration<double>(s);
+        }
       }
       MUSG_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(CGState), cudaMemcpyDeviceToHost, s));
       MUSG_CUDA(cudaStreamSynchronize(s));
       check_stop(stop);
-      if (verbose) {
+      if (verbose && (hst->active || !mixed)) {  // mixed: the last pass only finishes x
         printf("  at CG step %d: |r|/|b| = %15g, cg_tol = %g\n", hst->iter - 1,
                std::sqrt(hst->rdr / hst->rhs_norm2), tol);
         fflush(stdout);
       }
       if (!hst->active) break;
-    }
-    if (precision == MUSG_PRECISION_MIXED) {
-      unsigned fault = 0;
-      MUSG_CUDA(cudaMemcpyAsync(&fault, wait_fault_word(), sizeof fault, cudaMemcpyDeviceToHost, s));
-      MUSG_CUDA(cudaStreamSynchronize(s));
-      if (fault) {
-        MUSG_CUDA(cudaMemsetAsync(wait_fault_word(), 0, sizeof fault, s));
-        throw Error(MUSG_ERR_RUNTIME, "a spectral pass timed out waiting for its tile copy; a copy may still land in shared memory after its block exited, so later results of this CUDA context are suspect: check them or restart the process");
-      }
     }
     counter = hst->counter;
     if (hst->rdr < hst->tol2) {
@@ -751,11 +780,7 @@ struct musg_solver {
         << std::sqrt(hst->rdr / hst->rhs_norm2) << ", cg_tol = " << std::sqrt(hst->tol2 / hst->rhs_norm2);
       throw Error(MUSG_ERR_CONVERGENCE, e.str());
     }
-  }
-
-  void solve_device_any(const double *rhs) {
-    if (precision == MUSG_PRECISION_MIXED) solve_device<float>(rhs);
-    else solve_device<double>(rhs);
+    if (mixed) disp_solution(c.sp, vectors(), st.as<CGState>(), x.as<float>(), s);
   }
 
   void reset_counter() {
@@ -784,11 +809,13 @@ struct musg_batch {
   // grouped launch per pass over all of them (generic pass kernels)
   bool uniform = true;
   GroupedOp *gop = nullptr;
+  DispBatch *disp = nullptr;  // mixed: the displacement-space passes of all cells
   long long nmax = 0;  // the largest cell's vector length
   const int *stop = nullptr;  // musg_batch_set_stop_flag
 
   ~musg_batch() {
     if (gop) grouped_op_destroy(gop);
+    if (disp) disp_batch_destroy(disp);
     if (exec) cudaGraphExecDestroy(exec);
     if (hst) cudaFreeHost(hst);
     if (stream) cudaStreamDestroy(stream);
@@ -796,30 +823,37 @@ struct musg_batch {
   int B() const { return (int)cells.size(); }
   CGState *state(int b) const { return states.as<CGState>() + b; }
 
-  template <typename R> void build_tables() {
+  void build_tables_mixed() {
+    std::vector<DispProblem> probs(B());
+    for (int b = 0; b < B(); ++b) {
+      musg_cell &c = *cells[b];
+      probs[b] = {&c.sp, solvers[b]->vectors(), state(b), c.partial.as<double>(), c.tangent<float>()};
+    }
+    disp = disp_batch_create(probs, cells[0]->tkind32, uniform);
+  }
+
+  void build_tables() {
     std::vector<ProblemPtrsHost> tp(B());
-    std::vector<BatchVec<R>> tv(B());
+    std::vector<BatchVec<double>> tv(B());
     for (int b = 0; b < B(); ++b) {
       musg_cell &c = *cells[b];
       musg_solver &sv = *solvers[b];
-      const TangentData<R> td = c.tangent<R>();
-      tp[b].spec = sizeof(R) == 8 ? c.sp.spec64 : c.sp.spec32;
+      const TangentData<double> td = c.tangent<double>();
+      tp[b].spec = c.sp.spec64;
       tp[b].st = state(b);
       tp[b].r = sv.r.p;
-      tp[b].x = sv.x.p;
       tp[b].p = sv.p.p;
-      tp[b].Ap = sizeof(R) == 8 ? sv.Ap.p : nullptr;  // the FP32 passes do not store Ap
+      tp[b].Ap = sv.Ap.p;
       tp[b].partial = c.partial.as<double>();
-      static_assert(sizeof(TangentData<R>) == sizeof(tp[b].td), "tangent table layout");
+      static_assert(sizeof(td) == sizeof(tp[b].td), "tangent table layout");
       memcpy(tp[b].td, &td, sizeof(td));
       tv[b].st = state(b);
-      tv[b].x = sv.x.as<R>();
-      tv[b].r = sv.r.as<R>();
-      tv[b].p = sv.p.as<R>();
-      tv[b].Ap = sv.Ap.as<R>();
+      tv[b].x = sv.x.as<double>();
+      tv[b].r = sv.r.as<double>();
+      tv[b].p = sv.p.as<double>();
+      tv[b].Ap = sv.Ap.as<double>();
       tv[b].partial = c.partial.as<double>();
       tv[b].n = c.nb_dof();
-      tv[b].nparts = 0;
       nmax = std::max(nmax, c.nb_dof());
     }
     if (!uniform) {
@@ -828,38 +862,39 @@ struct musg_batch {
         probs[b].sp = &cells[b]->sp;
         probs[b].st = state(b);
         probs[b].r = tp[b].r;
-        probs[b].x = tp[b].x;
         probs[b].p = tp[b].p;
         probs[b].Ap = tp[b].Ap;
         probs[b].partial = tp[b].partial;
         memcpy(probs[b].td, tp[b].td, sizeof(probs[b].td));
       }
-      gop = grouped_op_create<R>(probs, cells[0]->tk<R>());
-      for (int b = 0; b < B(); ++b) tv[b].nparts = grouped_op_fwd_partials(gop, b);
+      gop = grouped_op_create<double>(probs, cells[0]->tkind);
     }
     tab_p.alloc(tp.size() * sizeof(ProblemPtrsHost));
-    tab_v.alloc(tv.size() * sizeof(BatchVec<R>));
+    tab_v.alloc(tv.size() * sizeof(BatchVec<double>));
     MUSG_CUDA(cudaMemcpy(tab_p.p, tp.data(), tab_p.bytes, cudaMemcpyHostToDevice));
     MUSG_CUDA(cudaMemcpy(tab_v.p, tv.data(), tab_v.bytes, cudaMemcpyHostToDevice));
   }
 
-  template <typename R> void iteration(cudaStream_t s) {
+  void iteration(cudaStream_t s) {
+    if (disp) {
+      disp_batch_run(disp, s);
+      return;
+    }
     musg_cell &c0 = *cells[0];
     if (uniform)
-      cg_operator_batch<R>(c0.sp, c0.tk<R>(), (const ProblemPtrs<R> *)tab_p.p, tab_v.as<BatchVec<R>>(), B(),
-                           s);  // and alpha (FP32: the whole iteration)
+      cg_operator_batch<double>(c0.sp, c0.tkind, (const ProblemPtrs<double> *)tab_p.p, B(), s);  // and alpha
     else
-      grouped_op_run<R>(gop, tab_v.as<BatchVec<R>>(), nmax, B(), s);
-    if (sizeof(R) == 8) cg_update_batch<R>(tab_v.as<BatchVec<R>>(), nmax, B(), s);  // and beta
+      grouped_op_run<double>(gop, s);
+    cg_update_batch<double>(tab_v.as<BatchVec<double>>(), nmax, B(), s);  // and beta
   }
 
-  template <typename R> void build_graph() {
+  void build_graph() {
     if (exec) return;
     cudaGraph_t g = nullptr;
     const unsigned long long before = g_launches.load();
     MUSG_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
     try {
-      for (int k = 0; k < chunk; ++k) iteration<R>(stream);
+      for (int k = 0; k < chunk; ++k) iteration(stream);
     } catch (...) {
       cudaStreamEndCapture(stream, &g);
       if (g) cudaGraphDestroy(g);
@@ -873,19 +908,24 @@ struct musg_batch {
   }
 
   // one batched SolverCG::solve over the cells whose `solve` flag is set
-  template <typename R> void solve(const std::vector<char> &solve_it, std::vector<std::string> &errors) {
-    const double t = (precision == MUSG_PRECISION_MIXED) ? std::max(tol, inner_tol) : tol;
+  void solve(const std::vector<char> &solve_it, std::vector<std::string> &errors) {
+    const bool mixed = precision == MUSG_PRECISION_MIXED;
     for (int b = 0; b < B(); ++b) {
       musg_cell &c = *cells[b];
+      musg_solver &sv = *solvers[b];
       double *part = c.partial.as<double>();
-      if (solve_it[b]) {
-        cg_init<R>(state(b), c.rhs.as<double>(), solvers[b]->r.as<R>(), solvers[b]->x.as<R>(), c.nb_dof(), t,
-                   (int)maxiter, part, part + 4096, stream);
-      } else {
+      if (!solve_it[b]) {
         MUSG_CUDA(cudaMemsetAsync(&state(b)->active, 0, sizeof(int), stream));
+        MUSG_CUDA(cudaMemsetAsync(&state(b)->go, 0, sizeof(int), stream));
+      } else if (mixed) {
+        disp_start(c.sp, sv.vectors(), c.rhat.p, state(b), std::max(tol, inner_tol), (int)maxiter, nullptr,
+                   c.scal.as<double>() + 32, stream);
+      } else {
+        cg_init<double>(state(b), c.rhs.as<double>(), sv.r.as<double>(), sv.x.as<double>(), c.nb_dof(), tol,
+                        (int)maxiter, part, part + 4096, stream);
       }
     }
-    build_graph<R>();
+    build_graph();
     for (;;) {
       MUSG_CUDA(cudaGraphLaunch(exec, stream));
       g_launches.fetch_add(graph_nodes);
@@ -905,6 +945,8 @@ struct musg_batch {
           << " steps, the solver  FAILED with  |r|/|b| = " << std::sqrt(hst[b].rdr / hst[b].rhs_norm2)
           << ", cg_tol = " << std::sqrt(hst[b].tol2 / hst[b].rhs_norm2);
         errors[b] = e.str();
+      } else if (mixed) {
+        disp_solution(cells[b]->sp, solvers[b]->vectors(), state(b), solvers[b]->x.as<float>(), stream);
       }
     }
   }
@@ -985,7 +1027,7 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
     double *ddelta = c.put_matrix(delta.data(), 16);
     if (!geus) add_macro(c.F.as<double>(), ddelta, D2, c.npx, s);
     c.residual_kept = false;  // the load step's first residual is projected in FP64
-    const bool incremental = solver->precision == MUSG_PRECISION_MIXED && solver->incremental_residual;
+    const bool mixed = solver->precision == MUSG_PRECISION_MIXED, incremental = solver->incremental_residual;
     std::string message = "Has not converged";
     double incr_norm = 2 * newton_tol, grad_norm = 1, stress_norm = 2 * equil_tol;
     bool has_converged = false;
@@ -1016,17 +1058,20 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
           tangent_operator<double>(c.sp, c.tkind, c.tangent<double>(), c.rhs.as<double>(), c.rhs.as<double>(), s);
           convert<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, -1.0, s);
           c.residual_kept = false;
+          if (mixed)
+            c.residual_from_rhs();
+          else
+            dot_device<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, c.partial.as<double>(), dscal + 32, s);
         } else {
           // rhs = -P, projected
-          c.project_residual(incremental);
+          c.residual(mixed, incremental);
         }
-        dot_device<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, c.partial.as<double>(), dscal + 32, s);
         MUSG_CUDA(cudaMemcpyAsync(c.hscal + 32, dscal + 32, sizeof(double), cudaMemcpyDeviceToHost, s));
         MUSG_CUDA(cudaStreamSynchronize(s));
         stress_norm = std::sqrt(c.hscal[32]);
       }
       if (convergence_test()) break;
-      solver->solve_device_any(c.rhs.as<double>());
+      solver->solve_device(mixed ? nullptr : c.rhs.as<double>());
       if (first_geus) add_macro(c.F.as<double>(), ddelta, D2, c.npx, s);
       if (solver->line_search && !first_geus) {
         // F = F0 + lam dF for lam = 1, 1/2, ... until the projected residual norm drops
@@ -1043,8 +1088,7 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
             newton_trial<double>(c.F.as<double>(), c.F0.as<double>(), solver->x.as<double>(), lam, n,
                                  c.partial.as<double>(), dscal + 34, s);
           c.evaluate(false);
-          c.project_residual(incremental);
-          dot_device<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, c.partial.as<double>(), dscal + 32, s);
+          c.residual(mixed, incremental);
           MUSG_CUDA(cudaMemcpyAsync(c.hscal + 32, dscal + 32, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
           MUSG_CUDA(cudaStreamSynchronize(s));
           stress_norm = std::sqrt(c.hscal[32]);
@@ -1157,9 +1201,7 @@ void batch_newton_impl(musg_batch *batch, const double *steps, int nsteps, doubl
         }
         musg_cell &c = *bt.cells[b];
         c.evaluate(false);
-        c.project_residual(bt.precision == MUSG_PRECISION_MIXED && bt.solvers[b]->incremental_residual);
-        dot_device<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), c.nb_dof(), c.partial.as<double>(),
-                                   c.scal.as<double>() + 32, s);
+        c.residual(bt.precision == MUSG_PRECISION_MIXED, bt.solvers[b]->incremental_residual);
         MUSG_CUDA(cudaMemcpyAsync(c.hscal + 32, c.scal.as<double>() + 32, sizeof(double), cudaMemcpyDeviceToHost, s));
       }
       MUSG_CUDA(cudaStreamSynchronize(s));
@@ -1175,8 +1217,7 @@ void batch_newton_impl(musg_batch *batch, const double *steps, int nsteps, doubl
       }
       if (!any) break;
       std::vector<std::string> errors(B);
-      if (bt.precision == MUSG_PRECISION_MIXED) bt.solve<float>(solve_it, errors);
-      else bt.solve<double>(solve_it, errors);
+      bt.solve(solve_it, errors);
       for (int b = 0; b < B; ++b) {
         if (!solve_it[b]) continue;
         if (!errors[b].empty()) {
@@ -1235,27 +1276,36 @@ void batch_newton_impl(musg_batch *batch, const double *steps, int nsteps, doubl
 
 // ====================================================================== C ABI
 namespace {
-template <typename R> void cg_operator_once(musg_cell &c, const double *dF, double *dP) {
+void cg_operator_once(musg_cell &c, const double *dF, double *dP) {
   const long long n = c.nb_dof();
   if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
   c.upload_field(dF, c.io2.as<double>());
-  DevBuf r, x, p, Ap, st;
-  r.alloc((size_t)n * sizeof(R));
-  x.alloc((size_t)n * sizeof(R));
-  p.alloc((size_t)n * sizeof(R));
-  Ap.alloc((size_t)n * sizeof(R));
-  MUSG_CUDA(cudaMemsetAsync(x.p, 0, (size_t)n * sizeof(R), c.stream));
+  DevBuf r, p, Ap, st;
+  for (DevBuf *b : {&r, &p, &Ap}) b->alloc((size_t)n * sizeof(double));
   st.alloc(sizeof(CGState));
   // first CG iteration: p = -r, so r = -dF gives p = dF and Ap = G(K:dF)
-  convert<R, double>(r.as<R>(), c.io2.as<double>(), n, -1.0, c.stream);
+  convert<double, double>(r.as<double>(), c.io2.as<double>(), n, -1.0, c.stream);
   CGState h{};
   h.maxiter = 1;
   h.active = 1;
   MUSG_CUDA(cudaMemcpyAsync(st.p, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream));
-  // the kernels of the solver's iteration; the FP32 ones store Ap because it is given
-  cg_operator<R>(c.sp, c.tk<R>(), c.tangent<R>(), st.as<CGState>(), r.as<R>(), x.as<R>(), p.as<R>(), Ap.as<R>(),
-                 c.partial.as<double>(), c.stream);
-  convert<double, R>(c.io2.as<double>(), Ap.as<R>(), n, 1.0, c.stream);
+  cg_operator<double>(c.sp, c.tkind, c.tangent<double>(), st.as<CGState>(), r.as<double>(), p.as<double>(),
+                      Ap.as<double>(), c.partial.as<double>(), c.stream);
+  convert<double, double>(c.io2.as<double>(), Ap.as<double>(), n, 1.0, c.stream);
+  c.download_field(c.io2.as<double>(), dP);
+}
+// the FP32 operator of the mixed method: the displacement-space passes, from a general
+// (not necessarily compatible) dF
+void cg_operator_once_mixed(musg_cell &c, const double *dF, double *dP) {
+  const long long n = c.nb_dof();
+  if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
+  c.upload_field(dF, c.io2.as<double>());
+  DevBuf qhat, out;
+  qhat.alloc(disp_vector_bytes(c.sp));
+  out.alloc((size_t)n * sizeof(float));
+  disp_operator(c.sp, c.tkind32, c.tangent<float>(), c.io2.as<double>(), qhat.p, out.as<float>(), c.partial.as<double>(),
+                c.stream);
+  convert<double, float>(c.io2.as<double>(), out.as<float>(), n, 1.0, c.stream);
   c.download_field(c.io2.as<double>(), dP);
 }
 }  // namespace
@@ -1521,14 +1571,14 @@ int musg_cell_cg_operator(musg_cell *cell, int precision, const double *dF, doub
     require(c.tangent_valid, MUSG_ERR_RUNTIME,
             "currently only implemented for cases where a stiffness matrix exists");
     if (precision == MUSG_PRECISION_FP64) {
-      cg_operator_once<double>(c, dF, dP);
+      cg_operator_once(c, dF, dP);
       return;
     }
     if (!c.need32 || !c.lam32.p) {
       c.alloc32();
       c.evaluate(false);  // the FP32 tangent data of the current strain
     }
-    cg_operator_once<float>(c, dF, dP);
+    cg_operator_once_mixed(c, dF, dP);
   });
 }
 
@@ -1778,7 +1828,7 @@ int musg_solver_solve(musg_solver *solver, const double *rhs, double *x_out) {
     require(c.tangent_valid, MUSG_ERR_RUNTIME, "currently only implemented for cases where a stiffness matrix exists");
     if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
     c.upload_field(rhs, c.io2.as<double>());
-    solver->solve_device_any(c.io2.as<double>());
+    solver->solve_device(c.io2.as<double>());
     if (solver->precision == MUSG_PRECISION_MIXED)
       convert<double, float>(c.io2.as<double>(), solver->x.as<float>(), c.nb_dof(), 1.0, c.stream);
     else
@@ -1849,8 +1899,8 @@ int musg_batch_create(musg_cell **cells, int nb_cells, double tol, unsigned maxi
     bt->states.alloc(nb_cells * sizeof(CGState));
     MUSG_CUDA(cudaMemset(bt->states.p, 0, bt->states.bytes));
     MUSG_CUDA(cudaMallocHost(&bt->hst, nb_cells * sizeof(CGState)));
-    if (precision == MUSG_PRECISION_MIXED) bt->build_tables<float>();
-    else bt->build_tables<double>();
+    if (precision == MUSG_PRECISION_MIXED) bt->build_tables_mixed();
+    else bt->build_tables();
     *out = bt.release();
   });
 }

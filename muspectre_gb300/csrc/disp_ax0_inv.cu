@@ -1,0 +1,45 @@
+// Launches of the displacement-space CG's update pass and of the plain axis-0 inverse
+// (disp.cuh).
+#include "disp_launch.cuh"
+
+namespace musg {
+namespace {
+
+template <typename R, int D, bool FIN>
+void ax0_step(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+              const DispGroup<R> *grp) {
+  if (grp) return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, true>, a, c, B, s, grp);
+  switch (pl.blu ? 0 : pl.m) {
+#define MUSG_C(M, A, BB) \
+  case M: return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, A, BB, false>, a, c, B, s);
+    MUSG_DISP_PLANS(MUSG_C)
+#undef MUSG_C
+    default: return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, false>, a, c, B, s);
+  }
+}
+}  // namespace
+
+template <typename R>
+void disp_ax0_step(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+              const DispGroup<R> *grp) {
+  const bool fin = disp_finite(sp);
+  if (sp.g.dim == 2) fin ? ax0_step<R, 2, true>(sp.tp[0], a, c, B, s, grp) : ax0_step<R, 2, false>(sp.tp[0], a, c, B, s, grp);
+  else fin ? ax0_step<R, 3, true>(sp.tp[0], a, c, B, s, grp) : ax0_step<R, 3, false>(sp.tp[0], a, c, B, s, grp);
+}
+
+template <typename R>
+void disp_ax0_field(const Spectral &sp, bool from_x, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
+#define MUSG_C(DD, FF)                                                                           \
+  if (sp.g.dim == DD && disp_finite(sp) == FF) {                                                             \
+    if (from_x) disp_launch<R>(k_ax0_inv<R, DD, FF, AX_X, -1, -1, false>, a, c, 1, s);     \
+    else disp_launch<R>(k_ax0_inv<R, DD, FF, AX_Q, -1, -1, false>, a, c, 1, s);            \
+  }
+  MUSG_C(2, true) MUSG_C(2, false) MUSG_C(3, true) MUSG_C(3, false)
+#undef MUSG_C
+}
+
+template void disp_ax0_step<float>(const Spectral &, const DispArgs<float> &, const DispShape &, int, cudaStream_t,
+                                   const DispGroup<float> *);
+template void disp_ax0_field<float>(const Spectral &, bool, const DispArgs<float> &, const DispShape &, cudaStream_t);
+
+}  // namespace musg

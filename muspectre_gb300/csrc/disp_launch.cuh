@@ -1,0 +1,195 @@
+// Host side of the displacement-space passes (disp.cuh): launch shapes, arguments and
+// the dispatch over compile-time plans, shared by disp.cu and the passes' translation units (one per pass, so that they build
+// side by side).
+#pragma once
+
+#include <algorithm>
+#include <vector>
+
+#include "disp.cuh"
+#include "launch_util.h"
+
+namespace musg {
+
+// launch shape of one pass
+struct DispShape {
+  int T = 0, G = 0, ntx = 0, nbx = 0, ng = 1, comps_at_once = 1, threads = 0, blocks = 0, sp = 0, sh = 31;
+  size_t smem = 0;
+};
+
+constexpr int kDispSms = 152;
+
+inline bool disp_finite(const Spectral &sp) { return sp.proj_kind != MUSG_PROJ_SMALL_STRAIN; }
+
+// about 16 points of the tile per thread: one radix-16 or two radix-8 butterflies.  A
+// multiple of `unit` (the pencils of a pencil-fast tile, or a warp).
+inline int disp_threads(long points, long unit) {
+  const long t = std::max(64L, std::min(512L, points / 16));
+  return (int)std::max(unit, std::min(512 / unit, (t + unit - 1) / unit) * unit);
+}
+inline long lcm32(long p) {
+  long a = p;
+  while (a % 32) a += p;
+  return a;
+}
+
+// axis-0 passes: tiles of T consecutive k-points.  16 complex values are a 128-byte
+// line; narrower tiles where the grid would otherwise leave SMs without a block.
+template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
+  const bool fin = disp_finite(sp);
+  const int D = sp.g.dim, na = fin ? 2 : D * (D + 1) / 2;
+  const TilePlan &pl = sp.tp[0];
+  const long long Rr = sp.g.nk / sp.g.n[0];
+  DispShape c;
+  c.ng = fin ? D : 1;
+  const long cb = 2 * (long)sizeof(R), per = (long)na * pl.m * cb * pl.buffers(), tw = pl.r1 ? pl.m * cb : 0;
+  auto fits = [&](long T, long cap) { return T * per + tw <= cap; };
+  long T = 16;
+  while (T > 1 && !fits(T, 100 << 10)) T >>= 1;
+  while (T > 4 && (Rr + T - 1) / T * c.ng < 2 * kDispSms) T >>= 1;
+  if (!pl.m || !fits(T, optin_smem())) throw Error(MUSG_ERR_ARGUMENT, "first-axis FFT too long for one thread block");
+  c.T = (int)T;
+  c.ntx = (int)((Rr + T - 1) / T);
+  // sums: a bounded number of blocks, so that every block of the next pass can add
+  // their sums up itself
+  c.nbx = sums ? std::min(c.ntx, 4 * kDispSms / c.ng) : c.ntx;
+  c.blocks = c.nbx * c.ng;
+  c.smem = (size_t)(T * per + tw);
+  c.threads = disp_threads((long)na * pl.m * T, lcm32(na * T));
+  return c;
+}
+
+template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
+  const bool fin = disp_finite(sp);
+  const TilePlan &pl = sp.tp[1];
+  DispShape c;
+  c.ng = fin ? 3 : 6;
+  c.comps_at_once = fin ? 3 : 1;
+  const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0, nh = sp.g.nh;
+  long per = (long)c.comps_at_once * pl.m * cb * pl.buffers();
+  if (fin && per + tw > optin_smem()) {
+    c.comps_at_once = 1;
+    per = (long)pl.m * cb * pl.buffers();
+  }
+  if (!pl.m || per + tw > optin_smem()) throw Error(MUSG_ERR_ARGUMENT, "FFT axis too long for one thread block");
+  long T = std::min<long>(fin ? 16 : 32, nh);
+  while (T > 1 && T * per + tw > (56 << 10)) T = (T + 1) / 2;
+  if (T * per + tw > optin_smem()) T = 1;
+  while (T > 4 && (long long)c.ng * sp.g.n[0] * ((nh + T - 1) / T) < 2 * kDispSms) T = (T + 1) / 2;
+  const long nt = (nh + T - 1) / T;
+  T = (nh + nt - 1) / nt;  // balanced: 65 -> 5 x 13
+  c.T = (int)T;
+  c.ntx = c.nbx = (int)nt;
+  c.blocks = (int)((long long)c.ng * sp.g.n[0] * nt);
+  c.smem = (size_t)(T * per + tw);
+  c.threads = disp_threads((long)c.comps_at_once * pl.m * T, c.comps_at_once * T);
+  return c;
+}
+
+// last-axis pass: pairs of rows of all components
+template <typename R> DispShape disp_last_shape(const Spectral &sp) {
+  const bool fin = disp_finite(sp);
+  const int D = sp.g.dim, nl = fin ? D * D : D * (D + 1) / 2;
+  const TilePlan &pl = sp.tp[D - 1];
+  DispShape c;
+  const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0;
+  c.sp = padded_pencil(pl.m);
+  c.sh = 4;
+  if ((long)nl * c.sp * cb * pl.buffers() + tw > optin_smem()) {  // the longest rows: no padding
+    c.sp = pl.m;
+    c.sh = 31;
+  }
+  const long per = (long)nl * c.sp * cb * pl.buffers();
+  if (!pl.m || per + tw > optin_smem()) throw Error(MUSG_ERR_ARGUMENT, "last-axis FFT too long for one thread block");
+  // rows until a block has about 160 threads, fewer where SMs would be without a block
+  long g2 = std::max(1L, 160 * 16 / ((long)nl * pl.m));
+  g2 = std::min<long>(g2, (sp.g.nrows + 1) / 2);
+  while (g2 > 1 && g2 * per + tw > (64 << 10)) --g2;
+  while (g2 > 1 && (sp.g.nrows + 2 * g2 - 1) / (2 * g2) < 2 * kDispSms) --g2;
+  c.G = (int)(2 * g2);
+  c.blocks = (int)((sp.g.nrows + c.G - 1) / c.G);
+  c.smem = (size_t)(g2 * per + tw);
+  c.threads = disp_threads((long)nl * pl.m * g2, 32);
+  return c;
+}
+
+// arguments common to the passes
+template <typename R> DispArgs<R> disp_base(Spectral &sp) {
+  DispArgs<R> a{};
+  const int D = sp.g.dim;
+  a.n0 = sp.g.n[0];
+  a.n1 = sp.g.n[1];
+  a.nh = sp.g.nh;
+  a.L = sp.g.nlast();
+  a.Rr = (int)(sp.g.nk / sp.g.n[0]);
+  a.nk = sp.g.nk;
+  a.npx = sp.g.npx;
+  a.nrows = sp.g.nrows;
+  a.xi0 = xi_table<R>(sp, 0);
+  a.xi1 = xi_table<R>(sp, 1);
+  a.xi2 = D == 3 ? xi_table<R>(sp, 2) : nullptr;
+  auto nyq = [&](int d) { return (sp.allow_even && sp.g.n[d] % 2 == 0) ? sp.g.n[d] / 2 : -1; };
+  a.nyq0 = nyq(0);
+  a.nyq1 = nyq(1);
+  a.nyq2 = D == 3 ? nyq(2) : -1;
+  a.scale = R(1.0 / std::sqrt((double)sp.g.npx));
+  a.in_scale = 1.0;
+  return a;
+}
+template <typename R> DispArgs<R> disp_with(DispArgs<R> a, const Spectral &sp, int axis, const DispShape &c) {
+  a.ap = sp.tp[axis].device<R>();
+  a.T = c.T;
+  a.G = c.G;
+  a.ntx = c.ntx;
+  a.nbx = c.nbx;
+  a.ng = c.ng;
+  a.comps_at_once = c.comps_at_once;
+  a.sp = c.sp;
+  a.sh = c.sh;
+  return a;
+}
+
+// one grouped launch: device tables of the problems' arguments and block prefix sums
+template <typename R> struct DispGroup {
+  const DispArgs<R> *tab = nullptr;
+  const int *blk0 = nullptr;
+  int B = 0;
+};
+
+template <typename R, typename K>
+void disp_launch(K kernel, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+                 const DispGroup<R> *grp = nullptr) {
+  allow_smem(kernel);
+  launch_pdl(kernel, dim3(c.blocks, B), dim3(c.threads), c.smem, s, a, grp ? grp->tab : nullptr,
+             grp ? grp->blk0 : nullptr, grp ? grp->B : 0);
+  MUSG_CHECK_LAUNCH();
+}
+
+// power-of-two axes have kernels with compile-time plans
+#define MUSG_DISP_PLANS(X) X(32, 8, 4) X(64, 8, 8) X(128, 16, 8) X(256, 16, 16)
+
+// the passes: of an iteration (solo, batched, or grouped with grp), and the plain ones
+template <typename R>
+void disp_ax0_step(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+                   const DispGroup<R> *grp);
+template <typename R>
+void disp_ax0_field(const Spectral &sp, bool from_x, const DispArgs<R> &a, const DispShape &c, cudaStream_t s);
+template <typename R>
+void disp_mid(const Spectral &sp, bool inv, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+              const DispGroup<R> *grp);
+template <typename R>
+void disp_ax0_dots(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+                   const DispGroup<R> *grp);
+template <typename R>
+void disp_ax0_contract(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, cudaStream_t s);
+template <typename R, int D>
+void disp_pixels(int tkind, const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+                 const DispGroup<R> *grp);
+// real field in (through the tangent, tkind TK_PLAIN: without it), spectrum out
+template <typename R, int D>
+void disp_pixels_in(bool fin, int tkind, bool delta, const DispArgs<R> &a, const DispShape &c, cudaStream_t s);
+// spectrum in, real field out
+template <typename R, int D>
+void disp_pixels_out(bool fin, const DispArgs<R> &a, const DispShape &c, cudaStream_t s);
+
+}  // namespace musg

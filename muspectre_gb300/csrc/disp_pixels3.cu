@@ -1,0 +1,6 @@
+// The displacement-space CG's pixel pass in 3-D.
+#include "disp_pixels.cuh"
+
+namespace musg {
+MUSG_INSTANTIATE_PIXELS(float, 3)
+}  // namespace musg

@@ -149,6 +149,36 @@ template <> struct PrimeCS<7> {
   }
 };
 
+// the larger prime radices: cos / sin of 2 pi j / P for j <= P/2, mirrored
+#define MUSG_PRIME_CS(P, CVALS, SVALS)                                                    \
+  template <> struct PrimeCS<P> {                                                         \
+    static __device__ __forceinline__ double c(int j) {                                   \
+      constexpr double t[] = CVALS;                                                       \
+      return t[j > P / 2 ? P - j : j];                                                    \
+    }                                                                                     \
+    static __device__ __forceinline__ double s(int j) {                                   \
+      constexpr double t[] = SVALS;                                                       \
+      return j > P / 2 ? -t[P - j] : t[j];                                                \
+    }                                                                                     \
+  };
+#define MUSG_LIST(...) {__VA_ARGS__}
+MUSG_PRIME_CS(11, MUSG_LIST(1.0, 0.8412535328311811688618, 0.4154150130018864255293, -0.1423148382732851404438,
+                        -0.6548607339452850640569, -0.9594929736144973898904),
+              MUSG_LIST(0.0, 0.5406408174555975821076, 0.9096319953545183714117, 0.9898214418809327323761,
+                        0.755749574354258283774, 0.2817325568414296977114))
+MUSG_PRIME_CS(13, MUSG_LIST(1.0, 0.8854560256532098959004, 0.5680647467311558025118, 0.1205366802553230533491,
+                        -0.3546048870425356259696, -0.7485107481711010986346, -0.970941817426052027157),
+              MUSG_LIST(0.0, 0.464723172043768545656, 0.8229838658936563945796, 0.9927088740980539928008,
+                        0.9350162426854148234398, 0.6631226582407952023768, 0.2393156642875577671488))
+MUSG_PRIME_CS(17, MUSG_LIST(1.0, 0.9324722294043558045731, 0.7390089172206591159245, 0.4457383557765382673965,
+                        0.09226835946330199523965, -0.2736629900720828635391, -0.6026346363792563891786,
+                        -0.8502171357296141521341, -0.9829730996839017782819),
+              MUSG_LIST(0.0, 0.3612416661871529487447, 0.6736956436465572117127, 0.895163291355062322067,
+                        0.9957341762950345218712, 0.9618256431728190704088, 0.7980172272802395033328,
+                        0.5264321628773558002446, 0.1837495178165703315744))
+#undef MUSG_PRIME_CS
+#undef MUSG_LIST
+
 // odd prime radix P via the symmetric pair decomposition
 //   y[k]   = x0 + sum_q a_q cos(2 pi kq/P) -+ i sum_q b_q sin(2 pi kq/P)
 //   y[P-k] = x0 + sum_q a_q cos(2 pi kq/P) +- i sum_q b_q sin(2 pi kq/P)
@@ -255,6 +285,62 @@ template <bool INV, typename T> struct Dft<5, INV, T> {
 };
 template <bool INV, typename T> struct Dft<7, INV, T> {
   static __device__ __forceinline__ void run(T *v) { DftPrime<7, INV, T>::run(v); }
+};
+
+// composite radix N = A * B with A and B coprime (Good 1958, Thomas 1963): no twiddles,
+// input n = (B n1 + A n2) mod N, output k = (B (B^-1 mod A) k1 + A (A^-1 mod B) k2) mod N
+__host__ __device__ constexpr int inverse_mod(int a, int m) {
+  for (int x = 1; x < m; ++x)
+    if (a * x % m == 1) return x;
+  return 1;
+}
+template <int A, int B, bool INV, typename T> struct DftCoprime {
+  static __device__ __forceinline__ void run(T *v) {
+    constexpr int N = A * B, EA = B * inverse_mod(B % A, A), EB = A * inverse_mod(A % B, B);
+    T a[B][A];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+#pragma unroll
+      for (int n1 = 0; n1 < A; ++n1) a[n2][n1] = v[(B * n1 + A * n2) % N];
+      Dft<A, INV, T>::run(a[n2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+      T b[B];
+#pragma unroll
+      for (int n2 = 0; n2 < B; ++n2) b[n2] = a[n2][k1];
+      Dft<B, INV, T>::run(b);
+#pragma unroll
+      for (int k2 = 0; k2 < B; ++k2) v[(EA * k1 + EB * k2) % N] = b[k2];
+    }
+  }
+};
+template <bool INV, typename T> struct Dft<1, INV, T> {
+  static __device__ __forceinline__ void run(T *) {}
+};
+template <bool INV, typename T> struct Dft<6, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 3, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<10, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 5, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<12, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<4, 3, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<14, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 7, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<15, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<3, 5, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<11, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftPrime<11, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<13, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftPrime<13, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<17, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftPrime<17, INV, T>::run(v); }
 };
 
 // -------------------------------------------------------------- one stage

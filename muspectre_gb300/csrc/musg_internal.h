@@ -103,6 +103,29 @@ struct AxisPlan {
   template <typename R> AxisPlanD<R> device() const;
 };
 
+// Plan of the in-place tile transforms (tile_fft.cuh): m = r1 r2 in two stages (r1 = 0:
+// three or more factors, the radix of stage s in bits [5s, 5s+5) of rcode), blu: a
+// Bluestein transform of length n over m.
+template <typename R> struct TilePlanD {
+  int n, m, r1, r2, blu, nst;
+  unsigned long long rcode;
+  const typename V2<R>::T *tw;     // m entries: exp(-2 pi i j / m)
+  const typename V2<R>::T *chirp;  // n entries (Bluestein)
+  const typename V2<R>::T *bf;     // m entries (Bluestein)
+};
+struct TilePlan {
+  int n = 0, m = 0, r1 = 0, r2 = 0, blu = 0, nst = 0;
+  int radix[kMaxStages] = {0};
+  void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;
+  void *tw32 = nullptr, *chirp32 = nullptr, *bf32 = nullptr;
+  // factors only (host); build() also makes the device tables
+  void factor(int n);
+  void build(int n);
+  void release();
+  template <typename R> TilePlanD<R> device() const;
+  int buffers() const { return r1 ? 1 : 2; }  // tile buffers a transform needs
+};
+
 // ---------------------------------------------------------------- geometry
 struct Geom {
   int dim = 0;
@@ -124,6 +147,7 @@ enum TangentKind : int {
   TK_FISO = 5,    // TK_FINITE with S rebuilt from F per application (isotropic LE1/LE3/LE4)
   TK_GSMALL = 6,  // small strain, per-material stiffness C (MaterialLinearElasticGeneric): dP = C:de
   TK_GFINITE = 7, // finite strain, per-material C: dP = dF S + F (C:(F^T dF))
+  TK_ANYFIN = 9,  // the displacement-space pixel pass (disp.cuh): any finite-strain kind, by DispArgs::tkind
   TK_FULL = 8,    // stored per-pixel tangent K(i,m,j,n) (D^4 planes): dP = K:dF (the consistent
                   // elasto-plastic tangent, and the elastic pixels of a cell that has it)
 };
@@ -158,6 +182,12 @@ struct CGState {
   int active;        // 1 while the loop runs
   int ticket;        // blocks of the running kernel that have written their partial sum
   unsigned long long counter;  // cumulative iterations (SolverBase::counter)
+  // displacement-space iteration (disp.cuh): whether another operator application follows
+  // (active: the update pass is still due), and the part of |rhs|^2 outside the range of
+  // the projection
+  int go;
+  double out2;
+  double xscale;  // the norm of the right-hand side, by which that solve is scaled
 };
 
 // ---------------------------------------------------------------- spectral ops
@@ -169,6 +199,7 @@ struct Spectral {
   bool allow_even = false;
   double lengths[3] = {1, 1, 1};
   AxisPlan ax[3];
+  TilePlan tp[3];           // the same axes for the displacement-space passes (disp.cu)
   // per-axis xi_d(k) = fftfreq_d(k)/L_d over the hermitian index range, FP64 and FP32
   void *xi64[3] = {nullptr, nullptr, nullptr};
   void *xi32[3] = {nullptr, nullptr, nullptr};
@@ -180,19 +211,14 @@ struct Spectral {
   // the defaults below or by spectral_autotune
   int tune_threads[2][3] = {{256, 256, 256}, {256, 256, 256}};
   long tune_bytes[2][3] = {{73728, 49152, 73728}, {73728, 49152, 73728}};
-  // TMA descriptor of the FP32 spectrum for the Green pass (an opaque CUtensorMap,
-  // encoded on first use for the tile width and mode below) and its persistent grid
-  unsigned char green_tmap[128] = {};
-  const void *green_tmap_spec = nullptr;
-  int green_tmap_T = 0, green_tmap_mode = -1, green_tmap_grid = 0;
   void init(int dim, const int *res, int ncomp, int proj_kind, const double *lengths,
             bool allow_even, bool want32);
   void ensure32();
   void release();
 };
 
-// Device word set by a kernel whose bounded wait on an asynchronous copy ran out
-// (spectral_tma.cuh); its device address, for a stream-ordered read by the host
+// Device word set by a kernel whose bounded wait ran out (probe.cu); its device address,
+// for a stream-ordered read by the host
 unsigned *wait_fault_word();
 // one block that waits on an mbarrier nothing arrives at, bounded by limit_ns
 // (self-test of the bounded waits: it sets the fault word and exits)
@@ -212,19 +238,14 @@ void spectral_inverse(Spectral &sp, R *out, R scale, cudaStream_t s);
 template <typename R>
 void spectral_project(Spectral &sp, const R *in, R *out, R in_scale, cudaStream_t s);
 
-// CG operator application with the iteration's vector work fused into its passes.
-// FP64 (the reference's order): p = -r + beta p (or p = -r on the first iteration),
-// Ap = G(K:p), and alpha = r.r / p.Ap in the state (last block of the last pass);
-// cg_update completes the iteration.  FP32 (the mixed path's inner solve): the whole
-// iteration: the first pass writes the block sums of p.(K:p), cg_update_x sets
-// alpha = r.r / p.(K:p) and applies x += alpha p, the last pass r += alpha Ap, beta
-// and the loop condition; x is not
-// read in FP64, and Ap is written in FP32 only when non-null.  Returns the number of
-// partial sums written by the last pass.  ev (optional): an event is recorded before
-// the first and after every kernel
+// CG operator application with the iteration's vector work fused into its passes (FP64,
+// the reference's order): p = -r + beta p (or p = -r on the first iteration), Ap =
+// G(K:p), and alpha = r.r / p.Ap in the state (last block of the last pass); cg_update
+// completes the iteration.  Returns the number of partial sums written by the last
+// pass.  ev (optional): an event is recorded before the first and after every kernel
 template <typename R>
 int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState *st,
-                R *r, R *x, R *p, R *Ap, double *partial, cudaStream_t s,
+                R *r, R *p, R *Ap, double *partial, cudaStream_t s,
                 cudaEvent_t *ev = nullptr);
 // plain operator (no CG state): out = G(K:in)
 template <typename R>
@@ -238,36 +259,66 @@ struct ProblemPtrsHost {
   void *spec;
   const CGState *st;
   void *r;
-  void *x;
   void *p;
   void *Ap;
   double *partial;
   unsigned char td[sizeof(TangentData<double>)];
 };
-template <typename R> struct BatchVec;
 template <typename R>
-int cg_operator_batch(Spectral &sp, int tkind, const ProblemPtrs<R> *tab, const BatchVec<R> *xtab, int B,
-                      cudaStream_t s);
+int cg_operator_batch(Spectral &sp, int tkind, const ProblemPtrs<R> *tab, int B, cudaStream_t s);
 // Grouped CG operator over problems of different grids (the same dimension,
 // projection and tangent kind): one launch per pass for all of them, problem b
 // owning a contiguous range of the one-dimensional grid (generic pass kernels, whose
 // plans and sizes are runtime values).  The per-problem arguments live in device
-// tables built once; run launches one CG iteration's passes (FP32: with cg_alpha /
-// cg_update_x over xtab between the forward and the middle passes).
+// tables built once; run launches one CG iteration's passes.
 struct GroupProblem {
   Spectral *sp;
   const CGState *st;
-  void *r, *x, *p, *Ap;
+  void *r, *p, *Ap;
   double *partial;
   unsigned char td[sizeof(TangentData<double>)];
 };
 struct GroupedOp;
 template <typename R> GroupedOp *grouped_op_create(const std::vector<GroupProblem> &probs, int tkind);
 void grouped_op_destroy(GroupedOp *op);
-// partial sums the grouped forward pass writes for problem b (its blocks x warps)
-int grouped_op_fwd_partials(const GroupedOp *op, int b);
-template <typename R>
-void grouped_op_run(GroupedOp *op, const BatchVec<R> *xtab, long long nmax, int B, cudaStream_t s);
+template <typename R> void grouped_op_run(GroupedOp *op, cudaStream_t s);
+// ---------------------------------------------------------------- displacement-space CG (disp.cu)
+// The FP32 inner solve of the mixed method (disp.cuh).  A vector in the range of the
+// projection is D complex values per half-spectrum point, [D][nk] float2.
+struct DispVectors {
+  void *r = nullptr, *q = nullptr, *p = nullptr, *x = nullptr;
+};
+inline size_t disp_vector_bytes(const Spectral &sp) { return (size_t)sp.g.nk * sp.g.dim * sizeof(float2); }
+// rhat (+)= the projection of scale * field (FP64 planes), or with prev of prev - field,
+// after which prev = field; *norm2 = |rhat|^2 (a device double)
+void disp_residual(Spectral &sp, void *rhat, const double *field, double *prev, double scale, bool accumulate,
+                   double *partial, double *norm2, cudaStream_t s);
+// state and vectors of a solve A x = rhat: tol is relative to *rhs2, or to *range2 =
+// |rhat|^2 when rhs2 is null (device doubles); what *rhs2 has beyond *range2 is outside
+// the range of the projection and stays in the residual
+void disp_start(Spectral &sp, const DispVectors &v, const void *rhat, CGState *st, double tol, int maxiter,
+                const double *rhs2, const double *range2, cudaStream_t s);
+// one CG iteration: five passes (3-D) or three (2-D)
+void disp_iteration(Spectral &sp, int tkind, const TangentData<float> &td, const DispVectors &v, CGState *st,
+                    double *partial, cudaStream_t s, cudaEvent_t *ev = nullptr);
+// the solution of the state's solve as real component planes
+void disp_solution(Spectral &sp, const DispVectors &v, CGState *st, float *x, cudaStream_t s);
+// out = G(K:in) of a real field (FP64 planes in, FP32 out); qhat: one vector of scratch
+void disp_operator(Spectral &sp, int tkind, const TangentData<float> &td, const double *in, void *qhat, float *out,
+                   double *partial, cudaStream_t s);
+// iterations of several problems per launch: of one grid (the solo kernels, problem =
+// blockIdx.y), or of different grids (each owning a range of the blocks)
+struct DispProblem {
+  Spectral *sp;
+  DispVectors v;
+  CGState *st;
+  double *partial;
+  TangentData<float> td;
+};
+struct DispBatch;
+DispBatch *disp_batch_create(const std::vector<DispProblem> &probs, int tkind, bool uniform);
+void disp_batch_destroy(DispBatch *b);
+void disp_batch_run(DispBatch *b, cudaStream_t s);
 // Times candidate launch shapes of each pass on this grid (CUDA events) and keeps
 // the fastest (FFT_PlanFlags::measure / patient); fp32 selects the FP32 passes.
 template <typename R> void spectral_autotune(Spectral &sp, cudaStream_t s, int effort);
@@ -294,25 +345,14 @@ template <typename R> struct BatchVec {
   const R *Ap;
   double *partial;
   long long n;  // entries of the problem's vectors
-  int nparts;   // the forward pass's partial sums of the problem (grouped launches)
 };
 template <typename R>
 void cg_update_batch(const BatchVec<R> *tab, long long n, int B, cudaStream_t s);
-// alpha from the forward pass's nparts block sums of p.(K:p) and x += alpha p of the
-// FP32 inner solve's iteration, launched between its forward and inverse passes
-// (solo / batched; a batch's problems have nparts sums each in their partial arrays)
-template <typename R>
-void cg_update_x(const CGState *st, R *x, const R *p, long long n, const double *partial, int nparts,
-                 cudaStream_t s);
-template <typename R> void cg_update_x_batch(const BatchVec<R> *tab, long long n, int nparts, int B, cudaStream_t s);
 // FP64 dot of a with b over n entries into *out_device (deterministic)
 template <typename Ra, typename Rb>
 void dot_device(const Ra *a, const Rb *b, long long n, double *partial, double *out,
                 cudaStream_t s);
 // y += x (promoting), with the dots x.x and y.y (after the update) into out[0], out[1]
-// d = (float)(rhs - (P - Pk)), Pk = P: the FP32 input of the mixed path's
-// incremental Newton residual
-void residual_input(const double *rhs, const double *P, double *Pk, float *d, long long n, cudaStream_t s);
 template <typename R>
 void newton_update(double *F, const R *x, long long n, double *partial, double *out,
                    cudaStream_t s);

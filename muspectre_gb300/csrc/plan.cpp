@@ -3,6 +3,7 @@
 // Twiddles are computed in long double from their definition exp(-2 pi i j/m)
 // and rounded once to double and to float; the Bluestein filter DFT_m(conj w)/m is
 // formed on the host by a direct DFT with compensated (Kahan) summation.
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstring>
@@ -78,25 +79,10 @@ void *upload_complex(const std::vector<std::complex<long double>> &v) {
   return upload(h.data(), h.size() * sizeof(T2));
 }
 
-}  // namespace
-
-void AxisPlan::build(int n_) {
-  release();
-  n = n_;
-  std::vector<int> rad;
-  if (factorize(n, rad)) {
-    blu = 0;
-    m = n;
-  } else {
-    blu = 1;
-    if (n > (1 << 28)) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
-    m = smooth_at_least(2 * n - 1);
-    factorize(m, rad);
-  }
-  if ((int)rad.size() > kMaxStages) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
-  nst = (int)rad.size();
-  for (int s = 0; s < nst; ++s) radix[s] = rad[s];
-
+// device tables of a length-n transform over m (FP64 and FP32): twiddles W_m^j, and for
+// Bluestein the chirp and the filter
+void build_tables(int n, int m, int blu, void *&tw64, void *&tw32, void *&chirp64, void *&chirp32, void *&bf64,
+                  void *&bf32) {
   std::vector<std::complex<long double>> tw(m);
   for (int j = 0; j < m; ++j) {
     long double a = -2.0L * kPi * (long double)j / (long double)m;
@@ -146,6 +132,28 @@ void AxisPlan::build(int n_) {
   }
 }
 
+}  // namespace
+
+void AxisPlan::build(int n_) {
+  release();
+  n = n_;
+  std::vector<int> rad;
+  if (factorize(n, rad)) {
+    blu = 0;
+    m = n;
+  } else {
+    blu = 1;
+    if (n > (1 << 28)) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
+    m = smooth_at_least(2 * n - 1);
+    factorize(m, rad);
+  }
+  if ((int)rad.size() > kMaxStages) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
+  nst = (int)rad.size();
+  for (int s = 0; s < nst; ++s) radix[s] = rad[s];
+
+  build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
+}
+
 void AxisPlan::release() {
   for (void **p : {&tw64, &chirp64, &bf64, &tw32, &chirp32, &bf32}) {
     if (*p) cudaFree(*p);
@@ -173,6 +181,113 @@ template <> AxisPlanD<float> AxisPlan::device<float>() const {
   d.chirp = (const float2 *)chirp32;
   d.bf = (const float2 *)bf32;
   return d;
+}
+
+namespace {
+
+// arithmetic per point of one radix-r stage, in units of one addition per point: what
+// the factor choice below weighs (small composites cost about 2 log2 r and a twiddle,
+// the direct primes about r)
+double stage_cost(int r) {
+  static const double c[18] = {0, 0, 2, 4.5, 4, 8, 6.5, 11, 6.5, 9, 10, 15, 8.5, 18, 13, 12.5, 9, 23};
+  return c[r] + 4.0;  // + twiddles and a shared-memory round trip
+}
+
+// the cheapest factorisation of m into radices 2..17: two factors if there are any,
+// else the fewest; false when a prime above 17 divides m
+bool tile_factor(int m, std::vector<int> &rad, double &cost) {
+  rad.clear();
+  cost = 1e30;
+  for (int a = 1; a <= 17; ++a)
+    if (m % a == 0 && m / a <= 17) {
+      const int b = m / a;
+      if (b < a) continue;
+      const double c = (a > 1 ? stage_cost(a) : 0.0) + (b > 1 ? stage_cost(b) : 0.0);
+      if (c < cost) {
+        cost = c;
+        rad = {b, a};  // r1 >= r2
+      }
+    }
+  if (!rad.empty()) return true;
+  // three or more: peel the largest factor that leaves the cheapest rest
+  for (int a = 17; a >= 2; --a) {
+    if (m % a) continue;
+    std::vector<int> rest;
+    double c = 0;
+    if (!tile_factor(m / a, rest, c)) continue;
+    rest.erase(std::remove(rest.begin(), rest.end(), 1), rest.end());
+    if (c + stage_cost(a) + 1.0 < cost) {
+      cost = c + stage_cost(a) + 1.0;
+      rad.assign(1, a);
+      rad.insert(rad.end(), rest.begin(), rest.end());
+    }
+  }
+  return !rad.empty();
+}
+
+}  // namespace
+
+void TilePlan::factor(int n_) {
+  n = n_;
+  m = nst = r1 = r2 = 0;
+  if (n > (1 << 16)) return;  // longer than any tile: the passes refuse it (m = 0)
+  std::vector<int> rad;
+  double cost = 0;
+  if (tile_factor(n, rad, cost)) {
+    blu = 0;
+    m = n;
+  } else {
+    // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass
+    blu = 1;
+    double best = 1e30;
+    std::vector<int> r;
+    for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
+      double c = 0;
+      if (!tile_factor(k, r, c)) continue;
+      c *= k;
+      if (c < best) {
+        best = c;
+        m = k;
+        rad = r;
+      }
+    }
+    if (best > 1e29) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
+  }
+  nst = (int)rad.size();
+  if (nst > kMaxStages) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
+  for (int s = 0; s < nst; ++s) radix[s] = rad[s];
+  r1 = nst == 2 ? rad[0] : 0;
+  r2 = nst == 2 ? rad[1] : 0;
+}
+
+void TilePlan::build(int n_) {
+  release();
+  factor(n_);
+  if (m) build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
+}
+
+void TilePlan::release() {
+  for (void **p : {&tw64, &chirp64, &bf64, &tw32, &chirp32, &bf32}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+}
+
+template <typename R, typename T>
+static TilePlanD<R> tile_plan_device(const TilePlan &t, const void *tw, const void *chirp, const void *bf) {
+  TilePlanD<R> d{};
+  d.n = t.n; d.m = t.m; d.r1 = t.r1; d.r2 = t.r2; d.blu = t.blu; d.nst = t.nst;
+  for (int s = 0; s < t.nst; ++s) d.rcode |= (unsigned long long)t.radix[s] << (5 * s);
+  d.tw = (const T *)tw;
+  d.chirp = (const T *)chirp;
+  d.bf = (const T *)bf;
+  return d;
+}
+template <> TilePlanD<double> TilePlan::device<double>() const {
+  return tile_plan_device<double, double2>(*this, tw64, chirp64, bf64);
+}
+template <> TilePlanD<float> TilePlan::device<float>() const {
+  return tile_plan_device<float, float2>(*this, tw32, chirp32, bf32);
 }
 
 // fftfreq(n)[k]/L (src/fft/fft_utils.cc:41-56)
@@ -220,11 +335,14 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
 
 void Spectral::ensure32() {
   want32 = true;
+  for (int d = 0; d < g.dim; ++d)
+    if (tp[d].n != g.n[d]) tp[d].build(g.n[d]);
   if (!spec32) MUSG_CUDA(cudaMalloc(&spec32, (size_t)ncomp * g.nk * sizeof(float2)));
 }
 
 void Spectral::release() {
   for (auto &a : ax) a.release();
+  for (auto &a : tp) a.release();
   for (int d = 0; d < 3; ++d) {
     if (xi64[d]) cudaFree(xi64[d]);
     if (xi32[d]) cudaFree(xi32[d]);

@@ -7,6 +7,12 @@
 // fused multiply-add chains (eight per thread, so that the pipe's latency is covered
 // by the chains of one warp and the warps of a block) and reports FLOP/s = 2 x FMAs /
 // CUDA-event time.
+//
+// Also the self-test of a bounded wait on an mbarrier (musg_selftest_wait_timeout): a
+// wait that nothing completes gives up after a wall-clock limit, records the fault in a
+// device word and leaves the device usable.
+#include <cstdint>
+
 #include "musg_internal.h"
 
 namespace musg {
@@ -28,7 +34,71 @@ __global__ void k_fp64_fma(double *sink, int iters, double a, double b) {
   if (s == 12345.678) sink[0] = s;  // keeps the chains live; never true for these inputs
 }
 
+__device__ unsigned int g_wait_fault;
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_init_fence() {
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// poll until the phase of the given parity completed or the wall-clock limit ran out
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity,
+                                                  unsigned long long limit_ns) {
+  const unsigned long long t0 = global_ns();
+  for (unsigned i = 0;; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && global_ns() - t0 > limit_ns) return false;
+  }
+}
+
+// Self-test of the bounded wait: one thread waits on an mbarrier that nothing arrives
+// at, gives up after limit_ns, records the fault word, and
+// the kernel exits (no copy is in flight).
+__global__ void k_wait_probe(unsigned long long limit_ns) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && !mbar_wait_bounded(&bar, 0, limit_ns)) atomicOr(&g_wait_fault, 1u);
+}
+
 }  // namespace
+
+void wait_probe(unsigned long long limit_ns, cudaStream_t s) {
+  k_wait_probe<<<1, 32, 0, s>>>(limit_ns);
+  MUSG_CHECK_LAUNCH();
+}
+
+unsigned *wait_fault_word() {
+  static unsigned *p = [] {
+    void *q = nullptr;
+    MUSG_CUDA(cudaGetSymbolAddress(&q, g_wait_fault));
+    return static_cast<unsigned *>(q);
+  }();
+  return p;
+}
 
 double fp64_fma_tflops(cudaStream_t s) {
   int dev = 0, nsm = 0;

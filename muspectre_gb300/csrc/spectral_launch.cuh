@@ -1,5 +1,5 @@
-// Host launchers of the spectral passes, instantiated once per precision by
-// spectral_f64.cu and spectral_f32.cu.
+// Host launchers of the FP64 spectral passes, instantiated by
+// spectral_f64.cu (the mixed method's FP32 passes are disp.cu).
 #pragma once
 
 #include <algorithm>
@@ -9,44 +9,13 @@
 #include <set>
 #include <vector>
 
+#include "launch_util.h"
 #include "spectral.cuh"
 #include "spectral_reg.cuh"
 
 namespace musg {
 
-// The FP32 Green pass through the TMA-fed persistent kernel (spectral_tma.cu) for a
-// tile of Tt pencils; false (nothing launched) when the spectrum, the tile or the
-// driver does not qualify, and the caller launches the register kernel instead.
-bool launch_green_tma(Spectral &sp, int mode, const GreenArgs<float> &a, int Tt, cudaStream_t s);
-// The FP32 last-axis inverse with the CG epilogue through the bulk-copy-fed
-// persistent kernel (spectral_tma.cu) for tiles of G rows; returns its number of
-// blocks (= partial sums), or 0 (nothing launched) when the shape does not qualify.
-int launch_last_inv_tma(Spectral &sp, const LastArgs<float> &a, int G, cudaStream_t s, int B = 1);
-
 namespace {
-
-int optin_smem() {
-  static int v = 0;
-  if (v == 0) {
-    int dev = 0;
-    MUSG_CUDA(cudaGetDevice(&dev));
-    int b = 0;
-    MUSG_CUDA(cudaDeviceGetAttribute(&b, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    v = b - 2048;  // room for the static shared memory of the reductions
-  }
-  return v;
-}
-
-// raise the dynamic shared-memory limit of a kernel once (keyed by its address)
-template <typename K> void allow_smem(K kernel) {
-  static std::mutex mu;
-  static std::set<const void *> done;
-  const void *key = (const void *)kernel;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done.count(key)) return;
-  MUSG_CUDA(cudaFuncSetAttribute(key, cudaFuncAttributeMaxDynamicSharedMemorySize, optin_smem()));
-  done.insert(key);
-}
 
 struct Cfg {
   int per;       // rows per block (last pass) or tile (axis / green passes)
@@ -156,9 +125,6 @@ void dispatch_fwd(int dim, int tk, const LastArgs<R> &a, const Cfg &c, cudaStrea
   MUSG_FWD_CASE(3, TK_SMALL) MUSG_FWD_CASE(3, TK_FINITE) MUSG_FWD_CASE(3, TK_KPRIME) MUSG_FWD_CASE(3, TK_MIXED)
   MUSG_FWD_CASE(2, TK_GSMALL) MUSG_FWD_CASE(2, TK_GFINITE) MUSG_FWD_CASE(3, TK_GSMALL) MUSG_FWD_CASE(3, TK_GFINITE)
   MUSG_FWD_CASE(2, TK_FULL) MUSG_FWD_CASE(3, TK_FULL)
-  if (sizeof(R) == 4) {
-    MUSG_FWD_CASE(2, TK_FISO) MUSG_FWD_CASE(3, TK_FISO)
-  }
 #undef MUSG_FWD_CASE
   throw Error(MUSG_ERR_ARGUMENT, "unsupported tangent kind");
 }
@@ -218,101 +184,6 @@ void launch_green_reg(int m, const GreenArgs<R> &a, dim3 grid, dim3 block, size_
   }
 #undef MUSG_GRR
   MUSG_CHECK_LAUNCH();
-}
-
-// last-axis register kernels (FP32 CG passes): rows per block G = 2 G2 with the
-// block (Y lanes, ncomp G2 pencils) a whole number of warps and at most 384 threads;
-// G = 0 when the axis or the shape does not allow them
-// Rows per block of the register last-axis passes (two rows share one complex
-// transform, so G is even; a block is Y lanes x ncomp components x G/2 row pairs).
-// Measured on 128^3 finite-strain cells (9 components, Y = 8): the forward pass is
-// fastest at 144 threads (77 us; 78-86 us at 72, 216, 288 threads, 92 us at 360) and
-// the inverse at 216 (70 us; 74 us at 288, 77 at 144, 91 at 72).  Small blocks keep
-// more of them resident between the stage barriers; the rule takes the most row
-// pairs whose block stays within those thread counts.  0 = no register path.
-template <typename R> int last_reg_rows(const Spectral &sp, bool inv) {
-  if (sizeof(R) != 4) return 0;
-  const AxisPlan &ap = sp.ax[sp.g.dim - 1];
-  if (!reg_axis(ap)) return 0;
-  const int m = ap.m, Y = reg_lanes(m), nc = sp.ncomp;
-  const long ps = (long)(m + m / RegLanesR1(m));
-  const long per_g2 = (long)nc * ps * (long)sizeof(typename V2<R>::T);
-  const long target = inv ? 224 : 160, bound = inv ? 384 : 512;  // launch bounds of the kernels
-  const long th1 = (long)Y * nc;
-  if (th1 > bound || per_g2 + (long)m * (long)sizeof(float2) > optin_smem()) return 0;
-  long g2 = std::max(1L, target / th1);
-  g2 = std::min<long>(g2, (sp.g.nrows + 1) / 2);
-  g2 = std::min<long>(g2, (optin_smem() - (long)m * (long)sizeof(float2)) / per_g2);  // + twiddle table
-  return (int)(2 * g2);
-}
-
-template <int D, int TK>
-void launch_fwd_reg(int m, const LastArgs<float> &a, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
-#define MUSG_LFR(M)                           \
-  case M: {                                   \
-    auto k = k_last_fwd_reg<M, D, TK>;        \
-    allow_smem(k);                            \
-    launch_pdl(k, grid, block, smem, s, a);           \
-    break;                                    \
-  }
-  switch (m) {
-    MUSG_LFR(16) MUSG_LFR(32) MUSG_LFR(64) MUSG_LFR(128) MUSG_LFR(256)
-    default: throw Error(MUSG_ERR_ARGUMENT, "no register FFT of this length");
-  }
-#undef MUSG_LFR
-  MUSG_CHECK_LAUNCH();
-}
-
-template <int D>
-void launch_inv_reg(int m, const LastArgs<float> &a, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
-#define MUSG_LIR(M)                           \
-  case M: {                                   \
-    auto k = k_last_inv_reg<M, D>;            \
-    allow_smem(k);                            \
-    launch_pdl(k, grid, block, smem, s, a);           \
-    break;                                    \
-  }
-  switch (m) {
-    MUSG_LIR(16) MUSG_LIR(32) MUSG_LIR(64) MUSG_LIR(128) MUSG_LIR(256)
-    default: throw Error(MUSG_ERR_ARGUMENT, "no register FFT of this length");
-  }
-#undef MUSG_LIR
-  MUSG_CHECK_LAUNCH();
-}
-
-// the two CG last-axis passes through the register kernels; returns the number of
-// partial sums (blocks)
-template <typename R>
-int last_cg_reg(Spectral &sp, int tkind, LastArgs<R> a, int G, bool inv, cudaStream_t s, int B) {
-  if constexpr (sizeof(R) != 4) {
-    throw Error(MUSG_ERR_RUNTIME, "register last-axis passes are FP32 only");
-  } else {
-    const int m = sp.ax[sp.g.dim - 1].m, Y = reg_lanes(m);
-    const int nc = sp.ncomp, G2 = G / 2;
-    const int blocks = (int)((sp.g.nrows + G - 1) / G);
-    const long ps = m + m / RegLanesR1(m);
-    a.G = G;
-    const dim3 grid(blocks, B), block(Y, nc * G2);
-    const int wpb = (Y * nc * G2 + 31) / 32;  // warps per block (the forward pass's partial sums per block)
-    const size_t smem = ((size_t)nc * G2 * ps + m) * sizeof(float2);  // pencils + twiddle table
-    if (!inv) {
-#define MUSG_FR(DD, TT) \
-  if (sp.g.dim == DD && tkind == TT) { launch_fwd_reg<DD, TT>(m, a, grid, block, smem, s); return blocks * wpb; }
-      MUSG_FR(2, TK_SMALL) MUSG_FR(2, TK_FINITE) MUSG_FR(2, TK_KPRIME) MUSG_FR(2, TK_MIXED) MUSG_FR(2, TK_FISO)
-      MUSG_FR(3, TK_SMALL) MUSG_FR(3, TK_FINITE) MUSG_FR(3, TK_KPRIME) MUSG_FR(3, TK_MIXED) MUSG_FR(3, TK_FISO)
-      MUSG_FR(2, TK_GSMALL) MUSG_FR(2, TK_GFINITE) MUSG_FR(3, TK_GSMALL) MUSG_FR(3, TK_GFINITE)
-      MUSG_FR(2, TK_FULL) MUSG_FR(3, TK_FULL)
-#undef MUSG_FR
-      throw Error(MUSG_ERR_ARGUMENT, "unsupported tangent kind");
-    }
-    {
-      const int nb = launch_last_inv_tma(sp, a, G, s, B);
-      if (nb) return nb;
-    }
-    if (sp.g.dim == 2) launch_inv_reg<2>(m, a, grid, block, smem, s);
-    else launch_inv_reg<3>(m, a, grid, block, smem, s);
-    return blocks;
-  }
 }
 
 template <typename R>
@@ -400,9 +271,6 @@ void run_green(Spectral &sp, int mode, const CGState *st, cudaStream_t s, const 
     if (tmax >= 1) {
       const long Tt = reg_tile(sp.tune_bytes[prec_index<R>()][2], (long)nc * m * sizeof(T), tmax, Rr);
       a.T = (int)Tt;
-      if constexpr (sizeof(R) == 4) {
-        if (!batch && B == 1 && launch_green_tma(sp, mode, a, (int)Tt, s)) return;
-      }
       const dim3 grid((unsigned)((Rr + Tt - 1) / Tt), mode == GM_FINITE ? dim : 1, B), block((unsigned)Tt, Y, nc);
       const size_t smem = (size_t)(nc * Tt + 1) * m * sizeof(T);  // tile + twiddle table
       if (mode == GM_FINITE && dim == 2) launch_green_reg<R, GM_FINITE, 2>(m, a, grid, block, smem, s);
@@ -476,17 +344,13 @@ void spectral_project(Spectral &sp, const R *in, R *out, R in_scale, cudaStream_
 }
 
 template <typename R>
-int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState *st, R *r, R *x, R *p,
-                R *Ap, double *partial, cudaStream_t s, cudaEvent_t *ev) {
-  // FP32 (the mixed path's inner solve): the fused iteration; FP64: the reference's
-  constexpr int kPro = sizeof(R) == 4 ? PRO_CGF : PRO_CG;
-  constexpr int kEpi = sizeof(R) == 4 ? EPI_CGF : EPI_CG;
+int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState *st, R *r, R *p, R *Ap,
+                double *partial, cudaStream_t s, cudaEvent_t *ev) {
   const int gm = green_mode_of(sp);
   const Cfg c = last_cfg<R>(sp);
   LastArgs<R> a = last_args<R>(sp, c);
   a.st = st;
   a.r = r;
-  a.x = x;
   a.p = p;
   a.Ap = Ap;
   a.partial = partial;
@@ -495,18 +359,9 @@ int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState
   auto mark = [&]() {
     if (ev) MUSG_CUDA(cudaEventRecord(ev[k++], s));
   };
-  const int gfwd = last_reg_rows<R>(sp, false), ginv = last_reg_rows<R>(sp, true);
-  const bool greg = gfwd && ginv;
   mark();
-  int nfwd = c.blocks * ((c.threads + 31) / 32);  // the forward pass's per-warp partial sums
-  if (greg) nfwd = last_cg_reg<R>(sp, tkind, a, gfwd, false, s, 1);
-  else dispatch_fwd<R, kPro>(sp.g.dim, tkind, a, c, s);
+  dispatch_fwd<R, PRO_CG>(sp.g.dim, tkind, a, c, s);
   mark();
-  if constexpr (sizeof(R) == 4) {
-    // alpha, and x += alpha p, between the forward pass and the one that may end the loop
-    cg_update_x<R>(st, x, p, sp.g.npx * sp.ncomp, partial, nfwd, s);
-    mark();
-  }
   if (sp.g.dim == 3) {
     run_axis<R>(sp, false, st, s);
     mark();
@@ -517,43 +372,27 @@ int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState
     run_axis<R>(sp, true, st, s);
     mark();
   }
-  int nb;
-  if (greg) {
-    nb = last_cg_reg<R>(sp, tkind, a, ginv, true, s, 1);
-  } else {
-    if (sp.g.dim == 2) launch_inv<R, kEpi, 2>(a, c, s);
-    else launch_inv<R, kEpi, 3>(a, c, s);
-    nb = c.blocks;
-  }
+  if (sp.g.dim == 2) launch_inv<R, EPI_CG, 2>(a, c, s);
+  else launch_inv<R, EPI_CG, 3>(a, c, s);
   mark();
-  return nb;
+  return c.blocks;
 }
 
-static_assert(sizeof(ProblemPtrs<float>) == sizeof(ProblemPtrsHost) &&
-                  sizeof(ProblemPtrs<double>) == sizeof(ProblemPtrsHost),
+static_assert(sizeof(ProblemPtrs<double>) == sizeof(ProblemPtrsHost),
               "host image of the batch table");
 
 template <typename R>
-int cg_operator_batch(Spectral &sp, int tkind, const ProblemPtrs<R> *tab, const BatchVec<R> *xtab, int B,
-                      cudaStream_t s) {
-  constexpr int kPro = sizeof(R) == 4 ? PRO_CGF : PRO_CG;
-  constexpr int kEpi = sizeof(R) == 4 ? EPI_CGF : EPI_CG;
+int cg_operator_batch(Spectral &sp, int tkind, const ProblemPtrs<R> *tab, int B, cudaStream_t s) {
   const int gm = green_mode_of(sp);
   const Cfg c = last_cfg<R>(sp);
   LastArgs<R> a = last_args<R>(sp, c);
   a.batch = tab;
-  const int gfwd = last_reg_rows<R>(sp, false), ginv = last_reg_rows<R>(sp, true);
-  const bool greg = gfwd && ginv;
-  int nfwd = c.blocks * ((c.threads + 31) / 32);
-  if (greg) nfwd = last_cg_reg<R>(sp, tkind, a, gfwd, false, s, B);
-  else dispatch_fwd<R, kPro>(sp.g.dim, tkind, a, c, s, B);
-  if constexpr (sizeof(R) == 4) cg_update_x_batch<R>(xtab, sp.g.npx * sp.ncomp, nfwd, B, s);
+  dispatch_fwd<R, PRO_CG>(sp.g.dim, tkind, a, c, s, B);
   if (sp.g.dim == 3) run_axis<R>(sp, false, nullptr, s, tab, B);
   run_green<R>(sp, gm, nullptr, s, tab, B);
   if (sp.g.dim == 3) run_axis<R>(sp, true, nullptr, s, tab, B);
-  if (greg) return last_cg_reg<R>(sp, tkind, a, ginv, true, s, B);
-  if (sp.g.dim == 2) launch_inv<R, kEpi, 2>(a, c, s, B);
-  else launch_inv<R, kEpi, 3>(a, c, s, B);
+  if (sp.g.dim == 2) launch_inv<R, EPI_CG, 2>(a, c, s, B);
+  else launch_inv<R, EPI_CG, 3>(a, c, s, B);
   return c.blocks;
 }
 
@@ -582,7 +421,6 @@ struct GroupedOp {
   int threads[3] = {0, 0, 0};
   size_t smem[3] = {0, 0, 0};
   int total[3] = {0, 0, 0};       // blocks of the last-axis, middle-axis and Green launches
-  std::vector<int> fwd_parts;     // per problem: the forward pass's per-warp partial sums
   DevBuf last, axisf, axisi, green, blk;  // argument tables; blk: 3 x (B + 1) prefix sums
 };
 
@@ -604,7 +442,6 @@ template <typename R> GroupedOp *grouped_op_create(const std::vector<GroupProble
   std::vector<AxisArgs<R>> axf(B), axi(B);
   std::vector<GreenArgs<R>> grn(B);
   std::vector<int> blk(3 * (B + 1), 0);
-  op->fwd_parts.resize(B);
   for (int b = 0; b < B; ++b) {
     Spectral &sp = *probs[b].sp;
     if (sp.g.dim != op->dim || green_mode_of(sp) != op->gm || sp.ncomp != s0.ncomp)
@@ -618,14 +455,12 @@ template <typename R> GroupedOp *grouped_op_create(const std::vector<GroupProble
     LastArgs<R> a = last_args<R>(sp, c);
     a.st = probs[b].st;
     a.r = static_cast<R *>(probs[b].r);
-    a.x = static_cast<R *>(probs[b].x);
     a.p = static_cast<R *>(probs[b].p);
     a.Ap = static_cast<R *>(probs[b].Ap);
     a.partial = probs[b].partial;
     memcpy(&a.td, probs[b].td, sizeof(a.td));
     last[b] = a;
     blk[b + 1] = blk[b] + c.blocks;
-    op->fwd_parts[b] = c.blocks * ((c.threads + 31) / 32);
     op->smem[0] = std::max(op->smem[0], c.smem);
     op->threads[0] = c.threads;
     // middle axis (3-D): the generic kernel's arguments of run_axis
@@ -696,26 +531,19 @@ void launch_fwd_g(const GroupedOp &op, cudaStream_t s) {
 }
 
 template <typename R>
-void grouped_op_run(GroupedOp *op, const BatchVec<R> *xtab, long long nmax, int B, cudaStream_t s) {
-  constexpr int kPro = sizeof(R) == 4 ? PRO_CGF : PRO_CG;
-  constexpr int kEpi = sizeof(R) == 4 ? EPI_CGF : EPI_CG;
+void grouped_op_run(GroupedOp *op, cudaStream_t s) {
   const int dim = op->dim, tk = op->tkind, Bp = op->B + 1;
   const int *blk = op->blk.as<const int>();
   // last-axis forward with the CG prologue
 #define MUSG_FWDG_CASE(DD, TT) \
-  if (dim == DD && tk == TT) { launch_fwd_g<R, kPro, DD, TT>(*op, s); goto fwd_done; }
+  if (dim == DD && tk == TT) { launch_fwd_g<R, PRO_CG, DD, TT>(*op, s); goto fwd_done; }
   MUSG_FWDG_CASE(2, TK_SMALL) MUSG_FWDG_CASE(2, TK_FINITE) MUSG_FWDG_CASE(2, TK_KPRIME) MUSG_FWDG_CASE(2, TK_MIXED)
   MUSG_FWDG_CASE(3, TK_SMALL) MUSG_FWDG_CASE(3, TK_FINITE) MUSG_FWDG_CASE(3, TK_KPRIME) MUSG_FWDG_CASE(3, TK_MIXED)
   MUSG_FWDG_CASE(2, TK_GSMALL) MUSG_FWDG_CASE(2, TK_GFINITE) MUSG_FWDG_CASE(3, TK_GSMALL) MUSG_FWDG_CASE(3, TK_GFINITE)
   MUSG_FWDG_CASE(2, TK_FULL) MUSG_FWDG_CASE(3, TK_FULL)
-  if constexpr (sizeof(R) == 4) {
-    MUSG_FWDG_CASE(2, TK_FISO) MUSG_FWDG_CASE(3, TK_FISO)
-  }
 #undef MUSG_FWDG_CASE
   throw Error(MUSG_ERR_ARGUMENT, "unsupported tangent kind");
 fwd_done:
-  // FP32: alpha from each problem's own partial sums (nparts < 0), x += alpha p
-  if constexpr (sizeof(R) == 4) cg_update_x_batch<R>(xtab, nmax, -1, B, s);
   if (dim == 3) {
     auto k = k_axis_g<R, false>;
     allow_smem(k);
@@ -746,7 +574,7 @@ fwd_done:
     MUSG_CHECK_LAUNCH();
   }
   {
-    auto k = dim == 2 ? k_last_inv_g<R, kEpi, 2> : k_last_inv_g<R, kEpi, 3>;
+    auto k = dim == 2 ? k_last_inv_g<R, EPI_CG, 2> : k_last_inv_g<R, EPI_CG, 3>;
     allow_smem(k);
     launch_pdl(k, dim3(op->total[0]), dim3(op->threads[0]), op->smem[0], s, op->last.as<const LastArgs<R>>(), blk,
                op->B);
@@ -838,13 +666,12 @@ template <typename R> void spectral_autotune(Spectral &sp, cudaStream_t s, int e
   template void spectral_inverse<R>(Spectral &, R *, R, cudaStream_t);                            \
   template void spectral_project<R>(Spectral &, const R *, R *, R, cudaStream_t);                 \
   template int cg_operator<R>(Spectral &, int, const TangentData<R> &, const CGState *, R *, R *,  \
-                              R *, R *, double *, cudaStream_t, cudaEvent_t *);                    \
+                              R *, double *, cudaStream_t, cudaEvent_t *);                         \
   template void tangent_operator<R>(Spectral &, int, const TangentData<R> &, const R *, R *,       \
                                     cudaStream_t);                                                 \
   template void spectral_autotune<R>(Spectral &, cudaStream_t, int);                               \
-  template int cg_operator_batch<R>(Spectral &, int, const ProblemPtrs<R> *, const BatchVec<R> *, int,         \
-                                    cudaStream_t);                                                             \
-  template GroupedOp *grouped_op_create<R>(const std::vector<GroupProblem> &, int);                         \
-  template void grouped_op_run<R>(GroupedOp *, const BatchVec<R> *, long long, int, cudaStream_t);
+  template int cg_operator_batch<R>(Spectral &, int, const ProblemPtrs<R> *, int, cudaStream_t);   \
+  template GroupedOp *grouped_op_create<R>(const std::vector<GroupProblem> &, int);               \
+  template void grouped_op_run<R>(GroupedOp *, cudaStream_t);
 
 }  // namespace musg

@@ -1,0 +1,124 @@
+"""The displacement-space passes of the mixed method (csrc/disp.cuh) at the edges of their
+plans: lengths of one factor, of two factors up to 17 x 17, of three and more factors,
+primes that need Bluestein, odd k-plane and row counts, axes of one and two points.
+
+One application of the FP32 operator G(K:dF) against the FP64 operator (which
+test_gpu_parity.py pins to the oracle) within 1e-5, the bound of the FP32 operator in
+test_gpu_fastpaths.py: about forty FP32 roundings of 6e-8 on the way through five
+transforms.  Mixed solves of the same grids against FP64 solves: homogenised stress
+within 1e-6, the metric's bound, alone and in a batch of uneven grids.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = {
+    'one_factor': [7, 13, 11],
+    'two_factors': [17, 12, 51],
+    'largest_two_factors': [2, 289, 15],
+    'three_factors': [3, 2, 405],
+    'many_factors': [1024, 6],
+    'bluestein': [19, 23, 29],
+    'bluestein_three_factors': [5, 331],
+    'power_of_two_axes': [32, 64, 16],
+    'compile_time_last_axis': [5, 7, 32],
+    'compile_time_first_axes': [64, 32, 9],
+    'one_point_axis': [1, 9, 15],
+    'two_point_axes': [2, 2, 2],
+    'thin': [301, 3],
+}
+
+
+@pytest.fixture(scope='module')
+def mu():
+    import muspectre_gb300 as m
+    if m.device_count() < 1:
+        pytest.fail('no CUDA device visible')
+    return m
+
+
+def _cell(mu, res, form, seed):
+    d, n = len(res), int(np.prod(res))
+    rng = np.random.default_rng(seed)
+    cell = mu.Cell(res, [1.0, 1.3, 0.7][:d], form, allow_even=True)
+    hard = rng.random(n) < 0.3
+    hard[0], hard[-1] = True, False
+    m = getattr(mu.material, 'MaterialLinearElastic1_%dd' % d)
+    m.make(cell, 'hard', 30e9, .3).add_pixels(hard)
+    m.make(cell, 'soft', 3e9, .25).add_pixels(~hard)
+    cell.initialise()
+    return cell
+
+
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('name', sorted(GRIDS))
+def test_operator(mu, name, form):
+    res = GRIDS[name]
+    d, n = len(res), int(np.prod(res))
+    cell = _cell(mu, res, form, 3)
+    rng = np.random.default_rng(5)
+    F = 0.01 * rng.normal(size=(d, d, n))
+    F = 0.5 * (F + F.transpose(1, 0, 2)) if form else F + np.eye(d)[:, :, None]
+    cell.evaluate_stress_tangent(F.reshape(d * d, n))
+    dF = rng.normal(size=(d * d, n))
+    ref = cell.directional_stiffness(dF)
+    got = cell.cg_operator(dF, 'mixed')
+    scale = max(np.linalg.norm(ref), 1e-12 * 30e9)  # a grid without a free mode projects to zero
+    assert np.linalg.norm(got - ref) <= 1e-5 * scale
+
+
+SOLVED = ['one_factor', 'two_factors', 'bluestein', 'many_factors', 'power_of_two_axes', 'thin']
+
+
+def _load(d, form):
+    load = np.zeros((d, d))
+    load[0, 0] = 0.01
+    load[0, 1] = 0.004
+    if form:
+        load[1, 0] = 0.004
+    return load
+
+
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('name', SOLVED)
+def test_mixed_solve(mu, name, form):
+    res = GRIDS[name]
+    load = _load(len(res), form)
+    hom = {}
+    for prec in ('fp64', 'mixed'):
+        cell = _cell(mu, res, form, 3)
+        r = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 2000, precision=prec), 1e-8, 0.0)
+        assert r.success, r.message
+        hom[prec] = r.hom_stress
+    assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
+def test_uneven_batch(mu):
+    grids = [GRIDS[k] for k in ('one_factor', 'two_factors', 'bluestein', 'power_of_two_axes', 'three_factors')]
+    cells = [_cell(mu, g, 0, 3) for g in grids]
+    load = _load(3, 0)
+    rs = mu.batch.BatchSolver(cells, 1e-8, 2000, precision='mixed').newton_cg(load, 1e-8, 0.0)
+    for g, r in zip(grids, rs):
+        cell = _cell(mu, g, 0, 3)
+        s = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 2000, precision='mixed'), 1e-8, 0.0)
+        assert r[0].success and s.success
+        assert np.linalg.norm(r[0].hom_stress - s.hom_stress) <= 1e-6 * np.linalg.norm(s.hom_stress)
+
+
+def test_rhs_outside_the_range_does_not_converge(mu):
+    """SolverCG.solve on a right-hand side with a part outside the range of the projection:
+    the iteration cannot reduce that part, so it ends in ConvergenceError, as with the
+    residual in real space; the part inside solves."""
+    cell = _cell(mu, [9, 8, 15], 0, 3)
+    n = cell.nb_pixels
+    rng = np.random.default_rng(5)
+    s = mu.solvers.SolverCG(cell, 1e-8, 200, precision='mixed', inner_tol=1e-4)
+    cell.evaluate_stress_tangent(np.tile(np.eye(3).reshape(9, 1), (1, n)))
+    rhs = rng.normal(size=(9, n))
+    inside = cell.project(rhs)
+    x = s.solve(np.ascontiguousarray(inside.T).reshape(-1))
+    back = cell.directional_stiffness(x.reshape(n, 9).T)
+    assert np.linalg.norm(back - inside) <= 2e-4 * np.linalg.norm(inside)
+    with pytest.raises(mu.ConvergenceError):
+        s.solve(np.ascontiguousarray(rhs.T).reshape(-1))
