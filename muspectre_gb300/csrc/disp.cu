@@ -76,10 +76,10 @@ __global__ void k_disp_init(const float2 *__restrict__ b, float2 *__restrict__ r
 
 // the fourth sums of the blocks, in a fixed order
 __global__ void k_disp_sum(const double *partial, int nparts, double *out) {
-  double s[4] = {0, 0, 0, 0};
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s[3] += partial[4 * i + 3];
-  block_sum4(s);
-  if (threadIdx.x == 0) *out = s[3];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += partial[4 * i + 3];
+  s = block_sum(s);
+  if (threadIdx.x == 0) *out = s;
 }
 
 template <typename R> DispProb<R> disp_prob(Spectral &sp, const DispVectors &v, CGState *st, double *partial) {
@@ -146,12 +146,12 @@ void disp_residual(Spectral &sp, void *rhat, const double *field, double *prev, 
 
 void disp_start(Spectral &sp, const DispVectors &v, const void *rhat, CGState *st, double tol, int maxiter,
                 const double *rhs2, const double *range2, cudaStream_t s) {
-  const long long n = sp.g.nk * sp.g.dim;
+  const long long n = disp_nk(sp) * sp.g.dim;
   if (n > 0xf0000000ll) throw Error(MUSG_ERR_ARGUMENT, "grid too large for the mixed method");
   k_disp_start<<<1, 1, 0, s>>>(st, rhs2, range2, tol, maxiter);
   MUSG_CHECK_LAUNCH();
   k_disp_init<<<reduce_blocks(n), 256, 0, s>>>((const float2 *)rhat, (float2 *)v.r, (float2 *)v.x, sp.g.dim,
-                                                 sp.g.n[0], sp.g.dim == 3 ? sp.g.n[1] : 1, sp.g.nh, st);
+                                                 sp.g.n[0], sp.g.dim == 3 ? sp.g.n[1] : 1, disp_nh(sp), st);
   MUSG_CHECK_LAUNCH();
 }
 

@@ -10,6 +10,8 @@
 //   finite  sum_k w_k Re(conj(a) . b)
 //   small   sum_k w_k Re(conj(a) . b + conj(a.xi) (b.xi)) / 2
 // and the iteration of solver_cg.cc:76-97 runs on v with the same scalars alpha, beta.
+// The Nyquist column of an even last axis is left out (the operator is zero there), so a
+// row of 128 pixels is 64 complex values, a whole number of 128-byte lines.
 // One iteration is five passes in 3-D and three in 2-D, R bytes per value:
 //   ax0_inv   r += alpha q, x += alpha p, p = -r + beta p, then p's field along axis 0
 //   mid_inv   axis 1 (3-D)
@@ -37,8 +39,10 @@
 // this one moves 101 and 78 in five.  One iteration on GB300, before -> now: 128^3 finite
 // 291 -> 268 us, 63^3 115 -> 80, 45x77x81 164 -> 83, 160^3 small strain 1279 -> 486 (the
 // odd and 5-smooth lengths also gain from the two-stage transforms of tile_fft.cuh).
-// What bounds the passes is latency and instruction issue at 25-30% of the warp slots,
-// not bandwidth: 128^3 moves 860 MB in 268 us.
+// Without the Nyquist column (64 instead of 65 columns: whole lines, 128^3 axis-1 passes
+// 39 -> 34 and 43 -> 33 us) and with the sums reduced in FP32 pairs (51 -> 45 us) the
+// 128^3 iteration takes 246 us.  What bounds the passes is latency and instruction issue
+// at 25-30% of the warp slots, not bandwidth: 128^3 moves 850 MB in 246 us.
 #pragma once
 
 #include "spectral.cuh"
@@ -57,7 +61,7 @@ template <typename R> struct DispProb {
 
 template <typename R> struct DispArgs {
   TilePlanD<R> ap;        // the axis of this pass
-  int n0, n1, nh, L;      // grid; nh = L/2 + 1
+  int n0, n1, nh, L;      // grid; nh: stored k-points of the last axis (disp_nh)
   int T, G;               // k-points per tile (strided axes), rows per tile (last axis)
   int ntx, nbx;           // tiles and blocks of a row group (component group)
   int ng;                 // row groups: D for the finite-strain axis passes
@@ -112,26 +116,34 @@ __device__ __forceinline__ void stage_tile_twiddles(typename V2<R>::T *dst, cons
 // 120 and halve the warps that hide the loads of all the others (they spill instead)
 template <int CR1> constexpr int kDispRegs = CR1 == 16 ? 72 : CR1 > 0 ? 64 : 80;
 
-// sums of four values over the block, valid in every thread
-__device__ __forceinline__ void block_sum4(double *v) {
-  __shared__ double red[4][33];
+// Sum of the threads' compensated accumulators over the block, by thread 0.  FP32: the
+// warps add (sum, correction) pairs with Knuth's two-sum, an error of about 2^-46 in FP32
+// instructions; FP64 shuffles and additions took 2 us a block on the slow FP64 pipe, all
+// blocks at once at the end of the pass.
+__device__ __forceinline__ void two_sum_add(Acc<float> &a, float s, float c) {
+  const float t = a.s + s, z = t - a.s;
+  a.c += ((a.s - (t - z)) + (s - z)) + c;
+  a.s = t;
+}
+template <int N> __device__ __forceinline__ void block_sums(Acc<float> (&v)[N], double *out) {
+  __shared__ float2 red[N][32];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  __syncthreads();
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float s = __shfl_down_sync(0xffffffffu, v[k].s, o), c = __shfl_down_sync(0xffffffffu, v[k].c, o);
+      two_sum_add(v[k], s, c);
+    }
   if (l == 0)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) red[k][w] = v[k];
+    for (int k = 0; k < N; ++k) red[k][w] = make_float2(v[k].s, v[k].c);
   __syncthreads();
-  if (threadIdx.x < 4) {
-    double s = 0.0;
-    for (int i = 0; i < nw; ++i) s += red[threadIdx.x][i];
-    red[threadIdx.x][32] = s;
+  if (threadIdx.x < N) {
+    Acc<float> t;
+    for (int i = 0; i < nw; ++i) two_sum_add(t, red[threadIdx.x][i].x, red[threadIdx.x][i].y);
+    out[threadIdx.x] = t.value();
   }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; ++k) v[k] = red[k][32];
 }
 
 __device__ __forceinline__ double disp_floor(float) { return 1e-6; }
@@ -142,34 +154,38 @@ __device__ __forceinline__ double disp_floor(double) { return 1e-14; }
 // (solver_cg.cc:76-97).  The next update pass applies alpha and beta; without a further
 // iteration it only finishes x.
 template <typename R> __device__ __forceinline__ void disp_finish(CGState *st, const double *partial, int nparts) {
-  // two 16-byte loads per block's sums, four blocks in flight per thread; added in index order
-  double s[4] = {0, 0, 0, 0};
-  const double2 *p2 = reinterpret_cast<const double2 *>(partial);
-  for (int i = threadIdx.x; i < nparts; i += 4 * blockDim.x) {
-    double2 v[4][2];
+  // a quarter of the warps per sum, eight loads in flight per thread, added in index order
+  __shared__ double red[4][8], total[4];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int k = w & 3, part = w >> 2, parts = max(1, nw >> 2);
+  for (int kk = k; kk < 4 && part < parts; kk += min(nw, 4)) {  // fewer than four warps: several sums each
+    double s = 0.0;
+    for (int i = part * 32 + l; i < nparts; i += 8 * 32 * parts) {
+      double t[8];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int q = i + u * blockDim.x;
-      v[u][0] = v[u][1] = make_double2(0.0, 0.0);
-      if (q < nparts) {
-        v[u][0] = __ldcg(p2 + 2 * q);
-        v[u][1] = __ldcg(p2 + 2 * q + 1);
+      for (int u = 0; u < 8; ++u) {
+        const int q = i + u * 32 * parts;
+        t[u] = q < nparts ? __ldcg(partial + (long long)4 * q + kk) : 0.0;
       }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += t[u];
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      s[0] += v[u][0].x;
-      s[1] += v[u][0].y;
-      s[2] += v[u][1].x;
-      s[3] += v[u][1].y;
-    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (l == 0) red[kk][part] = s;
   }
-  block_sum4(s);
+  __syncthreads();
+  if (threadIdx.x < 4) {
+    double s = 0.0;
+    for (int i = 0; i < parts; ++i) s += red[threadIdx.x][i];
+    total[threadIdx.x] = s;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    const double rr = s[3], alpha = rr / s[0];
-    double rn = rr + 2.0 * alpha * s[1] + alpha * alpha * s[2];
+    const double rr = total[3], alpha = rr / total[0];
+    double rn = rr + 2.0 * alpha * total[1] + alpha * alpha * total[2];
     if (rn < disp_floor(R(0)) * rr) rn = disp_floor(R(0)) * rr;  // a NaN stays
-    st->pAp = s[0];
+    st->pAp = total[0];
     st->alpha = alpha;
     st->beta = rn / rr;
     rn += st->out2;
@@ -470,7 +486,7 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_fwd(const DispArgs<R> a0, cons
   const int g = bid / a.nbx;
   const int t = map.p % Tt, c = map.p / Tt, comp = FIN ? g + D * c : c;
   const int de = (int)blockDim.x / Tt, e0 = (int)threadIdx.x / Tt < de ? (int)threadIdx.x / Tt : kNoRow;
-  Acc<R> s0, s1, s2, s3;
+  Acc<R> sum[4];
   __syncthreads();  // the twiddle copy
   for (int tile = bid - g * a.nbx; tile < a.ntx; tile += a.nbx) {
     const int rho = tile * Tt + t;
@@ -481,7 +497,7 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_fwd(const DispArgs<R> a0, cons
         [&](int, int s, int p, T v) { buf[map.at(s, p)] = v; });
     __syncthreads();
     const Wave<D, R> wv(a, ok ? rho : 0);
-    const R wt = (wv.kl == 0 || 2 * wv.kl == a.L) ? R(1) : R(2);
+    const R wt = wv.kl == 0 ? R(1) : R(2);
     const long long ob = (long long)(FIN ? g : 0) * a.nk + rho;
     constexpr int U = FIN ? 4 : 2;
     for (int eb = e0; eb < n0; eb += U * de) {
@@ -563,22 +579,18 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_fwd(const DispArgs<R> a0, cons
           return wt * acc;
         };
         if (MODE == AX_DOTS) {
-          s0.add(dot(pv[u], v));
-          s1.add(dot(rv[u], v));
-          s2.add(dot(v, v));
-          s3.add(dot(rv[u], rv[u]));
+          sum[0].add(dot(pv[u], v));
+          sum[1].add(dot(rv[u], v));
+          sum[2].add(dot(v, v));
+          sum[3].add(dot(rv[u], rv[u]));
         } else {
-          s3.add(dot(v, v));
+          sum[3].add(dot(v, v));
         }
       }
     }
     __syncthreads();  // the tile is free for the next one
   }
-  double s[4] = {s0.value(), s1.value(), s2.value(), s3.value()};
-  block_sum4(s);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a.pb.partial[4 * (long long)bid + k] = s[k];
+  block_sums(sum, a.pb.partial + 4 * (long long)bid);
   if (MODE == AX_DOTS && cg_last_block(a.pb.st, a.nparts)) disp_finish<R>(a.pb.st, a.pb.partial, a.nparts);
 }
 
@@ -615,7 +627,7 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_pixels(const DispArgs<R> a0, const
       return;
     }
   }
-  const int L = CR1 > 0 ? CR1 * CR2 : a.L, H = L / 2 + 1, G = a.G, G2 = G >> 1;
+  const int L = CR1 > 0 ? CR1 * CR2 : a.L, H = (L + 1) / 2, G = a.G, G2 = G >> 1;
   const int P = NL * G2;
   const RowMap<(CR1 > 0 ? CR1 * CR2 : 0)> lay{CR1 > 0 ? padded_pencil(CR1 * CR2) : a.sp, a.sh};
   T *buf = reinterpret_cast<T *>(smem_raw);
@@ -653,10 +665,10 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_pixels(const DispArgs<R> a0, const
         int k;
         const int q = fH.div(idx, k);
         T x = X[u], y = Y[u];
-        const bool selfconj = k == 0 || 2 * k == L;
-        if (selfconj) { x.y = R(0); y.y = R(0); }  // c2r uses the real part only
+        if (k == 0) { x.y = R(0); y.y = R(0); }  // c2r uses the real part only
         buf[lay.at(slots.nat(k), q)] = T{x.x - y.y, x.y + y.x};
-        if (!selfconj) buf[lay.at(slots.nat(L - k), q)] = T{x.x + y.y, y.x - x.y};
+        if (k > 0) buf[lay.at(slots.nat(L - k), q)] = T{x.x + y.y, y.x - x.y};
+        else if (L % 2 == 0) buf[lay.at(slots.nat(L / 2), q)] = T{R(0), R(0)};  // not stored: zero
       }
     }
     __syncthreads();

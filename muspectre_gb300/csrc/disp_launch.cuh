@@ -39,7 +39,7 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   const bool fin = disp_finite(sp);
   const int D = sp.g.dim, na = fin ? 2 : D * (D + 1) / 2;
   const TilePlan &pl = sp.tp[0];
-  const long long Rr = sp.g.nk / sp.g.n[0];
+  const long long Rr = disp_nk(sp) / sp.g.n[0];
   DispShape c;
   c.ng = fin ? D : 1;
   const long cb = 2 * (long)sizeof(R), per = (long)na * pl.m * cb * pl.buffers(), tw = pl.r1 ? pl.m * cb : 0;
@@ -65,7 +65,7 @@ template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
   DispShape c;
   c.ng = fin ? 3 : 6;
   c.comps_at_once = fin ? 3 : 1;
-  const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0, nh = sp.g.nh;
+  const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0, nh = disp_nh(sp);
   long per = (long)c.comps_at_once * pl.m * cb * pl.buffers();
   if (fin && per + tw > optin_smem()) {
     c.comps_at_once = 1;
@@ -119,10 +119,10 @@ template <typename R> DispArgs<R> disp_base(Spectral &sp) {
   const int D = sp.g.dim;
   a.n0 = sp.g.n[0];
   a.n1 = sp.g.n[1];
-  a.nh = sp.g.nh;
+  a.nh = disp_nh(sp);
   a.L = sp.g.nlast();
-  a.Rr = (int)(sp.g.nk / sp.g.n[0]);
-  a.nk = sp.g.nk;
+  a.Rr = (int)(disp_nk(sp) / sp.g.n[0]);
+  a.nk = disp_nk(sp);
   a.npx = sp.g.npx;
   a.nrows = sp.g.nrows;
   a.xi0 = xi_table<R>(sp, 0);

@@ -288,7 +288,11 @@ template <typename R> void grouped_op_run(GroupedOp *op, cudaStream_t s);
 struct DispVectors {
   void *r = nullptr, *q = nullptr, *p = nullptr, *x = nullptr;
 };
-inline size_t disp_vector_bytes(const Spectral &sp) { return (size_t)sp.g.nk * sp.g.dim * sizeof(float2); }
+// stored k-points of the last axis (the Nyquist column of an even axis is zero), and of
+// the half spectrum
+inline int disp_nh(const Spectral &sp) { return (sp.g.nlast() + 1) / 2; }
+inline long long disp_nk(const Spectral &sp) { return sp.g.nrows * disp_nh(sp); }
+inline size_t disp_vector_bytes(const Spectral &sp) { return (size_t)disp_nk(sp) * sp.g.dim * sizeof(float2); }
 // rhat (+)= the projection of scale * field (FP64 planes), or with prev of prev - field,
 // after which prev = field; *norm2 = |rhat|^2 (a device double)
 void disp_residual(Spectral &sp, void *rhat, const double *field, double *prev, double scale, bool accumulate,
