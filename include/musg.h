@@ -94,10 +94,10 @@ int musg_device_count(int *count);
 /* device used by the objects the calling thread creates afterwards (one process per
  * GPU; no counterpart in the reference, whose ranks are MPI processes) */
 int musg_set_device(int device);
-/* self-test of the bounded waits of the TMA-fed passes (no counterpart in the
- * reference): one block waits on an mbarrier that nothing completes, gives up after
- * limit_ms, and sets the device fault word; the host reads it the way it does after
- * every FP32 CG solve, clears it, and reports *timed_out = 1.  The device stays usable. */
+/* self-test of a bounded device-side wait (no counterpart in the reference): one block
+ * waits on an mbarrier that nothing completes, gives up after limit_ms, and sets a device
+ * fault word; the host reads and clears it and reports *timed_out = 1.  The device stays
+ * usable. */
 int musg_selftest_wait_timeout(double limit_ms, int *timed_out);
 
 /* -------------------------------------------------------------- cell
@@ -128,10 +128,11 @@ int musg_material_size(musg_cell *cell, int material, long long *count);
  * upload of the microstructure, FFT plans.  Called implicitly by the first
  * evaluation. plan_flags follows FFT_PlanFlags (estimate=0, measure=1, patient=2). */
 int musg_cell_initialise(musg_cell *cell, int plan_flags);
-/* launch shapes of the spectral passes (threads per block, shared-memory target
- * per block) for FP64 then FP32, passes last-axis / middle-axis / Green: 6 entries
- * each.  FFT_PlanFlags measure/patient at initialise times candidates on the cell's
- * grid (the FFTW_MEASURE analogue); no counterpart in the reference. */
+/* launch shapes of the FFT engine's passes on the cell's grid (threads per block,
+ * shared-memory target per block) for FP64 then FP32, passes last axis / middle axis /
+ * first axis: 6 entries each.  The CG and projection passes take their shapes from the
+ * grid by rule, whatever plan_flags musg_cell_initialise is given; no counterpart in the
+ * reference. */
 int musg_cell_tuning(musg_cell *cell, int *threads, long long *bytes);
 /* CellBase::set_uniform_strain (cell_base.cc:110-112); strain is D*D column-major */
 int musg_cell_set_uniform_strain(musg_cell *cell, const double *strain);
@@ -190,9 +191,9 @@ int musg_solver_destroy(musg_solver *solver);
  * Newton method), and newton_cg refines in FP64 */
 int musg_solver_set_inner_tol(musg_solver *solver, double inner_tol);
 /* MUSG_PRECISION_MIXED only (no counterpart in the reference; on by default): newton_cg
- * projects the first residual G(-P) of a load step in FP64 and every later one as
- * G(rhs_prev - (P - P_prev)) in FP32, the previous residual minus the stress change
- * since (one FP64 projection per load step instead of one per Newton iteration).
+ * projects the first two residuals G(-P) of a load step in FP64 and every later one as
+ * the previous residual minus G(P - P_prev) of the stress change since in FP32 (two
+ * FP64 projections per load step instead of one per Newton iteration).
  * enable = 0 projects every residual in FP64. */
 int musg_solver_set_incremental_residual(musg_solver *solver, int enable);
 /* newton_cg with a backtracking line search (no counterpart in the reference; off by

@@ -25,9 +25,9 @@ LIB = os.path.join(HERE, 'libmusg.so')
 
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
-# the out-of-line tile transforms are linked into kernels of 80 registers (device code is
-# relocatable; a kernel takes the registers of the functions it calls)
-EXTRA = {'tile_stages.cu': ['-maxrregcount=80']}
+# the out-of-line tile transforms are linked into kernels of 80 (FP32) and 128 registers
+# (device code is relocatable; a kernel takes the registers of the functions it calls)
+EXTRA = {'tile_stages_f32.cu': ['-maxrregcount=80'], 'tile_stages_f64.cu': ['-maxrregcount=128']}
 
 
 def _nvcc():

@@ -70,46 +70,6 @@ std::string ccoord_str(const int *res, int dim, long long idx) {
   return o.str();
 }
 
-// Launch shapes found by the autotuner, shared by every cell of the same grid,
-// component count and projection in this process (cf. FFTW wisdom).
-struct Wisdom {
-  int threads[3];
-  long bytes[3];
-};
-std::mutex g_wisdom_mu;
-std::map<std::string, Wisdom> g_wisdom;
-
-std::string wisdom_key(const Spectral &sp, int prec) {
-  std::ostringstream k;
-  k << sp.g.dim << ':' << sp.g.n[0] << 'x' << sp.g.n[1] << 'x' << sp.g.n[2] << ':' << sp.ncomp << ':'
-    << sp.proj_kind << ':' << sp.allow_even << ':' << prec;
-  return k.str();
-}
-
-template <typename R> void autotune_with_wisdom(Spectral &sp, cudaStream_t s, int effort) {
-  const int pi = sizeof(R) == 8 ? 0 : 1;
-  const std::string key = wisdom_key(sp, pi);
-  {
-    std::lock_guard<std::mutex> lock(g_wisdom_mu);
-    auto it = g_wisdom.find(key);
-    if (it != g_wisdom.end()) {
-      for (int k = 0; k < 3; ++k) {
-        sp.tune_threads[pi][k] = it->second.threads[k];
-        sp.tune_bytes[pi][k] = it->second.bytes[k];
-      }
-      return;
-    }
-  }
-  spectral_autotune<R>(sp, s, effort);
-  Wisdom w;
-  for (int k = 0; k < 3; ++k) {
-    w.threads[k] = sp.tune_threads[pi][k];
-    w.bytes[k] = sp.tune_bytes[pi][k];
-  }
-  std::lock_guard<std::mutex> lock(g_wisdom_mu);
-  g_wisdom[key] = w;
-}
-
 struct Material {
   int law = 0;
   std::string name;
@@ -160,8 +120,6 @@ struct musg_cell {
   bool initialised = false;
   bool tangent_valid = false;
   bool need32 = false;
-  int plan_flags = 0;      // FFT_PlanFlags: estimate 0, measure 1, patient 2
-  bool tuned64 = false;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::vector<Material> materials;
@@ -171,10 +129,10 @@ struct musg_cell {
   bool has_le2 = false, has_hep = false;
   bool has_consistent = false;  // an HEP1 material with the consistent tangent: TK_FULL cell
   // device fields (FP64 component planes)
-  DevBuf F, P, rhs, io, io2, F0;  // F0: the line search's Newton iterate
+  DevBuf F, P, io, io2, F0;  // F0: the line search's Newton iterate
   DevBuf Pk;                      // the stress of the last projected residual (incremental residual)
-  DevBuf rhat;                    // the mixed method's residual G(-P) in displacement space (disp.cuh)
-  bool residual_kept = false;     // Pk and rhat belong together (incremental residual)
+  DevBuf rhat64, rhat;            // the residual G(-P) in displacement space (disp.cuh); its FP32 form (mixed)
+  int residual_kept = 0;          // FP64 projections of this load step (incremental residual)
   DevBuf mat, params, law_kind, Ctab64, Ctab32;
   bool has_generic = false;
   DevBuf lam64, mu64, lam32, mu32, eig;
@@ -218,7 +176,8 @@ struct musg_cell {
     sp.init(dim, res, D2, proj, lengths, (flags & MUSG_FLAG_ALLOW_EVEN) != 0, false);
     F.alloc(field_bytes());
     P.alloc(field_bytes());
-    rhs.alloc(field_bytes());
+    sp.ensure_tiles();
+    rhat64.alloc(disp_vector_bytes<double>(sp));
     MUSG_CUDA(cudaMemsetAsync(F.p, 0, field_bytes(), stream));
     MUSG_CUDA(cudaMemsetAsync(P.p, 0, field_bytes(), stream));
     // reduction scratch: block or per-warp partial sums of the passes (at most 16 warps
@@ -391,24 +350,13 @@ struct musg_cell {
     }
     if (need32) alloc32();
     initialised = true;
-    autotune();
     MUSG_CUDA(cudaStreamSynchronize(stream));
-  }
-
-  // FFT_PlanFlags::measure / patient: time the launch shapes of the passes on this
-  // grid (the analogue of FFTW planning with FFTW_MEASURE)
-  void autotune() {
-    if (plan_flags < 1 || !initialised) return;
-    if (!tuned64) {
-      autotune_with_wisdom<double>(sp, stream, plan_flags);
-      tuned64 = true;
-    }
   }
 
   void alloc32() {
     need32 = true;
     sp.ensure32();
-    if (!rhat.p) rhat.alloc(disp_vector_bytes(sp));
+    if (!rhat.p) rhat.alloc(disp_vector_bytes<float>(sp));
     if (!initialised && !lam64.p) return;  // done at initialise
     if (!lam32.p) {
       lam32.alloc((size_t)npx * sizeof(float));
@@ -423,7 +371,6 @@ struct musg_cell {
       if (tkind == TK_FULL && !Kt32.p) Kt32.alloc((size_t)npx * D2 * D2 * sizeof(float));
     }
     tangent_valid = false;
-    autotune();
   }
 
   void evaluate(bool want_K) {
@@ -481,43 +428,36 @@ struct musg_cell {
     for (int k = 0; k < 9; ++k) out[k] = k < D2 ? hscal[40 + k] : 0.0;
   }
 
-  // rhs = -G(P) for the current stress (FP64, the plain method), its norm's square in
-  // scal[32]
+  // rhat64 = -G(P) for the current stress, its norm's square in scal[32]
   void project_residual() {
-    spectral_project<double>(sp, P.as<double>(), rhs.as<double>(), -1.0, stream);
-    dot_device<double, double>(rhs.as<double>(), rhs.as<double>(), nb_dof(), partial.as<double>(),
-                               scal.as<double>() + 32, stream);
+    disp_residual<double>(sp, TK_PLAIN, {}, rhat64.p, P.as<double>(), nullptr, -1.0, false, partial.as<double>(),
+                          scal.as<double>() + 32, stream);
   }
-  // The mixed method's residual rhat = -G(P) in displacement space, its norm's square in
-  // scal[32].  Incremental (the default): the first residual after residual_kept is
-  // cleared is projected in FP64 and its P kept in Pk; each later one is rhat + G(Pk - P)
-  // with the stress change projected in FP32, and the new P is kept.  The FP32 rounding
-  // is relative to that change and not to P (whose mean and fluctuation are far larger),
-  // and in displacement space no part of it can leave the range of G.  The FP64
-  // projections, bound by the FP64 pipe, drop to one per load step.
+  // The mixed method's residual rhat.  Incremental (the default): the first two residuals
+  // of a load step are projected in FP64 and the second one's P kept in Pk; each later one
+  // is rhat + G(Pk - P) with the stress change projected in FP32, and the new P is kept.
+  // The FP32 rounding is relative to that change and not to P (whose mean and fluctuation
+  // are far larger), and in displacement space no part of it can leave the range of G.
+  // The change after the first Newton step is as large as the first residual; projected
+  // in FP32 it left an error floor of 1e-6 of the strain, the later ones are a hundredth.
   void project_residual_mixed(bool incremental) {
-    double *part = partial.as<double>(), *norm2 = scal.as<double>() + 32;
-    if (incremental && residual_kept) {
-      disp_residual(sp, rhat.p, P.as<double>(), Pk.as<double>(), 1.0, true, part, norm2, stream);
+    if (incremental && residual_kept >= 2) {
+      disp_residual<float>(sp, TK_PLAIN, {}, rhat.p, P.as<double>(), Pk.as<double>(), 1.0, true, partial.as<double>(),
+                           scal.as<double>() + 32, stream);
       return;
     }
-    spectral_project<double>(sp, P.as<double>(), rhs.as<double>(), -1.0, stream);
-    residual_from_rhs();
-    if (incremental) {
+    project_residual();
+    disp_convert(sp, rhat64.p, rhat.p, stream);
+    if (incremental && ++residual_kept == 2) {
       if (Pk.bytes < field_bytes()) Pk.alloc(field_bytes());
       MUSG_CUDA(cudaMemcpyAsync(Pk.p, P.p, field_bytes(), cudaMemcpyDeviceToDevice, stream));
-      residual_kept = true;
     }
-  }
-  // rhat of the projected field in rhs
-  void residual_from_rhs() {
-    disp_residual(sp, rhat.p, rhs.as<double>(), nullptr, 1.0, false, partial.as<double>(), scal.as<double>() + 32,
-                  stream);
   }
   void residual(bool mixed, bool incremental) {
     if (mixed) project_residual_mixed(incremental);
     else project_residual();
   }
+  void residual_geus(double *delta, bool mixed);
 
   // host AoS vector -> device SoA planes (dst)
   void upload_field(const double *host, double *dst) {
@@ -561,6 +501,17 @@ template <> TangentData<float> musg_cell::tangent<float>() const {
   return t;
 }
 
+// the residual of de_geus' first Newton iteration, -G(K:DF) with DF the uniform field of
+// the device matrix delta
+void musg_cell::residual_geus(double *delta, bool mixed) {
+  if (io2.bytes < field_bytes()) io2.alloc(field_bytes());
+  fill_uniform(io2.as<double>(), delta, D2, npx, stream);
+  disp_residual<double>(sp, tkind, tangent<double>(), rhat64.p, io2.as<double>(), nullptr, -1.0, false,
+                        partial.as<double>(), scal.as<double>() + 32, stream);
+  if (mixed) disp_convert(sp, rhat64.p, rhat.p, stream);
+  residual_kept = 0;
+}
+
 // ---------------------------------------------------------------------- solver
 struct musg_solver {
   musg_cell *cell = nullptr;
@@ -570,9 +521,8 @@ struct musg_solver {
   int precision = MUSG_PRECISION_FP64;
   bool converged = false;
   unsigned long long counter = 0;
-  // FP64: the CG vectors; mixed: r, q, p, xh in displacement space (DispVectors) and x,
-  // the solution in real space
-  DevBuf x, r, p, Ap, q, xh, st;
+  // the CG vectors in displacement space (DispVectors), and x, the solution in real space
+  DevBuf x, r, q, p, xh, st;
   CGState *hst = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned long long graph_nodes = 0;
@@ -611,11 +561,9 @@ struct musg_solver {
     if (precision == MUSG_PRECISION_MIXED) cell->alloc32();
     const size_t n = (size_t)cell->nb_dof();
     x.alloc(n * rbytes());
-    if (precision == MUSG_PRECISION_MIXED) {
-      for (DevBuf *b : {&r, &q, &p, &xh}) b->alloc(disp_vector_bytes(cell->sp));
-    } else {
-      for (DevBuf *b : {&r, &p, &Ap}) b->alloc(n * rbytes());
-    }
+    const size_t vb = precision == MUSG_PRECISION_MIXED ? disp_vector_bytes<float>(cell->sp)
+                                                        : disp_vector_bytes<double>(cell->sp);
+    for (DevBuf *b : {&r, &q, &p, &xh}) b->alloc(vb);
     st.alloc(sizeof(CGState));
     MUSG_CUDA(cudaMemset(st.p, 0, sizeof(CGState)));
     MUSG_CUDA(cudaMallocHost(&hst, sizeof(CGState)));
@@ -634,38 +582,23 @@ struct musg_solver {
     return v;
   }
 
-  // one CG iteration (solver_cg.cc:76-97); ev, when given, receives an event
-  // before the first and after every kernel (profiling).  FP64: the operator passes
-  // (alpha by the last one) and cg_update (x, r, beta); mixed: the displacement-space
-  // passes, whose first one applies the updates of the iteration before.
+  // one CG iteration (solver_cg.cc:76-97): the displacement-space passes, whose first one
+  // applies the updates of the iteration before; ev, when given, receives an event
+  // before the first and after every kernel (profiling)
   template <typename R> void iteration(cudaStream_t s, cudaEvent_t *ev = nullptr) {
     musg_cell &c = *cell;
-    CGState *d = st.as<CGState>();
-    double *part = c.partial.as<double>();
-    if constexpr (sizeof(R) == 4) {
-      disp_iteration(c.sp, c.tkind32, c.tangent<float>(), vectors(), d, part, s, ev);
-    } else {
-      cg_operator<double>(c.sp, c.tkind, c.tangent<double>(), d, r.as<double>(), p.as<double>(), Ap.as<double>(), part, s,
-                          ev);
-      cg_update<double>(d, x.as<double>(), r.as<double>(), p.as<double>(), Ap.as<double>(), c.nb_dof(), part, s);
-      if (ev) MUSG_CUDA(cudaEventRecord(ev[nb_kernels()], s));
-    }
+    disp_iteration<R>(c.sp, sizeof(R) == 4 ? c.tkind32 : c.tkind, c.tangent<R>(), vectors(), st.as<CGState>(),
+                      c.partial.as<double>(), s, ev);
   }
 
-  // kernels per CG iteration: five (3-D) or three (2-D) passes, in FP64 and the update
-  int nb_kernels() const { return (cell->dim == 3 ? 5 : 3) + (precision == MUSG_PRECISION_MIXED ? 0 : 1); }
+  // kernels per CG iteration
+  int nb_kernels() const { return cell->dim == 3 ? 5 : 3; }
 
-  static const char *kernel_name(int dim, int precision, int k) {
-    static const char *n3[] = {"last_axis_fwd_tangent", "axis1_fwd", "green_axis0", "axis1_inv", "last_axis_inv_dot",
-                               "cg_update"};
-    static const char *n2[] = {"last_axis_fwd_tangent", "green_axis0", "last_axis_inv_dot", "cg_update"};
-    static const char *f3[] = {"axis0_inv_update", "axis1_inv_expand", "last_axis_tangent", "axis1_fwd_contract",
+  static const char *kernel_name(int dim, int k) {
+    static const char *n3[] = {"axis0_inv_update", "axis1_inv_expand", "last_axis_tangent", "axis1_fwd_contract",
                                "axis0_fwd_dots"};
-    static const char *f2[] = {"axis0_inv_update", "last_axis_tangent", "axis0_fwd_dots"};
-    const bool mixed = precision == MUSG_PRECISION_MIXED;
-    const char *const *t = mixed ? (dim == 3 ? f3 : f2) : (dim == 3 ? n3 : n2);
-    const int nk = (dim == 3 ? 5 : 3) + (mixed ? 0 : 1);
-    return (k >= 0 && k < nk) ? t[k] : "";
+    static const char *n2[] = {"axis0_inv_update", "last_axis_tangent", "axis0_fwd_dots"};
+    return (k >= 0 && k < (dim == 3 ? 5 : 3)) ? (dim == 3 ? n3 : n2)[k] : "";
   }
 
   // mean per-kernel durations (ms) over `iters` eagerly launched iterations started
@@ -674,12 +607,8 @@ struct musg_solver {
     musg_cell &c = *cell;
     cudaStream_t s = c.stream;
     require(c.tangent_valid, MUSG_ERR_RUNTIME, "profile needs an evaluated tangent");
-    const long long n = c.nb_dof();
-    double *part = c.partial.as<double>();
-    if constexpr (sizeof(R) == 4)
-      disp_start(c.sp, vectors(), c.rhat.p, st.as<CGState>(), 0.0, iters, nullptr, c.scal.as<double>() + 32, s);
-    else
-      cg_init<R>(st.as<CGState>(), c.rhs.as<double>(), r.as<R>(), x.as<R>(), n, 0.0, iters, part, part + 4096, s);
+    disp_start<R>(c.sp, vectors(), sizeof(R) == 4 ? c.rhat.p : c.rhat64.p, st.as<CGState>(), 0.0, iters, nullptr,
+                  c.scal.as<double>() + 32, s);
     const int nk = nb_kernels();
     std::vector<cudaEvent_t> ev(nk + 1);
     for (auto &e : ev) MUSG_CUDA(cudaEventCreate(&e));
@@ -725,46 +654,39 @@ struct musg_solver {
     cudaGraphDestroy(g);
   }
 
-  // SolverCG::solve (solver_cg.cc:54-110) on a device rhs (FP64 SoA planes; mixed: null
-  // for the cell's own residual rhat, whose norm's square is in scal[32])
-  void solve_device(const double *rhs) {
+  // SolverCG::solve (solver_cg.cc:54-110) on a device rhs (FP64 SoA planes, overwritten; null
+  // for the cell's own residual, whose norm's square is in scal[32])
+  template <typename R> void solve_device(double *rhs) {
     musg_cell &c = *cell;
     cudaStream_t s = c.stream;
-    const long long n = c.nb_dof();
     double *part = c.partial.as<double>(), *dscal = c.scal.as<double>();
-    const bool mixed = precision == MUSG_PRECISION_MIXED;
+    const double t = sizeof(R) == 4 ? std::max(tol, inner_tol) : tol;
     // r = A 0 - rhs = -rhs, p = -r (first iteration), x = 0
-    if (mixed) {
-      const double t = std::max(tol, inner_tol);
-      if (rhs) {
-        dot_device<double, double>(rhs, rhs, n, part, dscal + 36, s);
-        disp_residual(c.sp, q.p, rhs, nullptr, 1.0, false, part, dscal + 37, s);
-        disp_start(c.sp, vectors(), q.p, st.as<CGState>(), t, (int)maxiter, dscal + 36, dscal + 37, s);
-      } else {
-        disp_start(c.sp, vectors(), c.rhat.p, st.as<CGState>(), t, (int)maxiter, nullptr, dscal + 32, s);
-      }
-    } else {
-      cg_init<double>(st.as<CGState>(), rhs, r.as<double>(), x.as<double>(), n, tol, (int)maxiter, part, part + 4096, s);
+    if (rhs) {
+      // a general right-hand side: its part outside the range of the projection stays in
+      // the residual (|rhs - G rhs|^2)
+      if (c.io.bytes < c.field_bytes()) c.io.alloc(c.field_bytes());
+      c.sp.ensure_tiles();
+      disp_residual<double>(c.sp, TK_PLAIN, {}, c.rhat64.p, rhs, nullptr, 1.0, false, part, dscal + 37, s);
+      disp_field<double>(c.sp, c.rhat64.p, c.io.as<double>(), s);
+      diff2_device(rhs, c.io.as<double>(), c.nb_dof(), part, dscal + 36, s);
+      if (sizeof(R) == 4) disp_convert(c.sp, c.rhat64.p, c.rhat.p, s);
     }
+    disp_start<R>(c.sp, vectors(), sizeof(R) == 4 ? c.rhat.p : c.rhat64.p, st.as<CGState>(), t, (int)maxiter,
+                  rhs ? dscal + 36 : nullptr, dscal + (rhs ? 37 : 32), s);
     converged = false;
-    if (graphs && !verbose) {
-      if (mixed) build_graph<float>();
-      else build_graph<double>();
-    }
+    if (graphs && !verbose) build_graph<R>();
     for (;;) {
       if (exec) {
         MUSG_CUDA(cudaGraphLaunch(exec, s));
         g_launches.fetch_add(graph_nodes);
       } else {
-        for (int k = 0; k < chunk; ++k) {
-          if (mixed) iteration<float>(s);
-          else iteration<double>(s);
-        }
+        for (int k = 0; k < chunk; ++k) iteration<R>(s);
       }
       MUSG_CUDA(cudaMemcpyAsync(hst, st.p, sizeof(CGState), cudaMemcpyDeviceToHost, s));
       MUSG_CUDA(cudaStreamSynchronize(s));
       check_stop(stop);
-      if (verbose && (hst->active || !mixed)) {  // mixed: the last pass only finishes x
+      if (verbose && hst->active) {  // the last pass only finishes x
         printf("  at CG step %d: |r|/|b| = %15g, cg_tol = %g\n", hst->iter - 1,
                std::sqrt(hst->rdr / hst->rhs_norm2), tol);
         fflush(stdout);
@@ -780,7 +702,11 @@ struct musg_solver {
         << std::sqrt(hst->rdr / hst->rhs_norm2) << ", cg_tol = " << std::sqrt(hst->tol2 / hst->rhs_norm2);
       throw Error(MUSG_ERR_CONVERGENCE, e.str());
     }
-    if (mixed) disp_solution(c.sp, vectors(), st.as<CGState>(), x.as<float>(), s);
+    disp_solution<R>(c.sp, vectors(), st.as<CGState>(), x.as<R>(), s);
+  }
+  void solve_device_any(double *rhs) {
+    if (precision == MUSG_PRECISION_MIXED) solve_device<float>(rhs);
+    else solve_device<double>(rhs);
   }
 
   void reset_counter() {
@@ -800,7 +726,7 @@ struct musg_batch {
   double tol = 0, inner_tol = 1e-2;
   unsigned maxiter = 0;
   cudaStream_t stream = nullptr;
-  DevBuf states, tab_p, tab_v;
+  DevBuf states;
   CGState *hst = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned long long graph_nodes = 0;
@@ -808,13 +734,10 @@ struct musg_batch {
   // cells of different grids (the same dimension, formulation and tangent kind): one
   // grouped launch per pass over all of them (generic pass kernels)
   bool uniform = true;
-  GroupedOp *gop = nullptr;
-  DispBatch *disp = nullptr;  // mixed: the displacement-space passes of all cells
-  long long nmax = 0;  // the largest cell's vector length
+  DispBatch *disp = nullptr;  // the displacement-space passes of all cells
   const int *stop = nullptr;  // musg_batch_set_stop_flag
 
   ~musg_batch() {
-    if (gop) grouped_op_destroy(gop);
     if (disp) disp_batch_destroy(disp);
     if (exec) cudaGraphExecDestroy(exec);
     if (hst) cudaFreeHost(hst);
@@ -823,69 +746,15 @@ struct musg_batch {
   int B() const { return (int)cells.size(); }
   CGState *state(int b) const { return states.as<CGState>() + b; }
 
-  void build_tables_mixed() {
+  bool mixed() const { return precision == MUSG_PRECISION_MIXED; }
+
+  void build_tables() {
     std::vector<DispProblem> probs(B());
     for (int b = 0; b < B(); ++b) {
       musg_cell &c = *cells[b];
-      probs[b] = {&c.sp, solvers[b]->vectors(), state(b), c.partial.as<double>(), c.tangent<float>()};
+      probs[b] = {&c.sp, solvers[b]->vectors(), state(b), c.partial.as<double>(), c.tangent<float>(), c.tangent<double>()};
     }
-    disp = disp_batch_create(probs, cells[0]->tkind32, uniform);
-  }
-
-  void build_tables() {
-    std::vector<ProblemPtrsHost> tp(B());
-    std::vector<BatchVec<double>> tv(B());
-    for (int b = 0; b < B(); ++b) {
-      musg_cell &c = *cells[b];
-      musg_solver &sv = *solvers[b];
-      const TangentData<double> td = c.tangent<double>();
-      tp[b].spec = c.sp.spec64;
-      tp[b].st = state(b);
-      tp[b].r = sv.r.p;
-      tp[b].p = sv.p.p;
-      tp[b].Ap = sv.Ap.p;
-      tp[b].partial = c.partial.as<double>();
-      static_assert(sizeof(td) == sizeof(tp[b].td), "tangent table layout");
-      memcpy(tp[b].td, &td, sizeof(td));
-      tv[b].st = state(b);
-      tv[b].x = sv.x.as<double>();
-      tv[b].r = sv.r.as<double>();
-      tv[b].p = sv.p.as<double>();
-      tv[b].Ap = sv.Ap.as<double>();
-      tv[b].partial = c.partial.as<double>();
-      tv[b].n = c.nb_dof();
-      nmax = std::max(nmax, c.nb_dof());
-    }
-    if (!uniform) {
-      std::vector<GroupProblem> probs(B());
-      for (int b = 0; b < B(); ++b) {
-        probs[b].sp = &cells[b]->sp;
-        probs[b].st = state(b);
-        probs[b].r = tp[b].r;
-        probs[b].p = tp[b].p;
-        probs[b].Ap = tp[b].Ap;
-        probs[b].partial = tp[b].partial;
-        memcpy(probs[b].td, tp[b].td, sizeof(probs[b].td));
-      }
-      gop = grouped_op_create<double>(probs, cells[0]->tkind);
-    }
-    tab_p.alloc(tp.size() * sizeof(ProblemPtrsHost));
-    tab_v.alloc(tv.size() * sizeof(BatchVec<double>));
-    MUSG_CUDA(cudaMemcpy(tab_p.p, tp.data(), tab_p.bytes, cudaMemcpyHostToDevice));
-    MUSG_CUDA(cudaMemcpy(tab_v.p, tv.data(), tab_v.bytes, cudaMemcpyHostToDevice));
-  }
-
-  void iteration(cudaStream_t s) {
-    if (disp) {
-      disp_batch_run(disp, s);
-      return;
-    }
-    musg_cell &c0 = *cells[0];
-    if (uniform)
-      cg_operator_batch<double>(c0.sp, c0.tkind, (const ProblemPtrs<double> *)tab_p.p, B(), s);  // and alpha
-    else
-      grouped_op_run<double>(gop, s);
-    cg_update_batch<double>(tab_v.as<BatchVec<double>>(), nmax, B(), s);  // and beta
+    disp = disp_batch_create(probs, mixed() ? cells[0]->tkind32 : cells[0]->tkind, uniform, !mixed());
   }
 
   void build_graph() {
@@ -894,7 +763,7 @@ struct musg_batch {
     const unsigned long long before = g_launches.load();
     MUSG_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed));
     try {
-      for (int k = 0; k < chunk; ++k) iteration(stream);
+      for (int k = 0; k < chunk; ++k) disp_batch_run(disp, stream);
     } catch (...) {
       cudaStreamEndCapture(stream, &g);
       if (g) cudaGraphDestroy(g);
@@ -909,20 +778,18 @@ struct musg_batch {
 
   // one batched SolverCG::solve over the cells whose `solve` flag is set
   void solve(const std::vector<char> &solve_it, std::vector<std::string> &errors) {
-    const bool mixed = precision == MUSG_PRECISION_MIXED;
     for (int b = 0; b < B(); ++b) {
       musg_cell &c = *cells[b];
       musg_solver &sv = *solvers[b];
-      double *part = c.partial.as<double>();
       if (!solve_it[b]) {
         MUSG_CUDA(cudaMemsetAsync(&state(b)->active, 0, sizeof(int), stream));
         MUSG_CUDA(cudaMemsetAsync(&state(b)->go, 0, sizeof(int), stream));
-      } else if (mixed) {
-        disp_start(c.sp, sv.vectors(), c.rhat.p, state(b), std::max(tol, inner_tol), (int)maxiter, nullptr,
-                   c.scal.as<double>() + 32, stream);
+      } else if (mixed()) {
+        disp_start<float>(c.sp, sv.vectors(), c.rhat.p, state(b), std::max(tol, inner_tol), (int)maxiter, nullptr,
+                          c.scal.as<double>() + 32, stream);
       } else {
-        cg_init<double>(state(b), c.rhs.as<double>(), sv.r.as<double>(), sv.x.as<double>(), c.nb_dof(), tol,
-                        (int)maxiter, part, part + 4096, stream);
+        disp_start<double>(c.sp, sv.vectors(), c.rhat64.p, state(b), tol, (int)maxiter, nullptr,
+                           c.scal.as<double>() + 32, stream);
       }
     }
     build_graph();
@@ -945,8 +812,10 @@ struct musg_batch {
           << " steps, the solver  FAILED with  |r|/|b| = " << std::sqrt(hst[b].rdr / hst[b].rhs_norm2)
           << ", cg_tol = " << std::sqrt(hst[b].tol2 / hst[b].rhs_norm2);
         errors[b] = e.str();
-      } else if (mixed) {
-        disp_solution(cells[b]->sp, solvers[b]->vectors(), state(b), solvers[b]->x.as<float>(), stream);
+      } else if (mixed()) {
+        disp_solution<float>(cells[b]->sp, solvers[b]->vectors(), state(b), solvers[b]->x.as<float>(), stream);
+      } else {
+        disp_solution<double>(cells[b]->sp, solvers[b]->vectors(), state(b), solvers[b]->x.as<double>(), stream);
       }
     }
   }
@@ -1026,7 +895,7 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
     for (int k = 0; k < D2; ++k) delta[k] = macro[k] - previous[k];
     double *ddelta = c.put_matrix(delta.data(), 16);
     if (!geus) add_macro(c.F.as<double>(), ddelta, D2, c.npx, s);
-    c.residual_kept = false;  // the load step's first residual is projected in FP64
+    c.residual_kept = 0;  // the load step's first residuals are projected in FP64
     const bool mixed = solver->precision == MUSG_PRECISION_MIXED, incremental = solver->incremental_residual;
     std::string message = "Has not converged";
     double incr_norm = 2 * newton_tol, grad_norm = 1, stress_norm = 2 * equil_tol;
@@ -1054,14 +923,7 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
         c.evaluate(false);
         if (first_geus) {
           // rhs = -G(K:DF) with DF the uniform macroscopic increment (FP64)
-          fill_uniform(c.rhs.as<double>(), ddelta, D2, c.npx, s);
-          tangent_operator<double>(c.sp, c.tkind, c.tangent<double>(), c.rhs.as<double>(), c.rhs.as<double>(), s);
-          convert<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, -1.0, s);
-          c.residual_kept = false;
-          if (mixed)
-            c.residual_from_rhs();
-          else
-            dot_device<double, double>(c.rhs.as<double>(), c.rhs.as<double>(), n, c.partial.as<double>(), dscal + 32, s);
+          c.residual_geus(ddelta, mixed);
         } else {
           // rhs = -P, projected
           c.residual(mixed, incremental);
@@ -1071,7 +933,7 @@ void newton_cg_impl(musg_cell *cell, const double *steps, int nsteps, musg_solve
         stress_norm = std::sqrt(c.hscal[32]);
       }
       if (convergence_test()) break;
-      solver->solve_device(mixed ? nullptr : c.rhs.as<double>());
+      solver->solve_device_any(nullptr);
       if (first_geus) add_macro(c.F.as<double>(), ddelta, D2, c.npx, s);
       if (solver->line_search && !first_geus) {
         // F = F0 + lam dF for lam = 1, 1/2, ... until the projected residual norm drops
@@ -1187,7 +1049,7 @@ void batch_newton_impl(musg_batch *batch, const double *steps, int nsteps, doubl
       add_macro(c.F.as<double>(), c.put_matrix(delta.data(), 16), D2, c.npx, s);
       previous[b].assign(macro, macro + D2);
       running[b] = 1;
-      c.residual_kept = false;
+      c.residual_kept = 0;
     }
     for (;;) {
       check_stop(bt.stop);
@@ -1276,36 +1138,21 @@ void batch_newton_impl(musg_batch *batch, const double *steps, int nsteps, doubl
 
 // ====================================================================== C ABI
 namespace {
-void cg_operator_once(musg_cell &c, const double *dF, double *dP) {
+// G(K:dF) of a general (not necessarily compatible) dF through the displacement-space
+// passes, in FP64 or with the FP32 operator of the mixed method
+void cg_operator_once(musg_cell &c, const double *dF, double *dP, bool mixed) {
   const long long n = c.nb_dof();
   if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
   c.upload_field(dF, c.io2.as<double>());
-  DevBuf r, p, Ap, st;
-  for (DevBuf *b : {&r, &p, &Ap}) b->alloc((size_t)n * sizeof(double));
-  st.alloc(sizeof(CGState));
-  // first CG iteration: p = -r, so r = -dF gives p = dF and Ap = G(K:dF)
-  convert<double, double>(r.as<double>(), c.io2.as<double>(), n, -1.0, c.stream);
-  CGState h{};
-  h.maxiter = 1;
-  h.active = 1;
-  MUSG_CUDA(cudaMemcpyAsync(st.p, &h, sizeof(h), cudaMemcpyHostToDevice, c.stream));
-  cg_operator<double>(c.sp, c.tkind, c.tangent<double>(), st.as<CGState>(), r.as<double>(), p.as<double>(),
-                      Ap.as<double>(), c.partial.as<double>(), c.stream);
-  convert<double, double>(c.io2.as<double>(), Ap.as<double>(), n, 1.0, c.stream);
-  c.download_field(c.io2.as<double>(), dP);
-}
-// the FP32 operator of the mixed method: the displacement-space passes, from a general
-// (not necessarily compatible) dF
-void cg_operator_once_mixed(musg_cell &c, const double *dF, double *dP) {
-  const long long n = c.nb_dof();
-  if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
-  c.upload_field(dF, c.io2.as<double>());
-  DevBuf qhat, out;
-  qhat.alloc(disp_vector_bytes(c.sp));
-  out.alloc((size_t)n * sizeof(float));
-  disp_operator(c.sp, c.tkind32, c.tangent<float>(), c.io2.as<double>(), qhat.p, out.as<float>(), c.partial.as<double>(),
-                c.stream);
-  convert<double, float>(c.io2.as<double>(), out.as<float>(), n, 1.0, c.stream);
+  if (mixed) {
+    DevBuf out;
+    out.alloc((size_t)n * sizeof(float));
+    disp_operator<float>(c.sp, c.tkind32, c.tangent<float>(), c.io2.as<double>(), out.as<float>(), c.stream);
+    convert<double, float>(c.io2.as<double>(), out.as<float>(), n, 1.0, c.stream);
+    c.download_field(c.io2.as<double>(), dP);
+    return;
+  }
+  disp_operator<double>(c.sp, c.tkind, c.tangent<double>(), c.io2.as<double>(), c.io2.as<double>(), c.stream);
   c.download_field(c.io2.as<double>(), dP);
 }
 }  // namespace
@@ -1466,7 +1313,6 @@ int musg_cell_initialise(musg_cell *cell, int plan_flags) {
   return guard([&] {
     require(cell, MUSG_ERR_ARGUMENT, "null cell");
     require(plan_flags >= 0 && plan_flags <= 2, MUSG_ERR_ARGUMENT, "unknown planner flag type");
-    cell->plan_flags = plan_flags;
     cell->initialise();
   });
 }
@@ -1544,7 +1390,7 @@ int musg_cell_apply_projection(musg_cell *cell, double *vec) {
     musg_cell &c = *cell;
     if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
     c.upload_field(vec, c.io2.as<double>());
-    spectral_project<double>(c.sp, c.io2.as<double>(), c.io2.as<double>(), 1.0, c.stream);
+    disp_operator<double>(c.sp, TK_PLAIN, {}, c.io2.as<double>(), c.io2.as<double>(), c.stream);
     c.download_field(c.io2.as<double>(), vec);
   });
 }
@@ -1557,7 +1403,7 @@ int musg_cell_directional_stiffness(musg_cell *cell, const double *dF, double *d
             "currently only implemented for cases where a stiffness matrix exists");
     if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
     c.upload_field(dF, c.io2.as<double>());
-    tangent_operator<double>(c.sp, c.tkind, c.tangent<double>(), c.io2.as<double>(), c.io2.as<double>(), c.stream);
+    disp_operator<double>(c.sp, c.tkind, c.tangent<double>(), c.io2.as<double>(), c.io2.as<double>(), c.stream);
     c.download_field(c.io2.as<double>(), dP);
   });
 }
@@ -1571,14 +1417,14 @@ int musg_cell_cg_operator(musg_cell *cell, int precision, const double *dF, doub
     require(c.tangent_valid, MUSG_ERR_RUNTIME,
             "currently only implemented for cases where a stiffness matrix exists");
     if (precision == MUSG_PRECISION_FP64) {
-      cg_operator_once(c, dF, dP);
+      cg_operator_once(c, dF, dP, false);
       return;
     }
     if (!c.need32 || !c.lam32.p) {
       c.alloc32();
       c.evaluate(false);  // the FP32 tangent data of the current strain
     }
-    cg_operator_once_mixed(c, dF, dP);
+    cg_operator_once(c, dF, dP, true);
   });
 }
 
@@ -1828,7 +1674,7 @@ int musg_solver_solve(musg_solver *solver, const double *rhs, double *x_out) {
     require(c.tangent_valid, MUSG_ERR_RUNTIME, "currently only implemented for cases where a stiffness matrix exists");
     if (c.io2.bytes < c.field_bytes()) c.io2.alloc(c.field_bytes());
     c.upload_field(rhs, c.io2.as<double>());
-    solver->solve_device(c.io2.as<double>());
+    solver->solve_device_any(c.io2.as<double>());
     if (solver->precision == MUSG_PRECISION_MIXED)
       convert<double, float>(c.io2.as<double>(), solver->x.as<float>(), c.nb_dof(), 1.0, c.stream);
     else
@@ -1862,7 +1708,7 @@ int musg_solver_profile(musg_solver *solver, int iterations, double *ms_out, int
 
 const char *musg_solver_kernel_name(musg_solver *solver, int k) {
   if (!solver || !solver->cell) return "";
-  return musg_solver::kernel_name(solver->cell->dim, solver->precision, k);
+  return musg_solver::kernel_name(solver->cell->dim, k);
 }
 
 int musg_batch_create(musg_cell **cells, int nb_cells, double tol, unsigned maxiter, int precision,
@@ -1885,13 +1731,6 @@ int musg_batch_create(musg_cell **cells, int nb_cells, double tol, unsigned maxi
       bt->solvers.push_back(std::move(sv));
       bt->cells.push_back(&c);
     }
-    // the launch shapes of the first cell serve the whole batch
-    for (int b = 1; b < nb_cells; ++b)
-      for (int p = 0; p < 2; ++p)
-        for (int k = 0; k < 3; ++k) {
-          cells[b]->sp.tune_threads[p][k] = c0.sp.tune_threads[p][k];
-          cells[b]->sp.tune_bytes[p][k] = c0.sp.tune_bytes[p][k];
-        }
     bt->precision = precision;
     bt->tol = tol;
     bt->maxiter = maxiter;
@@ -1899,8 +1738,7 @@ int musg_batch_create(musg_cell **cells, int nb_cells, double tol, unsigned maxi
     bt->states.alloc(nb_cells * sizeof(CGState));
     MUSG_CUDA(cudaMemset(bt->states.p, 0, bt->states.bytes));
     MUSG_CUDA(cudaMallocHost(&bt->hst, nb_cells * sizeof(CGState)));
-    if (precision == MUSG_PRECISION_MIXED) bt->build_tables_mixed();
-    else bt->build_tables();
+    bt->build_tables();
     *out = bt.release();
   });
 }
@@ -2023,7 +1861,7 @@ int musg_projection_apply(musg_projection *proj, double *vec) {
     if (proj->b.bytes < rb) proj->b.alloc(rb);
     MUSG_CUDA(cudaMemcpyAsync(proj->a.p, vec, rb, cudaMemcpyHostToDevice, proj->stream));
     aos_to_soa(proj->a.as<double>(), proj->b.as<double>(), sp.ncomp, sp.g.npx, proj->stream);
-    spectral_project<double>(sp, proj->b.as<double>(), proj->b.as<double>(), 1.0, proj->stream);
+    disp_operator<double>(sp, TK_PLAIN, {}, proj->b.as<double>(), proj->b.as<double>(), proj->stream);
     soa_to_aos(proj->b.as<double>(), proj->a.as<double>(), sp.ncomp, sp.g.npx, proj->stream);
     MUSG_CUDA(cudaMemcpyAsync(vec, proj->a.p, rb, cudaMemcpyDeviceToHost, proj->stream));
     MUSG_CUDA(cudaStreamSynchronize(proj->stream));

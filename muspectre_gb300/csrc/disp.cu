@@ -1,4 +1,4 @@
-// The displacement-space CG of the mixed method (disp.cuh): launches of its passes.
+// The displacement-space CG (disp.cuh): iterations, projections and batches from its passes.
 #include <cstring>
 #include <memory>
 
@@ -35,15 +35,12 @@ template <typename R> DispPasses<R> disp_passes(Spectral &sp, const DispProb<R> 
 // The solve runs on the right-hand side scaled to unit norm: q.q grows with the square of
 // the stiffness and would leave the range of FP32 for residuals in Pa.  x is scaled back
 // when it is read (AX_X).
-__global__ void k_disp_start(CGState *st, const double *rhs2, const double *range2, double tol, int maxiter) {
-  const double in = *range2, all = rhs2 ? *rhs2 : in;
-  // FP32 noise of the transform is not a part outside the range
-  const double out = all - in;
+__global__ void k_disp_start(CGState *st, const double *out2, const double *range2, double tol, int maxiter) {
+  const double in = *range2, out = out2 ? *out2 : 0.0;
   st->xscale = sqrt(in);
-  st->out2 = out > 1e-5 * all ? out / in : 0.0;
-  st->rdr = 1.0 + st->out2;
-  st->rhs_norm2 = all / in;
-  st->tol2 = tol * tol * (all / in);
+  st->out2 = out / in;
+  st->rdr = st->rhs_norm2 = (in + out) / in;
+  st->tol2 = tol * tol * st->rhs_norm2;
   st->alpha = st->beta = st->pAp = 0.0;
   st->iter = 0;
   st->maxiter = maxiter;
@@ -52,25 +49,27 @@ __global__ void k_disp_start(CGState *st, const double *rhs2, const double *rang
   st->active = st->go = maxiter > 0 ? 1 : 0;
 }
 
-// r = -b / |b|, x = 0.  The points of the plane k_last = 0 come in pairs (k, -k) of one
-// real field; rounding leaves b unsymmetric there, the operator's inverse transform
+// r = -b (over the scale), x = 0.  The points of the plane k_last = 0 come in pairs (k, -k)
+// of one real field; rounding leaves b unsymmetric there, the operator's inverse transform
 // drops that part and no iteration could reduce it, so each pair takes its mean (in a
 // residual accumulated over Newton steps the rounding is that of the largest one, and
 // the CG stalled on it).
-__global__ void k_disp_init(const float2 *__restrict__ b, float2 *__restrict__ r, float2 *__restrict__ x, int D, int n0,
-                            int n1, int nh, const CGState *st) {
-  const float c = (float)(-1.0 / st->xscale);
+template <typename R>
+__global__ void k_disp_init(const typename V2<R>::T *__restrict__ b, typename V2<R>::T *__restrict__ r,
+                            typename V2<R>::T *__restrict__ x, int D, int n0, int n1, int nh, const CGState *st) {
+  using T = typename V2<R>::T;
+  const R c = (R)(-1.0 / st->xscale);
   const unsigned rows = (unsigned)D * n0 * n1, n = rows * (unsigned)nh;  // n1: 1 in 2-D
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float2 v = b[i];
+    T v = b[i];
     if (i % nh == 0) {
       const unsigned row = i / nh, k1 = row % n1, dk0 = row / n1, k0 = dk0 % n0;
       const unsigned m0 = k0 ? n0 - k0 : 0, m1 = k1 ? n1 - k1 : 0;
-      const float2 w = b[((size_t)(dk0 - k0 + m0) * n1 + m1) * nh];
-      v = make_float2(0.5f * (v.x - w.x), 0.5f * (v.y + w.y));  // xi is odd: v(-k) = -conj v(k)
+      const T w = b[((size_t)(dk0 - k0 + m0) * n1 + m1) * nh];
+      v = T{R(0.5) * (v.x - w.x), R(0.5) * (v.y + w.y)};  // xi is odd: v(-k) = -conj v(k)
     }
-    r[i] = make_float2(c * v.x, c * v.y);
-    x[i] = make_float2(0.f, 0.f);
+    r[i] = T{c * v.x, c * v.y};
+    x[i] = T{R(0), R(0)};
   }
 }
 
@@ -82,11 +81,27 @@ __global__ void k_disp_sum(const double *partial, int nparts, double *out) {
   if (threadIdx.x == 0) *out = s;
 }
 
+__global__ void k_disp_convert(const double2 *__restrict__ a, float2 *__restrict__ b, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double2 v = a[i];
+    b[i] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
+template <typename R> typename V2<R>::T *work_spectrum(Spectral &sp);
+template <> double2 *work_spectrum<double>(Spectral &sp) {
+  sp.ensure_tiles();
+  return (double2 *)sp.spec64;
+}
+template <> float2 *work_spectrum<float>(Spectral &sp) {
+  sp.ensure32();
+  return (float2 *)sp.spec32;
+}
+
 template <typename R> DispProb<R> disp_prob(Spectral &sp, const DispVectors &v, CGState *st, double *partial) {
   using T = typename V2<R>::T;
-  sp.ensure32();
   DispProb<R> pb;
-  pb.spec = (T *)sp.spec32;
+  pb.spec = work_spectrum<R>(sp);
   pb.r = (T *)v.r;
   pb.q = (T *)v.q;
   pb.p = (T *)v.p;
@@ -96,10 +111,11 @@ template <typename R> DispProb<R> disp_prob(Spectral &sp, const DispVectors &v, 
   return pb;
 }
 
-void pixels(const Spectral &sp, int tkind, const DispArgs<float> &a, const DispShape &c, int B, cudaStream_t s,
-            const DispGroup<float> *grp) {
-  if (sp.g.dim == 2) disp_pixels<float, 2>(tkind, sp.tp[1], a, c, B, s, grp);
-  else disp_pixels<float, 3>(tkind, sp.tp[2], a, c, B, s, grp);
+template <typename R>
+void pixels(const Spectral &sp, int tkind, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
+            const DispGroup<R> *grp) {
+  if (sp.g.dim == 2) disp_pixels<R, 2>(tkind, sp.tp[1], a, c, B, s, grp);
+  else disp_pixels<R, 3>(tkind, sp.tp[2], a, c, B, s, grp);
 }
 
 // q (the vectors' q) -> real planes, ungated
@@ -137,144 +153,187 @@ void forward_to(Spectral &sp, DispProb<R> pb, int tkind, const double *in, doubl
 
 }  // namespace
 
-void disp_residual(Spectral &sp, void *rhat, const double *field, double *prev, double scale, bool accumulate,
-                   double *partial, double *norm2, cudaStream_t s) {
+template <typename R>
+void disp_residual(Spectral &sp, int tkind, const TangentData<R> &td, void *rhat, const double *field, double *prev,
+                   double scale, bool accumulate, double *partial, double *norm2, cudaStream_t s) {
   DispVectors v;
   v.q = rhat;
-  forward_to<float>(sp, disp_prob<float>(sp, v, nullptr, partial), TK_PLAIN, field, prev, scale, accumulate, norm2, s);
-}
-
-void disp_start(Spectral &sp, const DispVectors &v, const void *rhat, CGState *st, double tol, int maxiter,
-                const double *rhs2, const double *range2, cudaStream_t s) {
-  const long long n = disp_nk(sp) * sp.g.dim;
-  if (n > 0xf0000000ll) throw Error(MUSG_ERR_ARGUMENT, "grid too large for the mixed method");
-  k_disp_start<<<1, 1, 0, s>>>(st, rhs2, range2, tol, maxiter);
-  MUSG_CHECK_LAUNCH();
-  k_disp_init<<<reduce_blocks(n), 256, 0, s>>>((const float2 *)rhat, (float2 *)v.r, (float2 *)v.x, sp.g.dim,
-                                                 sp.g.n[0], sp.g.dim == 3 ? sp.g.n[1] : 1, disp_nh(sp), st);
-  MUSG_CHECK_LAUNCH();
-}
-
-void disp_iteration(Spectral &sp, int tkind, const TangentData<float> &td, const DispVectors &v, CGState *st,
-                    double *partial, cudaStream_t s, cudaEvent_t *ev) {
-  DispProb<float> pb = disp_prob<float>(sp, v, st, partial);
+  DispProb<R> pb = disp_prob<R>(sp, v, nullptr, partial);
   pb.td = td;
-  const DispPasses<float> p = disp_passes<float>(sp, pb);
+  forward_to<R>(sp, pb, tkind, field, prev, scale, accumulate, norm2, s);
+}
+
+template <typename R>
+void disp_start(Spectral &sp, const DispVectors &v, const void *rhat, CGState *st, double tol, int maxiter,
+                const double *out2, const double *range2, cudaStream_t s) {
+  using T = typename V2<R>::T;
+  const long long n = disp_nk(sp) * sp.g.dim;
+  if (n > 0xf0000000ll) throw Error(MUSG_ERR_ARGUMENT, "grid too large for the CG solver");
+  k_disp_start<<<1, 1, 0, s>>>(st, out2, range2, tol, maxiter);
+  MUSG_CHECK_LAUNCH();
+  k_disp_init<R><<<reduce_blocks(n), 256, 0, s>>>((const T *)rhat, (T *)v.r, (T *)v.x, sp.g.dim, sp.g.n[0],
+                                                  sp.g.dim == 3 ? sp.g.n[1] : 1, disp_nh(sp), st);
+  MUSG_CHECK_LAUNCH();
+}
+
+template <typename R>
+void disp_iteration(Spectral &sp, int tkind, const TangentData<R> &td, const DispVectors &v, CGState *st,
+                    double *partial, cudaStream_t s, cudaEvent_t *ev) {
+  DispProb<R> pb = disp_prob<R>(sp, v, st, partial);
+  pb.td = td;
+  const DispPasses<R> p = disp_passes<R>(sp, pb);
   int k = 0;
   auto mark = [&]() {
     if (ev) MUSG_CUDA(cudaEventRecord(ev[k++], s));
   };
   mark();
-  disp_ax0_step<float>(sp, p.ai, p.ci, 1, s, nullptr);
+  disp_ax0_step<R>(sp, p.ai, p.ci, 1, s, nullptr);
   mark();
   if (sp.g.dim == 3) {
-    disp_mid<float>(sp, true, p.am, p.cm, 1, s, nullptr);
+    disp_mid<R>(sp, true, p.am, p.cm, 1, s, nullptr);
     mark();
   }
-  pixels(sp, tkind, p.al, p.cl, 1, s, nullptr);
+  pixels<R>(sp, tkind, p.al, p.cl, 1, s, nullptr);
   mark();
   if (sp.g.dim == 3) {
-    disp_mid<float>(sp, false, p.am, p.cm, 1, s, nullptr);
+    disp_mid<R>(sp, false, p.am, p.cm, 1, s, nullptr);
     mark();
   }
-  disp_ax0_dots<float>(sp, p.af, p.cf, 1, s, nullptr);
+  disp_ax0_dots<R>(sp, p.af, p.cf, 1, s, nullptr);
   mark();
 }
 
-void disp_solution(Spectral &sp, const DispVectors &v, CGState *st, float *x, cudaStream_t s) {
-  inverse_from<float>(sp, disp_prob<float>(sp, v, st, nullptr), true, x, s);
+template <typename R>
+void disp_solution(Spectral &sp, const DispVectors &v, CGState *st, R *x, cudaStream_t s) {
+  inverse_from<R>(sp, disp_prob<R>(sp, v, st, nullptr), true, x, s);
 }
 
-void disp_operator(Spectral &sp, int tkind, const TangentData<float> &td, const double *in, void *qhat, float *out,
-                   double *partial, cudaStream_t s) {
+template <typename R>
+void disp_operator(Spectral &sp, int tkind, const TangentData<R> &td, const double *in, R *out, cudaStream_t s) {
+  // q in the work spectrum itself: a block of the contraction has read its tile's
+  // components before it writes q over the first ones, and the inverse likewise
+  DispVectors v;
+  v.q = work_spectrum<R>(sp);
+  DispProb<R> pb = disp_prob<R>(sp, v, nullptr, nullptr);
+  pb.td = td;
+  forward_to<R>(sp, pb, tkind, in, nullptr, 1.0, false, nullptr, s);
+  inverse_from<R>(sp, pb, false, out, s);
+}
+
+template <typename R> void disp_field(Spectral &sp, void *qhat, R *out, cudaStream_t s) {
   DispVectors v;
   v.q = qhat;
-  DispProb<float> pb = disp_prob<float>(sp, v, nullptr, partial);
-  pb.td = td;
-  forward_to<float>(sp, pb, tkind, in, nullptr, 1.0, false, nullptr, s);
-  inverse_from<float>(sp, pb, false, out, s);
+  inverse_from<R>(sp, disp_prob<R>(sp, v, nullptr, nullptr), false, out, s);
 }
+
+void disp_convert(const Spectral &sp, const void *v64, void *v32, cudaStream_t s) {
+  const long long n = disp_nk(sp) * sp.g.dim;
+  k_disp_convert<<<reduce_blocks(n), 256, 0, s>>>((const double2 *)v64, (float2 *)v32, n);
+  MUSG_CHECK_LAUNCH();
+}
+
+#define MUSG_INSTANTIATE_DISP(R)                                                                                      \
+  template void disp_residual<R>(Spectral &, int, const TangentData<R> &, void *, const double *, double *, double,   \
+                                 bool, double *, double *, cudaStream_t);                                             \
+  template void disp_start<R>(Spectral &, const DispVectors &, const void *, CGState *, double, int, const double *,  \
+                              const double *, cudaStream_t);                                                          \
+  template void disp_iteration<R>(Spectral &, int, const TangentData<R> &, const DispVectors &, CGState *, double *,  \
+                                  cudaStream_t, cudaEvent_t *);                                                       \
+  template void disp_solution<R>(Spectral &, const DispVectors &, CGState *, R *, cudaStream_t);                      \
+  template void disp_field<R>(Spectral &, void *, R *, cudaStream_t);                                                 \
+  template void disp_operator<R>(Spectral &, int, const TangentData<R> &, const double *, R *, cudaStream_t);
+MUSG_INSTANTIATE_DISP(float)
+MUSG_INSTANTIATE_DISP(double)
 
 // ------------------------------------------------------------------ batches
 // problems of one grid: a device table indexed by blockIdx.y; of different grids: per
 // pass a table of arguments and the prefix sums of the problems' blocks
 struct DispBatch {
-  bool uniform = true;
-  int B = 0, dim = 0, tkind = 0;
-  Spectral *sp0 = nullptr;
-  DispPasses<float> p;                      // uniform: the shared shapes; else the launches' sizes
-  DevBuf tab, gi, gm, gl, gf, blk;          // tables; blk: four prefix sums of B + 1
+  virtual ~DispBatch() {}
+  virtual void run(cudaStream_t s) = 0;
 };
 
-template <typename T> static void upload(DevBuf &d, const std::vector<T> &v) {
+namespace {
+
+template <typename T> void upload(DevBuf &d, const std::vector<T> &v) {
   d.alloc(v.size() * sizeof(T));
   MUSG_CUDA(cudaMemcpy(d.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
-DispBatch *disp_batch_create(const std::vector<DispProblem> &probs, int tkind, bool uniform) {
-  auto b = std::make_unique<DispBatch>();
-  b->uniform = uniform;
-  b->B = (int)probs.size();
-  b->sp0 = probs[0].sp;
-  b->dim = b->sp0->g.dim;
-  b->tkind = tkind;
-  std::vector<DispProb<float>> tab;
-  for (const DispProblem &q : probs) {
-    DispProb<float> pb = disp_prob<float>(*q.sp, q.v, q.st, q.partial);
-    pb.td = q.td;
-    tab.push_back(pb);
-  }
-  if (uniform) {
-    upload(b->tab, tab);
-    b->p = disp_passes<float>(*b->sp0, DispProb<float>{});
-    for (DispArgs<float> *a : {&b->p.ai, &b->p.am, &b->p.al, &b->p.af}) a->tab = b->tab.as<DispProb<float>>();
-    return b.release();
-  }
-  const int n = b->B + 1;
-  std::vector<DispArgs<float>> gi, gm, gl, gf;
-  std::vector<int> blk(4 * n, 0);
-  for (int k = 0; k < b->B; ++k) {
-    Spectral &sp = *probs[k].sp;
-    if (sp.g.dim != b->dim || disp_finite(sp) != disp_finite(*b->sp0))
-      throw Error(MUSG_ERR_ARGUMENT, "a grouped operator needs one dimension, projection and component count");
-    const DispPasses<float> p = disp_passes<float>(sp, tab[k]);
-    DispArgs<float> al = p.al;
-    al.tkind = tkind;
-    gi.push_back(p.ai);
-    gm.push_back(p.am);
-    gl.push_back(al);
-    gf.push_back(p.af);
-    const DispShape *c[4] = {&p.ci, &p.cm, &p.cl, &p.cf};
-    DispShape *m[4] = {&b->p.ci, &b->p.cm, &b->p.cl, &b->p.cf};
-    for (int q = 0; q < 4; ++q) {  // one block size and shared-memory size per launch: the largest
-      blk[q * n + k + 1] = blk[q * n + k] + c[q]->blocks;
-      m[q]->blocks = blk[q * n + k + 1];
-      m[q]->threads = std::max(m[q]->threads, c[q]->threads);
-      m[q]->smem = std::max(m[q]->smem, c[q]->smem);
+template <typename R> struct DispBatchR : DispBatch {
+  bool uniform = true;
+  int B = 0, dim = 0, tkind = 0;
+  Spectral *sp0 = nullptr;
+  DispPasses<R> p;                  // uniform: the shared shapes; else the launches' sizes
+  DevBuf tab, gi, gm, gl, gf, blk;  // tables; blk: four prefix sums of B + 1
+
+  DispBatchR(const std::vector<DispProblem> &probs, int tkind_, bool uniform_)
+      : uniform(uniform_), B((int)probs.size()), dim(probs[0].sp->g.dim), tkind(tkind_), sp0(probs[0].sp) {
+    std::vector<DispProb<R>> tb;
+    for (const DispProblem &q : probs) {
+      DispProb<R> pb = disp_prob<R>(*q.sp, q.v, q.st, q.partial);
+      if constexpr (sizeof(R) == 4) pb.td = q.td32;
+      else pb.td = q.td64;
+      tb.push_back(pb);
     }
+    if (uniform) {
+      upload(tab, tb);
+      p = disp_passes<R>(*sp0, DispProb<R>{});
+      for (DispArgs<R> *a : {&p.ai, &p.am, &p.al, &p.af}) a->tab = tab.as<DispProb<R>>();
+      return;
+    }
+    const int n = B + 1;
+    std::vector<DispArgs<R>> vi, vm, vl, vf;
+    std::vector<int> bk(4 * n, 0);
+    for (int k = 0; k < B; ++k) {
+      Spectral &sp = *probs[k].sp;
+      if (sp.g.dim != dim || disp_finite(sp) != disp_finite(*sp0))
+        throw Error(MUSG_ERR_ARGUMENT, "a grouped operator needs one dimension, projection and component count");
+      const DispPasses<R> q = disp_passes<R>(sp, tb[k]);
+      DispArgs<R> al = q.al;
+      al.tkind = tkind;
+      vi.push_back(q.ai);
+      vm.push_back(q.am);
+      vl.push_back(al);
+      vf.push_back(q.af);
+      const DispShape *c[4] = {&q.ci, &q.cm, &q.cl, &q.cf};
+      DispShape *m[4] = {&p.ci, &p.cm, &p.cl, &p.cf};
+      for (int u = 0; u < 4; ++u) {  // one block size and shared-memory size per launch: the largest
+        bk[u * n + k + 1] = bk[u * n + k] + c[u]->blocks;
+        m[u]->blocks = bk[u * n + k + 1];
+        m[u]->threads = std::max(m[u]->threads, c[u]->threads);
+        m[u]->smem = std::max(m[u]->smem, c[u]->smem);
+      }
+    }
+    upload(gi, vi);
+    upload(gm, vm);
+    upload(gl, vl);
+    upload(gf, vf);
+    upload(blk, bk);
   }
-  upload(b->gi, gi);
-  upload(b->gm, gm);
-  upload(b->gl, gl);
-  upload(b->gf, gf);
-  upload(b->blk, blk);
-  return b.release();
-}
 
+  void run(cudaStream_t s) override {
+    const Spectral &sp = *sp0;
+    const int nb = uniform ? B : 1, n = B + 1;
+    DispGroup<R> g[4];
+    const DevBuf *t[4] = {&gi, &gm, &gl, &gf};
+    for (int q = 0; q < 4; ++q) g[q] = {t[q]->as<const DispArgs<R>>(), blk.as<const int>() + q * n, B};
+    auto grp = [&](int q) { return uniform ? nullptr : &g[q]; };
+    disp_ax0_step<R>(sp, p.ai, p.ci, nb, s, grp(0));
+    if (dim == 3) disp_mid<R>(sp, true, p.am, p.cm, nb, s, grp(1));
+    pixels<R>(sp, tkind, p.al, p.cl, nb, s, grp(2));
+    if (dim == 3) disp_mid<R>(sp, false, p.am, p.cm, nb, s, grp(1));
+    disp_ax0_dots<R>(sp, p.af, p.cf, nb, s, grp(3));
+  }
+};
+
+}  // namespace
+
+DispBatch *disp_batch_create(const std::vector<DispProblem> &probs, int tkind, bool uniform, bool fp64) {
+  if (fp64) return new DispBatchR<double>(probs, tkind, uniform);
+  return new DispBatchR<float>(probs, tkind, uniform);
+}
 void disp_batch_destroy(DispBatch *b) { delete b; }
-
-void disp_batch_run(DispBatch *b, cudaStream_t s) {
-  const Spectral &sp = *b->sp0;
-  const int B = b->uniform ? b->B : 1, n = b->B + 1;
-  DispGroup<float> g[4];
-  const DevBuf *t[4] = {&b->gi, &b->gm, &b->gl, &b->gf};
-  for (int q = 0; q < 4; ++q) g[q] = {t[q]->as<const DispArgs<float>>(), b->blk.as<const int>() + q * n, b->B};
-  auto grp = [&](int q) { return b->uniform ? nullptr : &g[q]; };
-  disp_ax0_step<float>(sp, b->p.ai, b->p.ci, B, s, grp(0));
-  if (b->dim == 3) disp_mid<float>(sp, true, b->p.am, b->p.cm, B, s, grp(1));
-  pixels(sp, b->tkind, b->p.al, b->p.cl, B, s, grp(2));
-  if (b->dim == 3) disp_mid<float>(sp, false, b->p.am, b->p.cm, B, s, grp(1));
-  disp_ax0_dots<float>(sp, b->p.af, b->p.cf, B, s, grp(3));
-}
+void disp_batch_run(DispBatch *b, cudaStream_t s) { b->run(s); }
 
 }  // namespace musg

@@ -1,4 +1,6 @@
-// CG iteration in displacement space (device code): the inner solve of the mixed method.
+// CG iteration in displacement space (device code), in FP64 (the plain method) and in FP32
+// (the inner solve of the mixed method); the projection and the operator G(K:dF) of a
+// general field run through the same passes.
 //
 // Every vector of the CG lies in the range of the projection G (the right-hand side is
 // G(-P), x0 = 0), and a field in that range has D scalars per k-point instead of D^2:
@@ -32,7 +34,8 @@
 // 30 us of the 128^3 update pass).  alpha = r.r / p.q, and the new r.r for beta and the
 // loop test is r.r + 2 alpha r.q + alpha^2 q.q, with r.r summed afresh in every
 // iteration, so it does not drift; a drop below 1e-6 (FP32) of the old value, where that
-// expression cancels, counts as 1e-6 and the next iteration's fresh r.r decides.
+// expression cancels, counts as 1e-6 (FP64 1e-14) and the next iteration's fresh r.r
+// decides.
 //
 // Why: the real-space iteration this replaces moved 16 real fields and the tangent data
 // (155 component spectra at 128^3 finite strain, 146 small strain) in eight launches;
@@ -43,6 +46,9 @@
 // 39 -> 34 and 43 -> 33 us) and with the sums reduced in FP32 pairs (51 -> 45 us) the
 // 128^3 iteration takes 246 us.  What bounds the passes is latency and instruction issue
 // at 25-30% of the warp slots, not bandwidth: 128^3 moves 850 MB in 246 us.
+// FP64 (bound by the FP64 pipe and, on small grids, latency): 51^2 252 -> 95 us, where
+// the factors 17 x 3 replace Bluestein over 105, 35^3 182 -> 147; a 55^3 projection
+// 2.05 -> 0.43 ms.
 #pragma once
 
 #include "spectral.cuh"
@@ -112,9 +118,10 @@ __device__ __forceinline__ void stage_tile_twiddles(typename V2<R>::T *dst, cons
   for (int k = threadIdx.x; k < m; k += blockDim.x) dst[k] = pl.tw[k];
 }
 
-// registers per thread: 80 for the runtime plans, whose radices above 12 would take up to
-// 120 and halve the warps that hide the loads of all the others (they spill instead)
-template <int CR1> constexpr int kDispRegs = CR1 == 16 ? 72 : CR1 > 0 ? 64 : 80;
+// registers per thread.  FP32: 80 for the runtime plans, whose radices above 12 would take
+// up to 120 and halve the warps that hide the loads of all the others (they spill
+// instead).  FP64 passes wait on the FP64 pipe, not on loads: 128.
+template <typename R, int CR1> constexpr int kDispRegs = sizeof(R) == 8 ? 128 : CR1 == 16 ? 72 : CR1 > 0 ? 64 : 80;
 
 // Sum of the threads' compensated accumulators over the block, by thread 0.  FP32: the
 // warps add (sum, correction) pairs with Knuth's two-sum, an error of about 2^-46 in FP32
@@ -148,6 +155,24 @@ template <int N> __device__ __forceinline__ void block_sums(Acc<float> (&v)[N], 
 
 __device__ __forceinline__ double disp_floor(float) { return 1e-6; }
 __device__ __forceinline__ double disp_floor(double) { return 1e-14; }
+
+template <int N> __device__ __forceinline__ void block_sums(Acc<double> (&v)[N], double *out) {
+  __shared__ double red[N][32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    double s = v[k].s;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (l == 0) red[k][w] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double t = 0.0;
+    for (int i = 0; i < nw; ++i) t += red[threadIdx.x][i];
+    out[threadIdx.x] = t;
+  }
+}
 
 // the end of an iteration, by the whole of its last block: the scalars from the nparts
 // blocks' sums (p.q, r.q, q.q, r.r), and whether another iteration follows
@@ -250,7 +275,7 @@ enum Ax0Mode : int {
 };
 
 template <typename R, int D, bool FIN, int MODE, int CR1, int CR2, bool GRP>
-__global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_inv(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
+__global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_inv(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
   dep_wait();
   using T = typename V2<R>::T;
   using C = DispComps<D, FIN>;
@@ -379,7 +404,7 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_inv(const DispArgs<R> a0, cons
 // column 2 before column 1 replaces it, the forward pass finds column 2's transform in
 // memory when it forms column 1's.  Small strain: one component per block.
 template <typename R, bool FIN, bool INV, int CR1, int CR2, bool GRP>
-__global__ void __maxnreg__(kDispRegs<CR1>) k_mid(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
+__global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
   dep_wait();
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -467,7 +492,7 @@ enum Ax0Sums : int {
 };
 
 template <typename R, int D, bool FIN, int MODE, int CR1, int CR2, bool GRP>
-__global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_fwd(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
+__global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_fwd(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
   dep_wait();
   using T = typename V2<R>::T;
   using C = DispComps<D, FIN>;
@@ -590,7 +615,7 @@ __global__ void __maxnreg__(kDispRegs<CR1>) k_ax0_fwd(const DispArgs<R> a0, cons
     }
     __syncthreads();  // the tile is free for the next one
   }
-  block_sums(sum, a.pb.partial + 4 * (long long)bid);
+  if (a.pb.partial) block_sums(sum, a.pb.partial + 4 * (long long)bid);  // null: plain projections
   if (MODE == AX_DOTS && cg_last_block(a.pb.st, a.nparts)) disp_finish<R>(a.pb.st, a.pb.partial, a.nparts);
 }
 
@@ -613,7 +638,7 @@ __device__ __forceinline__ void pixel_tangent(const TangentData<R> &td, long lon
 // of the tile pass through shared memory once between the inverse and the forward
 // transform, where the tangent is applied
 template <typename R, int D, bool FIN, int TK, int IN, int OUT, int CR1, int CR2, bool GRP>
-__global__ void __maxnreg__(kDispRegs<CR1>) k_pixels(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
+__global__ void __maxnreg__((kDispRegs<R, CR1>)) k_pixels(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
   dep_wait();
   using T = typename V2<R>::T;
   constexpr int NL = DispComps<D, FIN>::NL, D2 = D * D;

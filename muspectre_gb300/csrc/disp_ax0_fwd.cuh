@@ -1,5 +1,7 @@
 // Launches of the displacement-space CG's axis-0 forward passes (disp.cuh): with the
 // iteration's sums, and the plain contraction.
+#pragma once
+
 #include "disp_launch.cuh"
 
 namespace musg {
@@ -8,14 +10,17 @@ namespace {
 template <typename R, int D, bool FIN>
 void ax0_dots(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
               const DispGroup<R> *grp) {
-  if (grp) return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, 0, 0, true>, a, c, B, s, grp);
-  switch (pl.blu ? 0 : pl.m) {
+  if (grp) return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+  if constexpr (sizeof(R) == 4) {
+    switch (disp_fixed_plan(pl)) {
 #define MUSG_C(M, A, BB) \
   case M: return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, A, BB, false>, a, c, B, s);
-    MUSG_DISP_PLANS(MUSG_C)
+      MUSG_DISP_PLANS(MUSG_C)
 #undef MUSG_C
-    default: return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, 0, 0, false>, a, c, B, s);
+      default: break;
+    }
   }
+  disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, 0, 0, false>, a, c, B, s);
 }
 }  // namespace
 
@@ -35,8 +40,9 @@ void disp_ax0_contract(const Spectral &sp, const DispArgs<R> &a, const DispShape
 #undef MUSG_C
 }
 
-template void disp_ax0_dots<float>(const Spectral &, const DispArgs<float> &, const DispShape &, int, cudaStream_t,
-                                   const DispGroup<float> *);
-template void disp_ax0_contract<float>(const Spectral &, const DispArgs<float> &, const DispShape &, cudaStream_t);
+#define MUSG_INSTANTIATE_DISP_AX0_FWD(R) \
+template void disp_ax0_dots<R>(const Spectral &, const DispArgs<R> &, const DispShape &, int, cudaStream_t, \
+                                   const DispGroup<R> *); \
+template void disp_ax0_contract<R>(const Spectral &, const DispArgs<R> &, const DispShape &, cudaStream_t);
 
 }  // namespace musg

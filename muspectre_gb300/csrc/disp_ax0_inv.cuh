@@ -1,5 +1,7 @@
 // Launches of the displacement-space CG's update pass and of the plain axis-0 inverse
 // (disp.cuh).
+#pragma once
+
 #include "disp_launch.cuh"
 
 namespace musg {
@@ -8,14 +10,17 @@ namespace {
 template <typename R, int D, bool FIN>
 void ax0_step(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
               const DispGroup<R> *grp) {
-  if (grp) return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, true>, a, c, B, s, grp);
-  switch (pl.blu ? 0 : pl.m) {
+  if (grp) return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+  if constexpr (sizeof(R) == 4) {
+    switch (disp_fixed_plan(pl)) {
 #define MUSG_C(M, A, BB) \
   case M: return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, A, BB, false>, a, c, B, s);
-    MUSG_DISP_PLANS(MUSG_C)
+      MUSG_DISP_PLANS(MUSG_C)
 #undef MUSG_C
-    default: return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, false>, a, c, B, s);
+      default: break;
+    }
   }
+  disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, false>, a, c, B, s);
 }
 }  // namespace
 
@@ -38,8 +43,9 @@ void disp_ax0_field(const Spectral &sp, bool from_x, const DispArgs<R> &a, const
 #undef MUSG_C
 }
 
-template void disp_ax0_step<float>(const Spectral &, const DispArgs<float> &, const DispShape &, int, cudaStream_t,
-                                   const DispGroup<float> *);
-template void disp_ax0_field<float>(const Spectral &, bool, const DispArgs<float> &, const DispShape &, cudaStream_t);
+#define MUSG_INSTANTIATE_DISP_AX0_INV(R) \
+template void disp_ax0_step<R>(const Spectral &, const DispArgs<R> &, const DispShape &, int, cudaStream_t, \
+                                   const DispGroup<R> *); \
+template void disp_ax0_field<R>(const Spectral &, bool, const DispArgs<R> &, const DispShape &, cudaStream_t);
 
 }  // namespace musg

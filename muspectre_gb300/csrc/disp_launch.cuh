@@ -165,8 +165,12 @@ void disp_launch(K kernel, const DispArgs<R> &a, const DispShape &c, int B, cuda
   MUSG_CHECK_LAUNCH();
 }
 
-// power-of-two axes have kernels with compile-time plans
+// FP32: power-of-two axes have kernels with compile-time plans (0: none).  In FP64 the
+// arithmetic, not the indexing, sets the pace.
 #define MUSG_DISP_PLANS(X) X(32, 8, 4) X(64, 8, 8) X(128, 16, 8) X(256, 16, 16)
+inline int disp_fixed_plan(const TilePlan &pl) { return pl.blu ? 0 : pl.m; }
+// stages of the grouped kernels: inline in FP32, out of line in FP64 (build time)
+template <typename R> constexpr int kGroupPlan = sizeof(R) == 4 ? 0 : -1;
 
 // the passes: of an iteration (solo, batched, or grouped with grp), and the plain ones
 template <typename R>

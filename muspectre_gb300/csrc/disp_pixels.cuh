@@ -11,23 +11,27 @@ template <typename R, int D, bool FIN, int TK>
 void pixels_iteration(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
                       const DispGroup<R> *grp) {
   if (grp) {
-    disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, 0, 0, true>, a, c, B, s, grp);
+    disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
     return;
   }
-  // compile-time plans need the padded pencils (always there at these lengths)
-  switch (pl.blu || c.sh != 4 ? 0 : pl.m) {
+  if constexpr (sizeof(R) == 4) {
+    // compile-time plans need the padded pencils (always there at these lengths)
+    switch (c.sh != 4 ? 0 : disp_fixed_plan(pl)) {
 #define MUSG_PX(M, A, BB) \
   case M: disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, A, BB, false>, a, c, B, s); return;
-    MUSG_DISP_PLANS(MUSG_PX)
+      MUSG_DISP_PLANS(MUSG_PX)
 #undef MUSG_PX
-    default: disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, 0, 0, false>, a, c, B, s);
+      default: break;
+    }
   }
+  disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, 0, 0, false>, a, c, B, s);
 }
 
 }  // namespace
 
-// kernels of their own for the isotropic laws (LE1, LE3, LE4) and the generic small-strain
-// stiffness; the other finite-strain kinds share one that picks per launch
+// kernels of their own for the isotropic laws (LE1, LE3, LE4; FP64 stores S, FP32 rebuilds
+// it) and the generic small-strain stiffness; the other finite-strain kinds share one
+// that picks per launch
 template <typename R, int D>
 void disp_pixels(int tkind, const TilePlan &pl, const DispArgs<R> &a0, const DispShape &c, int B, cudaStream_t s,
                  const DispGroup<R> *grp) {
@@ -36,7 +40,8 @@ void disp_pixels(int tkind, const TilePlan &pl, const DispArgs<R> &a0, const Dis
   switch (tkind) {
     case TK_SMALL: return pixels_iteration<R, D, false, TK_SMALL>(pl, a, c, B, s, grp);
     case TK_GSMALL: return pixels_iteration<R, D, false, TK_GSMALL>(pl, a, c, B, s, grp);
-    case TK_FISO: return pixels_iteration<R, D, true, TK_FISO>(pl, a, c, B, s, grp);
+    case sizeof(R) == 4 ? TK_FISO : TK_FINITE:
+      return pixels_iteration<R, D, true, sizeof(R) == 4 ? TK_FISO : TK_FINITE>(pl, a, c, B, s, grp);
     default: return pixels_iteration<R, D, true, TK_ANYFIN>(pl, a, c, B, s, grp);
   }
 }

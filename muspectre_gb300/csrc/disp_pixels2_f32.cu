@@ -1,4 +1,4 @@
-// The displacement-space CG's pixel pass in 2-D.
+// The displacement-space CG's pixel pass in 2-D, FP32.
 #include "disp_pixels.cuh"
 
 namespace musg {

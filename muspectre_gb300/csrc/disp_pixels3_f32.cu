@@ -1,4 +1,4 @@
-// The displacement-space CG's pixel pass in 3-D.
+// The displacement-space CG's pixel pass in 3-D, FP32.
 #include "disp_pixels.cuh"
 
 namespace musg {

@@ -118,8 +118,9 @@ struct TilePlan {
   int radix[kMaxStages] = {0};
   void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;
   void *tw32 = nullptr, *chirp32 = nullptr, *bf32 = nullptr;
-  // factors only (host); build() also makes the device tables
-  void factor(int n);
+  // factors only (host); build() also makes the device tables.  smallest: the shortest
+  // Bluestein length instead of the cheapest
+  void factor(int n, bool smallest = false);
   void build(int n);
   void release();
   template <typename R> TilePlanD<R> device() const;
@@ -199,20 +200,21 @@ struct Spectral {
   bool allow_even = false;
   double lengths[3] = {1, 1, 1};
   AxisPlan ax[3];
-  TilePlan tp[3];           // the same axes for the displacement-space passes (disp.cu)
+  TilePlan tp[3];           // the same axes for the displacement-space passes (disp.cu), by ensure_tiles
   // per-axis xi_d(k) = fftfreq_d(k)/L_d over the hermitian index range, FP64 and FP32
   void *xi64[3] = {nullptr, nullptr, nullptr};
   void *xi32[3] = {nullptr, nullptr, nullptr};
   void *spec64 = nullptr;   // [ncomp][nk] complex double
   void *spec32 = nullptr;   // [ncomp][nk] complex float
   bool want32 = false;
-  // launch shapes per precision (0: FP64, 1: FP32) and pass (0: last, 1: axis,
-  // 2: green): threads per block and the shared memory a block aims for; set by
-  // the defaults below or by spectral_autotune
+  // launch shapes of the FFT engine's passes per precision (0: FP64, 1: FP32) and pass
+  // (0: last, 1: axis, 2: first axis): threads per block and the shared memory a block
+  // aims for
   int tune_threads[2][3] = {{256, 256, 256}, {256, 256, 256}};
   long tune_bytes[2][3] = {{73728, 49152, 73728}, {73728, 49152, 73728}};
   void init(int dim, const int *res, int ncomp, int proj_kind, const double *lengths,
             bool allow_even, bool want32);
+  void ensure_tiles();
   void ensure32();
   void release();
 };
@@ -230,61 +232,15 @@ constexpr int kPassThreads = 512;
 // Pass launchers (spectral_*.cu).  All run on `stream`.
 //  fwd: real field [ncomp][npx] (scaled) -> spectrum (r2c over all axes)
 //  inv: spectrum -> real field (c2r, unnormalised, scaled)
-//  project: real -> real through the Green operator of sp.proj_kind
 template <typename R>
 void spectral_forward(Spectral &sp, const R *in, R scale, cudaStream_t s);
 template <typename R>
 void spectral_inverse(Spectral &sp, R *out, R scale, cudaStream_t s);
-template <typename R>
-void spectral_project(Spectral &sp, const R *in, R *out, R in_scale, cudaStream_t s);
 
-// CG operator application with the iteration's vector work fused into its passes (FP64,
-// the reference's order): p = -r + beta p (or p = -r on the first iteration), Ap =
-// G(K:p), and alpha = r.r / p.Ap in the state (last block of the last pass); cg_update
-// completes the iteration.  Returns the number of partial sums written by the last
-// pass.  ev (optional): an event is recorded before the first and after every kernel
-template <typename R>
-int cg_operator(Spectral &sp, int tkind, const TangentData<R> &td, const CGState *st,
-                R *r, R *p, R *Ap, double *partial, cudaStream_t s,
-                cudaEvent_t *ev = nullptr);
-// plain operator (no CG state): out = G(K:in)
-template <typename R>
-void tangent_operator(Spectral &sp, int tkind, const TangentData<R> &td, const R *in,
-                      R *out, cudaStream_t s);
-// batched CG operator over B same-shape problems (one launch per pass; problem b
-// is blockIdx.y); tab is a device array of B ProblemPtrs (spectral.cuh), whose host
-// image is ProblemPtrsHost
-template <typename R> struct ProblemPtrs;
-struct ProblemPtrsHost {
-  void *spec;
-  const CGState *st;
-  void *r;
-  void *p;
-  void *Ap;
-  double *partial;
-  unsigned char td[sizeof(TangentData<double>)];
-};
-template <typename R>
-int cg_operator_batch(Spectral &sp, int tkind, const ProblemPtrs<R> *tab, int B, cudaStream_t s);
-// Grouped CG operator over problems of different grids (the same dimension,
-// projection and tangent kind): one launch per pass for all of them, problem b
-// owning a contiguous range of the one-dimensional grid (generic pass kernels, whose
-// plans and sizes are runtime values).  The per-problem arguments live in device
-// tables built once; run launches one CG iteration's passes.
-struct GroupProblem {
-  Spectral *sp;
-  const CGState *st;
-  void *r, *p, *Ap;
-  double *partial;
-  unsigned char td[sizeof(TangentData<double>)];
-};
-struct GroupedOp;
-template <typename R> GroupedOp *grouped_op_create(const std::vector<GroupProblem> &probs, int tkind);
-void grouped_op_destroy(GroupedOp *op);
-template <typename R> void grouped_op_run(GroupedOp *op, cudaStream_t s);
 // ---------------------------------------------------------------- displacement-space CG (disp.cu)
-// The FP32 inner solve of the mixed method (disp.cuh).  A vector in the range of the
-// projection is D complex values per half-spectrum point, [D][nk] float2.
+// The CG solver and the projection (disp.cuh), in FP64 and, for the mixed method's inner
+// solve, in FP32 (R).  A vector in the range of the projection is D complex values per
+// half-spectrum point, [D][disp_nk].
 struct DispVectors {
   void *r = nullptr, *q = nullptr, *p = nullptr, *x = nullptr;
 };
@@ -292,24 +248,36 @@ struct DispVectors {
 // the half spectrum
 inline int disp_nh(const Spectral &sp) { return (sp.g.nlast() + 1) / 2; }
 inline long long disp_nk(const Spectral &sp) { return sp.g.nrows * disp_nh(sp); }
-inline size_t disp_vector_bytes(const Spectral &sp) { return (size_t)disp_nk(sp) * sp.g.dim * sizeof(float2); }
-// rhat (+)= the projection of scale * field (FP64 planes), or with prev of prev - field,
-// after which prev = field; *norm2 = |rhat|^2 (a device double)
-void disp_residual(Spectral &sp, void *rhat, const double *field, double *prev, double scale, bool accumulate,
-                   double *partial, double *norm2, cudaStream_t s);
-// state and vectors of a solve A x = rhat: tol is relative to *rhs2, or to *range2 =
-// |rhat|^2 when rhs2 is null (device doubles); what *rhs2 has beyond *range2 is outside
-// the range of the projection and stays in the residual
+template <typename R> size_t disp_vector_bytes(const Spectral &sp) {
+  return (size_t)disp_nk(sp) * sp.g.dim * 2 * sizeof(R);
+}
+// rhat (+)= the projection of scale * field (FP64 planes), through the tangent unless
+// tkind is TK_PLAIN; or with prev of prev - field, after which prev = field.  *norm2 (may
+// be null) = |rhat|^2, a device double
+template <typename R>
+void disp_residual(Spectral &sp, int tkind, const TangentData<R> &td, void *rhat, const double *field, double *prev,
+                   double scale, bool accumulate, double *partial, double *norm2, cudaStream_t s);
+// state and vectors of a solve A x = rhs for the rhat of its right-hand side, *range2 =
+// |rhat|^2; *out2 (null: 0) is the part of |rhs|^2 outside the range of the projection,
+// which stays in the residual (device doubles)
+template <typename R>
 void disp_start(Spectral &sp, const DispVectors &v, const void *rhat, CGState *st, double tol, int maxiter,
-                const double *rhs2, const double *range2, cudaStream_t s);
+                const double *out2, const double *range2, cudaStream_t s);
 // one CG iteration: five passes (3-D) or three (2-D)
-void disp_iteration(Spectral &sp, int tkind, const TangentData<float> &td, const DispVectors &v, CGState *st,
+template <typename R>
+void disp_iteration(Spectral &sp, int tkind, const TangentData<R> &td, const DispVectors &v, CGState *st,
                     double *partial, cudaStream_t s, cudaEvent_t *ev = nullptr);
 // the solution of the state's solve as real component planes
-void disp_solution(Spectral &sp, const DispVectors &v, CGState *st, float *x, cudaStream_t s);
-// out = G(K:in) of a real field (FP64 planes in, FP32 out); qhat: one vector of scratch
-void disp_operator(Spectral &sp, int tkind, const TangentData<float> &td, const double *in, void *qhat, float *out,
-                   double *partial, cudaStream_t s);
+template <typename R>
+void disp_solution(Spectral &sp, const DispVectors &v, CGState *st, R *x, cudaStream_t s);
+// the real field of a vector
+template <typename R> void disp_field(Spectral &sp, void *qhat, R *out, cudaStream_t s);
+// out = G(K:in) of a real field (FP64 planes in), without the tangent when tkind is
+// TK_PLAIN; in and out may be the same
+template <typename R>
+void disp_operator(Spectral &sp, int tkind, const TangentData<R> &td, const double *in, R *out, cudaStream_t s);
+// an FP64 vector in FP32
+void disp_convert(const Spectral &sp, const void *v64, void *v32, cudaStream_t s);
 // iterations of several problems per launch: of one grid (the solo kernels, problem =
 // blockIdx.y), or of different grids (each owning a range of the blocks)
 struct DispProblem {
@@ -317,41 +285,21 @@ struct DispProblem {
   DispVectors v;
   CGState *st;
   double *partial;
-  TangentData<float> td;
+  TangentData<float> td32;
+  TangentData<double> td64;
 };
 struct DispBatch;
-DispBatch *disp_batch_create(const std::vector<DispProblem> &probs, int tkind, bool uniform);
+DispBatch *disp_batch_create(const std::vector<DispProblem> &probs, int tkind, bool uniform, bool fp64);
 void disp_batch_destroy(DispBatch *b);
 void disp_batch_run(DispBatch *b, cudaStream_t s);
-// Times candidate launch shapes of each pass on this grid (CUDA events) and keeps
-// the fastest (FFT_PlanFlags::measure / patient); fp32 selects the FP32 passes.
-template <typename R> void spectral_autotune(Spectral &sp, cudaStream_t s, int effort);
 
 // ---------------------------------------------------------------- CG kernels (cg.cu)
 int reduce_blocks(long long n);
 // per-component means of a field [ncomp][npx] into out[ncomp] (device); partial
 // holds ncomp * 1024 doubles
 void plane_means(const double *f, int ncomp, long long npx, double *partial, double *out, cudaStream_t s);
-// blocks (= partial sums) of cg_update / cg_update_batch for n entries
-int update_blocks(long long n);
-template <typename R>
-void cg_init(CGState *st, const double *rhs, R *r, R *x, long long n, double tol,
-             int maxiter, double *partial, double *partial2, cudaStream_t s);
-template <typename R>
-void cg_update(CGState *st, R *x, R *r, const R *p, const R *Ap, long long n,
-               double *partial, cudaStream_t s);
-// batched variants: per-problem pointer tables (device arrays of B entries)
-template <typename R> struct BatchVec {
-  CGState *st;
-  R *x;
-  R *r;
-  const R *p;
-  const R *Ap;
-  double *partial;
-  long long n;  // entries of the problem's vectors
-};
-template <typename R>
-void cg_update_batch(const BatchVec<R> *tab, long long n, int B, cudaStream_t s);
+// sum of (a - b)^2 over n entries into *out (device)
+void diff2_device(const double *a, const double *b, long long n, double *partial, double *out, cudaStream_t s);
 // FP64 dot of a with b over n entries into *out_device (deterministic)
 template <typename Ra, typename Rb>
 void dot_device(const Ra *a, const Rb *b, long long n, double *partial, double *out,

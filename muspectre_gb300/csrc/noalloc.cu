@@ -60,39 +60,6 @@ void *scratch_address() {
   return g_noalloc_addr[dev];
 }
 
-// radices of a 2/3/5/7-smooth length (the policy of the allocating plans); false
-// when another prime divides n
-bool factor_fixed(int n, int *rad, int &nst) {
-  nst = 0;
-  int k = 0;
-  while (n % 2 == 0) { n /= 2; ++k; }
-  auto push = [&](int r) {
-    if (nst < kMaxStages) rad[nst] = r;
-    ++nst;
-  };
-  while (k > 0) {
-    if (k >= 4 && k != 5 && k != 6) { push(16); k -= 4; }
-    else if (k == 6) { push(8); push(8); k = 0; }
-    else if (k == 5) { push(8); push(4); k = 0; }
-    else if (k == 3) { push(8); k = 0; }
-    else if (k == 2) { push(4); k = 0; }
-    else { push(2); k = 0; }
-  }
-  while (n % 9 == 0) { push(9); n /= 9; }
-  for (int r : {3, 5, 7})
-    while (n % r == 0) { push(r); n /= r; }
-  return n == 1 && nst <= kMaxStages;
-}
-
-int smooth_ge(int v) {
-  for (int m = v;; ++m) {
-    int t = m;
-    for (int r : {2, 3, 5, 7})
-      while (t % r == 0) t /= r;
-    if (t == 1) return m;
-  }
-}
-
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 // twiddles exp(-2 pi i j/m), Bluestein chirp exp(-pi i (j^2 mod 2n)/n) and the wave
@@ -193,16 +160,9 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
   off += align256((size_t)sp.ncomp * sp.g.nk * sizeof(double2));
   size_t off_tw[3], off_chirp[3], off_bf[3], off_xi[3];
   for (int d = 0; d < dim; ++d) {
-    AxisPlan &ap = sp.ax[d];
-    ap.n = sp.g.n[d];
-    if (factor_fixed(ap.n, ap.radix, ap.nst)) {
-      ap.blu = 0;
-      ap.m = ap.n;
-    } else {
-      ap.blu = 1;
-      ap.m = smooth_ge(2 * ap.n - 1);
-      if (!factor_fixed(ap.m, ap.radix, ap.nst)) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
-    }
+    TilePlan &ap = sp.tp[d];
+    ap.factor(sp.g.n[d], true);
+    if (!ap.m) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
     off_tw[d] = off;
     off += align256((size_t)ap.m * sizeof(double2));
     off_chirp[d] = off;
@@ -221,7 +181,7 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
   double *soa = reinterpret_cast<double *>(base + off_soa);
   sp.spec64 = base + off_spec;
   for (int d = 0; d < dim; ++d) {
-    AxisPlan &ap = sp.ax[d];
+    TilePlan &ap = sp.tp[d];
     ap.tw64 = base + off_tw[d];
     ap.chirp64 = ap.blu ? base + off_chirp[d] : nullptr;
     ap.bf64 = ap.blu ? base + off_bf[d] : nullptr;
@@ -238,7 +198,7 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
     }
   }
   aos_to_soa(in_device, soa, sp.ncomp, sp.g.npx, s);
-  spectral_project<double>(sp, soa, soa, 1.0, s);
+  disp_operator<double>(sp, TK_PLAIN, {}, soa, soa, s);
   soa_to_aos(soa, out_device, sp.ncomp, sp.g.npx, s);
 }
 

@@ -193,11 +193,12 @@ double stage_cost(int r) {
   return c[r] + 4.0;  // + twiddles and a shared-memory round trip
 }
 
-// the cheapest factorisation of m into radices 2..17: two factors if there are any,
-// else the fewest; false when a prime above 17 divides m
-bool tile_factor(int m, std::vector<int> &rad, double &cost) {
-  rad.clear();
+// the cheapest factorisation of m into radices up to 17 (no heap: the allocation-free
+// projection plans with it): two factors (r1 >= r2, possibly 1) if there are any, else the
+// fewest; the number of factors in rad, 0 when a prime above 17 divides m
+int tile_factor(int m, int *rad, double &cost) {
   cost = 1e30;
+  int n = 0;
   for (int a = 1; a <= 17; ++a)
     if (m % a == 0 && m / a <= 17) {
       const int b = m / a;
@@ -205,59 +206,59 @@ bool tile_factor(int m, std::vector<int> &rad, double &cost) {
       const double c = (a > 1 ? stage_cost(a) : 0.0) + (b > 1 ? stage_cost(b) : 0.0);
       if (c < cost) {
         cost = c;
-        rad = {b, a};  // r1 >= r2
+        rad[0] = b;
+        rad[1] = a;
+        n = 2;
       }
     }
-  if (!rad.empty()) return true;
-  // three or more: peel the largest factor that leaves the cheapest rest
+  if (n) return n;
+  // three or more: peel the factor that leaves the cheapest rest
   for (int a = 17; a >= 2; --a) {
     if (m % a) continue;
-    std::vector<int> rest;
+    int rest[kMaxStages];
     double c = 0;
-    if (!tile_factor(m / a, rest, c)) continue;
-    rest.erase(std::remove(rest.begin(), rest.end(), 1), rest.end());
-    if (c + stage_cost(a) + 1.0 < cost) {
-      cost = c + stage_cost(a) + 1.0;
-      rad.assign(1, a);
-      rad.insert(rad.end(), rest.begin(), rest.end());
-    }
+    int k = tile_factor(m / a, rest, c);
+    if (k == 2 && rest[1] == 1) k = 1;
+    if (k == 0 || k + 1 > kMaxStages || c + stage_cost(a) + 1.0 >= cost) continue;
+    cost = c + stage_cost(a) + 1.0;
+    rad[0] = a;
+    for (int q = 0; q < k; ++q) rad[q + 1] = rest[q];
+    n = k + 1;
   }
-  return !rad.empty();
+  return n;
 }
 
 }  // namespace
 
-void TilePlan::factor(int n_) {
+void TilePlan::factor(int n_, bool smallest) {
   n = n_;
-  m = nst = r1 = r2 = 0;
+  m = nst = r1 = r2 = blu = 0;
   if (n > (1 << 16)) return;  // longer than any tile: the passes refuse it (m = 0)
-  std::vector<int> rad;
   double cost = 0;
-  if (tile_factor(n, rad, cost)) {
-    blu = 0;
+  if ((nst = tile_factor(n, radix, cost))) {
     m = n;
   } else {
     // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass
     blu = 1;
     double best = 1e30;
-    std::vector<int> r;
     for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
+      int rad[kMaxStages];
       double c = 0;
-      if (!tile_factor(k, r, c)) continue;
+      const int ns = tile_factor(k, rad, c);
+      if (!ns) continue;
+      if (smallest && m) break;
       c *= k;
       if (c < best) {
         best = c;
         m = k;
-        rad = r;
+        nst = ns;
+        for (int q = 0; q < ns; ++q) radix[q] = rad[q];
       }
     }
-    if (best > 1e29) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
+    if (!m) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
   }
-  nst = (int)rad.size();
-  if (nst > kMaxStages) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
-  for (int s = 0; s < nst; ++s) radix[s] = rad[s];
-  r1 = nst == 2 ? rad[0] : 0;
-  r2 = nst == 2 ? rad[1] : 0;
+  r1 = nst == 2 ? radix[0] : 0;
+  r2 = nst == 2 ? radix[1] : 0;
 }
 
 void TilePlan::build(int n_) {
@@ -333,10 +334,14 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
   if (want32) ensure32();
 }
 
-void Spectral::ensure32() {
-  want32 = true;
+void Spectral::ensure_tiles() {
   for (int d = 0; d < g.dim; ++d)
     if (tp[d].n != g.n[d]) tp[d].build(g.n[d]);
+}
+
+void Spectral::ensure32() {
+  want32 = true;
+  ensure_tiles();
   if (!spec32) MUSG_CUDA(cudaMalloc(&spec32, (size_t)ncomp * g.nk * sizeof(float2)));
 }
 

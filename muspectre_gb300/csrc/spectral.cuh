@@ -1,36 +1,18 @@
-// Spectral passes of the FFT-Galerkin operator (device code + launchers).
+// Passes of the FFT engine, tangents and block reductions (device code).
 //
 // A real field is stored as component planes [c][pixel] (pixels row-major, last
 // index fastest); its half spectrum as [c][k] complex with the last axis halved to
-// n/2+1.  One transform = one pass per axis:
-//
-//   last axis   (pass "last"):  r2c / c2r of rows, two real rows packed into one
-//                               complex FFT (x + i y); fused prologue / epilogue
-//                               (tangent K:dF, CG vector updates, dot products)
-//   middle axis (pass "axis"):  c2c of strided pencils, 3-D only
-//   first axis  (pass "green"): c2c of strided pencils with all components of a
-//                               k-point in one block, so that the Green operator
-//                               (projection_small_strain.cc:56-86,
-//                               projection_finite_strain_fast.cc:61-87) is applied
-//                               between the forward and the inverse transform.
-//
-// The CG operator of one iteration is therefore: last(fwd, prologue) -> axis(fwd)
-// -> green -> axis(inv) -> last(inv, epilogue), the projection of
-// src/fft/projection_default.cc:54-63 with the tangent contraction of
-// src/cell/cell_base.cc:182-188 fused into the first pass.
+// n/2+1.  One transform = one pass per axis: the last axis r2c / c2r, two real rows packed
+// into one complex FFT (x + i y), then c2c of strided pencils along the others.
+// These passes serve the FFT engine; the projection and the CG operator run in
+// displacement space (disp.cuh), which takes the tangents and reductions from here.
 #pragma once
 
 #include "fft_device.cuh"
 
 namespace musg {
 
-// PRO_CG / EPI_CG: the reference's CG iteration (solver_cg.cc:76-97) split over the
-// passes: the last pass writes Ap and finishes alpha = r.r / p.Ap, and cg_update then
-// applies x += alpha p, r += alpha Ap and finishes beta.  (The FP32 inner solve of the
-// mixed method runs in displacement space, disp.cuh.)
-enum Prologue : int { PRO_PLAIN = 0, PRO_TANGENT = 1, PRO_CG = 2 };
-enum Epilogue : int { EPI_PLAIN = 0, EPI_CG = 1 };
-enum GreenMode : int { GM_SMALL = 0, GM_FINITE = 1, GM_FWD = 2, GM_INV = 3 };
+enum GreenMode : int { GM_FWD = 2, GM_INV = 3 };  // the FFT engine's first-axis pass
 
 // independent global loads each thread keeps in flight in the staging loops
 constexpr int kLoadBatch = 8;
@@ -85,8 +67,8 @@ __device__ __forceinline__ double block_sum(double v) {
 
 // ------------------------------------------------------------ CG scalar steps
 // The kernel that produces a dot product's partial sums also finishes it: every block
-// writes partial[blockIdx.x], and the block that finishes last (counted with the
-// state's ticket) sums all gridDim.x partials in a fixed order and updates the state.
+// writes its partial sums, and the block that finishes last (counted with the state's
+// ticket) sums them all in a fixed order and updates the state.
 // Deterministic like a separate reduction kernel, without its launch.
 __device__ __forceinline__ int lin_tid() { return threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z); }
 __device__ __forceinline__ int lin_nth() { return blockDim.x * blockDim.y * blockDim.z; }
@@ -103,7 +85,6 @@ __device__ __forceinline__ bool cg_last_block(CGState *st, int nblk) {
   __syncthreads();
   return last != 0;
 }
-__device__ __forceinline__ bool cg_last_block(CGState *st) { return cg_last_block(st, (int)gridDim.x); }
 
 // Grouped launches: problems of different grids in one launch, the blocks of problem b
 // being [blk0[b], blk0[b+1]) of a one-dimensional grid; b by binary search
@@ -115,49 +96,6 @@ __device__ __forceinline__ int group_problem(const int *blk0, int B) {
     else hi = mid;
   }
   return lo;
-}
-
-__device__ __forceinline__ double sum_partials_fresh(const double *partial, int n) {
-  // eight independent loads in flight per thread; each thread still adds its entries
-  // in index order, so the sum is the same as one load at a time (tens of thousands of
-  // per-warp partials took one 1024-thread block 11.5 us, serialised on L2 latency)
-  const int nth = lin_nth();
-  int i = lin_tid();
-  double v = 0.0;
-  for (; i + 7 * nth < n; i += 8 * nth) {
-    double t[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) t[u] = __ldcg(partial + i + u * nth);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v += t[u];
-  }
-  for (; i < n; i += nth) v += __ldcg(partial + i);
-  return block_sum(v);
-}
-
-// alpha = r.r / p.Ap (solver_cg.cc:81)
-__device__ __forceinline__ void cg_alpha_step(CGState *st, const double *partial, int n) {
-  const double pAp = sum_partials_fresh(partial, n);
-  if (lin_tid() == 0) {
-    st->pAp = pAp;
-    st->alpha = st->rdr / pAp;
-    st->ticket = 0;
-  }
-}
-
-// beta = new r.r / old r.r (solver_cg.cc:86-88) and the loop condition of the next
-// iteration; a non-finite residual fails the comparison and ends the loop, as in the
-// reference
-__device__ __forceinline__ void cg_beta_step(CGState *st, const double *partial, int n) {
-  const double nr = sum_partials_fresh(partial, n);
-  if (lin_tid() == 0) {
-    st->beta = nr / st->rdr;
-    st->rdr = nr;
-    st->iter += 1;
-    st->counter += 1;
-    if (!(st->iter < st->maxiter && st->rdr > st->tol2)) st->active = 0;
-    st->ticket = 0;
-  }
 }
 
 // ------------------------------------------------------------ tangents
@@ -390,18 +328,7 @@ template <int D, int TK, typename R> struct TangentLocal {
 };
 
 // ------------------------------------------------------------ pass "last"
-// Per-problem pointers of a batched launch: problem b = blockIdx.y of a grid that
-// covers a batch of same-shape RVEs (or right-hand sides) in one launch per stage.
-template <typename R> struct ProblemPtrs {
-  typename V2<R>::T *spec;
-  const CGState *st;
-  R *r;
-  R *p;
-  R *Ap;
-  double *partial;
-  TangentData<R> td;
-};
-
+// real rows <-> half spectra of the FFT engine
 template <typename R> struct LastArgs {
   AxisPlanD<R> ap;
   int L, H, G, ncomp;
@@ -410,104 +337,41 @@ template <typename R> struct LastArgs {
   const R *in;
   R *out;
   R scale;
-  const CGState *st;
-  R *r;
-  R *p;
-  R *Ap;
-  double *partial;
-  TangentData<R> td;
-  const ProblemPtrs<R> *batch;  // null: a single problem
-  __device__ __forceinline__ void bind() {
-    if (!batch) return;
-    const ProblemPtrs<R> &q = batch[blockIdx.y];
-    spec = q.spec;
-    st = q.st;
-    r = q.r;
-    p = q.p;
-    Ap = q.Ap;
-    partial = q.partial;
-    td = q.td;
-  }
 };
 
-// forward: real rows -> half spectra.  D is the tensor dimension for the tangent
-// prologues (0 for PRO_PLAIN).  bid: this block among the problem's blocks.
-template <typename R, int PRO, int D, int TK>
+// forward: real rows -> half spectra.  bid: this block among the blocks.
+template <typename R>
 __device__ __forceinline__ void last_fwd_body(const LastArgs<R> &a, long long bid) {
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *buf = reinterpret_cast<T *>(smem_raw);
-  constexpr bool kCG = PRO == PRO_CG;
-  if (kCG && !a.st->active) return;
   const int L = a.L, G = a.G, nc = a.ncomp, G2 = G >> 1;
   const int P = nc * G2;
   T *buf2 = buf + (size_t)P * a.ap.m;
   const long long row0 = bid * G;
   R *bufr = reinterpret_cast<R *>(buf);
   const FDiv fGL(G * L), fL(L);
-  if constexpr (PRO == PRO_PLAIN) {
-    const int total = nc * G * L;
-    for (int i0 = threadIdx.x; i0 < total; i0 += kLoadBatch * blockDim.x) {
-      R v[kLoadBatch];
-      int dst[kLoadBatch];
+  const int total = nc * G * L;
+  for (int i0 = threadIdx.x; i0 < total; i0 += kLoadBatch * blockDim.x) {
+    R v[kLoadBatch];
+    int dst[kLoadBatch];
 #pragma unroll
-      for (int u = 0; u < kLoadBatch; ++u) {
-        const int idx = i0 + u * blockDim.x;
-        dst[u] = -1;
-        v[u] = R(0);
-        if (idx < total) {
-          int rem, e;
-          const int c = fGL.div(idx, rem);
-          const int g = fL.div(rem, e);
-          const long long row = row0 + g;
-          if (row < a.nrows) v[u] = a.in[(long long)c * a.npx + row * L + e];
-          dst[u] = 2 * (e * P + c * G2 + (g >> 1)) + (g & 1);
-        }
+    for (int u = 0; u < kLoadBatch; ++u) {
+      const int idx = i0 + u * blockDim.x;
+      dst[u] = -1;
+      v[u] = R(0);
+      if (idx < total) {
+        int rem, e;
+        const int c = fGL.div(idx, rem);
+        const int g = fL.div(rem, e);
+        const long long row = row0 + g;
+        if (row < a.nrows) v[u] = a.in[(long long)c * a.npx + row * L + e];
+        dst[u] = 2 * (e * P + c * G2 + (g >> 1)) + (g & 1);
       }
-#pragma unroll
-      for (int u = 0; u < kLoadBatch; ++u)
-        if (dst[u] >= 0) bufr[dst[u]] = v[u] * a.scale;
     }
-  } else {
-    constexpr int D2 = D * D;
-    const bool first = kCG ? (a.st->iter == 0) : false;
-    const R beta = kCG ? R(a.st->beta) : R(0);
-    for (int idx = threadIdx.x; idx < G * L; idx += blockDim.x) {
-      int e;
-      const int g = fL.div(idx, e);
-      const long long row = row0 + g;
-      R out[D2];
-      if (row < a.nrows) {
-        const long long px = row * L + e;
-        R v[D2];
-        TangentLocal<D, TK, R> tl;
-        if (kCG) {
-          R rv[D2], pv[D2];
 #pragma unroll
-          for (int c = 0; c < D2; ++c) {
-            const long long o = (long long)c * a.npx + px;
-            rv[c] = a.r[o];
-            pv[c] = first ? R(0) : a.p[o];
-          }
-          tl.load(a.td, px, a.npx);
-#pragma unroll
-          for (int c = 0; c < D2; ++c) {
-            v[c] = first ? -rv[c] : -rv[c] + beta * pv[c];
-            a.p[(long long)c * a.npx + px] = v[c];
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < D2; ++c) v[c] = a.in[(long long)c * a.npx + px];
-          tl.load(a.td, px, a.npx);
-        }
-        tl.apply(v, out);
-      } else {
-#pragma unroll
-        for (int c = 0; c < D2; ++c) out[c] = R(0);
-      }
-#pragma unroll
-      for (int c = 0; c < D2; ++c) bufr[2 * (e * P + c * G2 + (g >> 1)) + (g & 1)] = out[c];
-    }
+    for (int u = 0; u < kLoadBatch; ++u)
+      if (dst[u] >= 0) bufr[dst[u]] = v[u] * a.scale;
   }
   __syncthreads();
   const T *res = fft_run<R, false>(buf, buf2, P, a.ap);
@@ -530,30 +394,18 @@ __device__ __forceinline__ void last_fwd_body(const LastArgs<R> &a, long long bi
   }
 }
 
-template <typename R, int PRO, int D, int TK>
-__global__ void __launch_bounds__(kPassThreads) k_last_fwd(const LastArgs<R> a0) {
+template <typename R>
+__global__ void __launch_bounds__(kPassThreads) k_last_fwd(const LastArgs<R> a) {
   dep_wait();
-  LastArgs<R> a = a0;
-  a.bind();
-  last_fwd_body<R, PRO, D, TK>(a, blockIdx.x);
+  last_fwd_body<R>(a, blockIdx.x);
 }
 
-template <typename R, int PRO, int D, int TK>
-__global__ void __launch_bounds__(kPassThreads) k_last_fwd_g(const LastArgs<R> *tab, const int *blk0, int B) {
-  dep_wait();
-  const int b = group_problem(blk0, B);
-  const LastArgs<R> a = tab[b];
-  last_fwd_body<R, PRO, D, TK>(a, blockIdx.x - blk0[b]);
-}
-
-// inverse: half spectra -> real rows.  PLAIN writes out = scale*x; CG writes Ap
-// and the block sums of p.Ap.
-template <typename R, int EPI, int D>
-__device__ __forceinline__ void last_inv_body(const LastArgs<R> &a, long long bid, int nblk) {
+// inverse: half spectra -> real rows, out = scale*x
+template <typename R>
+__device__ __forceinline__ void last_inv_body(const LastArgs<R> &a, long long bid) {
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *buf = reinterpret_cast<T *>(smem_raw);
-  if (EPI != EPI_PLAIN && !a.st->active) return;
   const int L = a.L, G = a.G, nc = a.ncomp, G2 = G >> 1, H = a.H;
   const int P = nc * G2;
   T *buf2 = buf + (size_t)P * a.ap.m;
@@ -594,52 +446,19 @@ __device__ __forceinline__ void last_inv_body(const LastArgs<R> &a, long long bi
   }
   __syncthreads();
   const R *bufr = reinterpret_cast<const R *>(fft_run<R, true>(buf, buf2, P, a.ap));
-  if constexpr (EPI == EPI_PLAIN) {
-    for (int idx = threadIdx.x; idx < nc * G * L; idx += blockDim.x) {
-      int rem, e;
-      const int c = fGL.div(idx, rem);
-      const int g = fL.div(rem, e);
-      const long long row = row0 + g;
-      if (row < a.nrows) a.out[(long long)c * a.npx + row * L + e] = a.scale * bufr[2 * (e * P + c * G2 + (g >> 1)) + (g & 1)];
-    }
-  } else {
-    constexpr int D2 = D * D;
-    Acc<R> acc;
-    for (int idx = threadIdx.x; idx < G * L; idx += blockDim.x) {
-      int e;
-      const int g = fL.div(idx, e);
-      const long long row = row0 + g;
-      if (row >= a.nrows) continue;
-      const long long px = row * L + e;
-#pragma unroll
-      for (int c = 0; c < D2; ++c) {
-        const R v = bufr[2 * (e * P + c * G2 + (g >> 1)) + (g & 1)];
-        const long long o = (long long)c * a.npx + px;
-        a.Ap[o] = v;
-        acc.add(a.p[o] * v);
-      }
-    }
-    const double bs = block_sum(acc.value());
-    if (threadIdx.x == 0) a.partial[bid] = bs;
-    CGState *st = const_cast<CGState *>(a.st);
-    if (cg_last_block(st, nblk)) cg_alpha_step(st, a.partial, nblk);
+  for (int idx = threadIdx.x; idx < nc * G * L; idx += blockDim.x) {
+    int rem, e;
+    const int c = fGL.div(idx, rem);
+    const int g = fL.div(rem, e);
+    const long long row = row0 + g;
+    if (row < a.nrows) a.out[(long long)c * a.npx + row * L + e] = a.scale * bufr[2 * (e * P + c * G2 + (g >> 1)) + (g & 1)];
   }
 }
 
-template <typename R, int EPI, int D>
-__global__ void __launch_bounds__(kPassThreads) k_last_inv(const LastArgs<R> a0) {
+template <typename R>
+__global__ void __launch_bounds__(kPassThreads) k_last_inv(const LastArgs<R> a) {
   dep_wait();
-  LastArgs<R> a = a0;
-  a.bind();
-  last_inv_body<R, EPI, D>(a, blockIdx.x, (int)gridDim.x);
-}
-
-template <typename R, int EPI, int D>
-__global__ void __launch_bounds__(kPassThreads) k_last_inv_g(const LastArgs<R> *tab, const int *blk0, int B) {
-  dep_wait();
-  const int b = group_problem(blk0, B);
-  const LastArgs<R> a = tab[b];
-  last_inv_body<R, EPI, D>(a, blockIdx.x - blk0[b], blk0[b + 1] - blk0[b]);
+  last_inv_body<R>(a, blockIdx.x);
 }
 
 // ------------------------------------------------------------ pass "axis"
@@ -648,8 +467,6 @@ template <typename R> struct AxisArgs {
   int nax, T, ntiles;
   long long se, inner, sb;
   typename V2<R>::T *spec;
-  const CGState *st;
-  const ProblemPtrs<R> *batch;
 };
 
 template <typename R, bool INV>
@@ -657,7 +474,6 @@ __device__ __forceinline__ void axis_body(const AxisArgs<R> &a, long long bid) {
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *buf = reinterpret_cast<T *>(smem_raw);
-  if (a.st && !a.st->active) return;
   const int tile = (int)(bid % a.ntiles);
   const long long batch = bid / a.ntiles;
   const int Tt = a.T;
@@ -696,105 +512,29 @@ __device__ __forceinline__ void axis_body(const AxisArgs<R> &a, long long bid) {
 }
 
 template <typename R, bool INV>
-__global__ void __launch_bounds__(kPassThreads) k_axis(const AxisArgs<R> a0) {
+__global__ void __launch_bounds__(kPassThreads) k_axis(const AxisArgs<R> a) {
   dep_wait();
-  AxisArgs<R> a = a0;
-  if (a0.batch) {
-    a.spec = a0.batch[blockIdx.y].spec;
-    a.st = a0.batch[blockIdx.y].st;
-  }
   axis_body<R, INV>(a, blockIdx.x);
 }
 
-template <typename R, bool INV>
-__global__ void __launch_bounds__(kPassThreads) k_axis_g(const AxisArgs<R> *tab, const int *blk0, int B) {
-  dep_wait();
-  const int b = group_problem(blk0, B);
-  const AxisArgs<R> a = tab[b];
-  axis_body<R, INV>(a, blockIdx.x - blk0[b]);
-}
-
-// ------------------------------------------------------------ Green operators
 // 1 / sqrt(n2): FP64 correctly rounded division of the square root (parity path);
 // FP32 the rsqrtf intrinsic (2 ulp, far inside the FP32 operator's rounding)
 __device__ __forceinline__ double inv_sqrt(double n2) { return 1.0 / sqrt(n2); }
 __device__ __forceinline__ float inv_sqrt(float n2) { return rsqrtf(n2); }
 
-// unit wave vector of k-point (xi0[e], xi1[k1], xi2[k2]); false where the operator
-// is zero (the zero mode, and every Nyquist index under the even-grid extension)
-template <int D, typename R>
-__device__ __forceinline__ bool unit_xi(R *xi, int e, int k1, int k2, int nyq0, int nyq1, int nyq2) {
-  if ((e == 0 && k1 == 0 && k2 == 0) || e == nyq0 || k1 == nyq1 || (D == 3 && k2 == nyq2)) return false;
-  R n2 = R(0);
-#pragma unroll
-  for (int d = 0; d < D; ++d) n2 += xi[d] * xi[d];
-  const R inv = inv_sqrt(n2);
-#pragma unroll
-  for (int d = 0; d < D; ++d) xi[d] *= inv;
-  return true;
-}
-
-// finite strain, one row i of f: f_i. <- (f_i. xi) xi^T / N
-// (projection_finite_strain_fast.cc:79-85)
-template <int D, typename T, typename R>
-__device__ __forceinline__ void green_finite_row(T *row, const R *xi, R norm) {
-  T fx = T{R(0), R(0)};
-#pragma unroll
-  for (int j = 0; j < D; ++j) {
-    fx.x += row[j].x * xi[j];
-    fx.y += row[j].y * xi[j];
-  }
-#pragma unroll
-  for (int j = 0; j < D; ++j) row[j] = T{fx.x * xi[j] * norm, fx.y * xi[j] * norm};
-}
-
-// small strain: Ghat f = 1/2 (xi a^T + a xi^T) - xi xi^T (xi^T f xi) with a = (f + f^T) xi,
-// the contraction of the operator of projection_small_strain.cc:64-77 with f, / N
-template <int D, typename T, typename R>
-__device__ __forceinline__ void green_small(const T *f, T *o, const R *xi, R norm) {
-  T av[D];
-  T s = T{R(0), R(0)};
-#pragma unroll
-  for (int i = 0; i < D; ++i) {
-    T v = T{R(0), R(0)};
-#pragma unroll
-    for (int j = 0; j < D; ++j) {
-      v.x += (f[i + D * j].x + f[j + D * i].x) * xi[j];
-      v.y += (f[i + D * j].y + f[j + D * i].y) * xi[j];
-      s.x += xi[i] * f[i + D * j].x * xi[j];
-      s.y += xi[i] * f[i + D * j].y * xi[j];
-    }
-    av[i] = v;
-  }
-#pragma unroll
-  for (int j = 0; j < D; ++j)
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      const R xx = xi[i] * xi[j];
-      o[i + D * j] = T{(R(0.5) * (xi[i] * av[j].x + av[i].x * xi[j]) - xx * s.x) * norm,
-                       (R(0.5) * (xi[i] * av[j].y + av[i].y * xi[j]) - xx * s.y) * norm};
-    }
-}
-
-// ------------------------------------------------------------ pass "green"
+// ------------------------------------------------------------ pass "first axis"
 template <typename R> struct GreenArgs {
   AxisPlanD<R> ap;
-  int n0, T, ncomp, n1, nh;
+  int n0, T, ncomp;
   long long Rr, nk;
   typename V2<R>::T *spec;
-  const R *xi0, *xi1, *xi2;
-  int nyq0, nyq1, nyq2;
-  R norm;
-  const CGState *st;
-  const ProblemPtrs<R> *batch;
 };
 
-template <typename R, int MODE, int D>
+template <typename R, int MODE>
 __device__ __forceinline__ void green_body(const GreenArgs<R> &a, long long bid) {
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *buf = reinterpret_cast<T *>(smem_raw);
-  if (a.st && !a.st->active) return;
   const int Tt = a.T, nc = a.ncomp, n0 = a.n0;
   const int P = nc * Tt;
   T *buf2 = buf + (size_t)P * a.ap.m;
@@ -825,51 +565,6 @@ __device__ __forceinline__ void green_body(const GreenArgs<R> &a, long long bid)
   __syncthreads();
   T *cur = buf;
   if (MODE != GM_INV) cur = fft_run<R, false>(buf, buf2, P, a.ap);
-  if constexpr (MODE == GM_SMALL || MODE == GM_FINITE) {
-    constexpr int D2 = D * D;
-    const FDiv fnh(a.nh);
-    for (int idx = threadIdx.x; idx < n0 * Tt; idx += blockDim.x) {
-      int t;
-      const int e = fT.div(idx, t);
-      const long long rho = rho0 + t;
-      if (rho >= a.Rr) continue;
-      int k1, k2 = 0;
-      if (D == 3) {
-        k1 = fnh.div((int)rho, k2);
-      } else {
-        k1 = (int)rho;
-      }
-      R xi[D];
-      xi[0] = a.xi0[e];
-      xi[1] = a.xi1[k1];
-      if (D == 3) xi[D - 1] = a.xi2[k2];
-      T f[D2];
-#pragma unroll
-      for (int c = 0; c < D2; ++c) f[c] = cur[e * P + c * Tt + t];
-      T o[D2];
-      if (!unit_xi<D>(xi, e, k1, k2, a.nyq0, a.nyq1, a.nyq2)) {
-#pragma unroll
-        for (int c = 0; c < D2; ++c) o[c] = T{R(0), R(0)};
-      } else {
-        if (MODE == GM_FINITE) {
-#pragma unroll
-          for (int i = 0; i < D; ++i) {
-            T row[D];
-#pragma unroll
-            for (int j = 0; j < D; ++j) row[j] = f[i + D * j];
-            green_finite_row<D>(row, xi, a.norm);
-#pragma unroll
-            for (int j = 0; j < D; ++j) o[i + D * j] = row[j];
-          }
-        } else {
-          green_small<D>(f, o, xi, a.norm);
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < D2; ++c) cur[e * P + c * Tt + t] = o[c];
-    }
-    __syncthreads();
-  }
   if (MODE != GM_FWD) cur = fft_run<R, true>(cur, cur == buf ? buf2 : buf, P, a.ap);
   for (int idx = threadIdx.x; idx < nc * n0 * Tt; idx += blockDim.x) {
     int t, e;
@@ -880,23 +575,10 @@ __device__ __forceinline__ void green_body(const GreenArgs<R> &a, long long bid)
   }
 }
 
-template <typename R, int MODE, int D>
-__global__ void __launch_bounds__(kPassThreads) k_green(const GreenArgs<R> a0) {
+template <typename R, int MODE>
+__global__ void __launch_bounds__(kPassThreads) k_green(const GreenArgs<R> a) {
   dep_wait();
-  GreenArgs<R> a = a0;
-  if (a0.batch) {
-    a.spec = a0.batch[blockIdx.y].spec;
-    a.st = a0.batch[blockIdx.y].st;
-  }
-  green_body<R, MODE, D>(a, blockIdx.x);
-}
-
-template <typename R, int MODE, int D>
-__global__ void __launch_bounds__(kPassThreads) k_green_g(const GreenArgs<R> *tab, const int *blk0, int B) {
-  dep_wait();
-  const int b = group_problem(blk0, B);
-  const GreenArgs<R> a = tab[b];
-  green_body<R, MODE, D>(a, blockIdx.x - blk0[b]);
+  green_body<R, MODE>(a, blockIdx.x);
 }
 
 }  // namespace musg

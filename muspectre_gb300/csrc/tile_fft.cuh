@@ -219,6 +219,10 @@ __device__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, uns
                             const float2 *tw, const float2 *chirp, const float2 *bf, const TileLay lay, uint32_t buf,
                             uint32_t buf2, int P, uint32_t tws);
 
+__device__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode, int blu,
+                            const double2 *tw, const double2 *chirp, const double2 *bf, const TileLay lay, uint32_t buf,
+                            uint32_t buf2, int P, uint32_t tws);
+
 #define MUSG_TILE_RADICES(X) \
   X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17)
 

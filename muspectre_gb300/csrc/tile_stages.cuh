@@ -1,6 +1,9 @@
 // Out-of-line tile transforms (tile_fft.cuh): every role of every radix, compiled once
 // and called by the kernels of the displacement-space CG through tile_fft_rt (relocatable
 // device code): all roles inline in every kernel were ten minutes of compilation.
+// Included by tile_stages_f32.cu and tile_stages_f64.cu.
+#pragma once
+
 #include "tile_fft.cuh"
 
 namespace musg {
@@ -122,11 +125,5 @@ __device__ __forceinline__ bool tile_fft_any(bool inv, int n, int m, int r1, int
 }
 
 }  // namespace
-
-__device__ __noinline__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode, int blu,
-                            const float2 *tw, const float2 *chirp, const float2 *bf, const TileLay lay, uint32_t buf,
-                            uint32_t buf2, int P, uint32_t tws) {
-  return tile_fft_any<float2>(inv, n, m, r1, r2, nst, rcode, blu, tw, chirp, bf, lay, buf, buf2, P, tws);
-}
 
 }  // namespace musg

@@ -8,10 +8,9 @@ return mapping) stays FP64.  The FP32 inner solve stops at max(tol, inner_tol)
 contracts the error by about inner_tol and the FP64 Newton loop refines to
 newton_tol, which takes fewer CG iterations in total than tight inner solves) and
 the FP64 Newton loop refines; for history-free materials the returned stress is
-evaluated at the returned strain.  The Newton residual G(-P) is projected in FP64
-once per load step; later ones are the FP32 projection of the previous residual
-minus the stress change since (``incremental_residual=False`` projects every
-residual in FP64).  ``newton_cg`` follows
+evaluated at the returned strain.  The first two Newton residuals G(-P) of a load
+step are projected in FP64; later ones add the FP32 projection of the stress change
+since (``incremental_residual=False`` projects every residual in FP64).  ``newton_cg`` follows
 src/solver/solvers.cc:44-217.
 """
 from __future__ import annotations
