@@ -73,7 +73,7 @@ template <typename R> struct DispArgs {
   int ng;                 // row groups: D for the finite-strain axis passes
   int comps_at_once;      // mid passes, finite strain: 3, or 1 where a tile holds no more
   int nparts;             // blocks of ax0_fwd
-  int sp, sh;             // last-axis pencil stride and pad shift
+  int sp, S;              // last-axis strides of pencils and slot groups
   int Rr;                 // k-points per e of axis 0 (a component holds fewer than 2^31)
   long long nk, npx, nrows;
   const R *xi0, *xi1, *xi2;
@@ -120,8 +120,10 @@ __device__ __forceinline__ void stage_tile_twiddles(typename V2<R>::T *dst, cons
 
 // registers per thread.  FP32: 80 for the runtime plans, whose radices above 12 would take
 // up to 120 and halve the warps that hide the loads of all the others (they spill
-// instead).  FP64 passes wait on the FP64 pipe, not on loads: 128.
-template <typename R, int CR1> constexpr int kDispRegs = sizeof(R) == 8 ? 128 : CR1 == 16 ? 72 : CR1 > 0 ? 64 : 80;
+// instead).  FP64 passes wait on the FP64 pipe, not on loads: 128.  2-D grids, whose
+// radices go up to 32, are small: 128 and 168.
+template <typename R, int CR1> constexpr int kDispRegs =
+    sizeof(R) == 8 ? (CR1 == -2 ? 168 : 128) : CR1 == -2 ? 128 : 80;
 
 // Sum of the threads' compensated accumulators over the block, by thread 0.  FP32: the
 // warps add (sum, correction) pairs with Knuth's two-sum, an error of about 2^-46 in FP32
@@ -276,12 +278,21 @@ enum Ax0Mode : int {
 
 template <typename R, int D, bool FIN, int MODE, int CR1, int CR2, bool GRP>
 __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_inv(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
-  dep_wait();
   using T = typename V2<R>::T;
   using C = DispComps<D, FIN>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int bid;
   const DispArgs<R> a = disp_args<GRP, R>(a0, gtab, blk0, B, bid);
+  const int Tt = a.T, n0 = CR1 > 0 ? CR1 * CR2 : a.n0;
+  const int P = C::NA * Tt;
+  T *buf = reinterpret_cast<T *>(smem_raw);
+  T *buf2 = buf + (size_t)P * (CR1 > 0 ? CR1 * CR2 : a.ap.m);
+  T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
+  stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
+  const SlotMap<CR1, CR2> slots(a.ap, CR1 > 0 ? CR1 : a.ap.r1);
+  const PencilMap map(P);
+  const int g = bid / a.nbx, tile = bid - g * a.nbx;
+  dep_wait();
   R alpha = R(0), beta = R(0);
   bool first = true, go = true;
   if (MODE == AX_STEP) {
@@ -295,15 +306,6 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_inv(const DispArgs<R> a0,
     }
   }
   const R scale = MODE == AX_X ? a.scale * R(a.pb.st->xscale) : a.scale;
-  const int Tt = a.T, n0 = CR1 > 0 ? CR1 * CR2 : a.n0;
-  const int P = C::NA * Tt;
-  T *buf = reinterpret_cast<T *>(smem_raw);
-  T *buf2 = buf + (size_t)P * (CR1 > 0 ? CR1 * CR2 : a.ap.m);
-  T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
-  stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
-  const SlotMap<CR1, CR2> slots(a.ap);
-  const PencilMap map(P);
-  const int g = bid / a.nbx, tile = bid - g * a.nbx;
   // a thread keeps its k-point column t (T divides P, which divides the block)
   const int t = map.p % Tt, de = (int)blockDim.x / Tt;
   const int e0 = (int)threadIdx.x / Tt < de ? (int)threadIdx.x / Tt : kNoRow;
@@ -312,7 +314,7 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_inv(const DispArgs<R> a0,
   const Wave<D, R> wv(a, ok ? rho : 0);
   const long long ob = (long long)(FIN ? g : 0) * a.nk + rho;
   // independent loads of U points in flight before the first store
-  constexpr int U = FIN ? 2 : 1;
+  constexpr int U = FIN ? 4 : 1;
   for (int eb = e0; eb < n0; eb += U * de) {
     T v[U][C::ND];
     if (MODE == AX_STEP) {
@@ -405,22 +407,22 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_inv(const DispArgs<R> a0,
 // memory when it forms column 1's.  Small strain: one component per block.
 template <typename R, bool FIN, bool INV, int CR1, int CR2, bool GRP>
 __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
-  dep_wait();
   using T = typename V2<R>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int bid;
   const DispArgs<R> a = disp_args<GRP, R>(a0, gtab, blk0, B, bid);
-  if (a.gated && !a.pb.st->go) return;
   const int Tt = a.T, n1 = CR1 > 0 ? CR1 * CR2 : a.n1, nc = FIN ? a.comps_at_once : 1;
   const int P = nc * Tt;
   T *buf = reinterpret_cast<T *>(smem_raw);
   T *buf2 = buf + (size_t)P * (CR1 > 0 ? CR1 * CR2 : a.ap.m);
   T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
   stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
-  const SlotMap<CR1, CR2> slots(a.ap);
+  const SlotMap<CR1, CR2> slots(a.ap, CR1 > 0 ? CR1 : a.ap.r1);
   const PencilMap map(P);
   const int slab = bid / a.nbx, tile = bid - slab * a.nbx;  // slab: (row or component) * n0 + k0
   const int g = slab / a.n0, z = slab - g * a.n0;
+  dep_wait();
+  if (a.gated && !a.pb.st->go) return;
   const int t = map.p % Tt, k2 = tile * Tt + t;
   const bool ok = k2 < a.nh;
   const int nh = a.nh;
@@ -493,25 +495,25 @@ enum Ax0Sums : int {
 
 template <typename R, int D, bool FIN, int MODE, int CR1, int CR2, bool GRP>
 __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_fwd(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
-  dep_wait();
   using T = typename V2<R>::T;
   using C = DispComps<D, FIN>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int bid;
   const DispArgs<R> a = disp_args<GRP, R>(a0, gtab, blk0, B, bid);
-  if (a.gated && !a.pb.st->go) return;
   const int Tt = a.T, n0 = CR1 > 0 ? CR1 * CR2 : a.n0;
   const int P = C::NA * Tt;
   T *buf = reinterpret_cast<T *>(smem_raw);
   T *buf2 = buf + (size_t)P * (CR1 > 0 ? CR1 * CR2 : a.ap.m);
   T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
   stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
-  const SlotMap<CR1, CR2> slots(a.ap);
+  const SlotMap<CR1, CR2> slots(a.ap, CR1 > 0 ? CR1 : a.ap.r1);
   const PencilMap map(P);
   const int g = bid / a.nbx;
   const int t = map.p % Tt, c = map.p / Tt, comp = FIN ? g + D * c : c;
   const int de = (int)blockDim.x / Tt, e0 = (int)threadIdx.x / Tt < de ? (int)threadIdx.x / Tt : kNoRow;
   Acc<R> sum[4];
+  dep_wait();
+  if (a.gated && !a.pb.st->go) return;
   __syncthreads();  // the twiddle copy
   for (int tile = bid - g * a.nbx; tile < a.ntx; tile += a.nbx) {
     const int rho = tile * Tt + t;
@@ -639,12 +641,21 @@ __device__ __forceinline__ void pixel_tangent(const TangentData<R> &td, long lon
 // transform, where the tangent is applied
 template <typename R, int D, bool FIN, int TK, int IN, int OUT, int CR1, int CR2, bool GRP>
 __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_pixels(const DispArgs<R> a0, const DispArgs<R> *gtab, const int *blk0, int B) {
-  dep_wait();
   using T = typename V2<R>::T;
   constexpr int NL = DispComps<D, FIN>::NL, D2 = D * D;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int bid;
   const DispArgs<R> a = disp_args<GRP, R>(a0, gtab, blk0, B, bid);
+  const int L = CR1 > 0 ? CR1 * CR2 : a.L, H = (L + 1) / 2, G = a.G, G2 = G >> 1;
+  const int P = NL * G2;
+  const RowMap<CR1, CR2> lay(a.S, a.sp);
+  T *buf = reinterpret_cast<T *>(smem_raw);
+  T *buf2 = buf + (size_t)P * lay.sp;
+  T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
+  stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
+  const SlotMap<CR1, CR2> slots(a.ap, lay.S);
+  const long long row0 = (long long)bid * G;
+  dep_wait();
   if (a.gated) {
     CGState *st = a.pb.st;
     if (!st->go) {
@@ -652,150 +663,160 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_pixels(const DispArgs<R> a0, 
       return;
     }
   }
-  const int L = CR1 > 0 ? CR1 * CR2 : a.L, H = (L + 1) / 2, G = a.G, G2 = G >> 1;
-  const int P = NL * G2;
-  const RowMap<(CR1 > 0 ? CR1 * CR2 : 0)> lay{CR1 > 0 ? padded_pencil(CR1 * CR2) : a.sp, a.sh};
-  T *buf = reinterpret_cast<T *>(smem_raw);
-  T *buf2 = buf + (size_t)P * lay.sp;
-  T *tws = (CR1 > 0 || a.ap.r1) ? buf2 : nullptr;
-  stage_tile_twiddles<R, CR1, CR2>(tws, a.ap);
-  const SlotMap<CR1, CR2> slots(a.ap);
-  const long long row0 = (long long)bid * G;
-  const FDiv fH(H), fG2(G2);
   T *cur = buf;
+  // (row pair, k) of a load or store task; the components of a task follow each other
+  const FDiv fH(H);
+  auto task = [&](int idx, int &k) {
+    if constexpr (CR1 > 0) {
+      k = idx % (CR1 * CR2 / 2);
+      return idx / (CR1 * CR2 / 2);
+    } else {
+      return fH.div(idx, k);
+    }
+  };
   if (IN == IN_SPEC) {
-    const int total = P * H;
-    constexpr int U = kLoadBatch / 2;
-    for (int i0 = threadIdx.x; i0 < total; i0 += U * blockDim.x) {
-      T X[U], Y[U];
+    for (int idx = threadIdx.x; idx < G2 * H; idx += blockDim.x) {
+      int k;
+      const int g2 = task(idx, k);
+      const long long rx = row0 + 2 * g2;
+      const bool okx = rx < a.nrows, oky = rx + 1 < a.nrows;
+      const T *src = a.pb.spec + rx * H + k;
+      T X[NL], Y[NL];  // every load of the task in flight together
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int idx = i0 + u * blockDim.x;
-        X[u] = T{R(0), R(0)};
-        Y[u] = T{R(0), R(0)};
-        if (idx < total) {
-          int k, g2;
-          const int q = fH.div(idx, k);
-          const int c = fG2.div(q, g2);
-          const long long rx = row0 + 2 * g2, ry = rx + 1;
-          const T *s = a.pb.spec + (long long)c * a.nk + k;
-          if (rx < a.nrows) X[u] = s[rx * H];
-          if (ry < a.nrows) Y[u] = s[ry * H];
-        }
+      for (int c = 0; c < NL; ++c) {
+        X[c] = okx ? src[(long long)c * a.nk] : T{R(0), R(0)};
+        Y[c] = oky ? src[(long long)c * a.nk + H] : T{R(0), R(0)};
       }
+      const int pk = lay.at(slots.nat(k), g2), pm = lay.at(slots.nat(k > 0 ? L - k : L / 2), g2);
+      const int pstep = G2 * lay.sp;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int idx = i0 + u * blockDim.x;
-        if (idx >= total) continue;
-        int k;
-        const int q = fH.div(idx, k);
-        T x = X[u], y = Y[u];
+      for (int c = 0; c < NL; ++c) {
+        T x = X[c], y = Y[c];
         if (k == 0) { x.y = R(0); y.y = R(0); }  // c2r uses the real part only
-        buf[lay.at(slots.nat(k), q)] = T{x.x - y.y, x.y + y.x};
-        if (k > 0) buf[lay.at(slots.nat(L - k), q)] = T{x.x + y.y, y.x - x.y};
-        else if (L % 2 == 0) buf[lay.at(slots.nat(L / 2), q)] = T{R(0), R(0)};  // not stored: zero
+        buf[pk + c * pstep] = T{x.x - y.y, x.y + y.x};
+        if (k > 0) buf[pm + c * pstep] = T{x.x + y.y, y.x - x.y};
+        else if (L % 2 == 0) buf[pm + c * pstep] = T{R(0), R(0)};  // the Nyquist column is not stored: zero
       }
     }
     __syncthreads();
     cur = TileRun<CR1, CR2>::template run<true, R>(a.ap, lay, buf, buf2, P, tws);
   }
-  // pixels: component values of (row pair, slot of e) in the real or imaginary part
-  R *curr = reinterpret_cast<R *>(cur);
+  // pixels: a thread takes the two rows of a pair at one e, the real and imaginary parts of
+  // the pair's pencils
   const FDiv fL(L);
-  for (int idx = threadIdx.x; idx < G * L; idx += blockDim.x) {
-    int e;
-    const int g = fL.div(idx, e);
-    const long long row = row0 + g;
-    const long long px = row * L + e;
-    const int at0 = 2 * lay.at(slots.split(e), g >> 1) + (g & 1), pstep = 2 * G2 * lay.sp;
-    const bool ok = row < a.nrows;
-    R v[D2], out[D2];
-    constexpr bool kLocal = TK != TK_PLAIN && TK != TK_ANYFIN;
-    TangentLocal<D, kLocal ? TK : TK_SMALL, R> tl;
-    if constexpr (kLocal)
-      if (ok) tl.load(a.pb.td, px, a.npx);  // in flight with the shared-memory reads
-    if (IN == IN_SPEC) {
-      R f[NL];
+  for (int idx = threadIdx.x; idx < G2 * L; idx += blockDim.x) {
+    int e, g2;
+    if constexpr (CR1 > 0) {
+      g2 = idx / (CR1 * CR2);
+      e = idx % (CR1 * CR2);
+    } else {
+      g2 = fL.div(idx, e);
+    }
+    const long long px0 = (row0 + 2 * g2) * L + e;
+    const int at0 = lay.at(slots.split(e), g2), pstep = G2 * lay.sp;
+    T f[NL];
+    if (IN == IN_SPEC)
 #pragma unroll
-      for (int c = 0; c < NL; ++c) f[c] = curr[at0 + c * pstep];
-      if constexpr (FIN) {
-#pragma unroll
-        for (int c = 0; c < D2; ++c) v[c] = f[c];
-      } else {
+      for (int c = 0; c < NL; ++c) f[c] = cur[at0 + c * pstep];
+    auto pixel = [&](auto part, long long px, bool ok) {
+      // part(c): the pixel's value of component c in f
+      R v[D2], out[D2];
+      constexpr bool kLocal = TK != TK_PLAIN && TK != TK_ANYFIN;
+      TangentLocal<D, kLocal ? TK : TK_SMALL, R> tl;
+      if constexpr (kLocal)
+        if (ok) tl.load(a.pb.td, px, a.npx);
+      if (IN == IN_SPEC) {
 #pragma unroll
         for (int j = 0; j < D; ++j)
 #pragma unroll
-          for (int i = 0; i < D; ++i) v[i + D * j] = f[Sym<D>::at(i < j ? i : j, i < j ? j : i)];
-      }
-    } else {
+          for (int i = 0; i < D; ++i) v[i + D * j] = part(FIN ? i + D * j : Sym<D>::at(i < j ? i : j, i < j ? j : i));
+      } else {
 #pragma unroll
-      for (int c = 0; c < D2; ++c) {
-        const long long o = (long long)c * a.npx + px;
-        v[c] = R(0);
+        for (int c = 0; c < D2; ++c) {
+          const long long o = (long long)c * a.npx + px;
+          v[c] = R(0);
+          if (ok) {
+            if (IN == IN_REAL) {
+              v[c] = R(a.in_scale * a.in64[o]);
+            } else {
+              const double now = a.in64[o];
+              v[c] = R(a.in_prev[o] - now);
+              a.in_prev[o] = now;
+            }
+          }
+        }
+      }
+      if constexpr (TK == TK_PLAIN) {
+#pragma unroll
+        for (int c = 0; c < D2; ++c) out[c] = v[c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < D2; ++c) out[c] = R(0);
         if (ok) {
-          if (IN == IN_REAL) {
-            v[c] = R(a.in_scale * a.in64[o]);
+          if constexpr (kLocal) {
+            tl.apply(v, out);
           } else {
-            const double now = a.in64[o];
-            v[c] = R(a.in_prev[o] - now);
-            a.in_prev[o] = now;
+            switch (a.tkind) {
+              case TK_FINITE: pixel_tangent<D, TK_FINITE>(a.pb.td, px, a.npx, v, out); break;
+              case TK_KPRIME: pixel_tangent<D, TK_KPRIME>(a.pb.td, px, a.npx, v, out); break;
+              case TK_MIXED: pixel_tangent<D, TK_MIXED>(a.pb.td, px, a.npx, v, out); break;
+              case TK_FISO: pixel_tangent<D, TK_FISO>(a.pb.td, px, a.npx, v, out); break;
+              case TK_GFINITE: pixel_tangent<D, TK_GFINITE>(a.pb.td, px, a.npx, v, out); break;
+              default: pixel_tangent<D, TK_FULL>(a.pb.td, px, a.npx, v, out); break;
+            }
           }
         }
       }
-    }
-    if constexpr (TK == TK_PLAIN) {
+      if (OUT == OUT_REAL) {
+        if (ok)
 #pragma unroll
-      for (int c = 0; c < D2; ++c) out[c] = v[c];
-    } else {
+          for (int c = 0; c < D2; ++c) a.out[(long long)c * a.npx + px] = out[c];
+      } else {
 #pragma unroll
-      for (int c = 0; c < D2; ++c) out[c] = R(0);
-      if (ok) {
-        if constexpr (kLocal) {
-          tl.apply(v, out);
-        } else {
-          switch (a.tkind) {
-            case TK_FINITE: pixel_tangent<D, TK_FINITE>(a.pb.td, px, a.npx, v, out); break;
-            case TK_KPRIME: pixel_tangent<D, TK_KPRIME>(a.pb.td, px, a.npx, v, out); break;
-            case TK_MIXED: pixel_tangent<D, TK_MIXED>(a.pb.td, px, a.npx, v, out); break;
-            case TK_FISO: pixel_tangent<D, TK_FISO>(a.pb.td, px, a.npx, v, out); break;
-            case TK_GFINITE: pixel_tangent<D, TK_GFINITE>(a.pb.td, px, a.npx, v, out); break;
-            default: pixel_tangent<D, TK_FULL>(a.pb.td, px, a.npx, v, out); break;
+        for (int c = 0; c < NL; ++c) {
+          if constexpr (FIN) {
+            part(c) = out[c];
+          } else {
+            const int i = Sym<D>::row(c), j = Sym<D>::col(c);
+            // a general input may be unsymmetric; the projection takes its symmetric part
+            part(c) = (IN == IN_SPEC || i == j) ? out[i + D * j] : R(0.5) * (out[i + D * j] + out[j + D * i]);
           }
         }
       }
-    }
-    if (OUT == OUT_REAL) {
-      if (ok)
+    };
+    const long long row = row0 + 2 * g2;
+    if constexpr (TK == TK_ANYFIN) {  // the kinds' code once, the parts swapped between
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        pixel([&](int c) -> R & { return f[c].x; }, px0 + h * L, row + h < a.nrows);
 #pragma unroll
-        for (int c = 0; c < D2; ++c) a.out[(long long)c * a.npx + px] = out[c];
-    } else {
-#pragma unroll
-      for (int c = 0; c < NL; ++c) {
-        R w;
-        if constexpr (FIN) {
-          w = out[c];
-        } else {
-          const int i = Sym<D>::row(c), j = Sym<D>::col(c);
-          // a general input may be unsymmetric; the projection takes its symmetric part
-          w = (IN == IN_SPEC || i == j) ? out[i + D * j] : R(0.5) * (out[i + D * j] + out[j + D * i]);
-        }
-        curr[at0 + c * pstep] = w;
+        for (int c = 0; c < NL; ++c) f[c] = T{f[c].y, f[c].x};
       }
+    } else {
+      pixel([&](int c) -> R & { return f[c].x; }, px0, row < a.nrows);
+      pixel([&](int c) -> R & { return f[c].y; }, px0 + L, row + 1 < a.nrows);
     }
+    if (OUT == OUT_SPEC)
+#pragma unroll
+      for (int c = 0; c < NL; ++c) cur[at0 + c * pstep] = f[c];
   }
   if (OUT == OUT_REAL) return;
   __syncthreads();
   const T *res = TileRun<CR1, CR2>::template run<false, R>(a.ap, lay, cur, cur == buf ? buf2 : buf, P, tws);
   // unpack the two real spectra: X = (Z_k + conj Z_{L-k})/2, Y = -i (Z_k - conj Z_{L-k})/2
-  for (int idx = threadIdx.x; idx < P * H; idx += blockDim.x) {
-    int k, g2;
-    const int q = fH.div(idx, k);
-    const int c = fG2.div(q, g2);
-    const long long rx = row0 + 2 * g2, ry = rx + 1;
-    const T z = res[lay.at(slots.nat(k), q)], zn = res[lay.at(slots.nat(k == 0 ? 0 : L - k), q)];
-    T *s = a.pb.spec + (long long)c * a.nk + k;
-    if (rx < a.nrows) s[rx * H] = T{R(0.5) * (z.x + zn.x), R(0.5) * (z.y - zn.y)};
-    if (ry < a.nrows) s[ry * H] = T{R(0.5) * (z.y + zn.y), R(-0.5) * (z.x - zn.x)};
+  for (int idx = threadIdx.x; idx < G2 * H; idx += blockDim.x) {
+    int k;
+    const int g2 = task(idx, k);
+    const long long rx = row0 + 2 * g2;
+    const bool okx = rx < a.nrows, oky = rx + 1 < a.nrows;
+    T *dst = a.pb.spec + rx * H + k;
+    const int pk = lay.at(slots.nat(k), g2), pm = lay.at(slots.nat(k == 0 ? 0 : L - k), g2), pstep = G2 * lay.sp;
+#pragma unroll
+    for (int c = 0; c < NL; ++c) {
+      const T z = res[pk + c * pstep], zn = res[pm + c * pstep];
+      if (okx) dst[(long long)c * a.nk] = T{R(0.5) * (z.x + zn.x), R(0.5) * (z.y - zn.y)};
+      if (oky) dst[(long long)c * a.nk + H] = T{R(0.5) * (z.y + zn.y), R(-0.5) * (z.x - zn.x)};
+    }
   }
 }
 

@@ -10,7 +10,7 @@ namespace {
 template <typename R, int D, bool FIN>
 void ax0_dots(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
               const DispGroup<R> *grp) {
-  if (grp) return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+  if (grp) return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, (kGroupPlan<R, D>), (kGroupPlan<R, D>), true>, a, c, B, s, grp);
   if constexpr (sizeof(R) == 4) {
     switch (disp_fixed_plan(pl)) {
 #define MUSG_C(M, A, BB) \
@@ -20,7 +20,7 @@ void ax0_dots(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int 
       default: break;
     }
   }
-  disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, 0, 0, false>, a, c, B, s);
+  disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, kRtPlan<D>, kRtPlan<D>, false>, a, c, B, s);
 }
 }  // namespace
 
@@ -35,7 +35,7 @@ void disp_ax0_dots(const Spectral &sp, const DispArgs<R> &a, const DispShape &c,
 template <typename R>
 void disp_ax0_contract(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
 #define MUSG_C(DD, FF) \
-  if (sp.g.dim == DD && disp_finite(sp) == FF) disp_launch<R>(k_ax0_fwd<R, DD, FF, AX_OUT, -1, -1, false>, a, c, 1, s);
+  if (sp.g.dim == DD && disp_finite(sp) == FF) disp_launch<R>(k_ax0_fwd<R, DD, FF, AX_OUT, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);
   MUSG_C(2, true) MUSG_C(2, false) MUSG_C(3, true) MUSG_C(3, false)
 #undef MUSG_C
 }

@@ -10,7 +10,7 @@ namespace {
 template <typename R, int D, bool FIN>
 void ax0_step(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
               const DispGroup<R> *grp) {
-  if (grp) return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+  if (grp) return disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, (kGroupPlan<R, D>), (kGroupPlan<R, D>), true>, a, c, B, s, grp);
   if constexpr (sizeof(R) == 4) {
     switch (disp_fixed_plan(pl)) {
 #define MUSG_C(M, A, BB) \
@@ -20,7 +20,7 @@ void ax0_step(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int 
       default: break;
     }
   }
-  disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, 0, 0, false>, a, c, B, s);
+  disp_launch<R>(k_ax0_inv<R, D, FIN, AX_STEP, kRtPlan<D>, kRtPlan<D>, false>, a, c, B, s);
 }
 }  // namespace
 
@@ -36,8 +36,8 @@ template <typename R>
 void disp_ax0_field(const Spectral &sp, bool from_x, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
 #define MUSG_C(DD, FF)                                                                           \
   if (sp.g.dim == DD && disp_finite(sp) == FF) {                                                             \
-    if (from_x) disp_launch<R>(k_ax0_inv<R, DD, FF, AX_X, -1, -1, false>, a, c, 1, s);     \
-    else disp_launch<R>(k_ax0_inv<R, DD, FF, AX_Q, -1, -1, false>, a, c, 1, s);            \
+    if (from_x) disp_launch<R>(k_ax0_inv<R, DD, FF, AX_X, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);     \
+    else disp_launch<R>(k_ax0_inv<R, DD, FF, AX_Q, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);            \
   }
   MUSG_C(2, true) MUSG_C(2, false) MUSG_C(3, true) MUSG_C(3, false)
 #undef MUSG_C

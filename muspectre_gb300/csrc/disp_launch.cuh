@@ -11,9 +11,14 @@
 
 namespace musg {
 
+// FP32: power-of-two axes have kernels with compile-time plans (0: none).  In FP64 the
+// arithmetic, not the indexing, sets the pace.
+#define MUSG_DISP_PLANS(X) X(32, 8, 4) X(64, 8, 8) X(128, 16, 8) X(256, 16, 16)
+inline int disp_fixed_plan(const TilePlan &pl) { return pl.blu ? 0 : pl.m; }
+
 // launch shape of one pass
 struct DispShape {
-  int T = 0, G = 0, ntx = 0, nbx = 0, ng = 1, comps_at_once = 1, threads = 0, blocks = 0, sp = 0, sh = 31;
+  int T = 0, G = 0, ntx = 0, nbx = 0, ng = 1, comps_at_once = 1, threads = 0, blocks = 0, sp = 0, S = 0;
   size_t smem = 0;
 };
 
@@ -21,12 +26,22 @@ constexpr int kDispSms = 152;
 
 inline bool disp_finite(const Spectral &sp) { return sp.proj_kind != MUSG_PROJ_SMALL_STRAIN; }
 
-// about 16 points of the tile per thread: one radix-16 or two radix-8 butterflies.  A
-// multiple of `unit` (the pencils of a pencil-fast tile, or a warp).
-inline int disp_threads(long points, long unit) {
-  const long t = std::max(64L, std::min(512L, points / 16));
-  return (int)std::max(unit, std::min(512 / unit, (t + unit - 1) / unit) * unit);
+// Threads per block for tiles of P pencils: about 16 points of the tile per thread (one
+// radix-16 or two radix-8 butterflies).  FP64, whose instructions take 16 cycles of an SM
+// each: on grids too small to fill the SMs up to one butterfly per thread (35^3 147 ->
+// 135 us an iteration; in FP32 the same rule cost more in per-thread setup than it
+// gained, 63^3 77 -> 92 us).  A multiple of `unit` (the pencils of a pencil-fast tile, or
+// a warp).
+template <typename R> int disp_threads(const TilePlan &pl, long P, long blocks, long unit, long most) {
+  const long tasks = P * (pl.r1 ? std::max(pl.r1, pl.r2) : pl.m / 4);
+  const long fill = kDispSms * 1024L / std::max(1L, blocks);
+  long t = P * pl.m / 16;
+  if (sizeof(R) == 8) t = std::max(t, std::min(tasks, fill));
+  t = std::max(64L, std::min(most, t));
+  return (int)std::max(unit, std::min(most / unit, (t + unit - 1) / unit) * unit);
 }
+// the kernels' registers (kDispRegs) allow 512 threads, of the FP64 2-D ones 384
+template <typename R> long disp_most(const Spectral &sp) { return sizeof(R) == 8 && sp.g.dim == 2 ? 384 : 512; }
 inline long lcm32(long p) {
   long a = p;
   while (a % 32) a += p;
@@ -55,7 +70,7 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   c.nbx = sums ? std::min(c.ntx, 4 * kDispSms / c.ng) : c.ntx;
   c.blocks = c.nbx * c.ng;
   c.smem = (size_t)(T * per + tw);
-  c.threads = disp_threads((long)na * pl.m * T, lcm32(na * T));
+  c.threads = disp_threads<R>(pl, na * T, c.blocks, lcm32(na * T), disp_most<R>(sp));
   return c;
 }
 
@@ -76,13 +91,14 @@ template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
   while (T > 1 && T * per + tw > (56 << 10)) T = (T + 1) / 2;
   if (T * per + tw > optin_smem()) T = 1;
   while (T > 4 && (long long)c.ng * sp.g.n[0] * ((nh + T - 1) / T) < 2 * kDispSms) T = (T + 1) / 2;
+  while (sizeof(R) == 8 && T > 1 && (long long)c.ng * sp.g.n[0] * ((nh + T - 1) / T) < kDispSms) T = (T + 1) / 2;
   const long nt = (nh + T - 1) / T;
   T = (nh + nt - 1) / nt;  // balanced: 65 -> 5 x 13
   c.T = (int)T;
   c.ntx = c.nbx = (int)nt;
   c.blocks = (int)((long long)c.ng * sp.g.n[0] * nt);
   c.smem = (size_t)(T * per + tw);
-  c.threads = disp_threads((long)c.comps_at_once * pl.m * T, c.comps_at_once * T);
+  c.threads = disp_threads<R>(pl, c.comps_at_once * T, c.blocks, c.comps_at_once * T, disp_most<R>(sp));
   return c;
 }
 
@@ -93,13 +109,24 @@ template <typename R> DispShape disp_last_shape(const Spectral &sp) {
   const TilePlan &pl = sp.tp[D - 1];
   DispShape c;
   const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0;
-  c.sp = padded_pencil(pl.m);
-  c.sh = 4;
-  if ((long)nl * c.sp * cb * pl.buffers() + tw > optin_smem()) {  // the longest rows: no padding
-    c.sp = pl.m;
-    c.sh = 31;
+  c.S = pl.r1;
+  c.sp = pl.m;
+  if (pl.r1) {
+    const RowStrides r = row_strides(pl.r1, pl.r2);
+    c.S = r.S;
+    c.sp = r.sp;
   }
-  const long per = (long)nl * c.sp * cb * pl.buffers();
+  long row = c.sp;
+  if (sizeof(R) == 4) {  // a compile-time plan has its own strides
+    switch (disp_fixed_plan(pl)) {
+#define MUSG_C(M, A, B) \
+  case M: row = std::max<long>(row, row_strides(A, B).sp); break;
+      MUSG_DISP_PLANS(MUSG_C)
+#undef MUSG_C
+      default: break;
+    }
+  }
+  const long per = (long)nl * row * cb * pl.buffers();
   if (!pl.m || per + tw > optin_smem()) throw Error(MUSG_ERR_ARGUMENT, "last-axis FFT too long for one thread block");
   // rows until a block has about 160 threads, fewer where SMs would be without a block
   long g2 = std::max(1L, 160 * 16 / ((long)nl * pl.m));
@@ -109,7 +136,7 @@ template <typename R> DispShape disp_last_shape(const Spectral &sp) {
   c.G = (int)(2 * g2);
   c.blocks = (int)((sp.g.nrows + c.G - 1) / c.G);
   c.smem = (size_t)(g2 * per + tw);
-  c.threads = disp_threads((long)nl * pl.m * g2, 32);
+  c.threads = disp_threads<R>(pl, nl * g2, c.blocks, 16, disp_most<R>(sp));
   return c;
 }
 
@@ -145,7 +172,7 @@ template <typename R> DispArgs<R> disp_with(DispArgs<R> a, const Spectral &sp, i
   a.ng = c.ng;
   a.comps_at_once = c.comps_at_once;
   a.sp = c.sp;
-  a.sh = c.sh;
+  a.S = c.S;
   return a;
 }
 
@@ -165,12 +192,11 @@ void disp_launch(K kernel, const DispArgs<R> &a, const DispShape &c, int B, cuda
   MUSG_CHECK_LAUNCH();
 }
 
-// FP32: power-of-two axes have kernels with compile-time plans (0: none).  In FP64 the
-// arithmetic, not the indexing, sets the pace.
-#define MUSG_DISP_PLANS(X) X(32, 8, 4) X(64, 8, 8) X(128, 16, 8) X(256, 16, 16)
-inline int disp_fixed_plan(const TilePlan &pl) { return pl.blu ? 0 : pl.m; }
-// stages of the grouped kernels: inline in FP32, out of line in FP64 (build time)
-template <typename R> constexpr int kGroupPlan = sizeof(R) == 4 ? 0 : -1;
+// runtime plans by dimension: radices up to 32 in 2-D (TileRun); of the passes that run
+// once per Newton step and of the FP64 grouped ones, out of line in 3-D (build time)
+template <int D> constexpr int kRtPlan = D == 2 ? -2 : 0;
+template <int D> constexpr int kPlainPlan = D == 2 ? -2 : -1;
+template <typename R, int D> constexpr int kGroupPlan = sizeof(R) == 4 ? kRtPlan<D> : kPlainPlan<D>;
 
 // the passes: of an iteration (solo, batched, or grouped with grp), and the plain ones
 template <typename R>

@@ -8,7 +8,7 @@ namespace {
 
 template <typename R, bool FIN, bool INV>
 void mid(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s, const DispGroup<R> *grp) {
-  if (grp) return disp_launch<R>(k_mid<R, FIN, INV, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+  if (grp) return disp_launch<R>(k_mid<R, FIN, INV, (kGroupPlan<R, 3>), (kGroupPlan<R, 3>), true>, a, c, B, s, grp);
   if constexpr (sizeof(R) == 4) {
     switch (disp_fixed_plan(pl)) {
 #define MUSG_C(M, A, BB) \

@@ -1,5 +1,6 @@
 // Launches of the displacement-space CG's pixel pass (disp.cuh) for one dimension,
-// included by disp_pixels2.cu and disp_pixels3.cu.
+// included by the disp_pixels*.cu (the iteration's
+// pass and the ones from and to real fields build side by side where they are long to build).
 #pragma once
 
 #include "disp_launch.cuh"
@@ -11,12 +12,11 @@ template <typename R, int D, bool FIN, int TK>
 void pixels_iteration(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
                       const DispGroup<R> *grp) {
   if (grp) {
-    disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, kGroupPlan<R>, kGroupPlan<R>, true>, a, c, B, s, grp);
+    disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, (kGroupPlan<R, D>), (kGroupPlan<R, D>), true>, a, c, B, s, grp);
     return;
   }
   if constexpr (sizeof(R) == 4) {
-    // compile-time plans need the padded pencils (always there at these lengths)
-    switch (c.sh != 4 ? 0 : disp_fixed_plan(pl)) {
+    switch (disp_fixed_plan(pl)) {
 #define MUSG_PX(M, A, BB) \
   case M: disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, A, BB, false>, a, c, B, s); return;
       MUSG_DISP_PLANS(MUSG_PX)
@@ -24,7 +24,7 @@ void pixels_iteration(const TilePlan &pl, const DispArgs<R> &a, const DispShape 
       default: break;
     }
   }
-  disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, 0, 0, false>, a, c, B, s);
+  disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, B, s);
 }
 
 }  // namespace
@@ -51,28 +51,29 @@ void disp_pixels_in(bool fin, int tkind, bool delta, const DispArgs<R> &a0, cons
   DispArgs<R> a = a0;
   a.tkind = tkind;
   if (tkind == TK_PLAIN) {
-    if (fin && delta) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_DELTA, OUT_SPEC, -1, -1, false>, a, c, 1, s);
-    else if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_REAL, OUT_SPEC, -1, -1, false>, a, c, 1, s);
-    else if (delta) disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_DELTA, OUT_SPEC, -1, -1, false>, a, c, 1, s);
-    else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_REAL, OUT_SPEC, -1, -1, false>, a, c, 1, s);
+    if (fin && delta) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_DELTA, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    else if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    else if (delta) disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_DELTA, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
   } else if (tkind == TK_SMALL) {
-    disp_launch<R>(k_pixels<R, D, false, TK_SMALL, IN_REAL, OUT_SPEC, -1, -1, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, false, TK_SMALL, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
   } else if (tkind == TK_GSMALL) {
-    disp_launch<R>(k_pixels<R, D, false, TK_GSMALL, IN_REAL, OUT_SPEC, -1, -1, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, false, TK_GSMALL, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
   } else {
-    disp_launch<R>(k_pixels<R, D, true, TK_ANYFIN, IN_REAL, OUT_SPEC, -1, -1, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, true, TK_ANYFIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
   }
 }
 
 template <typename R, int D>
 void disp_pixels_out(bool fin, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
-  if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_SPEC, OUT_REAL, -1, -1, false>, a, c, 1, s);
-  else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_SPEC, OUT_REAL, -1, -1, false>, a, c, 1, s);
+  if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_SPEC, OUT_REAL, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+  else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_SPEC, OUT_REAL, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
 }
 
 #define MUSG_INSTANTIATE_PIXELS(R, D)                                                                             \
   template void disp_pixels<R, D>(int, const TilePlan &, const DispArgs<R> &, const DispShape &, int, cudaStream_t, \
-                                  const DispGroup<R> *);                                                          \
+                                  const DispGroup<R> *);
+#define MUSG_INSTANTIATE_PIXELS_IO(R, D)                                                                          \
   template void disp_pixels_in<R, D>(bool, int, bool, const DispArgs<R> &, const DispShape &, cudaStream_t);      \
   template void disp_pixels_out<R, D>(bool, const DispArgs<R> &, const DispShape &, cudaStream_t);
 

@@ -3,4 +3,5 @@
 
 namespace musg {
 MUSG_INSTANTIATE_PIXELS(float, 3)
+MUSG_INSTANTIATE_PIXELS_IO(float, 3)
 }  // namespace musg

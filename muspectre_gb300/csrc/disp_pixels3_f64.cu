@@ -3,4 +3,5 @@
 
 namespace musg {
 MUSG_INSTANTIATE_PIXELS(double, 3)
+MUSG_INSTANTIATE_PIXELS_IO(double, 3)
 }  // namespace musg

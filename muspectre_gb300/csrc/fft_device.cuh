@@ -240,6 +240,49 @@ template <> struct CompCS<9> {
   }
 };
 
+// the larger composites: cos / sin of 2 pi j / N for j <= N/2, mirrored
+#define MUSG_COMP_CS(NN, CVALS, SVALS)                                                    \
+  template <> struct CompCS<NN> {                                                         \
+    static __device__ __forceinline__ double c(int j) {                                   \
+      constexpr double t[] = CVALS;                                                       \
+      return t[2 * j > NN ? NN - j : j];                                                  \
+    }                                                                                     \
+    static __device__ __forceinline__ double s(int j) {                                   \
+      constexpr double t[] = SVALS;                                                       \
+      return 2 * j > NN ? -t[NN - j] : t[j];                                              \
+    }                                                                                     \
+  };
+#define MUSG_LIST(...) {__VA_ARGS__}
+MUSG_COMP_CS(25, MUSG_LIST(1.0, 0.9685831611286311194902, 0.8763066800438635873081, 0.7289686274214115231467,
+                        0.5358267949789966182713, 0.3090169943749474241023, 0.06279051952931337607618,
+                        -0.1873813145857246305426, -0.4257792915650726488625, -0.6374239897486897101767,
+                        -0.8090169943749474241023, -0.9297764858882514036609, -0.9921147013144778310498),
+              MUSG_LIST(0.0, 0.2486898871648547882423, 0.4817536741017152749872, 0.6845471059286886737323,
+                        0.8443279255020150785486, 0.9510565162951535721164, 0.9980267284282715619523,
+                        0.9822872507286886810856, 0.9048270524660195277137, 0.770513242775789230803,
+                        0.5877852522924731291687, 0.3681245526846779591569, 0.1253332335643042453731))
+MUSG_COMP_CS(27, MUSG_LIST(1.0, 0.9730448705798238388329, 0.8936326403234122481926, 0.7660444431189780352024,
+                        0.5971585917027861648519, 0.396079766039156823696, 0.1736481776669303488517,
+                        -0.05814482891047582853875, -0.2868032327110902531033, -0.5, -0.6862416378687335857296,
+                        -0.8354878114129364196538, -0.9396926207859083840541, -0.9932383577419429885479),
+              MUSG_LIST(0.0, 0.2306158707424401784502, 0.448799180200462172785, 0.6427876096865393263226,
+                        0.8021231927550437850833, 0.918216106880274014759, 0.9848077530122080593667,
+                        0.9983081582712682080478, 0.9579895123154888744374, 0.8660254037844386467637,
+                        0.7273736415730486959872, 0.5495089780708060352628, 0.3420201433256687330441,
+                        0.1160929141252302296757))
+MUSG_COMP_CS(32, MUSG_LIST(1.0, 0.9807852804032304491262, 0.9238795325112867561282, 0.8314696123025452370788,
+                        0.7071067811865475244008, 0.5555702330196022247428, 0.3826834323650897717285,
+                        0.1950903220161282678483, 0.0, -0.1950903220161282678483, -0.3826834323650897717285,
+                        -0.5555702330196022247428, -0.7071067811865475244008, -0.8314696123025452370788,
+                        -0.9238795325112867561282, -0.9807852804032304491262, -1.0),
+              MUSG_LIST(0.0, 0.1950903220161282678483, 0.3826834323650897717285, 0.5555702330196022247428,
+                        0.7071067811865475244008, 0.8314696123025452370788, 0.9238795325112867561282,
+                        0.9807852804032304491262, 1.0, 0.9807852804032304491262, 0.9238795325112867561282,
+                        0.8314696123025452370788, 0.7071067811865475244008, 0.5555702330196022247428,
+                        0.3826834323650897717285, 0.1950903220161282678483, 0.0))
+#undef MUSG_COMP_CS
+#undef MUSG_LIST
+
 // composite radix N = N1 * N2 in registers (Cooley-Tukey): N2 DFTs of length N1 over
 // the stride-N2 subsequences, twiddles W_N^(n2 k1), then N1 DFTs of length N2
 template <int N1, int N2, bool INV, typename T> struct DftComposite {
@@ -341,6 +384,39 @@ template <bool INV, typename T> struct Dft<13, INV, T> {
 };
 template <bool INV, typename T> struct Dft<17, INV, T> {
   static __device__ __forceinline__ void run(T *v) { DftPrime<17, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<18, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 9, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<20, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<4, 5, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<21, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<3, 7, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<22, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 11, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<24, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<8, 3, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<26, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 13, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<28, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<4, 7, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<30, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftCoprime<2, 15, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<25, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftComposite<5, 5, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<27, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftComposite<9, 3, INV, T>::run(v); }
+};
+template <bool INV, typename T> struct Dft<32, INV, T> {
+  static __device__ __forceinline__ void run(T *v) { DftComposite<8, 4, INV, T>::run(v); }
 };
 
 // -------------------------------------------------------------- one stage

@@ -189,20 +189,22 @@ namespace {
 // the factor choice below weighs (small composites cost about 2 log2 r and a twiddle,
 // the direct primes about r)
 double stage_cost(int r) {
-  static const double c[18] = {0, 0, 2, 4.5, 4, 8, 6.5, 11, 6.5, 9, 10, 15, 8.5, 18, 13, 12.5, 9, 23};
+  static const double c[33] = {0,  0,  2,  4.5, 4,  8,    6.5, 11, 6.5, 9,  10, 15, 8.5, 18, 13, 12.5, 9,
+                               23, 11, 0,  12,  15, 17,   11,  0,  16,  20, 14, 15, 0,   15, 0,  11};
   return c[r] + 4.0;  // + twiddles and a shared-memory round trip
 }
+bool has_stage(int r) { return r <= 17 || (r <= 32 && r != 19 && r != 23 && r != 29 && r != 31); }
 
-// the cheapest factorisation of m into radices up to 17 (no heap: the allocation-free
-// projection plans with it): two factors (r1 >= r2, possibly 1) if there are any, else the
-// fewest; the number of factors in rad, 0 when a prime above 17 divides m
-int tile_factor(int m, int *rad, double &cost) {
+// the cheapest factorisation of m into radices (no heap: the allocation-free projection
+// plans with it): two factors up to `widest` (r1 >= r2, possibly 1) if there are any, else
+// the fewest up to 17; the number of factors in rad, 0 when a prime above 17 divides m
+int tile_factor(int m, int widest, int *rad, double &cost) {
   cost = 1e30;
   int n = 0;
-  for (int a = 1; a <= 17; ++a)
-    if (m % a == 0 && m / a <= 17) {
+  for (int a = 1; a <= widest; ++a)
+    if (m % a == 0 && m / a <= widest) {
       const int b = m / a;
-      if (b < a) continue;
+      if (b < a || !has_stage(a) || !has_stage(b)) continue;
       const double c = (a > 1 ? stage_cost(a) : 0.0) + (b > 1 ? stage_cost(b) : 0.0);
       if (c < cost) {
         cost = c;
@@ -217,7 +219,7 @@ int tile_factor(int m, int *rad, double &cost) {
     if (m % a) continue;
     int rest[kMaxStages];
     double c = 0;
-    int k = tile_factor(m / a, rest, c);
+    int k = tile_factor(m / a, 17, rest, c);
     if (k == 2 && rest[1] == 1) k = 1;
     if (k == 0 || k + 1 > kMaxStages || c + stage_cost(a) + 1.0 >= cost) continue;
     cost = c + stage_cost(a) + 1.0;
@@ -230,12 +232,12 @@ int tile_factor(int m, int *rad, double &cost) {
 
 }  // namespace
 
-void TilePlan::factor(int n_, bool smallest) {
+void TilePlan::factor(int n_, int widest, bool smallest) {
   n = n_;
   m = nst = r1 = r2 = blu = 0;
   if (n > (1 << 16)) return;  // longer than any tile: the passes refuse it (m = 0)
   double cost = 0;
-  if ((nst = tile_factor(n, radix, cost))) {
+  if ((nst = tile_factor(n, widest, radix, cost))) {
     m = n;
   } else {
     // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass
@@ -244,7 +246,7 @@ void TilePlan::factor(int n_, bool smallest) {
     for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
       int rad[kMaxStages];
       double c = 0;
-      const int ns = tile_factor(k, rad, c);
+      const int ns = tile_factor(k, 17, rad, c);
       if (!ns) continue;
       if (smallest && m) break;
       c *= k;
@@ -261,9 +263,9 @@ void TilePlan::factor(int n_, bool smallest) {
   r2 = nst == 2 ? radix[1] : 0;
 }
 
-void TilePlan::build(int n_) {
+void TilePlan::build(int n_, int widest) {
   release();
-  factor(n_);
+  factor(n_, widest);
   if (m) build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
 }
 
@@ -336,7 +338,7 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
 
 void Spectral::ensure_tiles() {
   for (int d = 0; d < g.dim; ++d)
-    if (tp[d].n != g.n[d]) tp[d].build(g.n[d]);
+    if (tp[d].n != g.n[d]) tp[d].build(g.n[d], g.dim == 2 ? 32 : 17);
 }
 
 void Spectral::ensure32() {

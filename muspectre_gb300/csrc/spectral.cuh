@@ -517,8 +517,8 @@ __global__ void __launch_bounds__(kPassThreads) k_axis(const AxisArgs<R> a) {
   axis_body<R, INV>(a, blockIdx.x);
 }
 
-// 1 / sqrt(n2): FP64 correctly rounded division of the square root (parity path);
-// FP32 the rsqrtf intrinsic (2 ulp, far inside the FP32 operator's rounding)
+// 1 / sqrt(n2) within 1 ulp (rsqrt; a square root and a division, each correctly rounded,
+// are no closer and twice the instructions of the FP64 pipe) and 2 ulp (rsqrtf)
 __device__ __forceinline__ double inv_sqrt(double n2) { return 1.0 / sqrt(n2); }
 __device__ __forceinline__ float inv_sqrt(float n2) { return rsqrtf(n2); }
 

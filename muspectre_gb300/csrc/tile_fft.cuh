@@ -1,7 +1,7 @@
 // In-place FFT of a tile of pencils in shared memory (device code), for the passes of
 // the displacement-space CG (disp.cuh).
 //
-// A length m = r1 * r2 (both at most 17) takes two stages on one buffer:
+// A length m = r1 * r2 (both at most 17, on 2-D grids 32) takes two stages on one buffer:
 //   forward  stage 1: for each y < r2, DFT_r1 over the slots y r1 + t (t < r1), which
 //                     hold x[y + r2 t] (the "split" order); results stay in their slots;
 //            stage 2: for each j < r1, slots j + r1 y times W_m^(j y), DFT_r2, giving
@@ -10,13 +10,13 @@
 //            slots j + r1 r, then IDFT_r1 over y r1 + t, split order out.
 // Both stages read and write the same slots of the same thread, so there is one
 // barrier per stage and no second buffer, and a forward transform takes the order an
-// inverse one leaves.  slot() maps an index to its place in split order.
+// inverse one leaves.
 //
 // Lengths with a prime factor above 17 run Bluestein's algorithm over such an m >=
 // 2 n - 1: chirp and zero padding ride on stage 1, the filter on the point between the
 // two middle stages (the same butterflies of the same thread), and the output chirp on
 // the last stage: four shared-memory passes, split order in and out.  Lengths that
-// need three or more factors (2-D grids above 289) ping-pong between two buffers in
+// need three or more factors ping-pong between two buffers in
 // natural order and read their twiddles from global memory (the table would not leave
 // room for the pencils of the longest axes).
 //
@@ -30,13 +30,13 @@
 
 namespace musg {
 
-// place of (slot, pencil): (slot + (slot >> sh)) * se + pencil * sp.  Pencil-fast
-// tiles (strided axes): se = P, sp = 1, sh = 31; slot-fast tiles (the contiguous
-// axis): se = 1, sp = the padded pencil, one pad entry per 16 slots, so that the
-// strides of 2 to 16 slots of a stage spread over the banks.
+// Slots of a pencil: groups of r1, S >= r1 places apart (S > r1 pads), so the inner stage
+// works on the places y S + t, the outer one on j + S r.  Place of (slot, pencil): slot *
+// se + pencil * sp.  Pencil-fast tiles (strided axes): se = P, sp = 1, S = r1; slot-fast
+// tiles (the contiguous axis): se = 1, sp = the pencil's stride.
 struct TileLay {
-  int se, sp, sh, pencil_fast;
-  __device__ __forceinline__ int at(int slot, int p) const { return (slot + (slot >> sh)) * se + p * sp; }
+  int se, sp, S, pencil_fast;
+  __device__ __forceinline__ int at(int slot, int p) const { return slot * se + p * sp; }
   // f(j, p) over the tasks (j < nj, p < P) of a stage, the faster one as the layout says
   template <typename F> __device__ __forceinline__ void each(int nj, int P, F f) const {
     const FDiv fd(pencil_fast ? P : nj);
@@ -59,20 +59,63 @@ struct PencilMap {
     j0 = f.div((int)threadIdx.x, p);
     if (j0 >= dj) j0 = kNoRow;
   }
+  __device__ __forceinline__ int stride(int r1) const { return r1; }
   __device__ __forceinline__ int at(int slot, int q) const { return slot * P + q; }
   template <typename F> __device__ __forceinline__ void each(int nj, int, F f) const {
     for (int j = j0; j < nj; j += dj) f(j, p);
   }
-  __device__ __forceinline__ TileLay lay() const { return TileLay{P, 1, 31, 1}; }
+  __device__ __forceinline__ TileLay lay(int r1) const { return TileLay{P, 1, r1, 1}; }
 };
-// a slot-fast tile; CM > 0: the length known at compile time
-template <int CM> struct RowMap {
-  int sp, sh;
-  __device__ __forceinline__ int at(int slot, int p) const {
-    return slot + (slot >> (CM > 0 ? 4 : sh)) + p * sp;
+// Strides of a slot-fast tile of two-stage pencils: S and the pencil stride with the
+// fewest bank conflicts over the four ways a half-warp walks it (16 lanes of 8 bytes:
+// consecutive indices in natural and in split order, the butterflies of the inner and of
+// the outer stage, going over to the next pencil), the smallest among equals.  At 16 x 8
+// the pixel phase had 4-way conflicts with one pad entry per 16 slots.
+struct RowStrides {
+  int S, sp;
+};
+__host__ __device__ constexpr int bank_cost(int r1, int r2, int S, int sp) {
+  int cost = 0;
+  for (int pat = 0; pat < 4; ++pat) {
+    int cnt[16] = {}, most = 0;
+    for (int i = 0; i < 16; ++i) {
+      const int a = pat == 0 ? (i / r1) * S + i % r1
+                    : pat == 1 ? (i % r2) * S + i / r2
+                    : pat == 2 ? (i % r2) * S + (i / r2) * sp
+                               : i % r1 + (i / r1) * sp;
+      const int k = ++cnt[a & 15];
+      if (k > most) most = k;
+    }
+    cost += most;
   }
+  return cost;
+}
+__host__ __device__ constexpr RowStrides row_strides(int r1, int r2) {
+  RowStrides best{r1, r1 * r2};
+  int cost = 1000;
+  for (int S = r1; S < r1 + 16; ++S)
+    for (int sp = (r2 - 1) * S + r1; sp < (r2 - 1) * S + r1 + 16; ++sp) {
+      const int c = bank_cost(r1, r2, S, sp);
+      if (c < cost || (c == cost && sp < best.sp)) {
+        cost = c;
+        best = RowStrides{S, sp};
+      }
+    }
+  return best;
+}
+
+// a slot-fast tile; CR1 > 0: factors known at compile time
+template <int CR1, int CR2> struct RowMap {
+  int S, sp;
+  __device__ __forceinline__ RowMap(int S_, int sp_) {
+    constexpr RowStrides r = row_strides(CR1 > 0 ? CR1 : 1, CR2 > 0 ? CR2 : 1);
+    S = CR1 > 0 ? r.S : S_;
+    sp = CR1 > 0 ? r.sp : sp_;
+  }
+  __device__ __forceinline__ int stride(int) const { return S; }
+  __device__ __forceinline__ int at(int slot, int p) const { return slot + p * sp; }
   template <typename F> __device__ __forceinline__ void each(int nj, int P, F f) const {
-    if constexpr (CM > 0) {  // nj is a power of two the compiler sees
+    if constexpr (CR1 > 0) {  // nj is a power of two the compiler sees
       for (int t = threadIdx.x; t < nj * P; t += blockDim.x) f(t % nj, t / nj);
     } else {
       const FDiv fd(nj);
@@ -83,9 +126,8 @@ template <int CM> struct RowMap {
       }
     }
   }
-  __device__ __forceinline__ TileLay lay() const { return TileLay{1, sp, CM > 0 ? 4 : sh, 0}; }
+  __device__ __forceinline__ TileLay lay(int) const { return TileLay{1, sp, S, 0}; }
 };
-__host__ __device__ constexpr int padded_pencil(int m) { return m + (m >> 4) + ((m + (m >> 4)) % 2 ? 0 : 1); }
 
 __device__ __forceinline__ uint32_t smem_window(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -129,7 +171,7 @@ enum TileOp : int {
   OP_B2 = 6   // Bluestein: inverse stage 2, chirp
 };
 template <typename T> struct TileStageArgs {
-  int P, ra;              // pencils; the other factor
+  int P, ra, S;           // pencils; the other factor; stride of the slot groups
   int n, conj;            // Bluestein: the transform's length; conj: the inverse transform
   const T *chirp, *bf;    // Bluestein tables (global memory)
 };
@@ -144,11 +186,11 @@ template <typename T> __device__ __forceinline__ T conj_if(T v, bool c) {
 template <int RAD, int OP, typename T, typename MAP, typename TWB, typename LD, typename ST>
 __device__ __forceinline__ void tile_stage(const MAP &map, const TWB tw, const TileStageArgs<T> &a, LD ld, ST st) {
   const int nj = a.ra;
-  constexpr bool kOuter = OP == OP_F2 || OP == OP_I1 || OP == OP_BM;  // slots j + ra r, else y RAD + t
+  constexpr bool kOuter = OP == OP_F2 || OP == OP_I1 || OP == OP_BM;  // slots j + S r, else y S + t
   map.each(nj, a.P, [&](int j, int p) {
     T v[RAD];
 #pragma unroll
-    for (int r = 0; r < RAD; ++r) v[r] = ld(j + nj * r, kOuter ? j + nj * r : j * RAD + r, p);
+    for (int r = 0; r < RAD; ++r) v[r] = ld(j + nj * r, kOuter ? j + a.S * r : j * a.S + r, p);
     if (OP == OP_B1) {
 #pragma unroll
       for (int r = 0; r < RAD; ++r) {
@@ -178,7 +220,7 @@ __device__ __forceinline__ void tile_stage(const MAP &map, const TWB tw, const T
       }
     }
 #pragma unroll
-    for (int r = 0; r < RAD; ++r) st(j + nj * r, kOuter ? j + nj * r : j * RAD + r, p, v[r]);
+    for (int r = 0; r < RAD; ++r) st(j + nj * r, kOuter ? j + a.S * r : j * a.S + r, p, v[r]);
   });
 }
 // Where an index sits in a tile: split order (what a forward transform takes and an
@@ -186,26 +228,34 @@ __device__ __forceinline__ void tile_stage(const MAP &map, const TWB tw, const T
 // compile time; <0, 0> and <-1, -1>: a runtime plan, where three and more factors keep natural order
 // throughout and Bluestein keeps split order throughout.
 template <int CR1, int CR2> struct SlotMap {
-  template <typename R> __device__ __forceinline__ explicit SlotMap(const TilePlanD<R> &) {}
-  __device__ __forceinline__ int split(int e) const { return (e % CR2) * CR1 + e / CR2; }
-  __device__ __forceinline__ int nat(int e) const { return e; }
+  int S;
+  template <typename R> __device__ __forceinline__ SlotMap(const TilePlanD<R> &, int S_) : S(S_) {}
+  __device__ __forceinline__ int split(int e) const { return (e % CR2) * S + e / CR2; }
+  __device__ __forceinline__ int nat(int e) const { return (e / CR1) * S + e % CR1; }
 };
 struct SlotMapRt {
-  int r1, blu;
-  FDiv f;
+  int r1, blu, S;
+  FDiv f, f1;
   template <typename R>
-  __device__ __forceinline__ explicit SlotMapRt(const TilePlanD<R> &pl)
-      : r1(pl.r1), blu(pl.blu), f(pl.r1 ? pl.r2 : 1) {}
+  __device__ __forceinline__ SlotMapRt(const TilePlanD<R> &pl, int S_)
+      : r1(pl.r1), blu(pl.blu), S(S_), f(pl.r1 ? pl.r2 : 1), f1(pl.r1 ? pl.r1 : 1) {}
   __device__ __forceinline__ int split(int e) const {
     if (!r1) return e;
     int lo;
     const int hi = f.div(e, lo);
-    return lo * r1 + hi;
+    return lo * S + hi;
   }
-  __device__ __forceinline__ int nat(int e) const { return blu ? split(e) : e; }
+  __device__ __forceinline__ int nat(int e) const {
+    if (blu) return split(e);
+    if (S == r1 || !r1) return e;
+    int lo;
+    const int hi = f1.div(e, lo);
+    return hi * S + lo;
+  }
 };
 template <> struct SlotMap<0, 0> : SlotMapRt { using SlotMapRt::SlotMapRt; };
 template <> struct SlotMap<-1, -1> : SlotMapRt { using SlotMapRt::SlotMapRt; };
+template <> struct SlotMap<-2, -2> : SlotMapRt { using SlotMapRt::SlotMapRt; };
 
 // The transform of P pencils.  run: from shared memory to shared memory, in place in buf
 // (buf2: the second buffer of a plan of three or more factors, unused otherwise); the
@@ -225,6 +275,9 @@ __device__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, uns
 
 #define MUSG_TILE_RADICES(X) \
   X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17)
+// two factors up to 32 cover the axes of 2-D grids up to 1024
+#define MUSG_TILE_RADICES_2D(X) \
+  X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) X(30) X(32)
 
 template <int CR1, int CR2> struct TileRun {
   template <bool INV, typename R, typename MAP, typename LD, typename ST>
@@ -232,7 +285,8 @@ template <int CR1, int CR2> struct TileRun {
                                             typename V2<R>::T *, int P, const typename V2<R>::T *tws, LD ld, ST st) {
     using T = typename V2<R>::T;
     const PtrBuf<T> tw{const_cast<T *>(tws)};
-    const TileStageArgs<T> a{P, CR2, CR1 * CR2, 0, nullptr, nullptr}, c{P, CR1, CR1 * CR2, 0, nullptr, nullptr};
+    const int S = map.stride(CR1);
+    const TileStageArgs<T> a{P, CR2, S, CR1 * CR2, 0, nullptr, nullptr}, c{P, CR1, S, CR1 * CR2, 0, nullptr, nullptr};
     auto rd = [&](int, int s, int p) { return buf[map.at(s, p)]; };
     auto wr = [&](int, int s, int p, T v) { buf[map.at(s, p)] = v; };
     if constexpr (INV) {
@@ -263,13 +317,13 @@ template <> struct TileRun<-1, -1> {
                                                            typename V2<R>::T *buf, typename V2<R>::T *buf2, int P,
                                                            const typename V2<R>::T *tws) {
     const bool second = tile_fft_rt(INV, pl.n, pl.m, pl.r1, pl.r2, pl.nst, pl.rcode, pl.blu, pl.tw, pl.chirp, pl.bf,
-                                    map.lay(), smem_window(buf), smem_window(buf2), P, smem_window(tws));
+                                    map.lay(pl.r1), smem_window(buf), smem_window(buf2), P, smem_window(tws));
     return second ? buf2 : buf;
   }
   template <bool INV, typename R, typename MAP, typename LD, typename ST>
   static __device__ __forceinline__ void io(const TilePlanD<R> &pl, const MAP &map, typename V2<R>::T *buf,
                                             typename V2<R>::T *buf2, int P, const typename V2<R>::T *tws, LD ld, ST st) {
-    const SlotMap<-1, -1> slots(pl);
+    const SlotMap<-1, -1> slots(pl, map.stride(pl.r1));
     map.each(pl.n, P, [&](int e, int p) {
       const int s = INV ? slots.nat(e) : slots.split(e);
       buf[map.at(s, p)] = ld(e, s, p);
@@ -282,16 +336,17 @@ template <> struct TileRun<-1, -1> {
     });
   }
 };
-// runtime plans of the iteration's passes: the two stages inline (one body per radix),
-// Bluestein and three or more factors out of line
-template <> struct TileRun<0, 0> {
+// runtime plans of the iteration's passes: the two stages inline (one body per radix; WIDE:
+// radices up to 32, 2-D), Bluestein and three or more factors out of line
+template <bool WIDE> struct TileRunRt {
   template <bool INV, typename R, typename MAP, typename LD, typename ST>
   static __device__ __forceinline__ void two(const TilePlanD<R> &pl, const MAP &map, typename V2<R>::T *buf, int P,
                                              const typename V2<R>::T *tws, LD ld, ST st) {
     using T = typename V2<R>::T;
     const PtrBuf<T> tw{const_cast<T *>(tws)};
-    const TileStageArgs<T> a{P, pl.r2, pl.n, 0, nullptr, nullptr};  // radix r1
-    const TileStageArgs<T> c{P, pl.r1, pl.n, 0, nullptr, nullptr};  // radix r2
+    const int S = map.stride(pl.r1);
+    const TileStageArgs<T> a{P, pl.r2, S, pl.n, 0, nullptr, nullptr};  // radix r1
+    const TileStageArgs<T> c{P, pl.r1, S, pl.n, 0, nullptr, nullptr};  // radix r2
     auto rd = [&](int, int s, int p) { return buf[map.at(s, p)]; };
     auto wr = [&](int, int s, int p, T v) { buf[map.at(s, p)] = v; };
     if constexpr (INV) {
@@ -300,12 +355,20 @@ template <> struct TileRun<0, 0> {
   case RAD: tile_stage<RAD, OP_I1, T>(map, tw, c, ld, wr); break;
         MUSG_TS(1) MUSG_TILE_RADICES(MUSG_TS)
 #undef MUSG_TS
+#define MUSG_TS(RAD) \
+  case RAD: if constexpr (WIDE) tile_stage<RAD, OP_I1, T>(map, tw, c, ld, wr); break;
+        MUSG_TILE_RADICES_2D(MUSG_TS)
+#undef MUSG_TS
       }
       __syncthreads();
       switch (pl.r1) {
 #define MUSG_TS(RAD) \
   case RAD: tile_stage<RAD, OP_I2, T>(map, tw, a, rd, st); break;
         MUSG_TILE_RADICES(MUSG_TS)
+#undef MUSG_TS
+#define MUSG_TS(RAD) \
+  case RAD: if constexpr (WIDE) tile_stage<RAD, OP_I2, T>(map, tw, a, rd, st); break;
+        MUSG_TILE_RADICES_2D(MUSG_TS)
 #undef MUSG_TS
         default: tile_stage<1, OP_I2, T>(map, tw, a, rd, st); break;
       }
@@ -315,6 +378,10 @@ template <> struct TileRun<0, 0> {
   case RAD: tile_stage<RAD, OP_F1, T>(map, tw, a, ld, wr); break;
         MUSG_TILE_RADICES(MUSG_TS)
 #undef MUSG_TS
+#define MUSG_TS(RAD) \
+  case RAD: if constexpr (WIDE) tile_stage<RAD, OP_F1, T>(map, tw, a, ld, wr); break;
+        MUSG_TILE_RADICES_2D(MUSG_TS)
+#undef MUSG_TS
         default: tile_stage<1, OP_F1, T>(map, tw, a, ld, wr); break;
       }
       __syncthreads();
@@ -322,6 +389,10 @@ template <> struct TileRun<0, 0> {
 #define MUSG_TS(RAD) \
   case RAD: tile_stage<RAD, OP_F2, T>(map, tw, c, rd, st); break;
         MUSG_TS(1) MUSG_TILE_RADICES(MUSG_TS)
+#undef MUSG_TS
+#define MUSG_TS(RAD) \
+  case RAD: if constexpr (WIDE) tile_stage<RAD, OP_F2, T>(map, tw, c, rd, st); break;
+        MUSG_TILE_RADICES_2D(MUSG_TS)
 #undef MUSG_TS
       }
     }
@@ -344,5 +415,8 @@ template <> struct TileRun<0, 0> {
     return buf;
   }
 };
+
+template <> struct TileRun<0, 0> : TileRunRt<false> {};
+template <> struct TileRun<-2, -2> : TileRunRt<true> {};
 
 }  // namespace musg

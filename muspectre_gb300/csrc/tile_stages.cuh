@@ -81,7 +81,7 @@ __device__ __forceinline__ bool tile_fft_any(bool inv, int n, int m, int r1, int
                                              int blu, const T *tw, const T *chirp, const T *bf, const TileLay lay,
                                              uint32_t buf, uint32_t buf2, int P, uint32_t tws) {
   if (r1) {
-    TileStageArgs<T> a{P, r2, n, inv ? 1 : 0, chirp, bf};  // radix r1
+    TileStageArgs<T> a{P, r2, lay.S, n, inv ? 1 : 0, chirp, bf};  // radix r1
     TileStageArgs<T> c = a;                                     // radix r2
     c.ra = r1;
     if (blu) {

@@ -68,6 +68,20 @@ def test_operator(mu, name, form):
     assert np.linalg.norm(got - ref) <= 1e-5 * scale
 
 
+@pytest.mark.parametrize('r', [18, 20, 21, 22, 24, 25, 26, 27, 28, 30, 32])
+def test_operator_wide_radix_2d(mu, r):
+    """2-D axes take radices up to 32: 17 * r leaves no other pair of factors than (r, 17)."""
+    for res in ([17 * r, 5], [6, 17 * r]):
+        n = int(np.prod(res))
+        cell = _cell(mu, res, 0, 3)
+        rng = np.random.default_rng(5)
+        F = 0.01 * rng.normal(size=(2, 2, n)) + np.eye(2)[:, :, None]
+        cell.evaluate_stress_tangent(F.reshape(4, n))
+        dF = rng.normal(size=(4, n))
+        ref = cell.directional_stiffness(dF)
+        assert np.linalg.norm(cell.cg_operator(dF, 'mixed') - ref) <= 1e-5 * np.linalg.norm(ref)
+
+
 SOLVED = ['one_factor', 'two_factors', 'bluestein', 'many_factors', 'power_of_two_axes', 'thin']
 
 
