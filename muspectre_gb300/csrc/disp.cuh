@@ -125,6 +125,7 @@ __device__ __forceinline__ void stage_tile_twiddles(typename V2<R>::T *dst, cons
 template <typename R, int CR1> constexpr int kDispRegs =
     sizeof(R) == 8 ? (CR1 == -2 ? 168 : 128) : CR1 == -2 ? 128 : 80;
 
+
 // Sum of the threads' compensated accumulators over the block, by thread 0.  FP32: the
 // warps add (sum, correction) pairs with Knuth's two-sum, an error of about 2^-46 in FP32
 // instructions; FP64 shuffles and additions took 2 us a block on the slow FP64 pipe, all
@@ -668,8 +669,9 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_pixels(const DispArgs<R> a0, 
   const FDiv fH(H);
   auto task = [&](int idx, int &k) {
     if constexpr (CR1 > 0) {
-      k = idx % (CR1 * CR2 / 2);
-      return idx / (CR1 * CR2 / 2);
+      constexpr int h = (CR1 * CR2 + 1) / 2;
+      k = idx % h;
+      return idx / h;
     } else {
       return fH.div(idx, k);
     }

@@ -17,7 +17,9 @@ void ax0_dots(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int 
   case M: return disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, A, BB, false>, a, c, B, s);
       MUSG_DISP_PLANS(MUSG_C)
 #undef MUSG_C
-      default: break;
+      default:
+        if constexpr (D == 3)
+          if (disp_odd_ax0(FIN, false, pl, a, c, B, s)) return;
     }
   }
   disp_launch<R>(k_ax0_fwd<R, D, FIN, AX_DOTS, kRtPlan<D>, kRtPlan<D>, false>, a, c, B, s);

@@ -11,9 +11,18 @@
 
 namespace musg {
 
-// FP32: power-of-two axes have kernels with compile-time plans (0: none).  In FP64 the
-// arithmetic, not the indexing, sets the pace.
-#define MUSG_DISP_PLANS(X) X(32, 8, 4) X(64, 8, 8) X(128, 16, 8) X(256, 16, 16)
+// FP32: axes with kernels of a compile-time plan.  The others' kernels hold a body per
+// radix, compute strides and divide by lengths known at run time only, and spill where a
+// radix above 12 does not fit their registers (160^3 small strain 382 -> 312 us an
+// iteration, 63^3 70 -> 62 us, 45x77x81 76 -> 66 us).  Multiples of 32 up to 256 and, in 3-D,
+// the odd lengths of two factors up to 121: one kernel per length, pass and law is what
+// a build of two minutes holds.  In FP64 the arithmetic, not the indexing, sets the pace.
+#define MUSG_DISP_PLANS(X) \
+  X(32, 8, 4) X(64, 8, 8) X(96, 12, 8) X(128, 16, 8) X(160, 16, 10) X(192, 16, 12) X(224, 16, 14) X(256, 16, 16)
+#define MUSG_DISP_PLANS_ODD(X) \
+  X(15, 5, 3) X(21, 7, 3) X(25, 5, 5) X(27, 9, 3) X(33, 11, 3) X(35, 7, 5) X(39, 13, 3) X(45, 9, 5) X(49, 7, 7) \
+  X(51, 17, 3) X(55, 11, 5) X(63, 9, 7) X(65, 13, 5) X(75, 15, 5) X(77, 11, 7) X(81, 9, 9) X(85, 17, 5) X(91, 13, 7) \
+  X(99, 11, 9) X(105, 15, 7) X(117, 13, 9) X(119, 17, 7) X(121, 11, 11)
 inline int disp_fixed_plan(const TilePlan &pl) { return pl.blu ? 0 : pl.m; }
 
 // launch shape of one pass
@@ -40,8 +49,10 @@ template <typename R> int disp_threads(const TilePlan &pl, long P, long blocks, 
   t = std::max(64L, std::min(most, t));
   return (int)std::max(unit, std::min(most / unit, (t + unit - 1) / unit) * unit);
 }
-// the kernels' registers (kDispRegs) allow 512 threads, of the FP64 2-D ones 384
-template <typename R> long disp_most(const Spectral &sp) { return sizeof(R) == 8 && sp.g.dim == 2 ? 384 : 512; }
+// Registers (kDispRegs): 512 threads of FP64 kernels fit, of their 2-D ones 384.  FP32: two
+// blocks of 384 threads an SM; one of 480 left nothing to run at its barriers (160^3 small
+// strain 422 -> 382 us an iteration).
+template <typename R> long disp_most(const Spectral &sp) { return sizeof(R) == 8 && sp.g.dim == 3 ? 512 : 384; }
 inline long lcm32(long p) {
   long a = p;
   while (a % 32) a += p;
@@ -65,12 +76,20 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   if (!pl.m || !fits(T, optin_smem())) throw Error(MUSG_ERR_ARGUMENT, "first-axis FFT too long for one thread block");
   c.T = (int)T;
   c.ntx = (int)((Rr + T - 1) / T);
-  // sums: a bounded number of blocks, so that every block of the next pass can add
-  // their sums up itself
-  c.nbx = sums ? std::min(c.ntx, 4 * kDispSms / c.ng) : c.ntx;
-  c.blocks = c.nbx * c.ng;
   c.smem = (size_t)(T * per + tw);
-  c.threads = disp_threads<R>(pl, na * T, c.blocks, lcm32(na * T), disp_most<R>(sp));
+  auto threads = [&] { return disp_threads<R>(pl, na * T, (long)c.nbx * c.ng, lcm32(na * T), disp_most<R>(sp)); };
+  // With sums a block walks over several tiles, so that few sums are left to add up.  FP32:
+  // as many blocks as are resident at once (128^3, 606 blocks of which 456 were resident:
+  // 44 us, 456: 40 us, one block a tile: 45 us)
+  c.nbx = c.ntx;
+  if (sums) {
+    c.threads = threads();
+    const int regs = 65536 / (kDispRegs<R, 0> * c.threads), mem = (int)((227l << 10) / (c.smem + 1024));
+    const int resident = sizeof(R) == 8 ? 4 : std::max(1, std::min(8, std::min(regs, mem)));
+    c.nbx = std::min(c.ntx, std::max(1, resident * kDispSms / c.ng));
+  }
+  c.blocks = c.nbx * c.ng;
+  c.threads = threads();
   return c;
 }
 
@@ -122,6 +141,7 @@ template <typename R> DispShape disp_last_shape(const Spectral &sp) {
 #define MUSG_C(M, A, B) \
   case M: row = std::max<long>(row, row_strides(A, B).sp); break;
       MUSG_DISP_PLANS(MUSG_C)
+      MUSG_DISP_PLANS_ODD(MUSG_C)
 #undef MUSG_C
       default: break;
     }
@@ -221,5 +241,11 @@ void disp_pixels_in(bool fin, int tkind, bool delta, const DispArgs<R> &a, const
 // spectrum in, real field out
 template <typename R, int D>
 void disp_pixels_out(bool fin, const DispArgs<R> &a, const DispShape &c, cudaStream_t s);
+
+// FP32 3-D kernels of the odd compile-time plans (disp_odd_*.cu): false if the axis has none
+bool disp_odd_ax0(bool fin, bool step, const TilePlan &, const DispArgs<float> &, const DispShape &, int B, cudaStream_t);
+bool disp_odd_mid(bool fin, bool inv, const TilePlan &, const DispArgs<float> &, const DispShape &, int B, cudaStream_t);
+bool disp_odd_pixels_finite(int tk, const TilePlan &, const DispArgs<float> &, const DispShape &, int B, cudaStream_t);
+bool disp_odd_pixels_small(int tk, const TilePlan &, const DispArgs<float> &, const DispShape &, int B, cudaStream_t);
 
 }  // namespace musg

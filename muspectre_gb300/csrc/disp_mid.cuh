@@ -15,7 +15,8 @@ void mid(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cu
   case M: return disp_launch<R>(k_mid<R, FIN, INV, A, BB, false>, a, c, B, s);
       MUSG_DISP_PLANS(MUSG_C)
 #undef MUSG_C
-      default: break;
+      default:
+        if (disp_odd_mid(FIN, INV, pl, a, c, B, s)) return;
     }
   }
   disp_launch<R>(k_mid<R, FIN, INV, 0, 0, false>, a, c, B, s);

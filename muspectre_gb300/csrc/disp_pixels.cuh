@@ -21,7 +21,11 @@ void pixels_iteration(const TilePlan &pl, const DispArgs<R> &a, const DispShape 
   case M: disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, A, BB, false>, a, c, B, s); return;
       MUSG_DISP_PLANS(MUSG_PX)
 #undef MUSG_PX
-      default: break;
+      default:
+        if constexpr (D == 3 && FIN)
+          if (disp_odd_pixels_finite(TK, pl, a, c, B, s)) return;
+        if constexpr (D == 3 && !FIN)
+          if (disp_odd_pixels_small(TK, pl, a, c, B, s)) return;
     }
   }
   disp_launch<R>(k_pixels<R, D, FIN, TK, IN_SPEC, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, B, s);

@@ -108,6 +108,25 @@ def test_mixed_solve(mu, name, form):
     assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
 
 
+FIXED = [15, 21, 25, 27, 32, 33, 35, 39, 45, 49, 51, 55, 63, 64, 65, 75, 77, 81, 85, 91, 96, 99, 105, 117, 119, 121,
+         128, 160, 192, 224, 256]
+
+
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('n', FIXED)
+def test_mixed_solve_compile_time_plan(mu, n, form):
+    """Each length with kernels of its own, along each axis."""
+    load = _load(3, form)
+    for res in ([n, 3, 3], [3, n, 5], [5, 3, n]):
+        hom = {}
+        for prec in ('fp64', 'mixed'):
+            cell = _cell(mu, res, form, 3)
+            r = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 2000, precision=prec), 1e-8, 0.0)
+            assert r.success, r.message
+            hom[prec] = r.hom_stress
+        assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
 def test_uneven_batch(mu):
     grids = [GRIDS[k] for k in ('one_factor', 'two_factors', 'bluestein', 'power_of_two_axes', 'three_factors')]
     cells = [_cell(mu, g, 0, 3) for g in grids]
