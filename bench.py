@@ -182,17 +182,16 @@ def fp64_flops(name, npx, nk, res, d2=9):
     """Floating-point operations of one launch of an FP64 CG-iteration kernel (finite-strain
     LE1 tangent), counted as 5 m log2 m per complex transform of length m (two real rows
     share one; 2 more per real entry to unpack), about 200 per pixel for dP = K:dF from F
-    and S, 100 per k-point for the Green operator of a row triple, 2 per vector entry
-    per axpy or dot."""
+    and S, 2 per real vector entry per axpy or dot, and per k-point the expansion or
+    contraction with the wave vector (1 / |k| about 30, 4 per product with a component)."""
     L, n1, n0 = res[2], res[1], res[0]
     last = d2 * (2.5 * np.log2(L) + 2.0)
     return {
-        'last_axis_fwd_tangent': npx * (last + 200 + 2 * d2),
-        'axis1_fwd': nk * d2 * 5 * np.log2(n1),
-        'green_axis0': nk * (d2 * 10 * np.log2(n0) + 100),
-        'axis1_inv': nk * d2 * 5 * np.log2(n1),
-        'last_axis_inv_dot': npx * (last + 2 * d2),
-        'cg_update': npx * d2 * 6,
+        'axis0_inv_update': nk * (6 * 5 * np.log2(n0) + 3 * 12 + 30 + 6 * 2),
+        'axis1_inv_expand': nk * (9 * 5 * np.log2(n1) + 9 * 2),
+        'last_axis_tangent': npx * (2 * last + 200),
+        'axis1_fwd_contract': nk * (9 * 5 * np.log2(n1) + 9 * 2 + 3 * 2),
+        'axis0_fwd_dots': nk * (6 * 5 * np.log2(n0) + 30 + 3 * 8 + 4 * 6 * 2),
     }.get(name, 0.0)
 
 

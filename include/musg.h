@@ -139,6 +139,9 @@ int musg_cell_set_uniform_strain(musg_cell *cell, const double *strain);
 /* Cell::get_strain_vector / get_stress_vector (cell_base.cc:96-106): copies */
 int musg_cell_get_strain(musg_cell *cell, double *out);
 int musg_cell_set_strain(musg_cell *cell, const double *in);
+/* The same from component planes [i + D j][pixel], the layout on the device: no
+ * transposition on either side. */
+int musg_cell_set_strain_planes(musg_cell *cell, const double *in);
 int musg_cell_get_stress(musg_cell *cell, double *out);
 /* Cell::evaluate_stress_tangent (cell_base.cc:129-146); either output may be NULL */
 int musg_cell_evaluate_stress_tangent(musg_cell *cell, double *stress_out,
@@ -152,6 +155,8 @@ int musg_cell_apply_projection(musg_cell *cell, double *vec);
 int musg_cell_homogenised_stress(musg_cell *cell, double *out);
 /* Cell::evaluate_projected_directional_stiffness (cell_base.cc:150-192) */
 int musg_cell_directional_stiffness(musg_cell *cell, const double *dF, double *dP);
+/* dF as component planes (musg_cell_set_strain_planes); dP pixel-major as above. */
+int musg_cell_directional_stiffness_planes(musg_cell *cell, const double *dF, double *dP);
 /* G(K:dF) through the kernels of one CG iteration (the operator SolverCG applies) in
  * the given precision (MUSG_PRECISION_FP64 or _MIXED = FP32 operator).  No reference
  * counterpart: it exposes the operator of the mixed-precision path for checking.

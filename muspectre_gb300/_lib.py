@@ -87,10 +87,12 @@ _SIGNATURES = {
     'musg_cell_set_uniform_strain': (C.c_int, [_P, _D]),
     'musg_cell_get_strain': (C.c_int, [_P, _D]),
     'musg_cell_set_strain': (C.c_int, [_P, _D]),
+    'musg_cell_set_strain_planes': (C.c_int, [_P, _D]),
     'musg_cell_get_stress': (C.c_int, [_P, _D]),
     'musg_cell_evaluate_stress_tangent': (C.c_int, [_P, _D, _D]),
     'musg_cell_apply_projection': (C.c_int, [_P, _D]),
     'musg_cell_directional_stiffness': (C.c_int, [_P, _D, _D]),
+    'musg_cell_directional_stiffness_planes': (C.c_int, [_P, _D, _D]),
     'musg_cell_cg_operator': (C.c_int, [_P, C.c_int, _D, _D]),
     'musg_cell_save_history_variables': (C.c_int, [_P]),
     'musg_cell_homogenised_stress': (C.c_int, [_P, _D]),

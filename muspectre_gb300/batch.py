@@ -7,7 +7,7 @@ graph.  Cells of one grid run the solo kernels with problem index = blockIdx.y, 
 each cell's results are those of a solo ``newton_cg`` call on it, bit for bit.  Cells
 of different grids (same dimension, formulation and material-law kind) run grouped
 launches: each cell owns a range of the grid's blocks and its own FFT plans and
-sizes (the generic pass kernels), with results equal to the solo ones within
+sizes (kernels of runtime plans), with results equal to the solo ones within
 rounding.
 """
 from __future__ import annotations

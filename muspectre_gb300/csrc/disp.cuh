@@ -28,7 +28,7 @@
 // transform; mid_inv expands w into the columns k1 w and k2 w, and mid_fwd contracts
 // the two columns again.  2-D uses the columns k0 w, k1 w directly.
 //
-// Scalars.  ax0_fwd leaves per-block sums; the last of its (at most 4 x 152) blocks to
+// Scalars.  ax0_fwd leaves per-block sums; the last of its (at most 8 x 152) blocks to
 // finish adds them up in a fixed order and sets alpha, beta and the loop flag, once:
 // the FP64 pipe is too slow to do it in every block of the next pass (2 us a block,
 // 30 us of the 128^3 update pass).  alpha = r.r / p.q, and the new r.r for beta and the
@@ -40,15 +40,16 @@
 // Why: the real-space iteration this replaces moved 16 real fields and the tangent data
 // (155 component spectra at 128^3 finite strain, 146 small strain) in eight launches;
 // this one moves 101 and 78 in five.  One iteration on GB300, before -> now: 128^3 finite
-// 291 -> 268 us, 63^3 115 -> 80, 45x77x81 164 -> 83, 160^3 small strain 1279 -> 486 (the
+// 291 -> 226 us, 63^3 115 -> 62, 45x77x81 164 -> 66, 160^3 small strain 1279 -> 309 (the
 // odd and 5-smooth lengths also gain from the two-stage transforms of tile_fft.cuh).
-// Without the Nyquist column (64 instead of 65 columns: whole lines, 128^3 axis-1 passes
-// 39 -> 34 and 43 -> 33 us) and with the sums reduced in FP32 pairs (51 -> 45 us) the
-// 128^3 iteration takes 246 us.  What bounds the passes is latency and instruction issue
-// at 25-30% of the warp slots, not bandwidth: 128^3 moves 850 MB in 246 us.
-// FP64 (bound by the FP64 pipe and, on small grids, latency): 51^2 252 -> 95 us, where
-// the factors 17 x 3 replace Bluestein over 105, 35^3 182 -> 147; a 55^3 projection
-// 2.05 -> 0.43 ms.
+// Of that at 128^3: without the Nyquist column (64 instead of 65 columns: whole lines)
+// the axis-1 passes 39 -> 34 and 43 -> 33 us, sums in FP32 pairs 51 -> 45 us, the last
+// axis by row pairs 88 -> 76 us.  What bounds the passes is latency between the barriers
+// of a tile and instruction issue, at 20-24 warps an SM (80 registers), not bandwidth:
+// 128^3 moves 850 MB in 226 us, 0.55 of the copy bandwidth.
+// FP64 (bound by the FP64 pipe and, on small grids, latency): 51^2 252 -> 88 us, where
+// the factors 17 x 3 replace Bluestein over 105, 35^3 182 -> 144; a 55^3 projection
+// 2.05 -> 0.40 ms.
 #pragma once
 
 #include "spectral.cuh"

@@ -1,6 +1,6 @@
 // Host side of the displacement-space passes (disp.cuh): launch shapes, arguments and
-// the dispatch over compile-time plans, shared by disp.cu and the passes' translation units (one per pass, so that they build
-// side by side).
+// the dispatch over compile-time plans, shared by disp.cu and the passes' translation
+// units (several, so that they build side by side).
 #pragma once
 
 #include <algorithm>
@@ -37,8 +37,8 @@ inline bool disp_finite(const Spectral &sp) { return sp.proj_kind != MUSG_PROJ_S
 
 // Threads per block for tiles of P pencils: about 16 points of the tile per thread (one
 // radix-16 or two radix-8 butterflies).  FP64, whose instructions take 16 cycles of an SM
-// each: on grids too small to fill the SMs up to one butterfly per thread (35^3 147 ->
-// 135 us an iteration; in FP32 the same rule cost more in per-thread setup than it
+// each: on grids too small to fill the SMs up to one butterfly per thread (35^3 149 ->
+// 142 us an iteration; in FP32 the same rule cost more in per-thread setup than it
 // gained, 63^3 77 -> 92 us).  A multiple of `unit` (the pencils of a pencil-fast tile, or
 // a warp).
 template <typename R> int disp_threads(const TilePlan &pl, long P, long blocks, long unit, long most) {

@@ -93,8 +93,8 @@ def voronoi(n=64, nseeds=32, nsteps=20, seed=11):
 
 
 def build_spheres_cell(mu, w, allow_even=True, flags=None):
-    """The GPU cell; ``flags`` = FFT_PlanFlags (default: measure, i.e. autotuned launch
-    shapes, as the reference's demonstrators plan with FFTW_MEASURE)."""
+    """The GPU cell; ``flags`` = FFT_PlanFlags (default: measure, as the reference's
+    demonstrators plan with FFTW_MEASURE; the launch shapes follow from the grid either way)."""
     cell = mu.Cell(w['res'], w['lengths'], mu.Formulation.finite_strain, allow_even=allow_even)
     mu.material.MaterialLinearElastic1_3d.make(cell, 'inclusions', w['E_incl'], w['nu']).add_pixels(w['inside'])
     mu.material.MaterialLinearElastic1_3d.make(cell, 'matrix', w['E_matrix'], w['nu']).add_pixels(~w['inside'])

@@ -82,6 +82,40 @@ def test_operator_wide_radix_2d(mu, r):
         assert np.linalg.norm(cell.cg_operator(dF, 'mixed') - ref) <= 1e-5 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('res', [[149, 5], [6, 157], [359, 4], [3, 359], [509, 3], [5, 509]])
+def test_operator_bluestein_2d(mu, res, form):
+    """Primes whose Bluestein length takes three factors, against FP64 and against NumPy."""
+    n = int(np.prod(res))
+    cell = _cell(mu, res, form, 3)
+    rng = np.random.default_rng(5)
+    F = 0.01 * rng.normal(size=(2, 2, n))
+    F = 0.5 * (F + F.transpose(1, 0, 2)) if form else F + np.eye(2)[:, :, None]
+    cell.evaluate_stress_tangent(F.reshape(4, n))
+    dF = rng.normal(size=(4, n))
+    ref = cell.directional_stiffness(dF)
+    assert np.linalg.norm(cell.cg_operator(dF, 'mixed') - ref) <= 1e-5 * np.linalg.norm(ref)
+    kx, ky = np.fft.fftfreq(res[0]) * res[0], np.fft.fftfreq(res[1]) * res[1] / 1.3
+    k = np.stack(np.meshgrid(kx, ky, indexing='ij')).reshape(2, n)
+    nyq = np.zeros(res, bool)
+    for d in range(2):
+        if res[d] % 2 == 0:
+            nyq[(slice(None),) * d + (res[d] // 2,)] = True
+    k2 = (k * k).sum(0)
+    xi = np.where((k2 > 0) & ~nyq.reshape(-1), k / np.sqrt(np.where(k2 > 0, k2, 1)), 0)
+    f = rng.normal(size=(4, n))  # the projection against NumPy's transform in FP64
+    f = 0.5 * (f + f[[0, 2, 1, 3]]) if form else f
+    fh = np.fft.fft2(f.reshape(2, 2, *res), axes=(2, 3)).reshape(2, 2, n)  # [j][i]
+    if form:
+        t = np.einsum('jin,jn->in', fh, xi)
+        v = 2 * t - np.einsum('in,in->n', t, xi) * xi
+        gh = 0.5 * (np.einsum('in,jn->jin', v, xi) + np.einsum('in,jn->ijn', v, xi))
+    else:
+        gh = np.einsum('jn,in->jin', xi, np.einsum('jin,jn->in', fh, xi))
+    g = np.fft.ifft2(gh.reshape(2, 2, *res), axes=(2, 3)).real.reshape(4, n)
+    assert np.linalg.norm(cell.project(f) - g) <= 1e-12 * np.linalg.norm(f)
+
+
 SOLVED = ['one_factor', 'two_factors', 'bluestein', 'many_factors', 'power_of_two_axes', 'thin']
 
 
@@ -125,6 +159,36 @@ def test_mixed_solve_compile_time_plan(mu, n, form):
             assert r.success, r.message
             hom[prec] = r.hom_stress
         assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
+@pytest.mark.parametrize('res', [[7, 5, 3], [3, 9], [1, 1, 1]])
+def test_inputs_as_planes_and_pixel_major(mu, res):
+    """A C-ordered (D², N) array goes up as it is; its Fortran-ordered copy, a strided view
+    and the flat pixel-major vector are transposed first.  The same values arrive."""
+    d, n = len(res), int(np.prod(res))
+    cell = _cell(mu, res, 0, 3) if n > 1 else None
+    if cell is None:
+        cell = mu.Cell(res, [1.0] * d, 0)
+        getattr(mu.material, 'MaterialLinearElastic1_%dd' % d).make(cell, 'm', 3e9, .25).add_pixels(np.ones(n, bool))
+        cell.initialise()
+    rng = np.random.default_rng(1)
+    F = 0.01 * rng.normal(size=(d * d, n)) + np.eye(d).reshape(-1, 1)
+    dF = rng.normal(size=(d * d, n))
+    wide = np.empty((d * d, 2 * n))
+    ways = [lambda a: a, np.asfortranarray, lambda a: a.T.reshape(-1).copy()]
+
+    def strided(a):
+        wide[:, ::2] = a
+        return wide[:, ::2]
+
+    got = []
+    for way in ways + [strided]:
+        P = cell.evaluate_stress_tangent(way(F)).copy()
+        got.append((cell.get_strain().copy(), P, cell.directional_stiffness(way(dF)).copy()))
+    assert np.array_equal(got[0][0], F)
+    for g in got[1:]:
+        for a, b in zip(got[0], g):
+            assert np.array_equal(a, b)
 
 
 def test_uneven_batch(mu):
