@@ -24,6 +24,10 @@ __device__ __forceinline__ void tile_stage_any(int rad, uint32_t buf, uint32_t t
   case RAD: tile_stage_rt<T, RAD, OP>(buf, tw, lay, a); break;
     MUSG_TILE_RADICES(MUSG_TS)
 #undef MUSG_TS
+#define MUSG_TS(RAD) \
+  case RAD: if constexpr (OP == OP_B1 || OP == OP_BM || OP == OP_B2) tile_stage_rt<T, RAD, OP>(buf, tw, lay, a); break;
+    MUSG_TILE_RADICES_2D(MUSG_TS)
+#undef MUSG_TS
     default: tile_stage_rt<T, 1, OP>(buf, tw, lay, a); break;
   }
 }

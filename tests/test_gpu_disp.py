@@ -85,7 +85,7 @@ def test_operator_wide_radix_2d(mu, r):
 @pytest.mark.parametrize('form', [0, 1])
 @pytest.mark.parametrize('res', [[149, 5], [6, 157], [359, 4], [3, 359], [509, 3], [5, 509]])
 def test_operator_bluestein_2d(mu, res, form):
-    """Primes whose Bluestein length takes three factors, against FP64 and against NumPy."""
+    """Primes whose Bluestein length takes three factors, or two radices above 17."""
     n = int(np.prod(res))
     cell = _cell(mu, res, form, 3)
     rng = np.random.default_rng(5)
