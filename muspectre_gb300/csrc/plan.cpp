@@ -242,7 +242,7 @@ void TilePlan::factor(int n_, int widest, bool smallest) {
   } else {
     // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass.  Two
     // wide radices in place of three factors above 256 only (324 x 359 mixed 14.1 -> 11.4
-    // ms, 127 x 509 14.6 -> 13.7): their registers spill, which costs FP64 more than the
+    // ms, 127 x 509 14.6 -> 13.1): their registers spill, which costs FP64 more than the
     // passes it saves (157 x 149 FP64 168 -> 195 ms)
     const int wide = n > 256 ? widest : 17;
     blu = 1;
