@@ -108,6 +108,9 @@ template <typename R> DispProb<R> disp_prob(Spectral &sp, const DispVectors &v, 
   pb.x = (T *)v.x;
   pb.st = st;
   pb.partial = partial;
+  pb.xi0 = xi_table<R>(sp, 0);
+  pb.xi1 = xi_table<R>(sp, 1);
+  pb.xi2 = sp.g.dim == 3 ? xi_table<R>(sp, 2) : nullptr;
   return pb;
 }
 

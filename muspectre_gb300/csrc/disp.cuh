@@ -63,6 +63,7 @@ template <typename R> struct DispProb {
   typename V2<R>::T *r, *q, *p, *x;   // [D][nk]
   CGState *st;
   double *partial;                    // 4 sums per block of ax0_fwd
+  const R *xi0, *xi1, *xi2;           // wave numbers: equal grids may have boxes of different lengths
   TangentData<R> td;
 };
 
@@ -77,7 +78,6 @@ template <typename R> struct DispArgs {
   int sp, S;              // last-axis strides of pencils and slot groups
   int Rr;                 // k-points per e of axis 0 (a component holds fewer than 2^31)
   long long nk, npx, nrows;
-  const R *xi0, *xi1, *xi2;
   int nyq0, nyq1, nyq2;
   R scale;                // 1 / sqrt(N)
   const double *in64;     // real input planes
@@ -254,8 +254,8 @@ template <int D, typename R> struct Wave {
     int i1, i2 = 0;
     if (D == 3) i1 = FDiv(a.nh).div(rho, i2);
     else i1 = rho;
-    k1 = a.xi1[i1];
-    k2 = D == 3 ? a.xi2[i2] : R(0);
+    k1 = a.pb.xi1[i1];
+    k2 = D == 3 ? a.pb.xi2[i2] : R(0);
     s = k1 * k1;
     if (D == 3) s += k2 * k2;
     e_zero = i1 == 0 && i2 == 0 ? 0 : -1;
@@ -263,7 +263,7 @@ template <int D, typename R> struct Wave {
     kl = D == 3 ? i2 : i1;
   }
   __device__ __forceinline__ R at(const DispArgs<R> &a, int e, R *k) const {
-    k[0] = a.xi0[e];
+    k[0] = a.pb.xi0[e];
     k[1] = k1;
     if (D == 3) k[D - 1] = k2;
     if (dead || e == e_zero || e == a.nyq0) return R(0);
@@ -439,7 +439,7 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, con
         });
   } else {
     T *b0 = a.pb.spec + b, *b1 = b0 + 3 * a.nk, *b2 = b1 + 3 * a.nk;
-    const R x2 = ok ? a.xi2[k2] : R(0);
+    const R x2 = ok ? a.pb.xi2[k2] : R(0);
     for (int hi = 2; hi >= 0; hi -= nc) {  // columns hi, hi - 1, ..., hi - nc + 1
       const int c0 = hi - nc + 1, c = c0 + map.p / Tt;  // this thread's column
       if (hi < 2) __syncthreads();                      // the previous column's tile is free
@@ -450,7 +450,7 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, con
         const R kc = c == 0 ? R(1) : x2;
         auto ld = [&](int e, int, int) {
           const T w = ok ? src[e * nh] : T{R(0), R(0)};
-          const R x1 = a.xi1[e], k = c == 1 ? x1 : kc;
+          const R x1 = a.pb.xi1[e], k = c == 1 ? x1 : kc;
           return T{k * w.x, k * w.y};
         };
         auto st = [&](int e, int, int, T v) {
@@ -476,7 +476,7 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, con
           const int s = slots.nat(e);
           if (c0 == 0) b0[e * nh] = buf[map.at(s, t)];
           if (c0 <= 1 && hi >= 1) {
-            const R k1 = a.xi1[e];
+            const R k1 = a.pb.xi1[e];
             const T f1 = buf[map.at(s, (1 - c0) * Tt + t)];
             const T f2 = hi == 2 ? buf[map.at(s, (2 - c0) * Tt + t)] : b2[e * nh];
             b1[e * nh] = T{k1 * f1.x + f2.x, k1 * f1.y + f2.y};

@@ -172,9 +172,6 @@ template <typename R> DispArgs<R> disp_base(Spectral &sp) {
   a.nk = disp_nk(sp);
   a.npx = sp.g.npx;
   a.nrows = sp.g.nrows;
-  a.xi0 = xi_table<R>(sp, 0);
-  a.xi1 = xi_table<R>(sp, 1);
-  a.xi2 = D == 3 ? xi_table<R>(sp, 2) : nullptr;
   auto nyq = [&](int d) { return (sp.allow_even && sp.g.n[d] % 2 == 0) ? sp.g.n[d] / 2 : -1; };
   a.nyq0 = nyq(0);
   a.nyq1 = nyq(1);

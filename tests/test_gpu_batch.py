@@ -126,3 +126,37 @@ def test_uneven_batch_matches_solo(mu, case, precision):
         hs = solo.homogenised_stress()
         assert np.linalg.norm(hb - hs) <= tol * np.linalg.norm(hs), (g, np.linalg.norm(hb - hs) / np.linalg.norm(hs))
         assert np.allclose(r.hom_stress, hb, rtol=0, atol=1e-12 * np.abs(hb).max())
+
+
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+def test_batch_of_equal_grids_in_boxes_of_different_lengths(mu, precision, form):
+    """Cells of one grid share the launches of a batch; each keeps the wave vectors of its
+    own box, along every axis: the results are the solo ones, bit for bit."""
+    boxes = ([1.0, 1.0, 1.0], [1.0, 2.5, 0.4], [3.0, 1.0, 1.0])
+    load = np.zeros((3, 3))
+    load[0, 0] = 0.01
+    load[0, 1] = load[1, 0] = 0.003
+
+    def cell(box):
+        rng = np.random.default_rng(7)
+        c = mu.Cell([16, 9, 32], box, form, allow_even=True)
+        hard = rng.random(16 * 9 * 32) < 0.3
+        make = mu.material.MaterialLinearElastic1_3d.make
+        make(c, 'hard', 30e9, .3).add_pixels(hard)
+        make(c, 'soft', 3e9, .25).add_pixels(~hard)
+        c.initialise()
+        return c
+
+    cells = [cell(b) for b in boxes]
+    rb = mu.batch.BatchSolver(cells, 1e-8, 2000, precision=precision).newton_cg(load, 1e-8, 0.0)
+    hom = []
+    for b, c, res in zip(boxes, cells, rb):
+        solo = cell(b)
+        rs = mu.solvers.newton_cg(solo, load, mu.solvers.SolverCG(solo, 1e-8, 2000, precision=precision), 1e-8, 0.0)
+        assert res[0].success and rs.success
+        assert (res[0].nb_it, res[0].nb_fev) == (rs.nb_it, rs.nb_fev)
+        assert np.array_equal(res[0].stress, rs.stress)
+        assert np.array_equal(c.get_strain(), solo.get_strain())
+        hom.append(rs.hom_stress)
+    assert np.linalg.norm(hom[0] - hom[1]) > 1e-4 * np.linalg.norm(hom[0])  # the boxes do differ
