@@ -122,10 +122,10 @@ struct TilePlan {
   void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;
   void *tw32 = nullptr, *chirp32 = nullptr, *bf32 = nullptr;
   // factors only (host), two up to `widest` (17, or 32 for the axes of a 2-D grid); build()
-  // also makes the device tables.  smallest: the shortest Bluestein length instead of the
-  // cheapest
-  void factor(int n, int widest, bool smallest = false);
-  void build(int n, int widest);
+  // also makes the device tables.  points: the longest plan of three or more factors that
+  // fits the axis' passes; smallest: the shortest Bluestein length instead of the cheapest
+  void factor(int n, int widest, long points, bool smallest = false);
+  void build(int n, int widest, long points);
   void release();
   template <typename R> TilePlanD<R> device() const;
   int buffers() const { return r1 ? 1 : 2; }  // tile buffers a transform needs
@@ -218,6 +218,9 @@ struct Spectral {
   long tune_bytes[2][3] = {{73728, 49152, 73728}, {73728, 49152, 73728}};
   void init(int dim, const int *res, int ncomp, int proj_kind, const double *lengths,
             bool allow_even, bool want32);
+  // points of a pencil of two buffers in `bytes` of shared memory, for the FP64 pass over
+  // `axis` that holds the most pencils at once (disp_launch.cuh)
+  long tile_points(int axis, long bytes) const;
   void ensure_tiles();
   void ensure32();
   void release();

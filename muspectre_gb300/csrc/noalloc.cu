@@ -161,7 +161,7 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
   size_t off_tw[3], off_chirp[3], off_bf[3], off_xi[3];
   for (int d = 0; d < dim; ++d) {
     TilePlan &ap = sp.tp[d];
-    ap.factor(sp.g.n[d], dim == 2 ? 32 : 17, true);
+    ap.factor(sp.g.n[d], dim == 2 ? 32 : 17, 1 << 16, true);
     if (!ap.m) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
     off_tw[d] = off;
     off += align256((size_t)ap.m * sizeof(double2));

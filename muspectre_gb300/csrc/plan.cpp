@@ -10,6 +10,7 @@
 #include <mutex>
 #include <vector>
 
+#include "launch_util.h"
 #include "musg_internal.h"
 
 namespace musg {
@@ -232,7 +233,7 @@ int tile_factor(int m, int widest, int *rad, double &cost) {
 
 }  // namespace
 
-void TilePlan::factor(int n_, int widest, bool smallest) {
+void TilePlan::factor(int n_, int widest, long points, bool smallest) {
   n = n_;
   m = nst = r1 = r2 = blu = 0;
   if (n > (1 << 16)) return;  // longer than any tile: the passes refuse it (m = 0)
@@ -246,20 +247,26 @@ void TilePlan::factor(int n_, int widest, bool smallest) {
     // passes it saves (157 x 149 FP64 168 -> 195 ms)
     const int wide = n > 256 ? widest : 17;
     blu = 1;
+    // the cheapest may be too long for its pass where a shorter one fits (899 in 2-D: 2048
+    // points of four components in two buffers are 262 KB, 1800 fit); where none fits, the
+    // pass refuses the length
     double best = 1e30;
-    for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
-      int rad[kMaxStages];
-      double c = 0;
-      const int ns = tile_factor(k, wide, rad, c);
-      if (!ns) continue;
-      if (smallest && m) break;
-      c *= k;
-      if (c < best) {
-        best = c;
-        m = k;
-        nst = ns;
-        for (int q = 0; q < ns; ++q) radix[q] = rad[q];
+    for (long most : {points, (long)(1 << 28)}) {
+      for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
+        int rad[kMaxStages];
+        double c = 0;
+        const int ns = tile_factor(k, wide, rad, c);
+        if (!ns || (ns > 2 && k > most)) continue;
+        if (smallest && m) break;
+        c *= k;
+        if (c < best) {
+          best = c;
+          m = k;
+          nst = ns;
+          for (int q = 0; q < ns; ++q) radix[q] = rad[q];
+        }
       }
+      if (m) break;
     }
     if (!m) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
   }
@@ -267,9 +274,9 @@ void TilePlan::factor(int n_, int widest, bool smallest) {
   r2 = nst == 2 ? radix[1] : 0;
 }
 
-void TilePlan::build(int n_, int widest) {
+void TilePlan::build(int n_, int widest, long points) {
   release();
-  factor(n_, widest);
+  factor(n_, widest, points);
   if (m) build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
 }
 
@@ -340,9 +347,17 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
   if (want32) ensure32();
 }
 
+long Spectral::tile_points(int axis, long bytes) const {
+  const int D = g.dim, sym = D * (D + 1) / 2;
+  const bool fin = proj_kind != MUSG_PROJ_SMALL_STRAIN;
+  // a pass over a middle axis falls back to one component at a time
+  const int pencils = axis == D - 1 ? (fin ? D * D : sym) : axis == 0 ? (fin ? 2 : sym) : 1;
+  return bytes / (pencils * 2 * (long)sizeof(double2));
+}
+
 void Spectral::ensure_tiles() {
   for (int d = 0; d < g.dim; ++d)
-    if (tp[d].n != g.n[d]) tp[d].build(g.n[d], g.dim == 2 ? 32 : 17);
+    if (tp[d].n != g.n[d]) tp[d].build(g.n[d], g.dim == 2 ? 32 : 17, tile_points(d, optin_smem()));
 }
 
 void Spectral::ensure32() {
