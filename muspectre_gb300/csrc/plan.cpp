@@ -188,18 +188,31 @@ namespace {
 
 // arithmetic per point of one radix-r stage, in units of one addition per point: what
 // the factor choice below weighs (small composites cost about 2 log2 r and a twiddle,
-// the direct primes about r)
-double stage_cost(int r) {
-  static const double c[33] = {0,  0,  2,  4.5, 4,  8,    6.5, 11, 6.5, 9,  10, 15, 8.5, 18, 13, 12.5, 9,
-                               23, 11, 0,  12,  15, 17,   11,  0,  16,  20, 14, 15, 0,   15, 0,  11};
-  return c[r] + 4.0;  // + twiddles and a shared-memory round trip
+// the direct primes about r; 24 by measurement: 360 points as 24 x 15 take 6.9 ms of a
+// 2-D solve, as 20 x 18 7.1 ms); 0: no such stage
+constexpr double kStageCost[33] = {0,  0,  2,  4.5, 4,  8,    6.5, 11, 6.5, 9,  10, 15, 8.5, 18, 13, 12.5, 9,
+                                   23, 11, 0,  12,  15, 17,   0,   10, 16,  20, 14, 15, 0,   15, 0,  11};
+constexpr bool has_stage(int r) { return r <= 17 || (r <= 32 && r != 19 && r != 23 && r != 29 && r != 31); }
+constexpr bool stage_costs_given() {
+  for (int r = 2; r <= 32; ++r)
+    if ((kStageCost[r] > 0) != has_stage(r)) return false;
+  return true;
 }
-bool has_stage(int r) { return r <= 17 || (r <= 32 && r != 19 && r != 23 && r != 29 && r != 31); }
+static_assert(stage_costs_given(), "a cost for every radix, and for no other number");
+double stage_cost(int r) { return kStageCost[r] + 4.0; }  // + twiddles and a shared-memory round trip
 
 // the cheapest factorisation of m into radices (no heap: the allocation-free projection
 // plans with it): two factors up to `widest` (r1 >= r2, possibly 1) if there are any, else
-// the fewest up to 17; the number of factors in rad, 0 when a prime above 17 divides m
+// the fewest up to 17; the number of factors in rad, 0 when a prime above 17 divides m.
+// Radices above 17 only where no two up to 17 do, and the most even pair among equals:
+// a thread runs a whole butterfly, so on grids that leave the SMs idle the widest one sets
+// the time (FP64 32^2 as 8 x 4 instead of one radix 32: 67 -> 32 ms, 64^2 as 8 x 8 instead
+// of 32 x 2: 74 -> 43 ms, 64^3 as 8 x 8 instead of 16 x 4: 316 -> 285 ms).
 int tile_factor(int m, int widest, int *rad, double &cost) {
+  if (widest > 17) {
+    const int k = tile_factor(m, 17, rad, cost);
+    if (k == 2) return k;
+  }
   cost = 1e30;
   int n = 0;
   for (int a = 1; a <= widest; ++a)
@@ -207,7 +220,7 @@ int tile_factor(int m, int widest, int *rad, double &cost) {
       const int b = m / a;
       if (b < a || !has_stage(a) || !has_stage(b)) continue;
       const double c = (a > 1 ? stage_cost(a) : 0.0) + (b > 1 ? stage_cost(b) : 0.0);
-      if (c < cost) {
+      if (c <= cost) {  // a rises: the later of equals is the more even
         cost = c;
         rad[0] = b;
         rad[1] = a;

@@ -1,6 +1,7 @@
 // Host check of the FFT plans of the displacement-space passes: every axis length whose
 // shortest 7-smooth plan fits the shared memory of a block gets a plan that fits its
-// passes too.  Prints the lengths that do not; exit status 1 if there are any.
+// passes too, and radices above 17 appear only where no two up to 17 make the length.
+// Prints the lengths that fail; exit status 1 if there are any.
 #include <algorithm>
 #include <cstdio>
 
@@ -45,6 +46,16 @@ int main() {
           }
         }
       }
+  for (int n = 1; n <= 1024; ++n) {
+    TilePlan t;
+    t.factor(n, 32, 1 << 28);
+    bool narrow = false;
+    for (int a = 1; a <= 17; ++a) narrow |= n % a == 0 && n / a <= 17;
+    if (narrow && (t.blu || t.nst != 2 || t.r1 > 17)) {
+      std::printf("length %d: %d x %d\n", n, t.r1, t.r2);
+      ++bad;
+    }
+  }
   std::printf("%d lengths checked, %d refused\n", checked, bad);
   return bad ? 1 : 0;
 }
