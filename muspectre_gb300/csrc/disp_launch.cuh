@@ -60,7 +60,11 @@ inline long lcm32(long p) {
 }
 
 // axis-0 passes: tiles of T consecutive k-points.  16 complex values are a 128-byte
-// line; narrower tiles where the grid would otherwise leave SMs without a block.
+// line; narrower tiles where the grid would otherwise leave SMs without a block.  A
+// Bluestein axis, several times the work per point, goes on below four points while most
+// SMs have none (16 bytes at least, FP32 only below half a wave): 157 x 149 FP64, 38 blocks
+// -> 150, 168 -> 109 ms; 359 x 324 small strain mixed, 41 -> 81, 12.8 -> 11.6 ms.  One
+// point of 8 bytes costs more than it gains on half-filled grids (401^2 19.6 -> 20.5 ms).
 template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   const bool fin = disp_finite(sp);
   const int D = sp.g.dim, na = fin ? 2 : D * (D + 1) / 2;
@@ -72,7 +76,9 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   auto fits = [&](long T, long cap) { return T * per + tw <= cap; };
   long T = 16;
   while (T > 1 && !fits(T, 100 << 10)) T >>= 1;
-  while (T > 4 && (Rr + T - 1) / T * c.ng < 2 * kDispSms) T >>= 1;
+  auto blocks = [&] { return (Rr + T - 1) / T * c.ng; };
+  while (T > 4 && blocks() < 2 * kDispSms) T >>= 1;
+  while (pl.blu && T > 1 && blocks() < (T * cb > 16 ? kDispSms : kDispSms / 2)) T >>= 1;
   if (!pl.m || !fits(T, optin_smem())) throw Error(MUSG_ERR_ARGUMENT, "first-axis FFT too long for one thread block");
   c.T = (int)T;
   c.ntx = (int)((Rr + T - 1) / T);

@@ -161,6 +161,23 @@ def test_mixed_solve_compile_time_plan(mu, n, form):
         assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
 
 
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('res', [[67, 9], [67, 400], [157, 149], [359, 62], [401, 640]])
+def test_solve_bluestein_first_axis_2d(mu, res, form):
+    """Tiles of one, two and four k-points on a Bluestein axis 0: the sums over partly filled
+    tiles; FP64 and mixed solves agree within 1e-6, and both equilibrate."""
+    load = _load(2, form)
+    hom = {}
+    for prec in ('fp64', 'mixed'):
+        cell = _cell(mu, res, form, 3)
+        r = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 3000, precision=prec), 1e-8, 0.0)
+        assert r.success, r.message
+        P = cell.evaluate_stress_tangent(cell.get_strain())
+        assert np.linalg.norm(cell.project(P)) <= 1e-5 * np.linalg.norm(P)
+        hom[prec] = r.hom_stress
+    assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
 @pytest.mark.parametrize('res', [[7, 5, 3], [3, 9], [1, 1, 1]])
 def test_inputs_as_planes_and_pixel_major(mu, res):
     """A C-ordered (D², N) array goes up as it is; its Fortran-ordered copy, a strided view
