@@ -25,9 +25,10 @@ LIB = os.path.join(HERE, 'libmusg.so')
 
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
-# the out-of-line tile transforms are linked into kernels of 80 (FP32) and 128 registers
-# (device code is relocatable; a kernel takes the registers of the functions it calls)
-EXTRA = {'tile_stages_f32.cu': ['-maxrregcount=80'], 'tile_stages_f64.cu': ['-maxrregcount=128']}
+# the out-of-line tile transforms take the registers of the kernels they are linked into
+# (device code is relocatable): 80 (FP32) and 128 in 3-D, 128 and 168 on 2-D grids
+EXTRA = {'tile_stages_f32.cu': ['-maxrregcount=80'], 'tile_stages_f64.cu': ['-maxrregcount=128'],
+         'tile_stages2_f32.cu': ['-maxrregcount=128'], 'tile_stages2_f64.cu': ['-maxrregcount=168']}
 
 
 def _nvcc():

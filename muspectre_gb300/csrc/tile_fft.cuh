@@ -22,7 +22,7 @@
 //
 // Kernels come with a compile-time plan (two stages inline, indices folded) or a runtime
 // one: its two stages are inline too, one body per radix; Bluestein and three or more
-// factors are one out-of-line function (tile_stages.cu, linked into every kernel that
+// factors are one out-of-line function (tile_stages.cuh, linked into every kernel that
 // calls it), which addresses shared memory by its 32-bit window address.
 #pragma once
 
@@ -264,14 +264,16 @@ template <> struct SlotMap<-2, -2> : SlotMapRt { using SlotMapRt::SlotMapRt; };
 // with the exchange between the stages in buf; the caller synchronises before if ld reads
 // shared memory, and after before buf is used again.
 
-// runtime plans, out of line (tile_stages.cu): true when the result is in the second buffer
-__device__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode, int blu,
-                            const float2 *tw, const float2 *chirp, const float2 *bf, const TileLay lay, uint32_t buf,
-                            uint32_t buf2, int P, uint32_t tws);
-
-__device__ bool tile_fft_rt(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode, int blu,
-                            const double2 *tw, const double2 *chirp, const double2 *bf, const TileLay lay, uint32_t buf,
-                            uint32_t buf2, int P, uint32_t tws);
+// runtime plans, out of line (tile_stages.cuh): true when the result is in the second buffer.
+// tile_fft_rt: radices up to 17, in the registers of the 3-D kernels; tile_fft_rt2: those of
+// 2-D grids, up to 32, in theirs (401^2 mixed 19.4 -> 17.6 ms, 449^2 23.1 -> 20.2)
+#define MUSG_TILE_FFT_RT(NAME, T)                                                                                    \
+  __device__ bool NAME(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode, int blu, const T *tw, \
+                       const T *chirp, const T *bf, const TileLay lay, uint32_t buf, uint32_t buf2, int P, uint32_t tws);
+MUSG_TILE_FFT_RT(tile_fft_rt, float2)
+MUSG_TILE_FFT_RT(tile_fft_rt, double2)
+MUSG_TILE_FFT_RT(tile_fft_rt2, float2)
+MUSG_TILE_FFT_RT(tile_fft_rt2, double2)
 
 #define MUSG_TILE_RADICES(X) \
   X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17)
@@ -310,14 +312,19 @@ template <int CR1, int CR2> struct TileRun {
     return buf;
   }
 };
-// runtime plans, every stage out of line (the passes that run once per Newton step)
-template <> struct TileRun<-1, -1> {
+// runtime plans, every stage out of line
+template <bool WIDE> struct TileRunOut {
   template <bool INV, typename R, typename MAP>
   static __device__ __forceinline__ typename V2<R>::T *run(const TilePlanD<R> &pl, const MAP &map,
                                                            typename V2<R>::T *buf, typename V2<R>::T *buf2, int P,
                                                            const typename V2<R>::T *tws) {
-    const bool second = tile_fft_rt(INV, pl.n, pl.m, pl.r1, pl.r2, pl.nst, pl.rcode, pl.blu, pl.tw, pl.chirp, pl.bf,
-                                    map.lay(pl.r1), smem_window(buf), smem_window(buf2), P, smem_window(tws));
+    bool second;
+    if constexpr (WIDE)
+      second = tile_fft_rt2(INV, pl.n, pl.m, pl.r1, pl.r2, pl.nst, pl.rcode, pl.blu, pl.tw, pl.chirp, pl.bf,
+                            map.lay(pl.r1), smem_window(buf), smem_window(buf2), P, smem_window(tws));
+    else
+      second = tile_fft_rt(INV, pl.n, pl.m, pl.r1, pl.r2, pl.nst, pl.rcode, pl.blu, pl.tw, pl.chirp, pl.bf,
+                           map.lay(pl.r1), smem_window(buf), smem_window(buf2), P, smem_window(tws));
     return second ? buf2 : buf;
   }
   template <bool INV, typename R, typename MAP, typename LD, typename ST>
@@ -336,6 +343,8 @@ template <> struct TileRun<-1, -1> {
     });
   }
 };
+// the passes of 3-D grids that run once per Newton step
+template <> struct TileRun<-1, -1> : TileRunOut<false> {};
 // runtime plans of the iteration's passes: the two stages inline (one body per radix; WIDE:
 // radices up to 32, 2-D), Bluestein and three or more factors out of line
 template <bool WIDE> struct TileRunRt {
@@ -400,7 +409,7 @@ template <bool WIDE> struct TileRunRt {
   template <bool INV, typename R, typename MAP, typename LD, typename ST>
   static __device__ __forceinline__ void io(const TilePlanD<R> &pl, const MAP &map, typename V2<R>::T *buf,
                                             typename V2<R>::T *buf2, int P, const typename V2<R>::T *tws, LD ld, ST st) {
-    if (!pl.r1 || pl.blu) TileRun<-1, -1>::template io<INV, R>(pl, map, buf, buf2, P, tws, ld, st);
+    if (!pl.r1 || pl.blu) TileRunOut<WIDE>::template io<INV, R>(pl, map, buf, buf2, P, tws, ld, st);
     else two<INV, R>(pl, map, buf, P, tws, ld, st);
   }
   template <bool INV, typename R, typename MAP>
@@ -408,7 +417,7 @@ template <bool WIDE> struct TileRunRt {
                                                            typename V2<R>::T *buf, typename V2<R>::T *buf2, int P,
                                                            const typename V2<R>::T *tws) {
     using T = typename V2<R>::T;
-    if (!pl.r1 || pl.blu) return TileRun<-1, -1>::template run<INV, R>(pl, map, buf, buf2, P, tws);
+    if (!pl.r1 || pl.blu) return TileRunOut<WIDE>::template run<INV, R>(pl, map, buf, buf2, P, tws);
     two<INV, R>(pl, map, buf, P, tws, [&](int, int s, int p) { return buf[map.at(s, p)]; },
                 [&](int, int s, int p, T v) { buf[map.at(s, p)] = v; });
     __syncthreads();

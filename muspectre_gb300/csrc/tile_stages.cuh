@@ -1,7 +1,7 @@
 // Out-of-line tile transforms (tile_fft.cuh): every role of every radix, compiled once
 // and called by the kernels of the displacement-space CG through tile_fft_rt (relocatable
 // device code): all roles inline in every kernel were ten minutes of compilation.
-// Included by tile_stages_f32.cu and tile_stages_f64.cu.
+// Included by tile_stages_f32.cu and tile_stages_f64.cu (3-D) and their tile_stages2_ twins (2-D).
 #pragma once
 
 #include "tile_fft.cuh"
@@ -16,7 +16,7 @@ __device__ __noinline__ void tile_stage_rt(uint32_t buf, uint32_t tw, const Tile
                          [&](int, int s, int p, T v) { b.st(lay.at(s, p), v); });
 }
 
-template <typename T, int OP>
+template <typename T, int OP, bool WIDE>
 __device__ __forceinline__ void tile_stage_any(int rad, uint32_t buf, uint32_t tw, const TileLay &lay,
                                                const TileStageArgs<T> &a) {
   switch (rad) {
@@ -25,7 +25,7 @@ __device__ __forceinline__ void tile_stage_any(int rad, uint32_t buf, uint32_t t
     MUSG_TILE_RADICES(MUSG_TS)
 #undef MUSG_TS
 #define MUSG_TS(RAD) \
-  case RAD: if constexpr (OP == OP_B1 || OP == OP_BM || OP == OP_B2) tile_stage_rt<T, RAD, OP>(buf, tw, lay, a); break;
+  case RAD: if constexpr (WIDE) tile_stage_rt<T, RAD, OP>(buf, tw, lay, a); break;
     MUSG_TILE_RADICES_2D(MUSG_TS)
 #undef MUSG_TS
     default: tile_stage_rt<T, 1, OP>(buf, tw, lay, a); break;
@@ -80,7 +80,7 @@ __device__ __forceinline__ bool tile_multi(int m, int nst, unsigned long long co
   return (nst & 1) != 0;
 }
 
-template <typename T>
+template <typename T, bool WIDE>
 __device__ __forceinline__ bool tile_fft_any(bool inv, int n, int m, int r1, int r2, int nst, unsigned long long rcode,
                                              int blu, const T *tw, const T *chirp, const T *bf, const TileLay lay,
                                              uint32_t buf, uint32_t buf2, int P, uint32_t tws) {
@@ -89,19 +89,21 @@ __device__ __forceinline__ bool tile_fft_any(bool inv, int n, int m, int r1, int
     TileStageArgs<T> c = a;                                     // radix r2
     c.ra = r1;
     if (blu) {
-      tile_stage_any<T, OP_B1>(r1, buf, tws, lay, a);
+      tile_stage_any<T, OP_B1, WIDE>(r1, buf, tws, lay, a);
       __syncthreads();
-      tile_stage_any<T, OP_BM>(r2, buf, tws, lay, c);
+      tile_stage_any<T, OP_BM, WIDE>(r2, buf, tws, lay, c);
       __syncthreads();
-      tile_stage_any<T, OP_B2>(r1, buf, tws, lay, a);
-    } else if (inv) {
-      tile_stage_any<T, OP_I1>(r2, buf, tws, lay, c);
-      __syncthreads();
-      tile_stage_any<T, OP_I2>(r1, buf, tws, lay, a);
-    } else {
-      tile_stage_any<T, OP_F1>(r1, buf, tws, lay, a);
-      __syncthreads();
-      tile_stage_any<T, OP_F2>(r2, buf, tws, lay, c);
+      tile_stage_any<T, OP_B2, WIDE>(r1, buf, tws, lay, a);
+    } else if constexpr (!WIDE) {  // (2-D kernels have these stages inline)
+      if (inv) {
+        tile_stage_any<T, OP_I1, WIDE>(r2, buf, tws, lay, c);
+        __syncthreads();
+        tile_stage_any<T, OP_I2, WIDE>(r1, buf, tws, lay, a);
+      } else {
+        tile_stage_any<T, OP_F1, WIDE>(r1, buf, tws, lay, a);
+        __syncthreads();
+        tile_stage_any<T, OP_F2, WIDE>(r2, buf, tws, lay, c);
+      }
     }
     __syncthreads();
     return false;
