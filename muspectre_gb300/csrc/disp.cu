@@ -117,8 +117,8 @@ template <typename R> DispProb<R> disp_prob(Spectral &sp, const DispVectors &v, 
 template <typename R>
 void pixels(const Spectral &sp, int tkind, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
             const DispGroup<R> *grp) {
-  if (sp.g.dim == 2) disp_pixels<R, 2>(tkind, sp.tp[1], a, c, B, s, grp);
-  else disp_pixels<R, 3>(tkind, sp.tp[2], a, c, B, s, grp);
+  if (sp.g.dim == 2) disp_pixels<R, 2>(tkind, sp.tile<R>(1), a, c, B, s, grp);
+  else disp_pixels<R, 3>(tkind, sp.tile<R>(2), a, c, B, s, grp);
 }
 
 // q (the vectors' q) -> real planes, ungated

@@ -30,8 +30,8 @@ template <typename R>
 void disp_ax0_step(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
               const DispGroup<R> *grp) {
   const bool fin = disp_finite(sp);
-  if (sp.g.dim == 2) fin ? ax0_step<R, 2, true>(sp.tp[0], a, c, B, s, grp) : ax0_step<R, 2, false>(sp.tp[0], a, c, B, s, grp);
-  else fin ? ax0_step<R, 3, true>(sp.tp[0], a, c, B, s, grp) : ax0_step<R, 3, false>(sp.tp[0], a, c, B, s, grp);
+  if (sp.g.dim == 2) fin ? ax0_step<R, 2, true>(sp.tile<R>(0), a, c, B, s, grp) : ax0_step<R, 2, false>(sp.tile<R>(0), a, c, B, s, grp);
+  else fin ? ax0_step<R, 3, true>(sp.tile<R>(0), a, c, B, s, grp) : ax0_step<R, 3, false>(sp.tile<R>(0), a, c, B, s, grp);
 }
 
 template <typename R>

@@ -68,7 +68,7 @@ inline long lcm32(long p) {
 template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   const bool fin = disp_finite(sp);
   const int D = sp.g.dim, na = fin ? 2 : D * (D + 1) / 2;
-  const TilePlan &pl = sp.tp[0];
+  const TilePlan &pl = sp.tile<R>(0);
   const long long Rr = disp_nk(sp) / sp.g.n[0];
   DispShape c;
   c.ng = fin ? D : 1;
@@ -101,7 +101,7 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
 
 template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
   const bool fin = disp_finite(sp);
-  const TilePlan &pl = sp.tp[1];
+  const TilePlan &pl = sp.tile<R>(1);
   DispShape c;
   c.ng = fin ? 3 : 6;
   c.comps_at_once = fin ? 3 : 1;
@@ -131,7 +131,7 @@ template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
 template <typename R> DispShape disp_last_shape(const Spectral &sp) {
   const bool fin = disp_finite(sp);
   const int D = sp.g.dim, nl = fin ? D * D : D * (D + 1) / 2;
-  const TilePlan &pl = sp.tp[D - 1];
+  const TilePlan &pl = sp.tile<R>(D - 1);
   DispShape c;
   const long cb = 2 * (long)sizeof(R), tw = pl.r1 ? pl.m * cb : 0;
   c.S = pl.r1;
@@ -187,7 +187,8 @@ template <typename R> DispArgs<R> disp_base(Spectral &sp) {
   return a;
 }
 template <typename R> DispArgs<R> disp_with(DispArgs<R> a, const Spectral &sp, int axis, const DispShape &c) {
-  a.ap = sp.tp[axis].device<R>();
+  const TilePlan &pl = sp.tile<R>(axis);
+  a.ap = pl.device<R>();
   a.T = c.T;
   a.G = c.G;
   a.ntx = c.ntx;

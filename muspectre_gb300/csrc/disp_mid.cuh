@@ -26,7 +26,7 @@ void mid(const TilePlan &pl, const DispArgs<R> &a, const DispShape &c, int B, cu
 template <typename R>
 void disp_mid(const Spectral &sp, bool inv, const DispArgs<R> &a, const DispShape &c, int B, cudaStream_t s,
              const DispGroup<R> *grp) {
-  const TilePlan &pl = sp.tp[1];
+  const TilePlan &pl = sp.tile<R>(1);
   if (disp_finite(sp)) inv ? mid<R, true, true>(pl, a, c, B, s, grp) : mid<R, true, false>(pl, a, c, B, s, grp);
   else inv ? mid<R, false, true>(pl, a, c, B, s, grp) : mid<R, false, false>(pl, a, c, B, s, grp);
 }

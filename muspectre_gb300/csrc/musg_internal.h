@@ -98,9 +98,7 @@ template <typename R> struct AxisPlanD {
 struct AxisPlan {
   int n = 0, m = 0, nst = 0, blu = 0;
   int radix[kMaxStages] = {0};
-  // device tables, double and float copies
-  void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;
-  void *tw32 = nullptr, *chirp32 = nullptr, *bf32 = nullptr;
+  void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;  // device tables
   void build(int n);
   void release();
   template <typename R> AxisPlanD<R> device() const;
@@ -119,17 +117,22 @@ template <typename R> struct TilePlanD {
 struct TilePlan {
   int n = 0, m = 0, r1 = 0, r2 = 0, blu = 0, nst = 0;
   int radix[kMaxStages] = {0};
-  void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;
-  void *tw32 = nullptr, *chirp32 = nullptr, *bf32 = nullptr;
-  // factors only (host), two up to `widest` (17, or 32 for the axes of a 2-D grid); build()
-  // also makes the device tables.  points: the longest plan of three or more factors that
-  // fits the axis' passes; smallest: the shortest Bluestein length instead of the cheapest
-  void factor(int n, int widest, long points, bool smallest = false);
-  void build(int n, int widest, long points);
+  void *tw = nullptr, *chirp = nullptr, *bf = nullptr;  // device tables of one precision
+  // factors only (host), two up to `widest` (17, or 32 for the axes of a 2-D grid; those of a
+  // Bluestein length up to `wide_blu`); build() also makes the device tables.  points: the
+  // longest plan of three or more factors that fits the axis' passes; smallest: the shortest
+  // Bluestein length instead of the cheapest
+  void factor(int n, int widest, int wide_blu, long points, bool smallest = false);
+  template <typename R> void build(int n, int dim, long points);
   void release();
   template <typename R> TilePlanD<R> device() const;
   int buffers() const { return r1 ? 1 : 2; }  // tile buffers a transform needs
 };
+// The largest radix of a Bluestein length on an axis of n points.  On 2-D grids two wide
+// radices replace three factors: in FP32 at every length (139^2 12.3 -> 8.9 ms, 701 x 211
+// 16.5 -> 14.5), in FP64, where they spill, only above 256 points (157 x 149 109 -> 161 ms
+// with them)
+template <typename R> int wide_bluestein(int n, int dim) { return dim == 2 && (sizeof(R) == 4 || n > 256) ? 32 : 17; }
 
 // ---------------------------------------------------------------- geometry
 struct Geom {
@@ -204,7 +207,8 @@ struct Spectral {
   bool allow_even = false;
   double lengths[3] = {1, 1, 1};
   AxisPlan ax[3];
-  TilePlan tp[3];           // the same axes for the displacement-space passes (disp.cu), by ensure_tiles
+  TilePlan tp64[3], tp32[3];  // the same axes for the displacement-space passes (disp.cu), by ensure_tiles, ensure32
+  template <typename R> const TilePlan &tile(int axis) const { return sizeof(R) == 8 ? tp64[axis] : tp32[axis]; }
   // per-axis xi_d(k) = fftfreq_d(k)/L_d over the hermitian index range, FP64 and FP32
   void *xi64[3] = {nullptr, nullptr, nullptr};
   void *xi32[3] = {nullptr, nullptr, nullptr};
@@ -218,9 +222,9 @@ struct Spectral {
   long tune_bytes[2][3] = {{73728, 49152, 73728}, {73728, 49152, 73728}};
   void init(int dim, const int *res, int ncomp, int proj_kind, const double *lengths,
             bool allow_even, bool want32);
-  // points of a pencil of two buffers in `bytes` of shared memory, for the FP64 pass over
-  // `axis` that holds the most pencils at once (disp_launch.cuh)
-  long tile_points(int axis, long bytes) const;
+  // points of a pencil of two buffers in `bytes` of shared memory, for the pass over `axis`
+  // that holds the most pencils at once (disp_launch.cuh)
+  template <typename R> long tile_points(int axis, long bytes) const;
   void ensure_tiles();
   void ensure32();
   void release();

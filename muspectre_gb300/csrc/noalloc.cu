@@ -160,8 +160,8 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
   off += align256((size_t)sp.ncomp * sp.g.nk * sizeof(double2));
   size_t off_tw[3], off_chirp[3], off_bf[3], off_xi[3];
   for (int d = 0; d < dim; ++d) {
-    TilePlan &ap = sp.tp[d];
-    ap.factor(sp.g.n[d], dim == 2 ? 32 : 17, 1 << 16, true);
+    TilePlan &ap = sp.tp64[d];
+    ap.factor(sp.g.n[d], dim == 2 ? 32 : 17, wide_bluestein<double>(sp.g.n[d], dim), 1 << 16, true);
     if (!ap.m) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
     off_tw[d] = off;
     off += align256((size_t)ap.m * sizeof(double2));
@@ -181,18 +181,18 @@ void noalloc_project(int dim, const int *resolutions, const double *lengths, int
   double *soa = reinterpret_cast<double *>(base + off_soa);
   sp.spec64 = base + off_spec;
   for (int d = 0; d < dim; ++d) {
-    TilePlan &ap = sp.tp[d];
-    ap.tw64 = base + off_tw[d];
-    ap.chirp64 = ap.blu ? base + off_chirp[d] : nullptr;
-    ap.bf64 = ap.blu ? base + off_bf[d] : nullptr;
+    TilePlan &ap = sp.tp64[d];
+    ap.tw = base + off_tw[d];
+    ap.chirp = ap.blu ? base + off_chirp[d] : nullptr;
+    ap.bf = ap.blu ? base + off_bf[d] : nullptr;
     sp.xi64[d] = base + off_xi[d];
     const int len = (d == dim - 1) ? sp.g.nh : sp.g.n[d];
     const int work = std::max(ap.m, std::max(ap.n, len));
-    k_fill_axis<<<(work + 255) / 256, 256, 0, s>>>((double2 *)ap.tw64, ap.m, (double2 *)ap.chirp64, ap.n,
+    k_fill_axis<<<(work + 255) / 256, 256, 0, s>>>((double2 *)ap.tw, ap.m, (double2 *)ap.chirp, ap.n,
                                                    (double *)sp.xi64[d], len, sp.lengths[d]);
     MUSG_CHECK_LAUNCH();
     if (ap.blu) {
-      k_fill_bluestein<<<(ap.m + 127) / 128, 128, 0, s>>>((const double2 *)ap.chirp64, ap.n, (double2 *)ap.bf64,
+      k_fill_bluestein<<<(ap.m + 127) / 128, 128, 0, s>>>((const double2 *)ap.chirp, ap.n, (double2 *)ap.bf,
                                                           ap.m);
       MUSG_CHECK_LAUNCH();
     }

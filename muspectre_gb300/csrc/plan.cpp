@@ -80,17 +80,16 @@ void *upload_complex(const std::vector<std::complex<long double>> &v) {
   return upload(h.data(), h.size() * sizeof(T2));
 }
 
-// device tables of a length-n transform over m (FP64 and FP32): twiddles W_m^j, and for
-// Bluestein the chirp and the filter
-void build_tables(int n, int m, int blu, void *&tw64, void *&tw32, void *&chirp64, void *&chirp32, void *&bf64,
-                  void *&bf32) {
+// device tables of a length-n transform over m: twiddles W_m^j, and for Bluestein the chirp
+// and the filter
+template <typename R> void build_tables(int n, int m, int blu, void *&tw_d, void *&chirp_d, void *&bf_d) {
+  using T = typename V2<R>::T;
   std::vector<std::complex<long double>> tw(m);
   for (int j = 0; j < m; ++j) {
     long double a = -2.0L * kPi * (long double)j / (long double)m;
     tw[j] = {cosl(a), sinl(a)};
   }
-  tw64 = upload_complex<double2, double>(tw);
-  tw32 = upload_complex<float2, float>(tw);
+  tw_d = upload_complex<T, R>(tw);
   if (blu) {
     std::vector<std::complex<long double>> w(n);
     for (int j = 0; j < n; ++j) {
@@ -126,10 +125,8 @@ void build_tables(int n, int m, int blu, void *&tw64, void *&tw32, void *&chirp6
       }
       bf[k] = {(long double)sr / m, (long double)ir / m};
     }
-    chirp64 = upload_complex<double2, double>(w);
-    chirp32 = upload_complex<float2, float>(w);
-    bf64 = upload_complex<double2, double>(bf);
-    bf32 = upload_complex<float2, float>(bf);
+    chirp_d = upload_complex<T, R>(w);
+    bf_d = upload_complex<T, R>(bf);
   }
 }
 
@@ -152,11 +149,11 @@ void AxisPlan::build(int n_) {
   nst = (int)rad.size();
   for (int s = 0; s < nst; ++s) radix[s] = rad[s];
 
-  build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
+  build_tables<double>(n, m, blu, tw64, chirp64, bf64);
 }
 
 void AxisPlan::release() {
-  for (void **p : {&tw64, &chirp64, &bf64, &tw32, &chirp32, &bf32}) {
+  for (void **p : {&tw64, &chirp64, &bf64}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
@@ -170,17 +167,6 @@ template <> AxisPlanD<double> AxisPlan::device<double>() const {
   d.tw = (const double2 *)tw64;
   d.chirp = (const double2 *)chirp64;
   d.bf = (const double2 *)bf64;
-  return d;
-}
-
-template <> AxisPlanD<float> AxisPlan::device<float>() const {
-  AxisPlanD<float> d{};
-  d.n = n; d.m = m; d.nst = nst; d.blu = blu;
-  d.rcode = 0;
-  for (int s = 0; s < nst; ++s) d.rcode |= (unsigned long long)radix[s] << (5 * s);
-  d.tw = (const float2 *)tw32;
-  d.chirp = (const float2 *)chirp32;
-  d.bf = (const float2 *)bf32;
   return d;
 }
 
@@ -246,7 +232,7 @@ int tile_factor(int m, int widest, int *rad, double &cost) {
 
 }  // namespace
 
-void TilePlan::factor(int n_, int widest, long points, bool smallest) {
+void TilePlan::factor(int n_, int widest, int wide_blu, long points, bool smallest) {
   n = n_;
   m = nst = r1 = r2 = blu = 0;
   if (n > (1 << 16)) return;  // longer than any tile: the passes refuse it (m = 0)
@@ -254,11 +240,7 @@ void TilePlan::factor(int n_, int widest, long points, bool smallest) {
   if ((nst = tile_factor(n, widest, radix, cost))) {
     m = n;
   } else {
-    // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass.  Two
-    // wide radices in place of three factors above 256 only (324 x 359 mixed 14.1 -> 11.4
-    // ms, 127 x 509 14.6 -> 13.1): their registers spill, which costs FP64 more than the
-    // passes it saves (157 x 149 FP64 168 -> 195 ms)
-    const int wide = n > 256 ? widest : 17;
+    // Bluestein: the cheapest m in [2n-1, 2.5n]; the two middle stages share a pass
     blu = 1;
     // the cheapest may be too long for its pass where a shorter one fits (899 in 2-D: 2048
     // points of four components in two buffers are 262 KB, 1800 fit); where none fits, the
@@ -268,7 +250,7 @@ void TilePlan::factor(int n_, int widest, long points, bool smallest) {
       for (int k = 2 * n - 1; k <= 2 * n - 1 + n / 2 + 16; ++k) {
         int rad[kMaxStages];
         double c = 0;
-        const int ns = tile_factor(k, wide, rad, c);
+        const int ns = tile_factor(k, wide_blu, rad, c);
         if (!ns || (ns > 2 && k > most)) continue;
         if (smallest && m) break;
         c *= k;
@@ -287,35 +269,31 @@ void TilePlan::factor(int n_, int widest, long points, bool smallest) {
   r2 = nst == 2 ? radix[1] : 0;
 }
 
-void TilePlan::build(int n_, int widest, long points) {
+template <typename R> void TilePlan::build(int n_, int dim, long points) {
   release();
-  factor(n_, widest, points);
-  if (m) build_tables(n, m, blu, tw64, tw32, chirp64, chirp32, bf64, bf32);
+  factor(n_, dim == 2 ? 32 : 17, wide_bluestein<R>(n_, dim), points);
+  if (m) build_tables<R>(n, m, blu, tw, chirp, bf);
 }
 
 void TilePlan::release() {
-  for (void **p : {&tw64, &chirp64, &bf64, &tw32, &chirp32, &bf32}) {
+  for (void **p : {&tw, &chirp, &bf}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
 }
 
-template <typename R, typename T>
-static TilePlanD<R> tile_plan_device(const TilePlan &t, const void *tw, const void *chirp, const void *bf) {
+template <typename R> TilePlanD<R> TilePlan::device() const {
+  using T = typename V2<R>::T;
   TilePlanD<R> d{};
-  d.n = t.n; d.m = t.m; d.r1 = t.r1; d.r2 = t.r2; d.blu = t.blu; d.nst = t.nst;
-  for (int s = 0; s < t.nst; ++s) d.rcode |= (unsigned long long)t.radix[s] << (5 * s);
+  d.n = n; d.m = m; d.r1 = r1; d.r2 = r2; d.blu = blu; d.nst = nst;
+  for (int s = 0; s < nst; ++s) d.rcode |= (unsigned long long)radix[s] << (5 * s);
   d.tw = (const T *)tw;
   d.chirp = (const T *)chirp;
   d.bf = (const T *)bf;
   return d;
 }
-template <> TilePlanD<double> TilePlan::device<double>() const {
-  return tile_plan_device<double, double2>(*this, tw64, chirp64, bf64);
-}
-template <> TilePlanD<float> TilePlan::device<float>() const {
-  return tile_plan_device<float, float2>(*this, tw32, chirp32, bf32);
-}
+template TilePlanD<double> TilePlan::device<double>() const;
+template TilePlanD<float> TilePlan::device<float>() const;
 
 // fftfreq(n)[k]/L (src/fft/fft_utils.cc:41-56)
 static double fft_freq(int n, int k) {
@@ -360,28 +338,33 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
   if (want32) ensure32();
 }
 
-long Spectral::tile_points(int axis, long bytes) const {
+template <typename R> long Spectral::tile_points(int axis, long bytes) const {
   const int D = g.dim, sym = D * (D + 1) / 2;
   const bool fin = proj_kind != MUSG_PROJ_SMALL_STRAIN;
   // a pass over a middle axis falls back to one component at a time
   const int pencils = axis == D - 1 ? (fin ? D * D : sym) : axis == 0 ? (fin ? 2 : sym) : 1;
-  return bytes / (pencils * 2 * (long)sizeof(double2));
+  return bytes / (pencils * 2 * (long)(2 * sizeof(R)));
 }
+template long Spectral::tile_points<double>(int, long) const;
+template long Spectral::tile_points<float>(int, long) const;
 
 void Spectral::ensure_tiles() {
   for (int d = 0; d < g.dim; ++d)
-    if (tp[d].n != g.n[d]) tp[d].build(g.n[d], g.dim == 2 ? 32 : 17, tile_points(d, optin_smem()));
+    if (tp64[d].n != g.n[d]) tp64[d].build<double>(g.n[d], g.dim, tile_points<double>(d, optin_smem()));
 }
 
 void Spectral::ensure32() {
   want32 = true;
   ensure_tiles();
+  for (int d = 0; d < g.dim; ++d)
+    if (tp32[d].n != g.n[d]) tp32[d].build<float>(g.n[d], g.dim, tile_points<float>(d, optin_smem()));
   if (!spec32) MUSG_CUDA(cudaMalloc(&spec32, (size_t)ncomp * g.nk * sizeof(float2)));
 }
 
 void Spectral::release() {
   for (auto &a : ax) a.release();
-  for (auto &a : tp) a.release();
+  for (auto &a : tp64) a.release();
+  for (auto &a : tp32) a.release();
   for (int d = 0; d < 3; ++d) {
     if (xi64[d]) cudaFree(xi64[d]);
     if (xi32[d]) cudaFree(xi32[d]);

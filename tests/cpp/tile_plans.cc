@@ -33,7 +33,7 @@ int main() {
           sp.g.dim = dim;
           sp.proj_kind = small ? MUSG_PROJ_SMALL_STRAIN : MUSG_PROJ_FINITE_STRAIN;
           TilePlan t;
-          t.factor(n, dim == 2 ? 32 : 17, sp.tile_points(axis, bytes));
+          t.factor(n, dim == 2 ? 32 : 17, wide_bluestein<double>(n, dim), sp.tile_points<double>(axis, bytes));
           // two stages: one buffer, its groups of r1 slots padded by at most 15 each way
           const long row = t.r1 ? (long)t.r2 * (t.r1 + 15) + 15 : 2L * t.m;
           const long need = 16 * (pencils * row + (t.r1 ? t.m : 0));
@@ -48,7 +48,7 @@ int main() {
       }
   for (int n = 1; n <= 1024; ++n) {
     TilePlan t;
-    t.factor(n, 32, 1 << 28);
+    t.factor(n, 32, 32, 1 << 28);
     bool narrow = false;
     for (int a = 1; a <= 17; ++a) narrow |= n % a == 0 && n / a <= 17;
     if (narrow && (t.blu || t.nst != 2 || t.r1 > 17)) {
