@@ -5,8 +5,10 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <complex>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <utility>
@@ -99,6 +101,7 @@ struct AxisPlan {
   int n = 0, m = 0, nst = 0, blu = 0;
   int radix[kMaxStages] = {0};
   void *tw64 = nullptr, *chirp64 = nullptr, *bf64 = nullptr;  // device tables
+  void factor(int n);  // host only; build() also makes the tables
   void build(int n);
   void release();
   template <typename R> AxisPlanD<R> device() const;
@@ -114,16 +117,21 @@ template <typename R> struct TilePlanD {
   const typename V2<R>::T *chirp;  // n entries (Bluestein)
   const typename V2<R>::T *bf;     // m entries (Bluestein)
 };
+struct FftTables {  // on the host: twiddles W_m^j; Bluestein: the chirp and the filter
+  std::vector<std::complex<long double>> tw, chirp, bf;
+};
 struct TilePlan {
   int n = 0, m = 0, r1 = 0, r2 = 0, blu = 0, nst = 0;
   int radix[kMaxStages] = {0};
   void *tw = nullptr, *chirp = nullptr, *bf = nullptr;  // device tables of one precision
+  std::shared_ptr<const FftTables> host;                // what they were rounded from
   // factors only (host), two up to `widest` (17, or 32 for the axes of a 2-D grid; those of a
-  // Bluestein length up to `wide_blu`); build() also makes the device tables.  points: the
+  // Bluestein length up to `wide_blu`); build() also makes the device tables, from those of
+  // the other precision's plan where both have one length.  points: the
   // longest plan of three or more factors that fits the axis' passes; smallest: the shortest
   // Bluestein length instead of the cheapest
   void factor(int n, int widest, int wide_blu, long points, bool smallest = false);
-  template <typename R> void build(int n, int dim, long points);
+  template <typename R> void build(int n, int dim, long points, const TilePlan *other);
   void release();
   template <typename R> TilePlanD<R> device() const;
   int buffers() const { return r1 ? 1 : 2; }  // tile buffers a transform needs

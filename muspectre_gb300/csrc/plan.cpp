@@ -80,60 +80,62 @@ void *upload_complex(const std::vector<std::complex<long double>> &v) {
   return upload(h.data(), h.size() * sizeof(T2));
 }
 
-// device tables of a length-n transform over m: twiddles W_m^j, and for Bluestein the chirp
-// and the filter
-template <typename R> void build_tables(int n, int m, int blu, void *&tw_d, void *&chirp_d, void *&bf_d) {
-  using T = typename V2<R>::T;
-  std::vector<std::complex<long double>> tw(m);
+// the tables of a length-n transform over m
+FftTables fft_tables(int n, int m, int blu) {
+  FftTables ft;
+  auto &tw = ft.tw, &w = ft.chirp, &bf = ft.bf;
+  tw.resize(m);
   for (int j = 0; j < m; ++j) {
     long double a = -2.0L * kPi * (long double)j / (long double)m;
     tw[j] = {cosl(a), sinl(a)};
   }
-  tw_d = upload_complex<T, R>(tw);
   if (blu) {
-    std::vector<std::complex<long double>> w(n);
+    w.resize(n);
     for (int j = 0; j < n; ++j) {
       long long q = ((long long)j * j) % (2LL * n);
       long double a = -kPi * (long double)q / (long double)n;
       w[j] = {cosl(a), sinl(a)};
     }
-    // b[t] = conj(w[|t|]) on the circle of length m
-    std::vector<std::complex<double>> b(m, {0.0, 0.0});
-    for (int t = 0; t < n; ++t) b[t] = std::conj(std::complex<double>((double)w[t].real(), (double)w[t].imag()));
-    for (int t = 1; t < n; ++t) b[m - t] = b[t];
-    std::vector<std::complex<long double>> bf(m);
-    std::vector<std::complex<double>> twd(m);
-    for (int j = 0; j < m; ++j) twd[j] = {(double)tw[j].real(), (double)tw[j].imag()};
-    for (int k = 0; k < m; ++k) {
-      // Kahan-compensated sum_t b[t] exp(-2 pi i t k / m)
-      double sr = 0, sc = 0, ir = 0, ic = 0;
-      long long idx = 0;
-      for (int t = 0; t < m; ++t) {
-        if (b[t].real() != 0.0 || b[t].imag() != 0.0) {
-          std::complex<double> term = b[t] * twd[idx];
-          double y = term.real() - sc;
-          double tt = sr + y;
-          sc = (tt - sr) - y;
-          sr = tt;
-          y = term.imag() - ic;
-          tt = ir + y;
-          ic = (tt - ir) - y;
-          ir = tt;
-        }
+    // the filter of b[t] = conj(w[|t|]) on the circle of length m: b is even, so
+    // bf[k] = bf[m - k] = (b[0] + 2 sum_{0 < t < n} b[t] cos(2 pi t k / m)) / m, Kahan-compensated
+    bf.resize(m);
+    std::vector<double> br(n), bi(n), co(m);
+    for (int t = 0; t < n; ++t) {
+      br[t] = 2.0 * (double)w[t].real();
+      bi[t] = -2.0 * (double)w[t].imag();
+    }
+    for (int j = 0; j < m; ++j) co[j] = (double)tw[j].real();
+    for (int k = 0; 2 * k <= m; ++k) {
+      double sr = 0.5 * br[0], sc = 0, ir = 0.5 * bi[0], ic = 0;
+      int idx = k;
+      for (int t = 1; t < n; ++t) {
+        const double yr = br[t] * co[idx] - sc, tr = sr + yr;
+        sc = (tr - sr) - yr;
+        sr = tr;
+        const double yi = bi[t] * co[idx] - ic, ti = ir + yi;
+        ic = (ti - ir) - yi;
+        ir = ti;
         idx += k;
         if (idx >= m) idx -= m;
       }
-      bf[k] = {(long double)sr / m, (long double)ir / m};
+      bf[k] = bf[(m - k) % m] = {(long double)sr / m, (long double)ir / m};
     }
-    chirp_d = upload_complex<T, R>(w);
-    bf_d = upload_complex<T, R>(bf);
   }
+  return ft;
+}
+
+// and on the device, in one precision
+template <typename R> void upload_tables(const FftTables &ft, void *&tw, void *&chirp, void *&bf) {
+  using T = typename V2<R>::T;
+  tw = upload_complex<T, R>(ft.tw);
+  if (ft.bf.empty()) return;
+  chirp = upload_complex<T, R>(ft.chirp);
+  bf = upload_complex<T, R>(ft.bf);
 }
 
 }  // namespace
 
-void AxisPlan::build(int n_) {
-  release();
+void AxisPlan::factor(int n_) {
   n = n_;
   std::vector<int> rad;
   if (factorize(n, rad)) {
@@ -148,8 +150,12 @@ void AxisPlan::build(int n_) {
   if ((int)rad.size() > kMaxStages) throw Error(MUSG_ERR_ARGUMENT, "FFT length too large");
   nst = (int)rad.size();
   for (int s = 0; s < nst; ++s) radix[s] = rad[s];
+}
 
-  build_tables<double>(n, m, blu, tw64, chirp64, bf64);
+void AxisPlan::build(int n_) {
+  release();
+  factor(n_);
+  upload_tables<double>(fft_tables(n, m, blu), tw64, chirp64, bf64);
 }
 
 void AxisPlan::release() {
@@ -269,10 +275,12 @@ void TilePlan::factor(int n_, int widest, int wide_blu, long points, bool smalle
   r2 = nst == 2 ? radix[1] : 0;
 }
 
-template <typename R> void TilePlan::build(int n_, int dim, long points) {
+template <typename R> void TilePlan::build(int n_, int dim, long points, const TilePlan *other) {
   release();
   factor(n_, dim == 2 ? 32 : 17, wide_bluestein<R>(n_, dim), points);
-  if (m) build_tables<R>(n, m, blu, tw, chirp, bf);
+  if (!m) return;
+  host = other && other->host && other->m == m ? other->host : std::make_shared<const FftTables>(fft_tables(n, m, blu));
+  upload_tables<R>(*host, tw, chirp, bf);
 }
 
 void TilePlan::release() {
@@ -280,6 +288,7 @@ void TilePlan::release() {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
+  host.reset();
 }
 
 template <typename R> TilePlanD<R> TilePlan::device() const {
@@ -321,7 +330,9 @@ void Spectral::init(int dim, const int *res, int ncomp_, int proj_kind_, const d
   proj_kind = proj_kind_;
   allow_even = allow_even_;
   want32 = want32_;
-  for (int d = 0; d < dim; ++d) ax[d].build(g.n[d]);
+  // the tables are the FFT engine's; cells and projections have those of their passes
+  // (ensure_tiles)
+  for (int d = 0; d < dim; ++d) proj_kind < 0 ? ax[d].build(g.n[d]) : ax[d].factor(g.n[d]);
   // xi tables over the hermitian index range of each axis
   for (int d = 0; d < dim; ++d) {
     int len = (d == dim - 1) ? g.nh : g.n[d];
@@ -350,14 +361,14 @@ template long Spectral::tile_points<float>(int, long) const;
 
 void Spectral::ensure_tiles() {
   for (int d = 0; d < g.dim; ++d)
-    if (tp64[d].n != g.n[d]) tp64[d].build<double>(g.n[d], g.dim, tile_points<double>(d, optin_smem()));
+    if (tp64[d].n != g.n[d]) tp64[d].build<double>(g.n[d], g.dim, tile_points<double>(d, optin_smem()), nullptr);
 }
 
 void Spectral::ensure32() {
   want32 = true;
   ensure_tiles();
   for (int d = 0; d < g.dim; ++d)
-    if (tp32[d].n != g.n[d]) tp32[d].build<float>(g.n[d], g.dim, tile_points<float>(d, optin_smem()));
+    if (tp32[d].n != g.n[d]) tp32[d].build<float>(g.n[d], g.dim, tile_points<float>(d, optin_smem()), &tp64[d]);
   if (!spec32) MUSG_CUDA(cudaMalloc(&spec32, (size_t)ncomp * g.nk * sizeof(float2)));
 }
 
