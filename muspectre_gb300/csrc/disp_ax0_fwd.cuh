@@ -37,7 +37,7 @@ void disp_ax0_dots(const Spectral &sp, const DispArgs<R> &a, const DispShape &c,
 template <typename R>
 void disp_ax0_contract(const Spectral &sp, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
 #define MUSG_C(DD, FF) \
-  if (sp.g.dim == DD && disp_finite(sp) == FF) disp_launch<R>(k_ax0_fwd<R, DD, FF, AX_OUT, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);
+  if (sp.g.dim == DD && disp_finite(sp) == FF) disp_launch<R>(k_ax0_fwd<R, DD, FF, AX_OUT, kRtPlan<DD>, kRtPlan<DD>, false>, a, c, 1, s);
   MUSG_C(2, true) MUSG_C(2, false) MUSG_C(3, true) MUSG_C(3, false)
 #undef MUSG_C
 }

@@ -38,8 +38,8 @@ template <typename R>
 void disp_ax0_field(const Spectral &sp, bool from_x, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
 #define MUSG_C(DD, FF)                                                                           \
   if (sp.g.dim == DD && disp_finite(sp) == FF) {                                                             \
-    if (from_x) disp_launch<R>(k_ax0_inv<R, DD, FF, AX_X, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);     \
-    else disp_launch<R>(k_ax0_inv<R, DD, FF, AX_Q, kPlainPlan<DD>, kPlainPlan<DD>, false>, a, c, 1, s);            \
+    if (from_x) disp_launch<R>(k_ax0_inv<R, DD, FF, AX_X, kRtPlan<DD>, kRtPlan<DD>, false>, a, c, 1, s);     \
+    else disp_launch<R>(k_ax0_inv<R, DD, FF, AX_Q, kRtPlan<DD>, kRtPlan<DD>, false>, a, c, 1, s);            \
   }
   MUSG_C(2, true) MUSG_C(2, false) MUSG_C(3, true) MUSG_C(3, false)
 #undef MUSG_C

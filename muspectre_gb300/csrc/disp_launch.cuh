@@ -216,11 +216,13 @@ void disp_launch(K kernel, const DispArgs<R> &a, const DispShape &c, int B, cuda
   MUSG_CHECK_LAUNCH();
 }
 
-// runtime plans by dimension: radices up to 32 in 2-D (TileRun); of the passes that run
-// once per Newton step and of the FP64 grouped ones, out of line in 3-D (build time)
+// runtime plans by dimension: radices up to 32 in 2-D (TileRun); of the FP64 grouped passes
+// out of line in 3-D (build time).  The passes that run once per Newton step and per operator
+// call have their stages inline like the iteration's: out of line they took two more
+// shared-memory passes and barriers an axis (directional stiffness at 64^3 0.77 -> 0.71 ms,
+// projection of 55^3 0.42 -> 0.40).
 template <int D> constexpr int kRtPlan = D == 2 ? -2 : 0;
-template <int D> constexpr int kPlainPlan = D == 2 ? -2 : -1;
-template <typename R, int D> constexpr int kGroupPlan = sizeof(R) == 4 ? kRtPlan<D> : kPlainPlan<D>;
+template <typename R, int D> constexpr int kGroupPlan = sizeof(R) == 4 || D == 2 ? kRtPlan<D> : -1;
 
 // the passes: of an iteration (solo, batched, or grouped with grp), and the plain ones
 template <typename R>

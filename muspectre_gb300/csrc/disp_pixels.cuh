@@ -55,23 +55,23 @@ void disp_pixels_in(bool fin, int tkind, bool delta, const DispArgs<R> &a0, cons
   DispArgs<R> a = a0;
   a.tkind = tkind;
   if (tkind == TK_PLAIN) {
-    if (fin && delta) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_DELTA, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
-    else if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
-    else if (delta) disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_DELTA, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
-    else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    if (fin && delta) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_DELTA, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
+    else if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_REAL, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
+    else if (delta) disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_DELTA, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
+    else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_REAL, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
   } else if (tkind == TK_SMALL) {
-    disp_launch<R>(k_pixels<R, D, false, TK_SMALL, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, false, TK_SMALL, IN_REAL, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
   } else if (tkind == TK_GSMALL) {
-    disp_launch<R>(k_pixels<R, D, false, TK_GSMALL, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, false, TK_GSMALL, IN_REAL, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
   } else {
-    disp_launch<R>(k_pixels<R, D, true, TK_ANYFIN, IN_REAL, OUT_SPEC, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+    disp_launch<R>(k_pixels<R, D, true, TK_ANYFIN, IN_REAL, OUT_SPEC, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
   }
 }
 
 template <typename R, int D>
 void disp_pixels_out(bool fin, const DispArgs<R> &a, const DispShape &c, cudaStream_t s) {
-  if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_SPEC, OUT_REAL, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
-  else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_SPEC, OUT_REAL, kPlainPlan<D>, kPlainPlan<D>, false>, a, c, 1, s);
+  if (fin) disp_launch<R>(k_pixels<R, D, true, TK_PLAIN, IN_SPEC, OUT_REAL, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
+  else disp_launch<R>(k_pixels<R, D, false, TK_PLAIN, IN_SPEC, OUT_REAL, kRtPlan<D>, kRtPlan<D>, false>, a, c, 1, s);
 }
 
 #define MUSG_INSTANTIATE_PIXELS(R, D)                                                                             \

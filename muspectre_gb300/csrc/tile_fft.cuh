@@ -343,7 +343,7 @@ template <bool WIDE> struct TileRunOut {
     });
   }
 };
-// the passes of 3-D grids that run once per Newton step
+// the FP64 grouped passes of 3-D grids
 template <> struct TileRun<-1, -1> : TileRunOut<false> {};
 // runtime plans of the iteration's passes: the two stages inline (one body per radix; WIDE:
 // radices up to 32, 2-D), Bluestein and three or more factors out of line
