@@ -14,11 +14,12 @@ namespace musg {
 // FP32: axes with kernels of a compile-time plan.  The others' kernels hold a body per
 // radix, compute strides and divide by lengths known at run time only, and spill where a
 // radix above 12 does not fit their registers (160^3 small strain 382 -> 312 us an
-// iteration, 63^3 70 -> 62 us, 45x77x81 76 -> 66 us).  Multiples of 32 up to 256 and, in 3-D,
-// the odd lengths of two factors up to 121: one kernel per length, pass and law is what
-// a build of two minutes holds.  In FP64 the arithmetic, not the indexing, sets the pace.
+// iteration, 63^3 70 -> 62 us, 45x77x81 76 -> 66 us, 16^3 54 -> 40 us).  16, multiples of 32 up
+// to 256 and, in 3-D, the odd lengths of two factors up to 121: one kernel per length, pass
+// and law is what a build of two minutes holds.  In FP64 the arithmetic, not the indexing,
+// sets the pace.
 #define MUSG_DISP_PLANS(X) \
-  X(32, 8, 4) X(64, 8, 8) X(96, 12, 8) X(128, 16, 8) X(160, 16, 10) X(192, 16, 12) X(224, 16, 14) X(256, 16, 16)
+  X(16, 4, 4) X(32, 8, 4) X(64, 8, 8) X(96, 12, 8) X(128, 16, 8) X(160, 16, 10) X(192, 16, 12) X(224, 16, 14) X(256, 16, 16)
 #define MUSG_DISP_PLANS_ODD(X) \
   X(15, 5, 3) X(21, 7, 3) X(25, 5, 5) X(27, 9, 3) X(33, 11, 3) X(35, 7, 5) X(39, 13, 3) X(45, 9, 5) X(49, 7, 7) \
   X(51, 17, 3) X(55, 11, 5) X(63, 9, 7) X(65, 13, 5) X(75, 15, 5) X(77, 11, 7) X(81, 9, 9) X(85, 17, 5) X(91, 13, 7) \

@@ -162,6 +162,19 @@ def test_mixed_solve_compile_time_plan(mu, n, form):
 
 
 @pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('res', [[16, 3, 3], [3, 16, 5], [5, 3, 16], [16, 16, 16], [16, 9], [9, 16], [16, 16]])
+def test_mixed_solve_compile_time_plan_of_16(mu, res, form):
+    load = _load(len(res), form)
+    hom = {}
+    for prec in ('fp64', 'mixed'):
+        cell = _cell(mu, res, form, 3)
+        r = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 2000, precision=prec), 1e-8, 0.0)
+        assert r.success, r.message
+        hom[prec] = r.hom_stress
+    assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
+@pytest.mark.parametrize('form', [0, 1])
 @pytest.mark.parametrize('res', [[67, 9], [67, 400], [157, 149], [359, 62], [401, 640]])
 def test_solve_bluestein_first_axis_2d(mu, res, form):
     """Tiles of one, two and four k-points on a Bluestein axis 0: the sums over partly filled
