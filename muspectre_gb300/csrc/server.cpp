@@ -55,26 +55,31 @@ struct Req {
   Clock::time_point t0;
 };
 
-unsigned long long footprint(int dim, const int *res, int form, bool has_hep, bool has_full, int precision) {
+// device bytes of a request's cell and solver: the buffers that musg_cell_create,
+// musg_cell_initialise, musg_solver_cg_create and a solve without field outputs allocate
+unsigned long long footprint(int dim, const int *res, int form, bool has_hep, bool has_full, bool has_le2, int precision) {
   unsigned long long npx = 1;
   for (int d = 0; d < dim; ++d) npx *= (unsigned long long)res[d];
   const unsigned long long d2 = (unsigned long long)dim * dim;
   const unsigned long long last = (unsigned long long)res[dim - 1];
   const unsigned long long nk = npx / last * (last / 2 + 1);
-  // fields F, P, rhs (FP64), the FP64 spectrum, strain/stress I/O staging, material
-  // index + lambda/mu, and 1 MiB of plans and reduction scratch
-  unsigned long long b = 3 * d2 * npx * 8 + d2 * nk * 16 + 2 * d2 * npx * 8 + npx * (1 + 16) + (1ull << 20);
+  const unsigned long long vec = dim * (npx / last * ((last + 1) / 2)) * 2;  // reals of a displacement-space vector
+  // fields F and P, the residual, the FP64 spectrum, material index, lambda and mu, and 1 MiB
+  // of plans and reduction scratch
+  unsigned long long b = 2 * d2 * npx * 8 + vec * 8 + d2 * nk * 16 + npx * (1 + 16) + (1ull << 20);
+  if (has_le2) b += d2 * npx * 8;                          // eigenstrain
   if (form == MUSG_FINITE_STRAIN) b += 2 * d2 * npx * 8;  // S and F of the tangent
-  if (has_hep) b += 38 * npx * 8;                          // plastic state
+  if (has_hep) b += (4 * d2 + 2) * npx * 8;                // plastic state
   const unsigned long long tplanes = has_full ? d2 * d2 : has_hep ? d2 * dim : 0;  // K or K'
   b += tplanes * npx * 8;
+  if (has_full) b += d2 * npx * 8;  // the line search's Newton iterate
   if (precision == MUSG_PRECISION_MIXED) {
-    b += npx * 8 + d2 * nk * 8 + 3 * d2 * npx * 4;  // FP32 lambda/mu, spectrum, CG vectors x r p
-    b += d2 * npx * (8 + 4);                         // incremental residual: kept stress, FP32 change
+    b += npx * 8 + d2 * nk * 8;                       // FP32 lambda/mu, spectrum
+    b += 5 * vec * 4 + d2 * npx * 4 + d2 * npx * 8;  // residual, CG vectors, solution, kept stress
     if (form == MUSG_FINITE_STRAIN) b += 2 * d2 * npx * 4;
     b += tplanes * npx * 4;
   } else {
-    b += 4 * d2 * npx * 8;  // FP64 CG vectors
+    b += 4 * vec * 8 + d2 * npx * 8;  // CG vectors, solution
   }
   return b;
 }
@@ -138,7 +143,7 @@ std::shared_ptr<Req> copy_request(const musg_request &src, int precision) {
        "MaterialHyperElastoPlastic1 needs the finite-strain formulation");
   int res[3] = {1, 1, 1};
   for (int d = 0; d < src.dim; ++d) res[d] = src.resolutions[d];
-  q->bytes = footprint(src.dim, res, src.formulation, q->has_hep, q->has_full, precision);
+  q->bytes = footprint(src.dim, res, src.formulation, q->has_hep, q->has_full, q->has_le2, precision);
   // batchable together = same dimension, formulation, flags, number of steps and
   // tangent kind (grids may differ: a batch of several grids runs grouped launches)
   q->key = std::make_tuple(src.dim, 0, 0, 0, src.formulation, src.flags, src.nb_steps, (int)q->has_hep,
@@ -377,7 +382,8 @@ int musg_request_bytes(const musg_request *req, int precision, unsigned long lon
     bool full = false;
     for (int m = 0; m < req->nb_materials; ++m)
       full |= req->laws[m] == MUSG_LAW_HEP1 && req->params && (int)req->params[5 * m + 4] == kHep1Consistent;
-    *bytes = footprint(req->dim, res, req->formulation, has_law(*req, MUSG_LAW_HEP1), full, precision);
+    *bytes = footprint(req->dim, res, req->formulation, has_law(*req, MUSG_LAW_HEP1), full, has_law(*req, MUSG_LAW_LE2),
+                       precision);
   });
 }
 
