@@ -52,8 +52,23 @@ template <typename R> int disp_threads(const TilePlan &pl, long P, long blocks, 
 }
 // Registers (kDispRegs): 512 threads of FP64 kernels fit, of their 2-D ones 384.  FP32: two
 // blocks of 384 threads an SM; one of 480 left nothing to run at its barriers (160^3 small
-// strain 422 -> 382 us an iteration).
-template <typename R> long disp_most(const Spectral &sp) { return sizeof(R) == 8 && sp.g.dim == 3 ? 512 : 384; }
+// strain 422 -> 382 us an iteration).  Of the 2-D kernels' 128 registers two blocks of 256,
+// where a grid has more blocks than SMs: 640^2 finite strain 75 -> 63 us, 613^2 327 -> 289.
+template <typename R> long disp_most(const Spectral &sp, long blocks) {
+  if (sizeof(R) == 8) return sp.g.dim == 3 ? 512 : 384;
+  return sp.g.dim == 2 && blocks > kDispSms ? 256 : 384;
+}
+// registers of an iteration's kernel for the axis plan pl
+template <typename R> int disp_regs(const Spectral &sp, const TilePlan &pl) {
+  if (sizeof(R) == 4)
+    switch (disp_fixed_plan(pl)) {
+#define MUSG_C(M, A, B) case M: return kDispRegs<R, 1>;
+      MUSG_DISP_PLANS(MUSG_C)
+#undef MUSG_C
+      default: break;
+    }
+  return sp.g.dim == 2 ? kDispRegs<R, -2> : kDispRegs<R, 0>;
+}
 inline long lcm32(long p) {
   long a = p;
   while (a % 32) a += p;
@@ -84,14 +99,16 @@ template <typename R> DispShape disp_ax0_shape(const Spectral &sp, bool sums) {
   c.T = (int)T;
   c.ntx = (int)((Rr + T - 1) / T);
   c.smem = (size_t)(T * per + tw);
-  auto threads = [&] { return disp_threads<R>(pl, na * T, (long)c.nbx * c.ng, lcm32(na * T), disp_most<R>(sp)); };
+  auto threads = [&] {
+    return disp_threads<R>(pl, na * T, (long)c.nbx * c.ng, lcm32(na * T), disp_most<R>(sp, (long)c.ntx * c.ng));
+  };
   // With sums a block walks over several tiles, so that few sums are left to add up.  FP32:
   // as many blocks as are resident at once (128^3, 606 blocks of which 456 were resident:
   // 44 us, 456: 40 us, one block a tile: 45 us)
   c.nbx = c.ntx;
   if (sums) {
     c.threads = threads();
-    const int regs = 65536 / (kDispRegs<R, 0> * c.threads), mem = (int)((227l << 10) / (c.smem + 1024));
+    const int regs = 65536 / (disp_regs<R>(sp, pl) * c.threads), mem = (int)((227l << 10) / (c.smem + 1024));
     const int resident = sizeof(R) == 8 ? 4 : std::max(1, std::min(8, std::min(regs, mem)));
     c.nbx = std::min(c.ntx, std::max(1, resident * kDispSms / c.ng));
   }
@@ -124,7 +141,7 @@ template <typename R> DispShape disp_mid_shape(const Spectral &sp) {
   c.ntx = c.nbx = (int)nt;
   c.blocks = (int)((long long)c.ng * sp.g.n[0] * nt);
   c.smem = (size_t)(T * per + tw);
-  c.threads = disp_threads<R>(pl, c.comps_at_once * T, c.blocks, c.comps_at_once * T, disp_most<R>(sp));
+  c.threads = disp_threads<R>(pl, c.comps_at_once * T, c.blocks, c.comps_at_once * T, disp_most<R>(sp, c.blocks));
   return c;
 }
 
@@ -163,7 +180,7 @@ template <typename R> DispShape disp_last_shape(const Spectral &sp) {
   c.G = (int)(2 * g2);
   c.blocks = (int)((sp.g.nrows + c.G - 1) / c.G);
   c.smem = (size_t)(g2 * per + tw);
-  c.threads = disp_threads<R>(pl, nl * g2, c.blocks, 16, disp_most<R>(sp));
+  c.threads = disp_threads<R>(pl, nl * g2, c.blocks, 16, disp_most<R>(sp, c.blocks));
   return c;
 }
 

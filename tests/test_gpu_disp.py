@@ -191,6 +191,21 @@ def test_solve_bluestein_first_axis_2d(mu, res, form):
     assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
 
 
+@pytest.mark.parametrize('form', [0, 1])
+@pytest.mark.parametrize('res', [[640, 630], [613, 307], [300, 1000], [1024, 400]])
+def test_solve_2d_with_more_blocks_than_sms(mu, res, form):
+    """256 threads a block and as many blocks of the pass with the sums as are resident, a tile
+    after the other in each: FP64 and mixed solves agree within 1e-6."""
+    load = _load(2, form)
+    hom = {}
+    for prec in ('fp64', 'mixed'):
+        cell = _cell(mu, res, form, 3)
+        r = mu.solvers.newton_cg(cell, load, mu.solvers.SolverCG(cell, 1e-8, 3000, precision=prec), 1e-8, 0.0)
+        assert r.success, r.message
+        hom[prec] = r.hom_stress
+    assert np.linalg.norm(hom['mixed'] - hom['fp64']) <= 1e-6 * np.linalg.norm(hom['fp64'])
+
+
 @pytest.mark.parametrize('res', [[7, 5, 3], [3, 9], [1, 1, 1]])
 def test_inputs_as_planes_and_pixel_major(mu, res):
     """A C-ordered (D², N) array goes up as it is; its Fortran-ordered copy, a strided view
