@@ -245,7 +245,7 @@ int musg_de_geus(musg_cell *cell, const double *load_steps, int nb_steps,
  * counterpart in the reference, which solves one cell at a time.  Cells of one grid
  * run the solo solve's kernels (results equal those of musg_newton_cg on each cell
  * alone, bit for bit); cells of different grids (same dimension, formulation and
- * material-law kind) run grouped launches of the generic pass kernels, each cell
+ * material-law kind) run grouped launches of the runtime plans' kernels, each cell
  * owning a range of blocks and its own plans (results equal to the solo ones within
  * rounding).  load_steps: nb_cells x nb_steps D*D column-major matrices; infos:
  * nb_cells x nb_steps records; stresses (may be NULL): for each cell in turn,
@@ -274,7 +274,7 @@ int musg_batch_newton_cg(musg_batch *batch, const double *load_steps, int nb_ste
  * device for all its load steps and return to the budget when it completes.  A
  * request batched with requests of its own grid gets the kernels of its solo solve in
  * the same order (the same result bit for bit); batched with other grids it runs the
- * generic pass kernels (the same result within rounding). */
+ * kernels of the runtime plans (the same result within rounding). */
 typedef struct musg_server musg_server;
 
 /* one request; the server copies everything at submission */

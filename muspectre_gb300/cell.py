@@ -194,7 +194,8 @@ class CellBase:
         return flat.reshape(self.nb_pixels, self.dim * self.dim).T
 
     def tuning(self):
-        """Launch shapes of the spectral passes {precision: {pass: (threads, smem bytes)}}."""
+        """Launch shapes of the FFT engine's passes {precision: {pass: (threads, smem bytes)}};
+        the CG and projection passes take theirs from the grid by rule."""
         t = np.zeros(6, dtype=np.int32)
         b = np.zeros(6, dtype=np.int64)
         L.check(L.lib().musg_cell_tuning(self._h, L.iptr(t), L.llptr(b)))

@@ -166,7 +166,7 @@ struct musg_cell {
   // device fields (FP64 component planes)
   DevBuf F, P, io, io2, F0;  // F0: the line search's Newton iterate
   DevBuf Pk;                      // the stress of the last projected residual (incremental residual)
-  DevBuf rhat64, rhat;            // the residual G(-P) in displacement space (disp.cuh); its FP32 form (mixed)
+  DevBuf rhat64, rhat;            // the residual G(-P) in displacement space (disp.cuh); the mixed method's, FP32
   int residual_kept = 0;          // FP64 projections of this load step (incremental residual)
   DevBuf mat, params, law_kind, Ctab64, Ctab32;
   bool has_generic = false;
@@ -572,7 +572,7 @@ struct musg_solver {
   // newton_cg with a backtracking line search on the projected residual norm (an
   // extension, off by default; needed by the consistent elasto-plastic tangent)
   bool line_search = false;
-  // mixed precision: the Newton residual by FP32 corrections after one FP64 projection
+  // mixed precision: the Newton residual by FP32 corrections after two FP64 projections
   // per load step (musg_cell::project_residual)
   bool incremental_residual = true;
   const int *stop = nullptr;  // musg_solver_set_stop_flag
@@ -767,7 +767,7 @@ struct musg_batch {
   unsigned long long graph_nodes = 0;
   int chunk = 16;
   // cells of different grids (the same dimension, formulation and tangent kind): one
-  // grouped launch per pass over all of them (generic pass kernels)
+  // grouped launch per pass over all of them (kernels of runtime plans)
   bool uniform = true;
   DispBatch *disp = nullptr;  // the displacement-space passes of all cells
   const int *stop = nullptr;  // musg_batch_set_stop_flag
@@ -1357,8 +1357,8 @@ int musg_cell_tuning(musg_cell *cell, int *threads, long long *bytes) {
     require(cell && threads && bytes, MUSG_ERR_ARGUMENT, "null argument");
     for (int p = 0; p < 2; ++p)
       for (int k = 0; k < 3; ++k) {
-        threads[3 * p + k] = cell->sp.tune_threads[p][k];
-        bytes[3 * p + k] = cell->sp.tune_bytes[p][k];
+        threads[3 * p + k] = kEngineThreads[k];
+        bytes[3 * p + k] = kEngineBytes[k];
       }
   });
 }

@@ -1,4 +1,4 @@
-// Vector kernels of the Newton level: dot products, updates, means, conversions.
+// Vector kernels of the Newton level: sums, updates, means, conversions.
 // Reductions are deterministic: a fixed block partition, then one block sums the partials
 // in a fixed order, so a rerun gives bit-identical scalars.
 #include <algorithm>
@@ -25,16 +25,7 @@ __device__ __forceinline__ double sum_partials(const double *partial, int nparts
   return block_sum(v);
 }
 
-// ------------------------------------------------------------------ dots
-template <typename Ra, typename Rb>
-__global__ void k_dot(const Ra *__restrict__ a, const Rb *__restrict__ b, long long n, double *partial) {
-  double acc = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    acc += (double)a[i] * (double)b[i];
-  const double bs = block_sum(acc);
-  if (threadIdx.x == 0) partial[blockIdx.x] = bs;
-}
-
+// ------------------------------------------------------------------ sums
 // (a - b)^2 summed
 __global__ void k_diff2(const double *__restrict__ a, const double *__restrict__ b, long long n, double *partial) {
   double acc = 0.0;
@@ -49,15 +40,6 @@ __global__ void k_diff2(const double *__restrict__ a, const double *__restrict__
 __global__ void k_sum_to(const double *partial, int nparts, double *out) {
   const double v = sum_partials(partial, nparts);
   if (threadIdx.x == 0) *out = v;
-}
-
-template <typename Ra, typename Rb>
-void dot_device(const Ra *a, const Rb *b, long long n, double *partial, double *out, cudaStream_t s) {
-  const int nb = reduce_blocks(n);
-  k_dot<Ra, Rb><<<nb, kRedThreads, 0, s>>>(a, b, n, partial);
-  MUSG_CHECK_LAUNCH();
-  k_sum_to<<<1, 1024, 0, s>>>(partial, nb, out);
-  MUSG_CHECK_LAUNCH();
 }
 
 void diff2_device(const double *a, const double *b, long long n, double *partial, double *out, cudaStream_t s) {
@@ -172,7 +154,6 @@ void convert(Rd *dst, const Rs *src, long long n, double scale, cudaStream_t s) 
   MUSG_CHECK_LAUNCH();
 }
 
-template void dot_device<double, double>(const double *, const double *, long long, double *, double *, cudaStream_t);
 template void newton_update<double>(double *, const double *, long long, double *, double *, cudaStream_t);
 template void newton_update<float>(double *, const float *, long long, double *, double *, cudaStream_t);
 template void newton_trial<double>(double *, const double *, const double *, double, long long, double *, double *,

@@ -223,11 +223,6 @@ struct Spectral {
   void *spec64 = nullptr;   // [ncomp][nk] complex double
   void *spec32 = nullptr;   // [ncomp][nk] complex float
   bool want32 = false;
-  // launch shapes of the FFT engine's passes per precision (0: FP64, 1: FP32) and pass
-  // (0: last, 1: axis, 2: first axis): threads per block and the shared memory a block
-  // aims for
-  int tune_threads[2][3] = {{256, 256, 256}, {256, 256, 256}};
-  long tune_bytes[2][3] = {{73728, 49152, 73728}, {73728, 49152, 73728}};
   void init(int dim, const int *res, int ncomp, int proj_kind, const double *lengths,
             bool allow_even, bool want32);
   // points of a pencil of two buffers in `bytes` of shared memory, for the pass over `axis`
@@ -245,8 +240,11 @@ unsigned *wait_fault_word();
 // (self-test of the bounded waits: it sets the fault word and exits)
 void wait_probe(unsigned long long limit_ns, cudaStream_t s);
 
-// Launch configuration limits of the pass kernels
+// The FFT engine's passes (last axis, middle axis, first axis): the most threads per block,
+// threads per block, and the shared memory a block aims for
 constexpr int kPassThreads = 512;
+constexpr int kEngineThreads[3] = {256, 256, 256};
+constexpr long kEngineBytes[3] = {73728, 49152, 73728};
 
 // Pass launchers (spectral_*.cu).  All run on `stream`.
 //  fwd: real field [ncomp][npx] (scaled) -> spectrum (r2c over all axes)
@@ -319,10 +317,6 @@ int reduce_blocks(long long n);
 void plane_means(const double *f, int ncomp, long long npx, double *partial, double *out, cudaStream_t s);
 // sum of (a - b)^2 over n entries into *out (device)
 void diff2_device(const double *a, const double *b, long long n, double *partial, double *out, cudaStream_t s);
-// FP64 dot of a with b over n entries into *out_device (deterministic)
-template <typename Ra, typename Rb>
-void dot_device(const Ra *a, const Rb *b, long long n, double *partial, double *out,
-                cudaStream_t s);
 // y += x (promoting), with the dots x.x and y.y (after the update) into out[0], out[1]
 template <typename R>
 void newton_update(double *F, const R *x, long long n, double *partial, double *out,

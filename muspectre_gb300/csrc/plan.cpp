@@ -7,7 +7,6 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "launch_util.h"

@@ -15,14 +15,13 @@ struct Cfg {
   int threads;
 };
 
-template <typename R> constexpr int prec_index() { return sizeof(R) == 8 ? 0 : 1; }
 
 // shared memory per block: two ping-pong buffers of (pencils x m) complex values
 template <typename R> Cfg last_cfg(const Spectral &sp) {
   const AxisPlan &ap = sp.ax[sp.g.dim - 1];
   const long per_pair = (long)sp.ncomp * ap.m;
   const long eb = 2 * sizeof(typename V2<R>::T);
-  const long target = sp.tune_bytes[prec_index<R>()][0];
+  const long target = kEngineBytes[0];
   long g2 = std::min(std::max(1L, target / (per_pair * eb)), (long)optin_smem() / (per_pair * eb));
   if (g2 < 1) throw Error(MUSG_ERR_ARGUMENT, "last-axis FFT too long for one thread block");
   g2 = std::min<long>(g2, 16);
@@ -31,14 +30,14 @@ template <typename R> Cfg last_cfg(const Spectral &sp) {
   c.per = (int)(2 * g2);
   c.blocks = (int)((sp.g.nrows + c.per - 1) / c.per);
   c.smem = (size_t)(g2 * per_pair * eb);
-  c.threads = sp.tune_threads[prec_index<R>()][0];
+  c.threads = kEngineThreads[0];
   return c;
 }
 
 template <typename R> Cfg axis_cfg(const Spectral &sp, int axis, long long inner, long long nbatch) {
   const AxisPlan &ap = sp.ax[axis];
   const long eb = 2 * sizeof(typename V2<R>::T);
-  const long target = sp.tune_bytes[prec_index<R>()][1];
+  const long target = kEngineBytes[1];
   long T = std::min(std::max(1L, target / (ap.m * eb)), (long)optin_smem() / (ap.m * eb));
   if (T < 1) throw Error(MUSG_ERR_ARGUMENT, "FFT axis too long for one thread block");
   T = std::min<long>(T, 32);
@@ -51,7 +50,7 @@ template <typename R> Cfg axis_cfg(const Spectral &sp, int axis, long long inner
   const long long ntiles = (inner + T - 1) / T;
   c.blocks = (int)(ntiles * nbatch);
   c.smem = (size_t)(T * ap.m * eb);
-  c.threads = sp.tune_threads[prec_index<R>()][1];
+  c.threads = kEngineThreads[1];
   return c;
 }
 
@@ -59,7 +58,7 @@ template <typename R> Cfg green_cfg(const Spectral &sp, long long Rr) {
   const AxisPlan &ap = sp.ax[0];
   const long per = (long)sp.ncomp * ap.m;
   const long eb = 2 * sizeof(typename V2<R>::T);
-  const long target = sp.tune_bytes[prec_index<R>()][2];
+  const long target = kEngineBytes[2];
   long T = std::min(std::max(1L, target / (per * eb)), (long)optin_smem() / (per * eb));
   if (T < 1) throw Error(MUSG_ERR_ARGUMENT, "first-axis FFT too long for one thread block");
   T = std::min<long>(T, 32);
@@ -68,7 +67,7 @@ template <typename R> Cfg green_cfg(const Spectral &sp, long long Rr) {
   c.per = (int)T;
   c.blocks = (int)((Rr + T - 1) / T);
   c.smem = (size_t)(T * per * eb);
-  c.threads = sp.tune_threads[prec_index<R>()][2];
+  c.threads = kEngineThreads[2];
   return c;
 }
 

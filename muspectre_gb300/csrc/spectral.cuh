@@ -71,9 +71,8 @@ __device__ __forceinline__ double block_sum(double v) {
 // ticket) sums them all in a fixed order and updates the state.
 // Deterministic like a separate reduction kernel, without its launch.
 __device__ __forceinline__ int lin_tid() { return threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z); }
-__device__ __forceinline__ int lin_nth() { return blockDim.x * blockDim.y * blockDim.z; }
 
-// call by the whole block after thread 0 wrote this block's partial sum; nblk = the
+// call by the whole block after its first threads wrote its partial sums; nblk = the
 // problem's blocks (gridDim.x, or a problem's share of a grouped launch)
 __device__ __forceinline__ bool cg_last_block(CGState *st, int nblk) {
   __shared__ int last;
@@ -517,8 +516,9 @@ __global__ void __launch_bounds__(kPassThreads) k_axis(const AxisArgs<R> a) {
   axis_body<R, INV>(a, blockIdx.x);
 }
 
-// 1 / sqrt(n2) within 1 ulp (rsqrt; a square root and a division, each correctly rounded,
-// are no closer and twice the instructions of the FP64 pipe) and 2 ulp (rsqrtf)
+// 1 / sqrt(n2).  FP64: a square root and a division, each correctly rounded, as the oracle
+// forms it; rsqrt is half the instructions, but its rounding moved CG counts at the tolerance
+// by two against the oracle's.  FP32: rsqrtf, within 2 ulp.
 __device__ __forceinline__ double inv_sqrt(double n2) { return 1.0 / sqrt(n2); }
 __device__ __forceinline__ float inv_sqrt(float n2) { return rsqrtf(n2); }
 

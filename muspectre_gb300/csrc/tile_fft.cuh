@@ -115,7 +115,7 @@ template <int CR1, int CR2> struct RowMap {
   __device__ __forceinline__ int stride(int) const { return S; }
   __device__ __forceinline__ int at(int slot, int p) const { return slot + p * sp; }
   template <typename F> __device__ __forceinline__ void each(int nj, int P, F f) const {
-    if constexpr (CR1 > 0) {  // nj is a power of two the compiler sees
+    if constexpr (CR1 > 0) {  // nj is a constant the compiler divides by with a multiplication
       for (int t = threadIdx.x; t < nj * P; t += blockDim.x) f(t % nj, t / nj);
     } else {
       const FDiv fd(nj);

@@ -12,7 +12,7 @@ request completes.  Latency = completion - submission.
 
 A request batched with requests of its own grid is computed by the kernels of its
 solo solve in the same order (per-request reductions in a fixed order), so its result
-is the same bit for bit; batched with other grids it runs the generic pass kernels
+is the same bit for bit; batched with other grids it runs the kernels of runtime plans
 and its result equals the solo one within rounding (``tests/test_gpu_serving.py``).
 """
 from __future__ import annotations

@@ -85,3 +85,17 @@ def test_fused_iteration_bytes():
     b_unfused = sum(bench.algorithmic_bytes(k, npx, nk, d2, s, tm) for k in unfused)
     assert abs(b_fused - (16 * u + tm * npx)) <= 2 / n * 16 * u
     assert abs(b_unfused - (19 * u + tm * npx)) <= 2 / n * 19 * u
+
+
+def test_displacement_iteration_bytes():
+    """The bytes counted for the five passes of the mixed CG iteration at finite strain: 90
+    component spectra (r, q, p, x in and r, p, x, q out, p and r in for the sums: 30; the
+    fields between the passes, 6 and 9 components: 60) and the tangent data once."""
+    sys.path.insert(0, ROOT)
+    import bench
+    n = 128
+    npx, nk, s = n ** 3, n * n * (n // 2), 4
+    tm = 4 * 9 + 1
+    names = ['axis0_inv_update', 'axis1_inv_expand', 'last_axis_tangent', 'axis1_fwd_contract', 'axis0_fwd_dots']
+    total = sum(bench.algorithmic_bytes(k, npx, nk, 9, s, tm) for k in names)
+    assert total == 90 * nk * 2 * s + tm * npx
