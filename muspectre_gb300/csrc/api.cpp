@@ -166,7 +166,7 @@ struct musg_cell {
   // device fields (FP64 component planes)
   DevBuf F, P, io, io2, F0;  // F0: the line search's Newton iterate
   DevBuf Pk;                      // the stress of the last projected residual (incremental residual)
-  DevBuf rhat64, rhat;            // the residual G(-P) in displacement space (disp.cuh); the mixed method's, FP32
+  DevBuf rhat64, rhat;            // the residual G(-P) in displacement space (disp.cuh); its FP32 form (mixed)
   int residual_kept = 0;          // FP64 projections of this load step (incremental residual)
   DevBuf mat, params, law_kind, Ctab64, Ctab32;
   bool has_generic = false;
@@ -465,20 +465,21 @@ struct musg_cell {
 
   // rhat64 = -G(P) for the current stress, its norm's square in scal[32]
   void project_residual() {
-    disp_residual<double>(sp, TK_PLAIN, {}, rhat64.p, P.as<double>(), nullptr, -1.0, false, partial.as<double>(),
+    disp_residual<double>(sp, TK_PLAIN, {}, rhat64.p, P.as<double>(), nullptr, -1.0, partial.as<double>(),
                           scal.as<double>() + 32, stream);
   }
-  // The mixed method's residual rhat.  Incremental (the default): the first two residuals
-  // of a load step are projected in FP64 and the second one's P kept in Pk; each later one
-  // is rhat + G(Pk - P) with the stress change projected in FP32, and the new P is kept.
+  // The mixed method's residual: rhat64, its norm in FP64, and rhat, the FP32 right-hand
+  // side of the inner solve.  Incremental (the default): the first two residuals of a load
+  // step are projected in FP64 and the second one's P kept in Pk; to each later one
+  // G(Pk - P) is added in FP64, the stress change projected in FP32, and the new P is kept.
   // The FP32 rounding is relative to that change and not to P (whose mean and fluctuation
   // are far larger), and in displacement space no part of it can leave the range of G.
   // The change after the first Newton step is as large as the first residual; projected
   // in FP32 it left an error floor of 1e-6 of the strain, the later ones are a hundredth.
   void project_residual_mixed(bool incremental) {
     if (incremental && residual_kept >= 2) {
-      disp_residual<float>(sp, TK_PLAIN, {}, rhat.p, P.as<double>(), Pk.as<double>(), 1.0, true, partial.as<double>(),
-                           scal.as<double>() + 32, stream);
+      disp_residual<float>(sp, TK_PLAIN, {}, rhat.p, P.as<double>(), Pk.as<double>(), 1.0, nullptr, nullptr, stream);
+      disp_accumulate(sp, rhat64.p, rhat.p, partial.as<double>(), scal.as<double>() + 32, stream);
       return;
     }
     project_residual();
@@ -541,7 +542,7 @@ template <> TangentData<float> musg_cell::tangent<float>() const {
 void musg_cell::residual_geus(double *delta, bool mixed) {
   if (io2.bytes < field_bytes()) io2.alloc(field_bytes());
   fill_uniform(io2.as<double>(), delta, D2, npx, stream);
-  disp_residual<double>(sp, tkind, tangent<double>(), rhat64.p, io2.as<double>(), nullptr, -1.0, false,
+  disp_residual<double>(sp, tkind, tangent<double>(), rhat64.p, io2.as<double>(), nullptr, -1.0,
                         partial.as<double>(), scal.as<double>() + 32, stream);
   if (mixed) disp_convert(sp, rhat64.p, rhat.p, stream);
   residual_kept = 0;
@@ -702,7 +703,7 @@ struct musg_solver {
       // the residual (|rhs - G rhs|^2)
       if (c.io.bytes < c.field_bytes()) c.io.alloc(c.field_bytes());
       c.sp.ensure_tiles();
-      disp_residual<double>(c.sp, TK_PLAIN, {}, c.rhat64.p, rhs, nullptr, 1.0, false, part, dscal + 37, s);
+      disp_residual<double>(c.sp, TK_PLAIN, {}, c.rhat64.p, rhs, nullptr, 1.0, part, dscal + 37, s);
       disp_field<double>(c.sp, c.rhat64.p, c.io.as<double>(), s);
       diff2_device(rhs, c.io.as<double>(), c.nb_dof(), part, dscal + 36, s);
       if (sizeof(R) == 4) disp_convert(c.sp, c.rhat64.p, c.rhat.p, s);

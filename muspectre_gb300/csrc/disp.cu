@@ -88,6 +88,46 @@ __global__ void k_disp_convert(const double2 *__restrict__ a, float2 *__restrict
   }
 }
 
+// The residual of the mixed method: r64 += change (the FP32 projection of the stress change,
+// in r32), r32 = r64 rounded, and a block's part of |r64|^2 in FP64 (Parseval's sum of the
+// header of disp.cuh) where k_disp_sum reads it.  Bound by its 40 bytes a value, 25 MB at
+// 128^3, once per Newton iteration.
+template <int D, bool FIN>
+__global__ void k_disp_add(double2 *__restrict__ r64, float2 *__restrict__ r32, const DispArgs<double> a, double *partial) {
+  double sum = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.nk; i += (long long)gridDim.x * blockDim.x) {
+    double2 v[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const long long o = (long long)d * a.nk + i;
+      const float2 c = r32[o];
+      v[d] = r64[o];
+      v[d].x += (double)c.x;
+      v[d].y += (double)c.y;
+      r64[o] = v[d];
+      r32[o] = make_float2((float)v[d].x, (float)v[d].y);
+    }
+    const int e = (int)(i / a.Rr), rho = (int)(i - (long long)e * a.Rr);
+    const Wave<D, double> wv(a, rho);
+    double acc = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) acc += v[d].x * v[d].x + v[d].y * v[d].y;
+    if constexpr (!FIN) {
+      double k[D], lx = 0.0, ly = 0.0;
+      const double w = wv.at(a, e, k);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        lx += v[d].x * k[d] * w;
+        ly += v[d].y * k[d] * w;
+      }
+      acc = 0.5 * (acc + lx * lx + ly * ly);
+    }
+    sum += wv.kl == 0 ? acc : 2.0 * acc;
+  }
+  sum = block_sum(sum);
+  if (threadIdx.x == 0) partial[4 * blockIdx.x + 3] = sum;
+}
+
 template <typename R> typename V2<R>::T *work_spectrum(Spectral &sp);
 template <> double2 *work_spectrum<double>(Spectral &sp) {
   sp.ensure_tiles();
@@ -135,14 +175,13 @@ template <typename R> void inverse_from(Spectral &sp, DispProb<R> pb, bool from_
 
 // real planes (through the tangent unless tkind is TK_PLAIN) -> q, its q.q in *sum2
 template <typename R>
-void forward_to(Spectral &sp, DispProb<R> pb, int tkind, const double *in, double *prev, double in_scale, bool accumulate,
-                double *sum2, cudaStream_t s) {
+void forward_to(Spectral &sp, DispProb<R> pb, int tkind, const double *in, double *prev, double in_scale, double *sum2,
+                cudaStream_t s) {
   DispPasses<R> p = disp_passes<R>(sp, pb);
   p.af.gated = p.am.gated = p.al.gated = 0;
   p.al.in64 = in;
   p.al.in_prev = prev;
   p.al.in_scale = in_scale;
-  p.af.accumulate = accumulate ? 1 : 0;
   const bool fin = disp_finite(sp);
   if (sp.g.dim == 2) disp_pixels_in<R, 2>(fin, tkind, prev != nullptr, p.al, p.cl, s);
   else disp_pixels_in<R, 3>(fin, tkind, prev != nullptr, p.al, p.cl, s);
@@ -158,12 +197,12 @@ void forward_to(Spectral &sp, DispProb<R> pb, int tkind, const double *in, doubl
 
 template <typename R>
 void disp_residual(Spectral &sp, int tkind, const TangentData<R> &td, void *rhat, const double *field, double *prev,
-                   double scale, bool accumulate, double *partial, double *norm2, cudaStream_t s) {
+                   double scale, double *partial, double *norm2, cudaStream_t s) {
   DispVectors v;
   v.q = rhat;
   DispProb<R> pb = disp_prob<R>(sp, v, nullptr, partial);
   pb.td = td;
-  forward_to<R>(sp, pb, tkind, field, prev, scale, accumulate, norm2, s);
+  forward_to<R>(sp, pb, tkind, field, prev, scale, norm2, s);
 }
 
 template <typename R>
@@ -219,7 +258,7 @@ void disp_operator(Spectral &sp, int tkind, const TangentData<R> &td, const doub
   v.q = work_spectrum<R>(sp);
   DispProb<R> pb = disp_prob<R>(sp, v, nullptr, nullptr);
   pb.td = td;
-  forward_to<R>(sp, pb, tkind, in, nullptr, 1.0, false, nullptr, s);
+  forward_to<R>(sp, pb, tkind, in, nullptr, 1.0, nullptr, s);
   inverse_from<R>(sp, pb, false, out, s);
 }
 
@@ -235,9 +274,26 @@ void disp_convert(const Spectral &sp, const void *v64, void *v32, cudaStream_t s
   MUSG_CHECK_LAUNCH();
 }
 
+void disp_accumulate(Spectral &sp, void *r64, void *r32, double *partial, double *norm2, cudaStream_t s) {
+  DispProb<double> pb{};
+  pb.xi0 = xi_table<double>(sp, 0);
+  pb.xi1 = xi_table<double>(sp, 1);
+  pb.xi2 = sp.g.dim == 3 ? xi_table<double>(sp, 2) : nullptr;
+  DispArgs<double> a = disp_base<double>(sp);
+  a.pb = pb;
+  const int nb = reduce_blocks(a.nk);
+  const bool fin = disp_finite(sp);
+  auto *k = sp.g.dim == 2 ? (fin ? k_disp_add<2, true> : k_disp_add<2, false>)
+                          : (fin ? k_disp_add<3, true> : k_disp_add<3, false>);
+  k<<<nb, 256, 0, s>>>((double2 *)r64, (float2 *)r32, a, partial);
+  MUSG_CHECK_LAUNCH();
+  k_disp_sum<<<1, 256, 0, s>>>(partial, nb, norm2);
+  MUSG_CHECK_LAUNCH();
+}
+
 #define MUSG_INSTANTIATE_DISP(R)                                                                                      \
   template void disp_residual<R>(Spectral &, int, const TangentData<R> &, void *, const double *, double *, double,   \
-                                 bool, double *, double *, cudaStream_t);                                             \
+                                 double *, double *, cudaStream_t);                                                   \
   template void disp_start<R>(Spectral &, const DispVectors &, const void *, CGState *, double, int, const double *,  \
                               const double *, cudaStream_t);                                                          \
   template void disp_iteration<R>(Spectral &, int, const TangentData<R> &, const DispVectors &, CGState *, double *,  \

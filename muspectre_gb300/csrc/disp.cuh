@@ -84,7 +84,6 @@ template <typename R> struct DispArgs {
   double *in_prev;        // their previous values (IN_DELTA)
   double in_scale;
   R *out;                 // real output planes
-  int accumulate;         // ax0_fwd: q += instead of q =
   int tkind;              // tangent kind (TK_ANYFIN kernels)
   int gated;              // passes of an iteration run only while the state is active
   DispProb<R> pb;
@@ -492,7 +491,7 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_mid(const DispArgs<R> a0, con
 // ------------------------------------------------------------ axis 0, forward
 enum Ax0Sums : int {
   AX_DOTS = 0,  // q and the sums p.q, r.q, q.q, r.r
-  AX_OUT = 1    // q (or q += with a.accumulate) and its own q.q in the fourth sum
+  AX_OUT = 1    // q and its own q.q in the fourth sum
 };
 
 template <typename R, int D, bool FIN, int MODE, int CR1, int CR2, bool GRP>
@@ -539,13 +538,9 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_fwd(const DispArgs<R> a0,
           const int e = eb + u * de;
           const long long o = ob + (long long)d * a.nk + e * a.Rr;
           pv[u][d] = rv[u][d] = T{R(0), R(0)};
-          if (e < n0) {
-            if (MODE == AX_DOTS) {
-              pv[u][d] = a.pb.p[o];
-              rv[u][d] = a.pb.r[o];
-            } else if (a.accumulate) {
-              rv[u][d] = a.pb.q[o];
-            }
+          if (MODE == AX_DOTS && e < n0) {
+            pv[u][d] = a.pb.p[o];
+            rv[u][d] = a.pb.r[o];
           }
         }
 #pragma unroll
@@ -582,10 +577,6 @@ __global__ void __maxnreg__((kDispRegs<R, CR1>)) k_ax0_fwd(const DispArgs<R> a0,
 #pragma unroll
           for (int i = 0; i < D; ++i)
             v[i] = T{(R(2) * tr[i].x - sc.x * k[i]) * a.scale, (R(2) * tr[i].y - sc.y * k[i]) * a.scale};
-        }
-        if (MODE == AX_OUT) {
-#pragma unroll
-          for (int d = 0; d < C::ND; ++d) v[d] = T{v[d].x + rv[u][d].x, v[d].y + rv[u][d].y};
         }
 #pragma unroll
         for (int d = 0; d < C::ND; ++d) a.pb.q[ob + (long long)d * a.nk + e * a.Rr] = v[d];

@@ -268,12 +268,14 @@ inline long long disp_nk(const Spectral &sp) { return sp.g.nrows * disp_nh(sp); 
 template <typename R> size_t disp_vector_bytes(const Spectral &sp) {
   return (size_t)disp_nk(sp) * sp.g.dim * 2 * sizeof(R);
 }
-// rhat (+)= the projection of scale * field (FP64 planes), through the tangent unless
-// tkind is TK_PLAIN; or with prev of prev - field, after which prev = field.  *norm2 (may
-// be null) = |rhat|^2, a device double
+// rhat = the projection of scale * field (FP64 planes), through the tangent unless tkind is
+// TK_PLAIN; or with prev of prev - field, after which prev = field.  *norm2 (may be null) =
+// |rhat|^2, a device double
 template <typename R>
 void disp_residual(Spectral &sp, int tkind, const TangentData<R> &td, void *rhat, const double *field, double *prev,
-                   double scale, bool accumulate, double *partial, double *norm2, cudaStream_t s);
+                   double scale, double *partial, double *norm2, cudaStream_t s);
+// r64 += r32 (an FP32 rhat), then r32 = r64 rounded, *norm2 = |r64|^2 summed in FP64
+void disp_accumulate(Spectral &sp, void *r64, void *r32, double *partial, double *norm2, cudaStream_t s);
 // state and vectors of a solve A x = rhs for the rhat of its right-hand side, *range2 =
 // |rhat|^2; *out2 (null: 0) is the part of |rhs|^2 outside the range of the projection,
 // which stays in the residual (device doubles)
