@@ -197,7 +197,7 @@ int musg_solver_destroy(musg_solver *solver);
 int musg_solver_set_inner_tol(musg_solver *solver, double inner_tol);
 /* MUSG_PRECISION_MIXED only (no counterpart in the reference; on by default): newton_cg
  * projects the first two residuals G(-P) of a load step in FP64 and every later one as
- * the previous residual minus G(P - P_prev) of the stress change since in FP32 (two
+ * the previous residual minus G(P - P_prev), the stress change since projected in FP32 (two
  * FP64 projections per load step instead of one per Newton iteration).
  * enable = 0 projects every residual in FP64. */
 int musg_solver_set_incremental_residual(musg_solver *solver, int enable);

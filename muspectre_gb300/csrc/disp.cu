@@ -90,8 +90,10 @@ __global__ void k_disp_convert(const double2 *__restrict__ a, float2 *__restrict
 
 // The residual of the mixed method: r64 += change (the FP32 projection of the stress change,
 // in r32), r32 = r64 rounded, and a block's part of |r64|^2 in FP64 (Parseval's sum of the
-// header of disp.cuh) where k_disp_sum reads it.  Bound by its 40 bytes a value, 25 MB at
-// 128^3, once per Newton iteration.
+// header of disp.cuh) where k_disp_sum reads it.  Bound by its 48 bytes a complex value, 151 MB
+// at 128^3, and on small grids by its launch; once per residual after the second of a load
+// step: 32^3 elasto-plastic, some hundred of them, 97.9 -> 99.6 ms a solve, 128^3 spheres 38.4
+// ms before and after.
 template <int D, bool FIN>
 __global__ void k_disp_add(double2 *__restrict__ r64, float2 *__restrict__ r32, const DispArgs<double> a, double *partial) {
   double sum = 0.0;
